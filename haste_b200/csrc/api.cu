@@ -30,24 +30,27 @@ int validate_shape(const char* who, int64_t B, int64_t D, int64_t F, int64_t L, 
   return HASTE_OK;
 }
 
-// Shape dispatch of the fused step: the tcgen05 kernel where its tile shapes apply — (G=128, F=64) or (G=64, F=128),
-// B % 8 == 0 (16-byte rows of xt for the tensor map), D*B < 2^32 (32-bit dxt row offsets), L < 2^31 — the warp-mma
+// Shape dispatch of the fused step: the tcgen05 kernel where its tile shapes apply — (G, F) in {(128, 64), (64, 128),
+// (64, 64), (32, 64), (32, 32), (32, 128)}, a row stride of xt that is a multiple of 8 (16-byte rows for the tensor map), D*B < 2^32 (32-bit dxt row offsets), L < 2^31 — the warp-mma
 // kernel for every other supported shape.
 static int g_max_ctas = 0;   // 0 = one CTA per SM
 
-static bool train_step_sm100_supported(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G) {
-  return ((G == 128 && F == 64) || (G == 64 && F == 128)) && (B % 8) == 0 && D * B < (int64_t(1) << 32) && L < (int64_t(1) << 31);
+static bool train_step_sm100_supported(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldxt) {
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
+  return shape && (ldxt % 8) == 0 && ldxt < (int64_t(1) << 31) && D * B < (int64_t(1) << 32) && L < (int64_t(1) << 31);
 }
 
 int launch_train_step(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                       const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind, float grad_scale,
-                      cudaStream_t st, const StepDump* dump) {
-  if (train_step_sm100_supported(B, D, F, L, G)) {
-    if (G == 128) return launch_train_step_sm100_g128f64(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, L, loss_kind, grad_scale, g_max_ctas, st, dump);
-    return launch_train_step_sm100_g64f128(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, L, loss_kind, grad_scale, g_max_ctas, st, dump);
+                      int64_t ldxt, cudaStream_t st, const StepDump* dump) {
+  if (train_step_sm100_supported(B, D, F, L, G, ldxt)) {
+    if (dump == nullptr && (G == 32 || (G == 64 && F == 64)))
+      return launch_train_step_sm100_small(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, ldxt, g_max_ctas, st);
+    if (G == 128) return launch_train_step_sm100_g128f64(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, L, loss_kind, grad_scale, ldxt, g_max_ctas, st, dump);
+    if (G == 64 && F == 128) return launch_train_step_sm100_g64f128(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, L, loss_kind, grad_scale, ldxt, g_max_ctas, st, dump);
   }
   if (dump != nullptr) return fail(HASTE_ERR_UNSUPPORTED, "debug outputs exist only in the tcgen05 fused step ((G,F) = (128,64) or (64,128), B%%8==0)");
-  return launch_train_step_mma(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, st);
+  return launch_train_step_mma(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, ldxt, st);
 }
 
 }  // namespace haste
@@ -77,17 +80,28 @@ int haste_ffi_forward(const int32_t* loc, const void* xt, const void* w, const v
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(w, who);
   if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
   if (ldz < L) return fail(HASTE_ERR_BAD_ARG, "%s: ldz=%lld < L=%lld", who, (long long)ldz, (long long)L);
-  return launch_forward(loc, xt, w, bias, z, B, D, F, L, G, ldz, ldz, static_cast<cudaStream_t>(stream));
+  return launch_forward(loc, xt, w, bias, z, B, D, F, L, G, ldz, ldz, B, static_cast<cudaStream_t>(stream));
+}
+
+static int check_ldxt(const char* who, int64_t B, int64_t ldxt) {
+  if (ldxt < B) return fail(HASTE_ERR_BAD_ARG, "%s: ldxt=%lld < B=%lld", who, (long long)ldxt, (long long)B);
+  return HASTE_OK;
 }
 
 int haste_ffi_forward_into(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
                            int64_t L, int64_t G, int64_t ldz, int64_t zcols, haste_stream_t stream) {
+  return haste_ffi_forward_ldx(loc, xt, w, bias, z, B, D, F, L, G, ldz, zcols, B, stream);
+}
+
+int haste_ffi_forward_ldx(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
+                          int64_t L, int64_t G, int64_t ldz, int64_t zcols, int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_ffi_forward_into";
   REQUIRE_PTR(loc, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(w, who); REQUIRE_PTR(z, who);
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(w, who);
   if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
   if (zcols < L || ldz < zcols) return fail(HASTE_ERR_BAD_ARG, "%s: need L <= zcols <= ldz (L=%lld zcols=%lld ldz=%lld)", who, (long long)L, (long long)zcols, (long long)ldz);
-  return launch_forward(loc, xt, w, bias, z, B, D, F, L, G, ldz, zcols, static_cast<cudaStream_t>(stream));
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
+  return launch_forward(loc, xt, w, bias, z, B, D, F, L, G, ldz, zcols, ldxt, static_cast<cudaStream_t>(stream));
 }
 
 int haste_ffi_backward_features(const void* w, const int32_t* loc, const void* dy, float* dxt, int64_t B, int64_t D, int64_t F, int64_t L,
@@ -102,26 +116,38 @@ int haste_ffi_backward_features(const void* w, const int32_t* loc, const void* d
     cudaError_t e = cudaMemsetAsync(dxt, 0, sizeof(float) * D * B, st);
     if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "%s: cudaMemsetAsync: %s", who, cudaGetErrorString(e));
   }
-  if (backward_sm100_supported(nullptr, w, dy, nullptr, B, D, F, L, G))
-    return launch_backward_sm100(nullptr, w, loc, dy, dxt, nullptr, nullptr, nullptr, B, D, F, L, G, ldy, st);
+  if (backward_sm100_supported(nullptr, w, dy, nullptr, B, D, F, L, G, B))
+    return launch_backward_sm100(nullptr, w, loc, dy, dxt, nullptr, nullptr, nullptr, B, D, F, L, G, ldy, B, st);
   return launch_bwd_features(w, loc, dy, dxt, B, D, F, L, G, ldy, st);
 }
 
 int haste_ffi_backward_weights(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias, int64_t B, int64_t D, int64_t F,
                                int64_t L, int64_t G, int64_t ldy, haste_stream_t stream) {
+  return haste_ffi_backward_weights_ldx(xt, loc, dy, dw, dbias, B, D, F, L, G, ldy, B, stream);
+}
+
+int haste_ffi_backward_weights_ldx(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias, int64_t B, int64_t D, int64_t F,
+                                   int64_t L, int64_t G, int64_t ldy, int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_ffi_backward_weights";
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
   REQUIRE_PTR(loc, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(dy, who); REQUIRE_PTR(dw, who);
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(dw, who);
   if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
   if (ldy < L) return fail(HASTE_ERR_BAD_ARG, "%s: ldy=%lld < L=%lld", who, (long long)ldy, (long long)L);
-  if (backward_sm100_supported(xt, nullptr, dy, dw, B, D, F, L, G))
-    return launch_backward_sm100(xt, nullptr, loc, dy, nullptr, dw, dbias, nullptr, B, D, F, L, G, ldy, static_cast<cudaStream_t>(stream));
-  return launch_bwd_weights(xt, loc, dy, dw, dbias, nullptr, B, D, F, L, G, ldy, static_cast<cudaStream_t>(stream));
+  if (backward_sm100_supported(xt, nullptr, dy, dw, B, D, F, L, G, ldxt))
+    return launch_backward_sm100(xt, nullptr, loc, dy, nullptr, dw, dbias, nullptr, B, D, F, L, G, ldy, ldxt, static_cast<cudaStream_t>(stream));
+  return launch_bwd_weights(xt, loc, dy, dw, dbias, nullptr, B, D, F, L, G, ldy, ldxt, static_cast<cudaStream_t>(stream));
 }
 
 int haste_ffi_backward(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias, int64_t B,
                        int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, uint32_t flags, haste_stream_t stream) {
+  return haste_ffi_backward_ldx(xt, w, loc, dy, dxt, dw, dbias, B, D, F, L, G, ldy, flags, B, stream);
+}
+
+int haste_ffi_backward_ldx(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias, int64_t B,
+                           int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, uint32_t flags, int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_ffi_backward";
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
   REQUIRE_PTR(loc, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(w, who); REQUIRE_PTR(dy, who); REQUIRE_PTR(dxt, who); REQUIRE_PTR(dw, who);
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(w, who); REQUIRE_ALIGNED(dxt, who); REQUIRE_ALIGNED(dw, who);
   if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
@@ -131,9 +157,10 @@ int haste_ffi_backward(const void* xt, const void* w, const int32_t* loc, const 
     cudaError_t e = cudaMemsetAsync(dxt, 0, sizeof(float) * D * B, st);
     if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "%s: cudaMemsetAsync: %s", who, cudaGetErrorString(e));
   }
-  if (backward_sm100_supported(xt, w, dy, dw, B, D, F, L, G)) return launch_backward_sm100(xt, w, loc, dy, dxt, dw, dbias, nullptr, B, D, F, L, G, ldy, st);
+  if (backward_sm100_supported(xt, w, dy, dw, B, D, F, L, G, ldxt))
+    return launch_backward_sm100(xt, w, loc, dy, dxt, dw, dbias, nullptr, B, D, F, L, G, ldy, ldxt, st);
   if (int rc = launch_bwd_features(w, loc, dy, dxt, B, D, F, L, G, ldy, st)) return rc;
-  return launch_bwd_weights(xt, loc, dy, dw, dbias, nullptr, B, D, F, L, G, ldy, st);
+  return launch_bwd_weights(xt, loc, dy, dw, dbias, nullptr, B, D, F, L, G, ldy, ldxt, st);
 }
 
 int haste_pad_rows_bf16(const void* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows, int64_t cols, haste_stream_t stream) {
@@ -156,9 +183,9 @@ int haste_ffi_bww_sr_sgd(const void* xt, const int32_t* loc, const void* dy, voi
   u.w = static_cast<__nv_bfloat16*>(w); u.bias = static_cast<__nv_bfloat16*>(bias);
   u.mom_w = (mu != 0.f) ? mom_w : nullptr; u.mom_b = (mu != 0.f) ? mom_b : nullptr;
   u.lr = lr; u.wd = wd; u.mu = mu; u.seed = seed; u.step = step; u.flags = flags; u.label0 = label0;
-  if (backward_sm100_supported(xt, nullptr, dy, w, B, D, F, L, G))
-    return launch_backward_sm100(xt, nullptr, loc, dy, nullptr, nullptr, nullptr, &u, B, D, F, L, G, ldy, static_cast<cudaStream_t>(stream));
-  return launch_bwd_weights(xt, loc, dy, nullptr, nullptr, &u, B, D, F, L, G, ldy, static_cast<cudaStream_t>(stream));
+  if (backward_sm100_supported(xt, nullptr, dy, w, B, D, F, L, G, B))
+    return launch_backward_sm100(xt, nullptr, loc, dy, nullptr, nullptr, nullptr, &u, B, D, F, L, G, ldy, B, static_cast<cudaStream_t>(stream));
+  return launch_bwd_weights(xt, loc, dy, nullptr, nullptr, &u, B, D, F, L, G, ldy, B, static_cast<cudaStream_t>(stream));
 }
 
 int haste_targets_bucket(const int32_t* coo, int64_t nnz, int64_t label0, int64_t L, int64_t G, int32_t* tgt_ptr, uint32_t* tgt_ent,
@@ -179,19 +206,24 @@ int haste_targets_bucket_noalloc(const int32_t* coo, int64_t nnz, int64_t label0
   return launch_targets_bucket_noalloc(coo, nnz, label0, L, G, tgt_ptr, tgt_ent, static_cast<cudaStream_t>(stream));
 }
 
-int haste_ffi_step_prepare(const void* x, void* xt, float* dxt, float* loss, const int32_t* coo, int64_t nnz, int64_t label0, int64_t L,
-                           int64_t G, int32_t* tgt_ptr, uint32_t* tgt_ent, int64_t B, int64_t D, haste_stream_t stream) {
+static int step_prepare_impl(const void* x, void* xt, float* dxt, float* loss, const int32_t* coo, int64_t nnz, int64_t label0, int64_t L,
+                             int64_t G, int32_t* tgt_ptr, uint32_t* tgt_ent, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_ffi_step_prepare";
   REQUIRE_PTR(x, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(dxt, who); REQUIRE_PTR(tgt_ptr, who);
   if (nnz < 0 || L < 1 || G < 1 || G > 256 || B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad sizes", who);
   if (nnz > 0) { REQUIRE_PTR(coo, who); REQUIRE_PTR(tgt_ent, who); }
-  return launch_step_prepare(x, xt, dxt, loss, coo, nnz, label0, L, G, tgt_ptr, tgt_ent, B, D, static_cast<cudaStream_t>(stream));
+  return launch_step_prepare(x, xt, dxt, loss, coo, nnz, label0, L, G, tgt_ptr, tgt_ent, B, D, ldxt, static_cast<cudaStream_t>(stream));
+}
+
+int haste_ffi_step_prepare(const void* x, void* xt, float* dxt, float* loss, const int32_t* coo, int64_t nnz, int64_t label0, int64_t L,
+                           int64_t G, int32_t* tgt_ptr, uint32_t* tgt_ent, int64_t B, int64_t D, haste_stream_t stream) {
+  return step_prepare_impl(x, xt, dxt, loss, coo, nnz, label0, L, G, tgt_ptr, tgt_ent, B, D, B, stream);
 }
 
 static int train_step_impl(const StepDump* dump, const int32_t* loc, const void* xt, void* w, void* bias, float* mom_w, float* mom_b, const int32_t* tgt_ptr,
                          const uint32_t* tgt_ent, float* dxt, float* loss, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G,
                          int64_t label0, int32_t loss_kind, float grad_scale, float lr, float wd, float mu, uint64_t seed, uint32_t step,
-                         uint32_t flags, haste_stream_t stream) {
+                         uint32_t flags, int64_t ldxt, haste_stream_t stream) {
   const char* who = dump ? "haste_ffi_train_step_dbg" : "haste_ffi_train_step";
   REQUIRE_PTR(loc, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(w, who); REQUIRE_PTR(tgt_ptr, who); REQUIRE_PTR(dxt, who);
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(w, who); REQUIRE_ALIGNED(dxt, who);
@@ -208,7 +240,7 @@ static int train_step_impl(const StepDump* dump, const int32_t* loc, const void*
   u.w = static_cast<__nv_bfloat16*>(w); u.bias = static_cast<__nv_bfloat16*>(bias);
   u.mom_w = (mu != 0.f) ? mom_w : nullptr; u.mom_b = (mu != 0.f) ? mom_b : nullptr;
   u.lr = lr; u.wd = wd; u.mu = mu; u.seed = seed; u.step = step; u.flags = flags; u.label0 = label0;
-  return launch_train_step(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, st, dump);
+  return launch_train_step(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, ldxt, st, dump);
 }
 
 int haste_ffi_train_step(const int32_t* loc, const void* xt, void* w, void* bias, float* mom_w, float* mom_b, const int32_t* tgt_ptr,
@@ -216,18 +248,36 @@ int haste_ffi_train_step(const int32_t* loc, const void* xt, void* w, void* bias
                          int64_t label0, int32_t loss_kind, float grad_scale, float lr, float wd, float mu, uint64_t seed, uint32_t step,
                          uint32_t flags, haste_stream_t stream) {
   return train_step_impl(nullptr, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, B, D, F, L, G, label0, loss_kind, grad_scale,
-                         lr, wd, mu, seed, step, flags, stream);
+                         lr, wd, mu, seed, step, flags, B, stream);
+}
+
+int haste_ffi_train_step_ldx(const int32_t* loc, const void* xt, void* w, void* bias, float* mom_w, float* mom_b, const int32_t* tgt_ptr,
+                             const uint32_t* tgt_ent, float* dxt, float* loss, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G,
+                             int64_t label0, int32_t loss_kind, float grad_scale, float lr, float wd, float mu, uint64_t seed,
+                             uint32_t step, uint32_t flags, int64_t ldxt, haste_stream_t stream) {
+  if (int rc = check_ldxt("haste_ffi_train_step", B, ldxt)) return rc;
+  return train_step_impl(nullptr, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, B, D, F, L, G, label0, loss_kind, grad_scale,
+                         lr, wd, mu, seed, step, flags, ldxt, stream);
 }
 
 int haste_ffi_step(const void* x, const int32_t* coo, int64_t nnz, const int32_t* loc, void* xt, void* w, void* bias, float* mom_w,
                    float* mom_b, int32_t* tgt_ptr, uint32_t* tgt_ent, float* dxt, float* loss, int64_t B, int64_t D, int64_t F, int64_t L,
                    int64_t G, int64_t label0, int32_t loss_kind, float grad_scale, float lr, float wd, float mu, uint64_t seed,
                    uint32_t step, uint32_t flags, haste_stream_t stream) {
-  if (int rc = haste_ffi_step_prepare(x, xt, dxt, loss, coo, nnz, label0, L, G, tgt_ptr, tgt_ent, B, D, stream)) return rc;
+  return haste_ffi_step_ldx(x, coo, nnz, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, B, D, F, L, G, label0, loss_kind,
+                            grad_scale, lr, wd, mu, seed, step, flags, B, stream);
+}
+
+int haste_ffi_step_ldx(const void* x, const int32_t* coo, int64_t nnz, const int32_t* loc, void* xt, void* w, void* bias, float* mom_w,
+                       float* mom_b, int32_t* tgt_ptr, uint32_t* tgt_ent, float* dxt, float* loss, int64_t B, int64_t D, int64_t F,
+                       int64_t L, int64_t G, int64_t label0, int32_t loss_kind, float grad_scale, float lr, float wd, float mu,
+                       uint64_t seed, uint32_t step, uint32_t flags, int64_t ldxt, haste_stream_t stream) {
+  if (int rc = check_ldxt("haste_ffi_step", B, ldxt)) return rc;
+  if (int rc = step_prepare_impl(x, xt, dxt, loss, coo, nnz, label0, L, G, tgt_ptr, tgt_ent, B, D, ldxt, stream)) return rc;
   // the step follows its own preparation kernel in the same stream: its set-up may overlap that kernel's tail
   dependent_launch_scope(1);
   const int rc = train_step_impl(nullptr, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, B, D, F, L, G, label0, loss_kind,
-                                 grad_scale, lr, wd, mu, seed, step, flags & ~static_cast<uint32_t>(HASTE_F_ZERO_DXT), stream);
+                                 grad_scale, lr, wd, mu, seed, step, flags & ~static_cast<uint32_t>(HASTE_F_ZERO_DXT), ldxt, stream);
   dependent_launch_scope(0);
   return rc;
 }
@@ -239,7 +289,7 @@ int haste_ffi_train_step_dbg(const int32_t* loc, const void* xt, void* w, void* 
                              haste_stream_t stream) {
   StepDump d{z_dump, ldz, dw_dump, dbias_dump};
   return train_step_impl(&d, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, B, D, F, L, G, label0, loss_kind, grad_scale, lr,
-                         wd, mu, seed, step, flags, stream);
+                         wd, mu, seed, step, flags, B, stream);
 }
 
 int haste_sr_round(const float* x, void* out, int64_t n, uint64_t seed, haste_stream_t stream) {
@@ -266,10 +316,15 @@ int haste_dxt_to_dx_sr(const float* dxt, void* dx, int64_t B, int64_t D, uint64_
 }
 
 int haste_transpose_bf16(const void* x, void* xt, int64_t B, int64_t D, haste_stream_t stream) {
+  return haste_transpose_bf16_ldx(x, xt, B, D, B, stream);
+}
+
+int haste_transpose_bf16_ldx(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_transpose_bf16";
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
   REQUIRE_PTR(x, who); REQUIRE_PTR(xt, who);
   if (B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad shape", who);
-  return launch_transpose(x, xt, B, D, static_cast<cudaStream_t>(stream));
+  return launch_transpose(x, xt, B, D, ldxt, static_cast<cudaStream_t>(stream));
 }
 
 int haste_ffi_rewire(void* w, int32_t* loc, float* mom_w, int64_t D, int64_t F, int64_t L, int64_t G, int64_t group0, int32_t prune_mode,
@@ -354,11 +409,18 @@ int haste_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t 
 int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void* bias, void* zbuf, int64_t ldz, int64_t B, int64_t D,
                    int64_t F, int64_t L, int64_t G, int64_t groups_per_chunk, int32_t k, int64_t label0, float* vals, int32_t* idx,
                    haste_stream_t stream) {
+  return haste_ffi_topk_ldx(loc, xt, w, bias, zbuf, ldz, B, D, F, L, G, groups_per_chunk, k, label0, vals, idx, B, stream);
+}
+
+int haste_ffi_topk_ldx(const int32_t* loc, const void* xt, const void* w, const void* bias, void* zbuf, int64_t ldz, int64_t B, int64_t D,
+                       int64_t F, int64_t L, int64_t G, int64_t groups_per_chunk, int32_t k, int64_t label0, float* vals, int32_t* idx,
+                       int64_t ldxt, haste_stream_t stream) {
   const char* who = "haste_ffi_topk";
   REQUIRE_PTR(loc, who); REQUIRE_PTR(xt, who); REQUIRE_PTR(w, who); REQUIRE_PTR(zbuf, who); REQUIRE_PTR(vals, who); REQUIRE_PTR(idx, who);
   REQUIRE_ALIGNED(xt, who); REQUIRE_ALIGNED(w, who); REQUIRE_ALIGNED(zbuf, who);
   if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
   if (k < 1 || k > 128) return fail(HASTE_ERR_UNSUPPORTED, "%s: k=%d outside [1,128]", who, k);
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
   if (groups_per_chunk < 1 || label0 < 0) return fail(HASTE_ERR_BAD_ARG, "%s: bad chunk size or label offset", who);
   if (ldz < groups_per_chunk * G || (ldz % 8) != 0)
     return fail(HASTE_ERR_BAD_ARG, "%s: the logit buffer needs a row stride of at least groups_per_chunk * G columns, a multiple of 8", who);
@@ -371,7 +433,7 @@ int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void
     const int64_t g1 = g0 + groups_per_chunk < NG ? g0 + groups_per_chunk : NG;
     const int64_t l0 = g0 * G, l1 = g1 * G < L ? g1 * G : L, C = l1 - l0;
     const int64_t zw = (C + 7) / 8 * 8;        // the forward writes zeros into the columns that pad the last group's row
-    if (int rc = launch_forward(loc + g0 * F, xt, wb + l0 * F * 2, bias ? bb + l0 * 2 : nullptr, zbuf, B, D, F, C, G, ldz, zw, st)) return rc;
+    if (int rc = launch_forward(loc + g0 * F, xt, wb + l0 * F * 2, bias ? bb + l0 * 2 : nullptr, zbuf, B, D, F, C, G, ldz, zw, ldxt, st)) return rc;
     if (int rc = launch_topk_update(zbuf, ldz, B, C, label0 + l0, k, vals, idx, st)) return rc;
   }
   return HASTE_OK;

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) dxt_to_dx_sr_kernel(const float* __restri
   }
 }
 
-__global__ void __launch_bounds__(256) transpose_bf16_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ xt, int64_t B, int64_t D) {
+__global__ void __launch_bounds__(256) transpose_bf16_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ xt, int64_t B, int64_t D, int64_t ldxt) {
   __shared__ uint16_t tile[32][34];
   const int64_t d0 = static_cast<int64_t>(blockIdx.x) * 32, b0 = static_cast<int64_t>(blockIdx.y) * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) transpose_bf16_kernel(const uint16_t* __r
   __syncthreads();
   for (int j = ty; j < 32; j += 8) {
     const int64_t d = d0 + j, b = b0 + tx;
-    if (d < D && b < B) xt[d * B + b] = tile[tx][j];
+    if (d < D && b < ldxt) xt[d * ldxt + b] = tile[tx][j];      // columns B .. ldxt-1 receive zeros
   }
 }
 
@@ -177,18 +177,19 @@ __global__ void tgt_fill_kernel(const int32_t* __restrict__ coo, int64_t nnz, in
 }
 
 // ---------------------------------------------------------------- per-step preparation in one launch
+// Columns B .. ldxt-1 of xt (a padded row stride) are written as zeros.
 // Block 0 buckets the COO targets entirely in shared memory (count, scan, fill: no global scratch) and clears
 // the loss scalar; every other block transposes one 32x32 tile of x [B,D] -> xt [D,B] and clears the same tile
 // of dxt [D,B].  Replaces one memset, the three bucketing kernels, the transpose and two fills.
 constexpr int PREP_THREADS = 1024;
-// VEC: B and D are multiples of 8 and the three arrays are 16-byte aligned; a block then moves a 64 (batch) x 128
+// VEC: D and the row stride of xt are multiples of 8 and the three arrays are 16-byte aligned; a block then moves a 64 (batch) x 128
 // (feature) tile with 16-byte accesses on both sides, so that the whole preparation is a few dozen blocks and still
 // finishes in microseconds when most SMs are held by a persistent kernel of another stream.
 template <bool VEC>
 __global__ void __launch_bounds__(PREP_THREADS) step_prepare_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ xt, float* __restrict__ dxt,
                                                                     float* __restrict__ loss, const int32_t* __restrict__ coo, int64_t nnz,
                                                                     int64_t label0, int64_t L, int G, int NG, int32_t* __restrict__ ptr,
-                                                                    uint32_t* __restrict__ ent, int64_t B, int64_t D, int tiles_d) {
+                                                                    uint32_t* __restrict__ ent, int64_t B, int64_t D, int64_t ldxt, int tiles_d) {
   extern __shared__ int32_t cnt[];          // NG counters, then reused as fill cursors
   __shared__ int part[PREP_THREADS];
   const int tid = threadIdx.x;
@@ -266,19 +267,20 @@ __global__ void __launch_bounds__(PREP_THREADS) step_prepare_kernel(const uint16
     {
       const int dl = tid >> 3, b8 = tid & 7;                 // 8 lanes write one 128-byte run of a row of xt
       const int64_t d = d0 + dl, b = b0 + b8 * 8;
-      if (d < D && b < B) {
+      if (d < D && b < ldxt) {                               // columns B .. ldxt-1 receive the zeros of the tile
         const int col = (((dl >> 3) ^ b8) << 3) | (dl & 7);  // rows b8*8 .. b8*8+7 all lie in 8-row group b8
         uint32_t w[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = static_cast<uint32_t>(tile[b8 * 8 + 2 * i][col]) | (static_cast<uint32_t>(tile[b8 * 8 + 2 * i + 1][col]) << 16);
-        *reinterpret_cast<uint4*>(xt + d * B + b) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(xt + d * ldxt + b) = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int idx = tid + k * PREP_THREADS, dl = idx >> 4, c = idx & 15;
-      const int64_t d = d0 + dl, b = b0 + c * 4;
-      if (d < D && b < B) *reinterpret_cast<float4*>(dxt + d * B + b) = make_float4(0.f, 0.f, 0.f, 0.f);
+      // dxt is cleared as one flat array (D % 8 == 0, so D * B is a multiple of 4): the blocks' shares of 128 x 64 floats
+      // together cover it for every B
+      const int64_t i4 = static_cast<int64_t>(blk) * (128 * 64 / 4) + tid + k * PREP_THREADS;
+      if (i4 * 4 < D * B) reinterpret_cast<float4*>(dxt)[i4] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     return;
   }
@@ -292,24 +294,25 @@ __global__ void __launch_bounds__(PREP_THREADS) step_prepare_kernel(const uint16
   __syncthreads();
   {
     const int64_t d = d0 + ty, b = b0 + tx;
-    if (d < D && b < B) { xt[d * B + b] = tile[tx][ty]; dxt[d * B + b] = 0.f; }
+    if (d < D && b < ldxt) xt[d * ldxt + b] = tile[tx][ty];
+    if (d < D && b < B) dxt[d * B + b] = 0.f;
   }
 }
 
 int launch_step_prepare(const void* x, void* xt, float* dxt, float* loss, const int32_t* coo, int64_t nnz, int64_t label0, int64_t L,
-                        int64_t G, int32_t* ptr, uint32_t* ent, int64_t B, int64_t D, cudaStream_t st) {
+                        int64_t G, int32_t* ptr, uint32_t* ent, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st) {
   const int64_t NG = (L + G - 1) / G;
   if (reinterpret_cast<uintptr_t>(coo) & 7) return fail(HASTE_ERR_BAD_ARG, "haste_ffi_step_prepare: the COO target pairs must start on an 8-byte boundary");
   const size_t sm = sizeof(int32_t) * static_cast<size_t>(NG);
   if (sm > 200 * 1024) return fail(HASTE_ERR_TOO_LARGE, "haste_ffi_step_prepare: %lld label groups need more shared memory than one block has; "
                                    "use haste_transpose_bf16 + haste_targets_bucket", (long long)NG);
-  const bool vec = (B % 8) == 0 && (D % 8) == 0 && aligned16(x) && aligned16(xt) && aligned16(dxt);
+  const bool vec = (ldxt % 8) == 0 && (D % 8) == 0 && aligned16(x) && aligned16(xt) && aligned16(dxt);
   auto k = vec ? step_prepare_kernel<true> : step_prepare_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
   if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  const int tiles_d = static_cast<int>(vec ? (D + 127) / 128 : (D + 31) / 32), tiles_b = static_cast<int>(vec ? (B + 63) / 64 : (B + 31) / 32);
+  const int tiles_d = static_cast<int>(vec ? (D + 127) / 128 : (D + 31) / 32), tiles_b = static_cast<int>(vec ? (ldxt + 63) / 64 : (ldxt + 31) / 32);
   k<<<1 + tiles_d * tiles_b, PREP_THREADS, sm, st>>>((const uint16_t*)x, (uint16_t*)xt, dxt, loss, coo, nnz, label0, L, int(G), int(NG), ptr, ent, B, D,
-                                                     tiles_d);
+                                                     ldxt, tiles_d);
   return check_launch("step_prepare_kernel");
 }
 
@@ -369,9 +372,9 @@ int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t 
   return check_launch("dxt_to_dx_sr_kernel");
 }
 
-int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, cudaStream_t st) {
-  dim3 grid(static_cast<unsigned>((D + 31) / 32), static_cast<unsigned>((B + 31) / 32));
-  transpose_bf16_kernel<<<grid, 256, 0, st>>>((const uint16_t*)x, (uint16_t*)xt, B, D);
+int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st) {
+  dim3 grid(static_cast<unsigned>((D + 31) / 32), static_cast<unsigned>((ldxt + 31) / 32));
+  transpose_bf16_kernel<<<grid, 256, 0, st>>>((const uint16_t*)x, (uint16_t*)xt, B, D, ldxt);
   return check_launch("transpose_bf16_kernel");
 }
 

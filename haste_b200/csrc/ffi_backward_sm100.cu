@@ -1,5 +1,5 @@
-// Unfused backward of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size 128, fan-in 64) and
-// (group size 64, fan-in 128): one pass over dY [B, ldy] produces both gradients of the autograd surface,
+// Unfused backward of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size, fan-in) = (128, 64), (64, 128), (64, 64)
+// and, with two consecutive groups per tile, (32, 64) and (32, 32): one pass over dY [B, ldy] produces both gradients of the autograd surface,
 //     dxt[loc[g,k], b] += sum_{l in g} w[l,k] * dy[b,l]          (fp32, reduced into dxt with red.global.add)
 //     dw [l, k]         = sum_b dy[b,l] * xt[loc[g,k], b]          (bf16, round to nearest)
 //     dbias[l]          = sum_b dy[b,l]                            (bf16; via a row of ones under the X tile)
@@ -30,10 +30,13 @@ namespace haste {
 namespace b100 {
 using namespace sm100;
 
-template <int G_, int F_>
+template <int GG_, int FF_, int P_>
 struct Cfg {
-  static constexpr int G = G_, F = F_, BT = 128;
-  static_assert((G == 128 && F == 64) || (G == 64 && F == 128), "shapes with a tcgen05 backward");
+  static constexpr int GG = GG_, FF = FF_, P = P_;     // label group, fan-in, groups per tile
+  static constexpr int G = P * GG, F = P * FF, BT = 128;
+  static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)), "tile shapes with a tcgen05 backward");
+  static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
+  static constexpr int WROW = FF == 32 ? 64 : 128;    // bytes of one swizzled row of a W block
   static constexpr int FR = F + 16;                   // X block rows: F gathered rows, one row of ones, 15 zero rows
   // Shared memory goes to the dY ring first: dY streams from HBM (several microseconds from request to arrival under
   // load, and a tile that has arrived still has to be shifted), the X rows come out of L2.
@@ -42,7 +45,7 @@ struct Cfg {
   static constexpr int NDX = 2;                       // dXg accumulator stages
   static constexpr int NDW = (F == 64) ? 2 : 1;       // dW accumulator stages
   static constexpr int XBLK = FR * 128, XSTAGE = 2 * XBLK;
-  static constexpr int NWB = F / 64, WBLK = G * 128, WSTAGE = NWB * WBLK;
+  static constexpr int NWB = FF == 32 ? 1 : FF / 64, WBLK = G * WROW, WSTAGE = NWB * WBLK;
   static constexpr int NYB = G / 64, YBLK = BT * 128, YSTAGE = NYB * YBLK;
   static constexpr int NCH = G / 8;                   // 16-byte chunks of a row slice
   static constexpr int YSIDE = BT * 16;               // one more aligned chunk per row (the tail of a misaligned slice)
@@ -72,6 +75,7 @@ struct Cfg {
   static constexpr uint32_t TM_DX = 0, TM_DW = NDX * F, TM_COLS = 512;
   static_assert(TM_DW + NDW * FR <= TM_COLS, "TMEM budget");
   static constexpr int ROWS_PER_Q = G / 4;            // label rows of the dW accumulator in one TMEM lane quarter
+  static_assert(GG % ROWS_PER_Q == 0, "the rows of a lane quarter belong to one group");
 };
 
 struct BwdArgs {
@@ -82,7 +86,7 @@ struct BwdArgs {
   __nv_bfloat16* dbias;
   int* err;
   int64_t B, L, ldy;
-  int D, NG;
+  int D, NG, NGR;      // NG: tiles of G labels; NGR: label groups
   long long wait_limit;
 };
 
@@ -94,12 +98,13 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // DX / DW: which gradients this instantiation produces (the roles of the other one are compiled out: its issuer, its
 // operand loads, its epilogue warps).  UPD (with DW): the dW writer warps apply SGD + weight decay (+ momentum) +
 // stochastic rounding to the weights and bias in global memory instead of storing the gradient.
-template <int G_, int F_, bool DX, bool DW, bool UPD>
-__global__ void __launch_bounds__(Cfg<G_, F_>::NTHREADS, 1)
+template <int GG_, int FF_, int P_, bool DX, bool DW, bool UPD>
+__global__ void __launch_bounds__(Cfg<GG_, FF_, P_>::NTHREADS, 1)
 ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w) {
   static_assert(DX || DW, "nothing to compute");
   static_assert(!UPD || DW, "the update consumes the weight gradient");
-  using C = Cfg<G_, F_>;
+  using C = Cfg<GG_, FF_, P_>;
+  constexpr int GG = C::GG, FF = C::FF, P = C::P;
   constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX, NDW = C::NDW;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE, NCH = C::NCH;
   extern __shared__ uint8_t smem_raw[];
@@ -158,7 +163,11 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
       int locv[F / 32];
 #pragma unroll
-      for (int j = 0; j < F / 32; ++j) locv[j] = min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1);   // clamped: never addresses outside xt / dxt
+      for (int j = 0; j < F / 32; ++j) {
+        // the last tile may hold one group less: its slots gather row 0 and meet zero weights and zero dY
+        const bool there = P == 1 || lane + 32 * j < (a.NGR - g * P) * FF;
+        locv[j] = there ? min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1) : 0;   // clamped: never addresses outside xt / dxt
+      }
       if (DX && prod_id == 0) {
         bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 31, WL, 100);
         ok = mbar_wait(bar(C::B_LEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 31, WL, 100) && ok;
@@ -311,10 +320,10 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     cp_async_wait<0>();
   } else if (warp == 1 || warp == 3) {
     // ================================================================ MMA issuers (one elected lane each)
-    constexpr uint32_t ID_BWX = make_idesc(128, F, 0, 1);
+    constexpr uint32_t ID_BWX = make_idesc(128, FF, 0, 1);
     constexpr uint32_t ID_BWW = make_idesc(G, FR, 1, 0);
     const uint64_t D_XB = make_sdesc(sbase + C::OFF_X, 16, 1024);      // X tile as K-major  B   (backward-weights)
-    const uint64_t D_WM = make_sdesc(sbase + C::OFF_W, WBLK, 1024);    // W tile as MN-major B   (backward-features)
+    const uint64_t D_WM = FF == 32 ? make_sdesc64(sbase + C::OFF_W, WBLK, 512) : make_sdesc(sbase + C::OFF_W, WBLK, 1024);   // W tile as MN-major B   (backward-features)
     const uint64_t D_YA = make_sdesc(sbase + C::OFF_Y, 16, 1024);      // Y tile as K-major  A   (backward-features)
     const uint64_t D_YM = make_sdesc(sbase + C::OFF_Y, YBLK, 1024);    // Y tile as MN-major A   (backward-weights)
     if (warp == 1 && DX) {
@@ -334,10 +343,15 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
           const uint32_t tdx = tmem + C::TM_DX + ds * F;
           // dXg[b,k] = sum over label chunks of Y[b, l-chunk] * W[l-chunk, k]
           if (ok && elect_one()) {
-            umma_bf16_lohi<false>(tdx, ya, ya_hi, wm, wm_hi, id_bwx);
 #pragma unroll
-            for (int ks = 1; ks < G / 16; ++ks)
-              umma_bf16_lohi<true>(tdx, ya + (((ks >> 2) * YBLK + (ks & 3) * 32) >> 4), ya_hi, wm + ((ks * 2048) >> 4), wm_hi, id_bwx);
+            for (int p = 0; p < P; ++p) {        // group p of the tile: its labels against its slots
+              constexpr int KS = GG / 16;
+              umma_bf16_lohi<false>(tdx + p * FF, ya + ((((p * KS) >> 2) * YBLK + ((p * KS) & 3) * 32) >> 4), ya_hi,
+                                    wm + ((p * KS * 16 * C::WROW) >> 4), wm_hi, id_bwx);
+#pragma unroll
+              for (int ks = p * KS + 1; ks < (p + 1) * KS; ++ks)
+                umma_bf16_lohi<true>(tdx + p * FF, ya + (((ks >> 2) * YBLK + (ks & 3) * 32) >> 4), ya_hi, wm + ((ks * 16 * C::WROW) >> 4), wm_hi, id_bwx);
+            }
             tc_commit(bar(C::B_DXFULL + ds));
             tc_commit(bar(C::B_YEMPTY + ys));
             if (t + 1 == T) tc_commit(bar(C::B_WEMPTY + ws));
@@ -443,14 +457,15 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       mbar_wait(bar(C::B_DWFULL + dws), (gi / NDW) & 1, abort_flag, a.err, 42, WL);
       tc_fence_after();
       const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW + dws * FR;
+      const uint32_t tg = ta + (q * C::ROWS_PER_Q) / GG * FF;      // the columns of this quarter's group: its block on the diagonal
       const bool do_row = row < rows_real && !*abort_flag;
       const int64_t l = l0 + row, gl = u.label0 + l;
       const bool fast = UPD && u.mom_w == nullptr && (u.flags & HASTE_F_SR) && (u.flags & HASTE_F_CONTRACT);
 #pragma unroll
-      for (int pc = 0; pc < F / 32; ++pc) {
+      for (int pc = 0; pc < FF / 32; ++pc) {
         uint32_t r0[32];
         __syncwarp();
-        tmem_ld32(ta + pc * 32, r0);
+        tmem_ld32(tg + pc * 32, r0);
         tmem_ld_wait();
         if (SPLIT) {
 #pragma unroll
@@ -463,7 +478,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
 #pragma unroll
           for (int c4 = 0; c4 < NCL; ++c4) {
             const int s0 = pc * 32 + half * 16 + c4 * 8;        // first of this chunk's 8 slots
-            uint4* out = reinterpret_cast<uint4*>((UPD ? u.w : a.dw) + l * F + s0);
+            uint4* out = reinterpret_cast<uint4*>((UPD ? u.w : a.dw) + l * FF + s0);
             // the gradient as the unfused kernel would store it: rounded to bf16
             const uint4 g8 = make_uint4(pack2(__uint_as_float(r0[8 * c4]), __uint_as_float(r0[8 * c4 + 1])),
                                         pack2(__uint_as_float(r0[8 * c4 + 2]), __uint_as_float(r0[8 * c4 + 3])),
@@ -482,7 +497,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
                 } else {
 #pragma unroll
                   for (int x = 0; x < 4; ++x)
-                    rnd[x] = rand16_reference(u.seed, gl * F + s0 + 2 * x) | (rand16_reference(u.seed, gl * F + s0 + 2 * x + 1) << 16);
+                    rnd[x] = rand16_reference(u.seed, gl * FF + s0 + 2 * x) | (rand16_reference(u.seed, gl * FF + s0 + 2 * x + 1) << 16);
                 }
               }
               uint32_t ob[4];
@@ -497,7 +512,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
                   ob[x] = __byte_perm(__float_as_uint(n0) + (rnd[x] & 0xFFFFu), __float_as_uint(n1) + (rnd[x] >> 16), 0x7632);
                 }
               } else {
-                float* mrow = u.mom_w != nullptr ? u.mom_w + l * F + s0 : nullptr;
+                float* mrow = u.mom_w != nullptr ? u.mom_w + l * FF + s0 : nullptr;
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                   float m0 = 0.f, m1 = 0.f;
@@ -543,10 +558,10 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
   if (warp == 1) tmem_dealloc(tmem, C::TM_COLS);
 }
 
-template <int G_, int F_>
+template <int GG_, int FF_, int P_>
 static int launch_shape(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias,
-                        const UpdateArgs* upd, int64_t B, int64_t D, int64_t L, int64_t ldy, cudaStream_t st) {
-  using C = Cfg<G_, F_>;
+                        const UpdateArgs* upd, int64_t B, int64_t D, int64_t L, int64_t ldy, int64_t ldxt, cudaStream_t st) {
+  using C = Cfg<GG_, FF_, P_>;
   if (int rc = report_pending_status("tcgen05 backward")) return rc;
   int* err_dev = nullptr;
   if (int rc = device_status_word(&err_dev)) return rc;
@@ -555,6 +570,7 @@ static int launch_shape(const void* xt, const void* w, const int32_t* loc, const
   a.loc = loc; a.dy = static_cast<const __nv_bfloat16*>(dy); a.dxt = dxt; a.dw = static_cast<__nv_bfloat16*>(dw);
   a.dbias = static_cast<__nv_bfloat16*>(dbias); a.err = err_dev;
   a.B = B; a.L = L; a.ldy = ldy; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::G - 1) / C::G);
+  a.NGR = static_cast<int>((L + C::GG - 1) / C::GG);
   a.wait_limit = wait_limit_cycles();
   UpdateArgs u{};
   if (upd) u = *upd;
@@ -562,8 +578,8 @@ static int launch_shape(const void* xt, const void* w, const int32_t* loc, const
   CUtensorMap tm_x, tm_w;
   const void* w_map = want_dx ? w : xt;
   const void* x_map = want_dw ? xt : w;
-  if (want_dw) { if (int rc = make_tmap_bf16_2d(&tm_x, x_map, static_cast<uint64_t>(B), static_cast<uint64_t>(D), static_cast<uint64_t>(B) * 2, 64, 1)) return rc; }
-  if (want_dx) { if (int rc = make_tmap_bf16_2d(&tm_w, w_map, static_cast<uint64_t>(C::F), static_cast<uint64_t>(L), static_cast<uint64_t>(C::F) * 2, 64, C::G)) return rc; }
+  if (want_dw) { if (int rc = make_tmap_bf16_2d(&tm_x, x_map, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc; }
+  if (want_dx) { if (int rc = make_tmap_bf16_2d(&tm_w, w_map, static_cast<uint64_t>(C::FF), static_cast<uint64_t>(L), static_cast<uint64_t>(C::FF) * 2, C::FF == 32 ? 32 : 64, C::G)) return rc; }
   if (!want_dw) tm_x = tm_w;
   if (!want_dx) tm_w = tm_x;
   int dev = 0, sms = 148;
@@ -572,7 +588,7 @@ static int launch_shape(const void* xt, const void* w, const int32_t* loc, const
   const int grid = a.NG < sms ? a.NG : sms;
 #define HASTE_B100_LAUNCH(DXF, DWF, UPDF)                                                                     \
   {                                                                                                          \
-    auto k = ffi_backward_sm100_kernel<G_, F_, DXF, DWF, UPDF>;                                              \
+    auto k = ffi_backward_sm100_kernel<GG_, FF_, P_, DXF, DWF, UPDF>;                                         \
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);     \
     if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));  \
     k<<<grid, C::NTHREADS, C::SMEM_BYTES, st>>>(a, u, tm_x, tm_w);                                           \
@@ -590,19 +606,23 @@ static int launch_shape(const void* xt, const void* w, const int32_t* loc, const
 
 // xt / w / dw may be NULL when the gradient that needs them is not asked for.
 bool backward_sm100_supported(const void* xt, const void* w, const void* dy, const void* dw, int64_t B, int64_t D, int64_t F, int64_t L,
-                              int64_t G) {
+                              int64_t G, int64_t ldxt) {
   // tensor maps need 16-byte aligned bases and row strides; dxt row offsets and tile coordinates are 32-bit; dy only
   // needs its natural 2-byte alignment
-  return ((G == 128 && F == 64) || (G == 64 && F == 128)) && (B % 8) == 0 && aligned16(xt) && aligned16(w) && aligned16(dw) &&
-         (reinterpret_cast<uintptr_t>(dy) & 1u) == 0 && D * B < (int64_t(1) << 32) && L < (int64_t(1) << 31) && B < (int64_t(1) << 31);
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 64 || F == 32));
+  return shape && (xt == nullptr || (ldxt % 8) == 0) && aligned16(xt) && aligned16(w) && aligned16(dw) &&
+         (reinterpret_cast<uintptr_t>(dy) & 1u) == 0 && D * B < (int64_t(1) << 32) && L < (int64_t(1) << 31) && ldxt < (int64_t(1) << 31);
 }
 
 // dxt == NULL: weight gradient only; dw == NULL and upd == NULL: feature gradient only; upd != NULL (with dxt == NULL):
 // backward-weights fused with the update of upd->w / upd->bias.
 int launch_backward_sm100(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias,
-                          const UpdateArgs* upd, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, cudaStream_t st) {
-  if (G == 128 && F == 64) return b100::launch_shape<128, 64>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, st);
-  if (G == 64 && F == 128) return b100::launch_shape<64, 128>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, st);
+                          const UpdateArgs* upd, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, int64_t ldxt, cudaStream_t st) {
+  if (G == 128 && F == 64) return b100::launch_shape<128, 64, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
+  if (G == 64 && F == 128) return b100::launch_shape<64, 128, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
+  if (G == 64 && F == 64) return b100::launch_shape<64, 64, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
+  if (G == 32 && F == 64) return b100::launch_shape<32, 64, 2>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
+  if (G == 32 && F == 32) return b100::launch_shape<32, 32, 2>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
   return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 backward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }
 

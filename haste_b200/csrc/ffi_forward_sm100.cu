@@ -1,5 +1,5 @@
-// Forward gather-GEMM of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size 128, fan-in 64) and
-// (group size 64, fan-in 128):
+// Forward gather-GEMM of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size, fan-in) = (128, 64), (64, 128),
+// (64, 64), and, with two consecutive groups per tile, (32, 64) and (32, 32):
 //     z[b, l] = sum_k xt[loc[l/G, k], b] * w[l, k] + bias[l]        (bf16 in, fp32 accumulate, bf16 out)
 // This is the unfused forward of the autograd surface: it has to write the [B, L] logits, so it is bound by
 // that HBM write (2*B*L bytes), not by the tensor pipe.
@@ -23,16 +23,19 @@ namespace haste {
 namespace f100 {
 using namespace sm100;
 
-template <int G_, int F_>
+template <int GG_, int FF_, int P_>
 struct Cfg {
-  static constexpr int G = G_, F = F_, BT = 128;
-  static_assert((G == 128 && F == 64) || (G == 64 && F == 128), "shapes with a tcgen05 forward");
+  static constexpr int GG = GG_, FF = FF_, P = P_;     // label group, fan-in, groups per tile
+  static constexpr int G = P * GG, F = P * FF, BT = 128;
+  static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)), "tile shapes with a tcgen05 forward");
+  static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
+  static constexpr int WROW = FF == 32 ? 64 : 128;    // bytes of one swizzled row of a W block
   static constexpr int FR = F + 16;                   // rows of an X block: F gathered rows, one row of ones, 15 zero rows
   static constexpr int NXS = (F == 64) ? 5 : 4;       // X ring stages
   static constexpr int XBLK = FR * 128;               // one 64-batch block of an X stage (bytes)
   static constexpr int XSTAGE = 2 * XBLK;
-  static constexpr int NWB = F / 64;                  // 64-slot blocks of a W stage
-  static constexpr int WBLK = G * 128;
+  static constexpr int NWB = FF == 32 ? 1 : FF / 64;  // blocks of a W stage (64 slots each, 32 at fan-in 32)
+  static constexpr int WBLK = G * WROW;
   static constexpr int WSTAGE = NWB * WBLK;
   static constexpr int NCB = G / 64;                  // 64-label blocks of a staging tile
   static constexpr int CBLK = BT * 128;
@@ -66,7 +69,7 @@ struct FwdArgs {
   __nv_bfloat16* z;
   int* err;
   int64_t B, L, ldz, zw;
-  int D, NG;
+  int D, NG, NGR;      // NG: tiles of G labels; NGR: label groups
   long long wait_limit;
 };
 
@@ -75,11 +78,12 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int G_, int F_>
-__global__ void __launch_bounds__(Cfg<G_, F_>::NTHREADS, 1)
+template <int GG_, int FF_, int P_>
+__global__ void __launch_bounds__(Cfg<GG_, FF_, P_>::NTHREADS, 1)
 ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_z) {
-  using C = Cfg<G_, F_>;
+  using C = Cfg<GG_, FF_, P_>;
+  constexpr int GG = C::GG, FF = C::FF, P = C::P;
   constexpr int G = C::G, F = C::F, BT = C::BT, NXS = C::NXS, XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -134,7 +138,11 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
       const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
       int locv[F / 32];
 #pragma unroll
-      for (int j = 0; j < F / 32; ++j) locv[j] = min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1);   // clamped: never addresses outside xt
+      for (int j = 0; j < F / 32; ++j) {
+        // the last tile may hold one group less: its slots gather row 0 and meet zero weights
+        const bool there = P == 1 || lane + 32 * j < (a.NGR - g * P) * FF;
+        locv[j] = there ? min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1) : 0;   // clamped: never addresses outside xt
+      }
       if (prod_id == 0) {
         uint16_t bv[G / 32];
 #pragma unroll
@@ -196,14 +204,15 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
     // ================================================================ MMA issuer
     // The warp runs its control flow converged; one elected lane issues the products and commits (descriptors stay
     // in uniform registers this way).
-    constexpr uint32_t ID_FWD = make_idesc(128, G, 1, 0);
+    constexpr uint32_t ID_FWD = make_idesc(128, GG, 1, 0);
+    constexpr uint32_t ID_BIAS = make_idesc(128, G, 1, 0);
     const uint64_t D_XA = make_sdesc(sbase + C::OFF_X, XBLK, 1024);            // X tile as MN-major A
-    const uint64_t D_WB = make_sdesc(sbase + C::OFF_W, 16, 1024);              // W tile as K-major B
+    const uint64_t D_WB = FF == 32 ? make_sdesc64(sbase + C::OFF_W, 16, 512) : make_sdesc(sbase + C::OFF_W, 16, 1024);   // W tile as K-major B
     const uint64_t D_BB = make_sdesc_noswizzle(sbase + C::OFF_BT, 128, 256);   // bias tile as K-major B (last K step)
     const uint32_t xa_lo = static_cast<uint32_t>(D_XA), xa_hi = static_cast<uint32_t>(D_XA >> 32);
     const uint32_t wb_lo = static_cast<uint32_t>(D_WB), wb_hi = static_cast<uint32_t>(D_WB >> 32);
     const uint32_t bb_lo = static_cast<uint32_t>(D_BB), bb_hi = static_cast<uint32_t>(D_BB >> 32);
-    const uint32_t id_fwd = ID_FWD;
+    const uint32_t id_fwd = ID_FWD, id_bias = ID_BIAS;
     int it = 0, xs = 0, xph = 0;
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int ws = gi & 1;
@@ -217,11 +226,15 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
         const uint32_t bb = bb_lo + (ws ? (C::BTILE >> 4) : 0u);
         const uint32_t tz = tmem + zs * G;
         if (ok && elect_one()) {          // after an abort nothing more is issued
-          umma_bf16_lohi<false>(tz, xa, xa_hi, wb, wb_hi, id_fwd);
 #pragma unroll
-          for (int ks = 1; ks < F / 16; ++ks)
-            umma_bf16_lohi<true>(tz, xa + ((ks * 2048) >> 4), xa_hi, wb + (((ks >> 2) * WBLK + (ks & 3) * 32) >> 4), wb_hi, id_fwd);
-          umma_bf16_lohi<true>(tz, xa + (((F / 16) * 2048) >> 4), xa_hi, bb, bb_hi, id_fwd);
+          for (int p = 0; p < P; ++p) {          // group p of the tile: its slots against its labels' weight rows
+            const uint32_t xp = xa + ((p * FF * 128) >> 4), wp = wb + ((p * GG * C::WROW) >> 4);
+            umma_bf16_lohi<false>(tz + p * GG, xp, xa_hi, wp, wb_hi, id_fwd);
+#pragma unroll
+            for (int ks = 1; ks < FF / 16; ++ks)
+              umma_bf16_lohi<true>(tz + p * GG, xp + ((ks * 2048) >> 4), xa_hi, wp + (((ks >> 2) * WBLK + (ks & 3) * 32) >> 4), wb_hi, id_fwd);
+          }
+          umma_bf16_lohi<true>(tz, xa + (((F / 16) * 2048) >> 4), xa_hi, bb, bb_hi, id_bias);
           tc_commit(bar(C::B_ZFULL + zs));
           tc_commit(bar(C::B_XEMPTY + xs));
           if (t + 1 == T) tc_commit(bar(C::B_WEMPTY + ws));
@@ -312,20 +325,21 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
   if (warp == 1) tmem_dealloc(tmem, C::TM_COLS);
 }
 
-template <int G_, int F_>
+template <int GG_, int FF_, int P_>
 static int launch_shape(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t L,
-                        int64_t ldz, int64_t zw, cudaStream_t st) {
-  using C = Cfg<G_, F_>;
+                        int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
+  using C = Cfg<GG_, FF_, P_>;
   if (int rc = report_pending_status("tcgen05 forward")) return rc;
   int* err_dev = nullptr;
   if (int rc = device_status_word(&err_dev)) return rc;
   FwdArgs a;
   a.loc = loc; a.bias = static_cast<const __nv_bfloat16*>(bias); a.z = static_cast<__nv_bfloat16*>(z); a.err = err_dev;
   a.B = B; a.L = L; a.ldz = ldz; a.zw = zw; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::G - 1) / C::G);
+  a.NGR = static_cast<int>((L + C::GG - 1) / C::GG);
   a.wait_limit = wait_limit_cycles();
   CUtensorMap tm_x, tm_w, tm_z;
-  if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(B), static_cast<uint64_t>(D), static_cast<uint64_t>(B) * 2, 64, 1)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tm_w, w, static_cast<uint64_t>(C::F), static_cast<uint64_t>(L), static_cast<uint64_t>(C::F) * 2, 64, C::G)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tm_w, w, static_cast<uint64_t>(C::FF), static_cast<uint64_t>(L), static_cast<uint64_t>(C::FF) * 2, C::FF == 32 ? 32 : 64, C::G)) return rc;
   // the store clips at the writable width, in whole 16-byte chunks (columns L..zw-1 of the last group receive the
   // zeros its absent weight rows produce); the kernel writes the remaining zw % 8 columns itself
   if (zw < 8) return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: writable width below 8 columns");
@@ -334,7 +348,7 @@ static int launch_shape(const int32_t* loc, const void* xt, const void* w, const
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = a.NG < sms ? a.NG : sms;
-  auto k = ffi_forward_sm100_kernel<G_, F_>;
+  auto k = ffi_forward_sm100_kernel<GG_, FF_, P_>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   k<<<grid, C::NTHREADS, C::SMEM_BYTES, st>>>(a, tm_x, tm_w, tm_z);
@@ -343,16 +357,20 @@ static int launch_shape(const int32_t* loc, const void* xt, const void* w, const
 
 }  // namespace f100
 
-bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz) {
+bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t ldxt) {
   // tensor maps need 16-byte aligned bases and row strides; coordinates are 32-bit
-  return ((G == 128 && F == 64) || (G == 64 && F == 128)) && (B % 8) == 0 && (ldz % 8) == 0 && aligned16(z) && aligned16(xt) &&
-         aligned16(w) && L < (int64_t(1) << 31) && B < (int64_t(1) << 31);
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 64 || F == 32));
+  return shape && (ldxt % 8) == 0 && (ldz % 8) == 0 && aligned16(z) && aligned16(xt) &&
+         aligned16(w) && L < (int64_t(1) << 31) && ldxt < (int64_t(1) << 31);
 }
 
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
-                         int64_t L, int64_t G, int64_t ldz, int64_t zw, cudaStream_t st) {
-  if (G == 128 && F == 64) return f100::launch_shape<128, 64>(loc, xt, w, bias, z, B, D, L, ldz, zw, st);
-  if (G == 64 && F == 128) return f100::launch_shape<64, 128>(loc, xt, w, bias, z, B, D, L, ldz, zw, st);
+                         int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
+  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
+  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
+  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
+  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
+  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
   return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }
 

@@ -114,9 +114,9 @@ __device__ __forceinline__ void load_W(__nv_bfloat16* Ws, int ldw, const __nv_bf
   load_tile(Ws, ldw, G, F, F, [&](int r) { return r < rows_real ? w + (l0 + r) * F : nullptr; }, tid);
 }
 __device__ __forceinline__ void load_X(__nv_bfloat16* Xs, int ldx, const __nv_bfloat16* xt, const int* locs, int F, int64_t B,
-                                       int64_t b0, int tid) {
+                                       int64_t ldx_g, int64_t b0, int tid) {
   const int valid = static_cast<int>(imin64(BT, B - b0));
-  load_tile(Xs, ldx, F, BT, valid, [&](int r) { return xt + static_cast<int64_t>(locs[r]) * B + b0; }, tid);
+  load_tile(Xs, ldx, F, BT, valid, [&](int r) { return xt + static_cast<int64_t>(locs[r]) * ldx_g + b0; }, tid);
 }
 __device__ __forceinline__ void load_Y(__nv_bfloat16* Ys, int ldy_s, const __nv_bfloat16* dy, int64_t ldy, int64_t B, int64_t b0,
                                        int64_t l0, int rows_real, int G, int tid) {
@@ -129,7 +129,7 @@ template <int G>
 __global__ void __launch_bounds__(NT) ffi_forward_kernel(const int32_t* __restrict__ loc, const __nv_bfloat16* __restrict__ xt,
                                                          const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
                                                          __nv_bfloat16* __restrict__ z, int64_t B, int D, int F, int64_t L,
-                                                         int64_t ldz, int64_t zw) {
+                                                         int64_t ldz, int64_t zw, int64_t ldxt) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = blockIdx.x;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(NT) ffi_forward_kernel(const int32_t* __restri
   load_loc(locs, loc + static_cast<int64_t>(g) * F, F, D, tid);
   load_W(Ws, ldw, w, l0, rows_real, G, F, tid);
   __syncthreads();
-  load_X(Xs, ldx, xt, locs, F, B, b0, tid);
+  load_X(Xs, ldx, xt, locs, F, B, ldxt, b0, tid);
   __syncthreads();
 
   float acc[1][G / 8][4];
@@ -338,7 +338,7 @@ template <int G, int FMAX, bool FUSED>
 __global__ void __launch_bounds__(NT) ffi_bwd_weights_kernel(const __nv_bfloat16* __restrict__ xt, const int32_t* __restrict__ loc,
                                                              const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dw,
                                                              __nv_bfloat16* __restrict__ dbias, UpdateArgs u, int64_t B, int D, int F,
-                                                             int64_t L, int64_t ldy) {
+                                                             int64_t L, int64_t ldy, int64_t ldxt) {
   using T = BwwTiling<G, FMAX>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(NT) ffi_bwd_weights_kernel(const __nv_bfloat16
   const int ni_n = max(0, min(T::NI, (F - n0) / 8));
   float bsum = 0.f;
   for (int64_t b0 = 0; b0 < B; b0 += BT) {
-    load_X(Xs, ldx, xt, locs, F, B, b0, tid);
+    load_X(Xs, ldx, xt, locs, F, B, ldxt, b0, tid);
     load_Y(Ys, ldys, dy, ldy, B, b0, l0, rows_real, G, tid);
     __syncthreads();
     if (ni_n > 0) warp_gemm_tn<1, T::NI>(acc, Ys, ldys, Xs, ldx, m0, n0, BT, 1, ni_n, lane);
@@ -385,7 +385,7 @@ template <int G, int FMAX, int LOSS, bool WITH_LOSS>
 __global__ void __launch_bounds__(NT, 1) ffi_train_step_mma_kernel(const int32_t* __restrict__ loc, const __nv_bfloat16* __restrict__ xt,
                                                                    const int32_t* __restrict__ tgt_ptr, const uint32_t* __restrict__ tgt_ent,
                                                                    float* __restrict__ dxt, float* __restrict__ loss, UpdateArgs u,
-                                                                   int64_t B, int D, int F, int64_t L, float grad_scale) {
+                                                                   int64_t B, int D, int F, int64_t L, float grad_scale, int64_t ldxt) {
   using T = BwwTiling<G, FMAX>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(NT, 1) ffi_train_step_mma_kernel(const int32_t
 
   for (int64_t b0 = 0; b0 < B; b0 += BT) {
     const int bvalid = static_cast<int>(imin64(BT, B - b0));
-    load_X(Xs, ldx, xt, locs, F, B, b0, tid);
+    load_X(Xs, ldx, xt, locs, F, B, ldxt, b0, tid);
     for (int i = tid; i < BT * YW; i += NT) ybits[i] = 0u;
     __syncthreads();
     for (int i = t_beg + tid; i < t_end; i += NT) {
@@ -510,9 +510,9 @@ static int set_smem(K kernel, size_t bytes) {
   else { constexpr int F_ = 128; __VA_ARGS__; }
 
 int launch_forward(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
-                   int64_t L, int64_t G, int64_t ldz, int64_t zw, cudaStream_t st) {
+                   int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
   // Shape dispatch: the tcgen05 kernel where its tile shapes apply, the warp-mma kernel otherwise
-  if (zw >= 8 && forward_sm100_supported(z, xt, w, B, F, L, G, ldz)) return launch_forward_sm100(loc, xt, w, bias, z, B, D, F, L, G, ldz, zw, st);
+  if (zw >= 8 && forward_sm100_supported(z, xt, w, B, F, L, G, ldz, ldxt)) return launch_forward_sm100(loc, xt, w, bias, z, B, D, F, L, G, ldz, zw, ldxt, st);
   const int64_t NG = (L + G - 1) / G;
   dim3 grid(static_cast<unsigned>(NG), static_cast<unsigned>((B + BT - 1) / BT));
   const size_t sm = fwd_smem(int(G), int(F));
@@ -520,7 +520,7 @@ int launch_forward(const int32_t* loc, const void* xt, const void* w, const void
     auto k = ffi_forward_kernel<G_>;
     if (int rc = set_smem(k, sm)) return rc;
     k<<<grid, NT, sm, st>>>(loc, (const __nv_bfloat16*)xt, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)z, B,
-                            int(D), int(F), L, ldz, zw);
+                            int(D), int(F), L, ldz, zw, ldxt);
   });
   return check_launch("ffi_forward_kernel");
 }
@@ -539,7 +539,7 @@ int launch_bwd_features(const void* w, const int32_t* loc, const void* dy, float
 }
 
 int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias, const UpdateArgs* upd, int64_t B,
-                       int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, cudaStream_t st) {
+                       int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, int64_t ldxt, cudaStream_t st) {
   const int64_t NG = (L + G - 1) / G;
   dim3 grid(static_cast<unsigned>(NG));
   const size_t sm = bww_smem(int(G), int(F));
@@ -549,12 +549,12 @@ int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void*
     if (upd) {
       auto k = ffi_bwd_weights_kernel<G_, F_, true>;
       if (int rc = set_smem(k, sm)) return rc;
-      k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)xt, loc, (const __nv_bfloat16*)dy, nullptr, nullptr, u, B, int(D), int(F), L, ldy);
+      k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)xt, loc, (const __nv_bfloat16*)dy, nullptr, nullptr, u, B, int(D), int(F), L, ldy, ldxt);
     } else {
       auto k = ffi_bwd_weights_kernel<G_, F_, false>;
       if (int rc = set_smem(k, sm)) return rc;
       k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)xt, loc, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dw, (__nv_bfloat16*)dbias, u, B,
-                              int(D), int(F), L, ldy);
+                              int(D), int(F), L, ldy, ldxt);
     }
   }));
   return check_launch("ffi_bwd_weights_kernel");
@@ -562,7 +562,7 @@ int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void*
 
 int launch_train_step_mma(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                           const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind, float grad_scale,
-                          cudaStream_t st) {
+                          int64_t ldxt, cudaStream_t st) {
   const int64_t NG = (L + G - 1) / G;
   dim3 grid(static_cast<unsigned>(NG));
   const size_t sm = step_smem(int(G), int(F));
@@ -571,7 +571,7 @@ int launch_train_step_mma(const int32_t* loc, const void* xt, const int32_t* tgt
   {                                                                                                           \
     auto k = ffi_train_step_mma_kernel<G_, F_, LOSSK, WL>;                                                    \
     if (int rc = set_smem(k, sm)) return rc;                                                                  \
-    k<<<grid, NT, sm, st>>>(loc, (const __nv_bfloat16*)xt, tgt_ptr, tgt_ent, dxt, loss, u, B, int(D), int(F), L, grad_scale); \
+    k<<<grid, NT, sm, st>>>(loc, (const __nv_bfloat16*)xt, tgt_ptr, tgt_ent, dxt, loss, u, B, int(D), int(F), L, grad_scale, ldxt); \
   }
   HASTE_DISPATCH_G(G, HASTE_DISPATCH_F(F, {
     if (loss_kind == HASTE_LOSS_BCE) { if (wl) HASTE_LAUNCH_STEP(HASTE_LOSS_BCE, true) else HASTE_LAUNCH_STEP(HASTE_LOSS_BCE, false) }

@@ -1,5 +1,15 @@
-// Fused FFI train step on the 5th-generation tensor cores (tcgen05 + TMEM), as a template over the two layer
-// shapes the benchmark configurations use: (group size 128, fan-in 64) and (group size 64, fan-in 128).
+// Fused FFI train step on the 5th-generation tensor cores (tcgen05 + TMEM), as a template over the layer shape
+// (group size GG, fan-in FF) and the number P of consecutive label groups that share a tile: (128, 64, 1), (64, 128, 1),
+// (64, 64, 1), (32, 64, 2), (32, 32, 2) and (32, 128, 1).
+//
+// A tile is G = P * GG labels by F = P * FF slots by 128 batch rows.  Groups of 32 labels are paired because the
+// backward-weights accumulator needs M = G >= 64 rows and because the hand-offs of a tile cost the same whatever it holds.
+// The index rows, weights and labels of consecutive groups are contiguous, so a pair loads like one group; the forward
+// and backward-features products run once per group of the pair (its own slots, its own labels), backward-weights
+// once for the pair: it also fills the two blocks that belong to no group, which nobody reads (the tensor pipe is far from
+// being the bound at these sizes).  A pair of (32, 128) groups would need a 256-slot X tile, which shared memory and TMEM
+// do not hold: there a tile has G = 64 label columns of which the upper 32 are absent (zero dY).  That shape is bound by its
+// dX reductions, F = 128 per 32 labels, which the absent columns do not add to.
 //
 // One persistent CTA per SM walks label groups g = blockIdx.x, += gridDim.x (the incomplete last round goes to the
 // highest-numbered CTAs).  Per group and per 128-row batch tile three UMMA products run out of the same three
@@ -40,18 +50,28 @@ __device__ __noinline__ static uint32_t rand16_call(uint32_t flags, uint64_t see
 
 using namespace sm100;
 
-template <int G_, int F_>
+// Loss of the kernel's template: BCE with the sigmoid from one tanh.approx (absolute error about 2^-12), squared hinge,
+// or BCE with the sigmoid from ex2 and rcp (relative error about 2^-22).
+constexpr int LOSS_BCE_EXP = 2;
+static_assert(LOSS_BCE_EXP != HASTE_LOSS_BCE && LOSS_BCE_EXP != HASTE_LOSS_SQHINGE, "distinct template values");
+
+template <int GG_, int FF_, int P_>
 struct Cfg {
-  static constexpr int G = G_, F = F_, BT = 128;
-  static_assert((G == 128 && F == 64) || (G == 64 && F == 128), "shapes with a tcgen05 fused step");
+  static constexpr int GG = GG_, FF = FF_, P = P_;     // label group, fan-in, groups per tile
+  static constexpr int LS = P * GG;                    // labels of a tile
+  static constexpr int G = LS < 64 ? 64 : LS, F = P * FF, BT = 128;      // label columns and slots of a tile
+  static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)), "tile shapes with a tcgen05 fused step");
+  static_assert(P == 1 || P == 2, "groups per tile");
+  static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
   static constexpr int FR = F + 16;                   // rows of an X block: F gathered rows, one row of ones, 15 zero rows
   static constexpr int NXS = (F == 64) ? 5 : 4;       // X ring stages
   static constexpr int NYS = 2;                       // dY ring stages
   static constexpr int NDX = (F == 64) ? 2 : 1;       // dXg accumulator stages in TMEM
   static constexpr int XBLK = FR * 128;               // one 64-batch block of an X stage (bytes)
   static constexpr int XSTAGE = 2 * XBLK;
-  static constexpr int NWB = F / 64;                  // 64-slot blocks of a W stage
-  static constexpr int WBLK = G * 128;
+  static constexpr int WROW = FF == 32 ? 64 : 128;    // bytes of one swizzled row of a W block
+  static constexpr int NWB = FF == 32 ? 1 : FF / 64;  // blocks of a W stage (64 slots each, 32 at fan-in 32)
+  static constexpr int WBLK = G * WROW;
   static constexpr int WSTAGE = NWB * WBLK;
   static constexpr int NYB = G / 64;                  // 64-label blocks of a dY stage
   static constexpr int YBLK = BT * 128;
@@ -92,8 +112,14 @@ struct Cfg {
   static constexpr int NTHREADS = (W_XP + (NPW > 2 ? NPW - 2 : 0)) * 32;
   static_assert(NTHREADS <= 1024, "thread budget");
   static constexpr int EA_COLS = G * 4 / N_EA;        // label columns of a tile handled by one loss-epilogue warp
-  static constexpr int UPS = F / 2;                   // slots updated by one update warp
+  static constexpr int UPS = FF / 2;                  // slots updated by one update warp
   static constexpr int ROWS_PER_Q = G / 4;            // label rows of the dW accumulator in one TMEM lane quarter (32, or 16 for M = 64)
+  static_assert(GG % ROWS_PER_Q == 0, "the rows of a lane quarter belong to one group");
+  // byte offset of 16-byte chunk c (8 slots) of label row `row` in a W stage
+  __device__ static __forceinline__ int w_chunk(int row, int c) {
+    if (FF == 32) return row * 64 + ((c ^ ((row >> 1) & 3)) << 4);
+    return (c >> 3) * WBLK + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+  }
 };
 
 struct StepArgs {
@@ -105,7 +131,8 @@ struct StepArgs {
   float* loss;
   int* err;
   int64_t B, L;
-  int D, NG;
+  int D, NG;           // NG: tiles of LS labels
+  int NGR;             // label groups (index rows, target buckets)
   float grad_scale;
   long long wait_limit;
   int stall_tile;      // debug builds: the first loss-epilogue warp withholds its "dY ready" arrival at this tile (-1 = never)
@@ -133,16 +160,24 @@ __device__ __forceinline__ float round_bf16_as_f32(float v) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(v), "f"(0.f));
   return __uint_as_float(d);
 }
+// 1 / (1 + e^-z), relative error about 2^-22 (ex2.approx and rcp.approx); e^-z may overflow, the quotient is then 0.
+__device__ __forceinline__ float sigmoid_exp(float z) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
-template <int G_, int F_, int LOSS, bool WITH_LOSS, bool MOM, bool DEBUG>
-__global__ void __launch_bounds__(Cfg<G_, F_>::NTHREADS, 1)
+template <int GG_, int FF_, int P_, int LOSS, bool WITH_LOSS, bool MOM, bool DEBUG>
+__global__ void __launch_bounds__(Cfg<GG_, FF_, P_>::NTHREADS, 1)
 ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w) {
-  using C = Cfg<G_, F_>;
+  using C = Cfg<GG_, FF_, P_>;
+  constexpr int GG = C::GG, FF = C::FF, P = C::P, LS = C::LS;
   constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE;
   constexpr int N_EA = C::N_EA, N_EB = C::N_EB, N_UP = C::N_UP, EA_COLS = C::EA_COLS, UPS = C::UPS;
@@ -228,12 +263,16 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int ws = gi & 1;
-      const int64_t l0 = static_cast<int64_t>(g) * G;
-      const int rows_real = static_cast<int>(imin64(G, a.L - l0));
+      const int64_t l0 = static_cast<int64_t>(g) * LS;
+      const int rows_real = static_cast<int>(imin64(LS, a.L - l0));
       const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
       int locv[F / 32];
 #pragma unroll
-      for (int j = 0; j < F / 32; ++j) locv[j] = min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1);   // clamped: never addresses outside xt / dxt
+      for (int j = 0; j < F / 32; ++j) {
+        // the last tile may hold one group less: its slots gather row 0 and meet zero weights and zero dY
+        const bool there = P == 1 || lane + 32 * j < (a.NGR - g * P) * FF;
+        locv[j] = there ? min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1) : 0;   // clamped: never addresses outside xt / dxt
+      }
       if (prod_id == 0) {
       uint16_t bv[G / 32];
 #pragma unroll
@@ -303,17 +342,18 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     // Feeding the tensor pipe from a single thread costs more cycles per tcgen05.mma than the small (N = 64..144)
     // products take to execute, so the work is split: warp 1 issues forward + backward-features, warp 3 issues
     // backward-weights.  Both hang off the same mbarriers; the pipe executes in arrival order.
-    constexpr uint32_t ID_FWD = make_idesc(128, G, 1, 0);
-    constexpr uint32_t ID_BWX = make_idesc(128, F, 0, 1);
+    constexpr uint32_t ID_FWD = make_idesc(128, GG, 1, 0);
+    constexpr uint32_t ID_BIAS = make_idesc(128, LS, 1, 0);
+    constexpr uint32_t ID_BWX = make_idesc(128, FF, 0, 1);
     constexpr uint32_t ID_BWW = make_idesc(G, FR, 1, 0);
     // Descriptors are built once.  Per MMA only the start-address field (low word, 16-byte units) moves, by
     // compile-time constants; it never carries out of its 14-bit field because every operand lies inside the
     // CTA's shared memory window.
     const uint64_t D_XA = make_sdesc(sbase + C::OFF_X, XBLK, 1024);            // X tile as MN-major A   (forward)
     const uint64_t D_XB = make_sdesc(sbase + C::OFF_X, 16, 1024);              // X tile as K-major  B   (backward-weights)
-    const uint64_t D_WB = make_sdesc(sbase + C::OFF_W, 16, 1024);              // W tile as K-major  B   (forward)
+    const uint64_t D_WB = FF == 32 ? make_sdesc64(sbase + C::OFF_W, 16, 512) : make_sdesc(sbase + C::OFF_W, 16, 1024);   // W tile as K-major  B   (forward)
     const uint64_t D_BB = make_sdesc_noswizzle(sbase + C::OFF_BT, 128, 256);   // bias tile as K-major B (forward, last K step)
-    const uint64_t D_WM = make_sdesc(sbase + C::OFF_W, WBLK, 1024);            // W tile as MN-major B   (backward-features)
+    const uint64_t D_WM = FF == 32 ? make_sdesc64(sbase + C::OFF_W, WBLK, 512) : make_sdesc(sbase + C::OFF_W, WBLK, 1024);   // W tile as MN-major B   (backward-features)
     const uint64_t D_YA = make_sdesc(sbase + C::OFF_Y, 16, 1024);              // Y tile as K-major  A   (backward-features)
     const uint64_t D_YM = make_sdesc(sbase + C::OFF_Y, YBLK, 1024);            // Y tile as MN-major A   (backward-weights)
     if (warp == 1) {
@@ -323,7 +363,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       const uint32_t bb_lo = static_cast<uint32_t>(D_BB), bb_hi = static_cast<uint32_t>(D_BB >> 32);
       const uint32_t wm_lo = static_cast<uint32_t>(D_WM), wm_hi = static_cast<uint32_t>(D_WM >> 32);
       const uint32_t ya_lo = static_cast<uint32_t>(D_YA), ya_hi = static_cast<uint32_t>(D_YA >> 32);
-      const uint32_t id_fwd = ID_FWD, id_bwx = ID_BWX;
+      const uint32_t id_fwd = ID_FWD, id_bias = ID_BIAS, id_bwx = ID_BWX;
       // Order of issue: forward(it) first, then backward-features of tile it - 1.  Both become possible at the same
       // moment (the loss epilogue finished a tile); the forward product goes first because the epilogue warps are
       // waiting for it, while nothing waits for the backward product's dY stage yet.
@@ -339,10 +379,15 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         // dXg[b,k] = sum over label chunks of Y[b, l-chunk] * W[l-chunk, k]
         const bool last_of_group = j_t + 1 == T;
         if (ok && elect_one()) {          // after an abort nothing more is issued
-          umma_bf16_lohi<false>(tdx, ya, ya_hi, wm, wm_hi, id_bwx);
 #pragma unroll
-          for (int ks = 1; ks < G / 16; ++ks)
-            umma_bf16_lohi<true>(tdx, ya + (((ks >> 2) * YBLK + (ks & 3) * 32) >> 4), ya_hi, wm + ((ks * 2048) >> 4), wm_hi, id_bwx);
+          for (int p = 0; p < P; ++p) {          // group p of the tile: its labels against its slots
+            constexpr int KS = GG / 16;
+            umma_bf16_lohi<false>(tdx + p * FF, ya + ((((p * KS) >> 2) * YBLK + ((p * KS) & 3) * 32) >> 4), ya_hi,
+                                  wm + ((p * KS * 16 * C::WROW) >> 4), wm_hi, id_bwx);
+#pragma unroll
+            for (int ks = p * KS + 1; ks < (p + 1) * KS; ++ks)
+              umma_bf16_lohi<true>(tdx + p * FF, ya + (((ks >> 2) * YBLK + (ks & 3) * 32) >> 4), ya_hi, wm + ((ks * 16 * C::WROW) >> 4), wm_hi, id_bwx);
+          }
           tc_commit(bar(C::B_DXFULL + ds));
           tc_commit(bar(C::B_YEMPTY + jy));
           if (last_of_group) tc_commit(bar(C::B_WEMPTY + ws));   // every product that reads this group's W tile has been issued
@@ -368,11 +413,15 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           const uint32_t tz = tmem + C::TM_Z + zs * G;
           // Z[b,l] = sum over slot chunks of X[k-chunk, b]^T * W[l, k-chunk], then ones^T * bias
           if (ok && elect_one()) {
-            umma_bf16_lohi<false>(tz, xa, xa_hi, wb, wb_hi, id_fwd);
 #pragma unroll
-            for (int ks = 1; ks < F / 16; ++ks)
-              umma_bf16_lohi<true>(tz, xa + ((ks * 2048) >> 4), xa_hi, wb + (((ks >> 2) * WBLK + (ks & 3) * 32) >> 4), wb_hi, id_fwd);
-            umma_bf16_lohi<true>(tz, xa + (((F / 16) * 2048) >> 4), xa_hi, bb, bb_hi, id_fwd);
+            for (int p = 0; p < P; ++p) {        // group p of the tile: its slots against its labels' weight rows
+              const uint32_t xp = xa + ((p * FF * 128) >> 4), wp = wb + ((p * GG * C::WROW) >> 4);
+              umma_bf16_lohi<false>(tz + p * GG, xp, xa_hi, wp, wb_hi, id_fwd);
+#pragma unroll
+              for (int ks = 1; ks < FF / 16; ++ks)
+                umma_bf16_lohi<true>(tz + p * GG, xp + ((ks * 2048) >> 4), xa_hi, wp + (((ks >> 2) * WBLK + (ks & 3) * 32) >> 4), wb_hi, id_fwd);
+            }
+            umma_bf16_lohi<true>(tz, xa + (((F / 16) * 2048) >> 4), xa_hi, bb, bb_hi, id_bias);
             tc_commit(bar(C::B_ZFULL + zs));
           }
           __syncwarp();
@@ -430,8 +479,10 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int ws = gi & 1;
-      const int rows_real = static_cast<int>(imin64(G, a.L - static_cast<int64_t>(g) * G));
-      const int t_beg = __ldg(a.tgt_ptr + g), t_end = __ldg(a.tgt_ptr + g + 1);
+      const int rows_real = static_cast<int>(imin64(LS, a.L - static_cast<int64_t>(g) * LS));
+      // entries of the tile's groups are contiguous; those from t_mid on belong to the second group of a pair
+      const int t_beg = __ldg(a.tgt_ptr + g * P), t_end = __ldg(a.tgt_ptr + min(g * P + P, a.NGR));
+      const int t_mid = P == 1 ? t_end : __ldg(a.tgt_ptr + g * P + 1);
       const bool has_t = t_end > t_beg;
       for (int t = 0; t < T; ++t) {
         const int zs = it & 1;
@@ -443,7 +494,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           const uint32_t rowkey = static_cast<uint32_t>(b0 + row);
           for (int i = t_beg; i < t_end; ++i) {
             const uint32_t e = __ldg(a.tgt_ent + i);
-            const uint32_t c = (e & 0xFFu) - static_cast<uint32_t>(h * EA_COLS);
+            const uint32_t c = (e & 0xFFu) + (P == 2 && i >= t_mid ? GG : 0) - static_cast<uint32_t>(h * EA_COLS);
             if ((e >> 8) == rowkey && c < static_cast<uint32_t>(EA_COLS)) ym |= 1ull << c;
           }
         } else if (has_t) {
@@ -462,7 +513,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
               const int rb = static_cast<int>(e8[x] >> 8) - b0;
-              const int c = e8[x] & 0xFF;
+              const int c = (e8[x] & 0xFF) + (P == 2 && i0 + x * N_EA * 32 >= t_mid ? GG : 0);
               if (rb >= 0 && rb < BT && c < G) atomicOr(&yb[rb * YBW + (c >> 5)], 1u << (c & 31));
             }
           }
@@ -480,7 +531,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_Z + zs * G + col0;
         const float gs2 = 2.f * gs;
         const float inv_gs2_sq = row_valid ? inv_4gs2_sq : 0.f;
-        const bool ragged = col0 + EA_COLS > rows_real;     // only the last group of the layer can be ragged
+        const bool ragged = col0 + EA_COLS > rows_real;     // only the last tile of the layer can be ragged (and absent columns)
         float tile_loss = 0.f, fast_loss = 0.f;             // fast_loss: hinge (4s)^2-scaled squares, or BCE raw log2 terms
         const float hgs = 0.5f * gs;
         // 16 label columns per iteration.  Nearly every chunk has no positive label in the warp's 32 rows and no
@@ -491,6 +542,13 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         constexpr int CH = 16;                             // label columns per TMEM load
 #pragma unroll 1
         for (int c16 = 0; c16 < EA_COLS; c16 += CH) {
+          if (LS < G && col0 + c16 >= LS) {                // columns no tile of this shape has
+            uint8_t* yblk = yrow + ((col0 + c16) >> 6) * YBLK;
+            const int chunk0 = ((col0 + c16) & 63) >> 3;
+#pragma unroll
+            for (int e = 0; e < CH / 8; ++e) *reinterpret_cast<uint4*>(yblk + (((chunk0 + e) ^ (row & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+            continue;
+          }
           uint32_t r[CH];
           __syncwarp();
           tmem_ld(ta + c16, r);
@@ -517,6 +575,17 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   if (WITH_LOSS) { const float m2 = x[i] + fabsf(x[i]); fl[i & 3] = fmaf(m2, m2, fl[i & 3]); }
                 }
                 pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
+              } else if (LOSS == LOSS_BCE_EXP) {
+                // dLoss/dz = s sigmoid(z) = s / (1 + e^-z); loss term softplus(z) = max(z,0) - ln(max(sigmoid, 1 - sigmoid)),
+                // whose logarithm arguments lie in [0.5, 1] as below
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
+                  const float sg = sigmoid_exp(zr);
+                  x[i] = sg * gs;
+                  if (WITH_LOSS) { fl[i & 1] += zr; fl[2 + (i & 1)] += fabsf(zr); bce_prod *= fmaxf(sg, 1.f - sg); }
+                }
+                pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
               } else {
                 // dLoss/dz = s sigmoid(z) = s/2 + s/2 tanh(z/2) (one MUFU op, one fma); loss term softplus(z) =
                 // max(z,0) - ln(0.5 + 0.5 |tanh(z/2)|).  max(z,0) is summed as (z + |z|) / 2; the logarithm arguments
@@ -533,7 +602,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
               *reinterpret_cast<uint4*>(yblk + (((chunk0 + (e8 >> 3)) ^ (row & 7)) << 4)) = pk;
             }
             if (WITH_LOSS) {
-              if (LOSS == HASTE_LOSS_BCE) { fast_loss += __log2f(bce_prod); tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]); }
+              if (LOSS != HASTE_LOSS_SQHINGE) { fast_loss += __log2f(bce_prod); tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]); }
               else fast_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
             }
           } else {
@@ -552,6 +621,11 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   const float m = fmaxf(fmaf(ns, zr, 1.f), 0.f);
                   gl = (ns * m) * gs2;
                   la = m * m;
+                } else if (LOSS == LOSS_BCE_EXP) {
+                  const float y = static_cast<float>(pos);
+                  const float sg = sigmoid_exp(zr);
+                  gl = (sg - y) * gs;
+                  la = 2.f * (fmaxf(zr, 0.f) - y * zr - 0.69314718f * __log2f(fmaxf(sg, 1.f - sg)));
                 } else {
                   // dLoss/dz = sigmoid(z) - y, loss = max(z,0) - y z - ln(0.5 + 0.5 |tanh(z/2)|); the factor 2 matches
                   // the (z + |z|) sums of the other branch, halved once per tile
@@ -565,7 +639,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 x[i] = gl;
                 if (DEBUG) {
                   if (a.z_dump != nullptr && row_valid && e8 + i < nvalid)
-                    reinterpret_cast<uint16_t*>(a.z_dump)[(static_cast<int64_t>(b0) + row) * a.ldz + static_cast<int64_t>(g) * G + col0 + c16 + e8 + i] =
+                    reinterpret_cast<uint16_t*>(a.z_dump)[(static_cast<int64_t>(b0) + row) * a.ldz + static_cast<int64_t>(g) * LS + col0 + c16 + e8 + i] =
                         static_cast<uint16_t>(__float_as_uint(zr) >> 16);
                 }
               }
@@ -667,12 +741,13 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     for (int gu = 0; gu < n_my_groups; ++gu) {
       const int gg = group_of(gu);
       const int wsu = gu & 1;
-      const int64_t l0 = static_cast<int64_t>(gg) * G;
-      const int rows_real_u = static_cast<int>(imin64(G, a.L - l0));
+      const int64_t l0 = static_cast<int64_t>(gg) * LS;
+      const int rows_real_u = static_cast<int>(imin64(LS, a.L - l0));
       mbar_wait(bar(C::B_WFULL + wsu), (gu >> 1) & 1, abort_flag, a.err, 14, WL);   // W tile and bias column are in place
       mbar_wait(bar(C::B_DWFULL), gu & 1, abort_flag, a.err, 15, WL);
       tc_fence_after();
       const uint32_t tdw = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW;
+      const uint32_t tdg = tdw + (P == 1 ? 0 : (q * C::ROWS_PER_Q) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
       uint32_t gw[UPS / 2];                       // this TMEM lane's gradients, bf16 pairs (garbage in lanes 16-31 when SPLIT)
       float gb = 0.f;
       {
@@ -680,7 +755,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
 #pragma unroll
         for (int pc = 0; pc < NPC; ++pc) {
           uint32_t rr[16];
-          tmem_ld16(tdw + kh * UPS + pc * 16, rr);
+          tmem_ld16(tdg + kh * UPS + pc * 16, rr);
           tmem_ld_wait();
 #pragma unroll
           for (int x = 0; x < 8; ++x) gw[pc * 8 + x] = pack_bf16x2(__uint_as_float(rr[2 * x]), __uint_as_float(rr[2 * x + 1]));
@@ -704,7 +779,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                                  ? *reinterpret_cast<const uint16_t*>(sm + C::OFF_BT + wsu * C::BTILE + (row >> 3) * 256 + (row & 7) * 16)
                                  : uint16_t(0);
       if (do_row) {
-        __nv_bfloat16* wrow = u.w + l * F;
+        __nv_bfloat16* wrow = u.w + l * FF;
 #pragma unroll 1
         for (int pc = 0; pc < NPC; ++pc) {          // pieces of 16 slots
           uint32_t p8[8];
@@ -730,19 +805,18 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           const int s0 = kh * UPS + pc * 16 + half * 8;        // first slot of this lane's part of the piece
           {
             // the old weights: one (SPLIT) or two 16-byte chunks of the row in the W tile
-            const uint8_t* wsm = sm + C::OFF_W + wsu * WSTAGE + (s0 >> 6) * WBLK + row * 128;
-            const int c0 = (s0 & 63) >> 3;
-            const uint4 wa = *reinterpret_cast<const uint4*>(wsm + ((c0 ^ (row & 7)) << 4));
+            const uint8_t* wsm = sm + C::OFF_W + wsu * WSTAGE;
+            const uint4 wa = *reinterpret_cast<const uint4*>(wsm + C::w_chunk(row, s0 >> 3));
             w8[0] = wa.x; w8[1] = wa.y; w8[2] = wa.z; w8[3] = wa.w;
             if (!SPLIT) {
-              const uint4 wb = *reinterpret_cast<const uint4*>(wsm + (((c0 + 1) ^ (row & 7)) << 4));
+              const uint4 wb = *reinterpret_cast<const uint4*>(wsm + C::w_chunk(row, (s0 >> 3) + 1));
               w8[NSL / 2 - 4] = wb.x; w8[NSL / 2 - 3] = wb.y; w8[NSL / 2 - 2] = wb.z; w8[NSL / 2 - 1] = wb.w;
             }
           }
           if (DEBUG) {
             if (a.dw_dump != nullptr) {
 #pragma unroll
-              for (int x = 0; x < NSL / 2; ++x) reinterpret_cast<uint32_t*>(a.dw_dump + l * F + s0)[x] = g8[x];
+              for (int x = 0; x < NSL / 2; ++x) reinterpret_cast<uint32_t*>(a.dw_dump + l * FF + s0)[x] = g8[x];
             }
           }
           uint32_t rnd[NSL / 2];           // NSL x 16 random bits, two per word
@@ -759,7 +833,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             } else {
 #pragma unroll
               for (int x = 0; x < NSL; x += 2)
-                rnd[x >> 1] = rand16_reference_call(u.seed, gl * F + s0 + x) | (rand16_reference_call(u.seed, gl * F + s0 + x + 1) << 16);
+                rnd[x >> 1] = rand16_reference_call(u.seed, gl * FF + s0 + x) | (rand16_reference_call(u.seed, gl * FF + s0 + x + 1) << 16);
             }
           }
           uint32_t ob[NSL / 2];
@@ -777,7 +851,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             }
           } else {
             float mv[NSL];
-            float* mrow = MOM ? u.mom_w + l * F + s0 : nullptr;
+            float* mrow = MOM ? u.mom_w + l * FF + s0 : nullptr;
             if (MOM) {
 #pragma unroll
               for (int x = 0; x < NSL / 4; ++x) {
@@ -824,24 +898,28 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
 }
 
 // Launch one shape.  `dump` selects the debug instantiation (always accumulates the loss).
-template <int G_, int F_>
+// The batch sizes and shapes that the warp-mma kernel used to serve computed the sigmoid to fp32 accuracy; they keep
+// that here (LOSS_BCE_EXP): the newer shapes always, (128, 64) and (64, 128) when B is not a multiple of 8.
+template <int GG_, int FF_, int P_>
 int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
-                      const UpdateArgs& u, int64_t B, int64_t D, int64_t L, int loss_kind, float grad_scale, int max_ctas, cudaStream_t st,
+                      const UpdateArgs& u, int64_t B, int64_t D, int64_t L, int loss_kind, float grad_scale, int64_t ldxt, int max_ctas, cudaStream_t st,
                       const StepDump* dump) {
-  using C = Cfg<G_, F_>;
+  using C = Cfg<GG_, FF_, P_>;
+  constexpr bool FIRST = P_ == 1 && GG_ * FF_ == 128 * 64;     // (128, 64) and (64, 128)
   if (int rc = report_pending_status("fused train step")) return rc;
   StepArgs a;
   a.loc = loc; a.xt = static_cast<const __nv_bfloat16*>(xt); a.tgt_ptr = tgt_ptr; a.tgt_ent = tgt_ent; a.dxt = dxt; a.loss = loss;
   if (int rc = device_status_word(&a.err)) return rc;
-  a.B = B; a.L = L; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + G_ - 1) / G_); a.grad_scale = grad_scale;
+  a.B = B; a.L = L; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::LS - 1) / C::LS);
+  a.NGR = static_cast<int>((L + GG_ - 1) / GG_); a.grad_scale = grad_scale;
   a.wait_limit = wait_limit_cycles();
   a.stall_tile = dump ? take_stall_tile() : -1;
   a.z_dump = dump ? static_cast<__nv_bfloat16*>(dump->z) : nullptr; a.ldz = dump ? dump->ldz : 0;
   a.dw_dump = dump ? static_cast<__nv_bfloat16*>(dump->dw) : nullptr; a.db_dump = dump ? static_cast<__nv_bfloat16*>(dump->dbias) : nullptr;
   CUtensorMap tm_x, tm_w;
-  // xt [D][B]: one box = 64 batch columns of one row (gather4 stacks four rows); W [L][F]: one box = 64 slots x G labels
-  if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(B), static_cast<uint64_t>(D), static_cast<uint64_t>(B) * 2, 64, 1)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tm_w, u.w, static_cast<uint64_t>(F_), static_cast<uint64_t>(L), static_cast<uint64_t>(F_) * 2, 64, G_)) return rc;
+  // xt [D][ldxt]: one box = 64 batch columns of one row (gather4 stacks four rows); W [L][FF]: one box = 64 slots (32 at fan-in 32) x G labels
+  if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tm_w, u.w, static_cast<uint64_t>(FF_), static_cast<uint64_t>(L), static_cast<uint64_t>(FF_) * 2, FF_ == 32 ? 32 : 64, C::G)) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -851,7 +929,7 @@ int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
   const bool mom = u.mom_w != nullptr;
 #define HASTE_S100_LAUNCH(LK, WLOSS, MOMF, DBG)                                                                     \
   {                                                                                                                \
-    auto k = ffi_train_step_sm100_kernel<G_, F_, LK, WLOSS, MOMF, DBG>;                                             \
+    auto k = ffi_train_step_sm100_kernel<GG_, FF_, P_, LK, WLOSS, MOMF, DBG>;                                           \
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);            \
     if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));         \
     cudaLaunchConfig_t cfg = {};                                                                                   \
@@ -866,6 +944,19 @@ int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
   }
 #define HASTE_S100_BY_LOSS(WLOSS, MOMF, DBG)                                                                       \
   { if (loss_kind == HASTE_LOSS_BCE) HASTE_S100_LAUNCH(HASTE_LOSS_BCE, WLOSS, MOMF, DBG) else HASTE_S100_LAUNCH(HASTE_LOSS_SQHINGE, WLOSS, MOMF, DBG) }
+  if (!FIRST || (B % 8) != 0) {
+    if (dump != nullptr) return fail(HASTE_ERR_UNSUPPORTED, "debug outputs exist only for (G,F) = (128,64) or (64,128), B%%8==0");
+#define HASTE_S100_EXP(WLOSS, MOMF)                                                                                 \
+  { if (loss_kind == HASTE_LOSS_BCE) HASTE_S100_LAUNCH(LOSS_BCE_EXP, WLOSS, MOMF, false) else HASTE_S100_LAUNCH(HASTE_LOSS_SQHINGE, WLOSS, MOMF, false) }
+    if (wl) {
+      if (mom) HASTE_S100_EXP(true, true) else HASTE_S100_EXP(true, false)
+    } else {
+      if (mom) HASTE_S100_EXP(false, true) else HASTE_S100_EXP(false, false)
+    }
+#undef HASTE_S100_EXP
+    return check_launch("ffi_train_step_sm100_kernel");
+  }
+  if constexpr (FIRST) {
   if (dump != nullptr) {
     if (loss == nullptr) return fail(HASTE_ERR_BAD_ARG, "debug step needs a loss pointer");
     if (mom) return fail(HASTE_ERR_UNSUPPORTED, "debug step: momentum is not supported");
@@ -874,6 +965,7 @@ int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
     if (mom) HASTE_S100_BY_LOSS(true, true, false) else HASTE_S100_BY_LOSS(true, false, false)
   } else {
     if (mom) HASTE_S100_BY_LOSS(false, true, false) else HASTE_S100_BY_LOSS(false, false, false)
+  }
   }
 #undef HASTE_S100_BY_LOSS
 #undef HASTE_S100_LAUNCH

@@ -18,19 +18,21 @@ struct UpdateArgs {
   int64_t label0;   // global index of the shard's first label (random-bit counters are global)
 };
 
+// ldxt (here and below): row stride of xt in elements, >= B.  With a stride that is a multiple of 8, columns B .. ldxt-1 hold
+// zeros and the rows are 16-byte aligned whatever B is.
 // zw: writable width of a row of z, L <= zw <= ldz (columns L..zw-1 receive zeros)
 int launch_forward(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
-                   int64_t L, int64_t G, int64_t ldz, int64_t zw, cudaStream_t st);
-bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz);
+                   int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st);
+bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t ldxt);
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
-                         int64_t L, int64_t G, int64_t ldz, int64_t zw, cudaStream_t st);
+                         int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st);
 int launch_bwd_features(const void* w, const int32_t* loc, const void* dy, float* dxt, int64_t B, int64_t D, int64_t F, int64_t L,
                         int64_t G, int64_t ldy, cudaStream_t st);
 int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias, const UpdateArgs* upd, int64_t B,
-                       int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, cudaStream_t st);
+                       int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, int64_t ldxt, cudaStream_t st);
 int launch_train_step_mma(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                           const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind, float grad_scale,
-                          cudaStream_t st);
+                          int64_t ldxt, cudaStream_t st);
 // Optional debug outputs of the tcgen05 fused step (tests only).
 struct StepDump {
   void* z;       // bf16 [B, ldz] logits as rounded by the epilogue
@@ -43,28 +45,31 @@ struct StepDump {
 // kernels of other streams).
 int launch_train_step_sm100_g128f64(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt,
                                     float* loss, const UpdateArgs& u, int64_t B, int64_t D, int64_t L, int loss_kind, float grad_scale,
-                                    int max_ctas, cudaStream_t st, const StepDump* dump);
+                                    int64_t ldxt, int max_ctas, cudaStream_t st, const StepDump* dump);
 int launch_train_step_sm100_g64f128(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt,
                                     float* loss, const UpdateArgs& u, int64_t B, int64_t D, int64_t L, int loss_kind, float grad_scale,
-                                    int max_ctas, cudaStream_t st, const StepDump* dump);
+                                    int64_t ldxt, int max_ctas, cudaStream_t st, const StepDump* dump);
+int launch_train_step_sm100_small(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt,
+                                  float* loss, const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind,
+                                  float grad_scale, int64_t ldxt, int max_ctas, cudaStream_t st);
 int launch_train_step(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                       const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind, float grad_scale,
-                      cudaStream_t st, const StepDump* dump = nullptr);
+                      int64_t ldxt, cudaStream_t st, const StepDump* dump = nullptr);
 int launch_sr_round(const float* x, void* out, int64_t n, uint64_t seed, cudaStream_t st);
 int launch_sgd_sr(void* w, const void* g, float* m, int64_t rows, int64_t cols, int64_t row0, float lr, float wd, float mu, uint64_t seed,
                   uint32_t step, uint32_t flags, cudaStream_t st);
 int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t seed, cudaStream_t st);
-int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, cudaStream_t st);
+int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st);
 int launch_targets_bucket(const int32_t* coo, int64_t nnz, int64_t label0, int64_t L, int64_t G, int32_t* ptr, uint32_t* ent,
                           int32_t* scratch, cudaStream_t st);
 int launch_targets_bucket_noalloc(const int32_t* coo, int64_t nnz, int64_t label0, int64_t L, int64_t G, int32_t* ptr, uint32_t* ent,
                                   cudaStream_t st);
 int launch_step_prepare(const void* x, void* xt, float* dxt, float* loss, const int32_t* coo, int64_t nnz, int64_t label0, int64_t L,
-                        int64_t G, int32_t* ptr, uint32_t* ent, int64_t B, int64_t D, cudaStream_t st);
+                        int64_t G, int32_t* ptr, uint32_t* ent, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st);
 bool backward_sm100_supported(const void* xt, const void* w, const void* dy, const void* dw, int64_t B, int64_t D, int64_t F, int64_t L,
-                              int64_t G);
+                              int64_t G, int64_t ldxt);
 int launch_backward_sm100(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias,
-                          const UpdateArgs* upd, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, cudaStream_t st);
+                          const UpdateArgs* upd, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, int64_t ldxt, cudaStream_t st);
 int launch_pad_rows(const void* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows, int64_t cols, cudaStream_t st);
 int launch_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t col0, int k, float* vals, int32_t* idx, cudaStream_t st);
 int launch_check_loc(const int32_t* loc, int64_t n, int64_t D, cudaStream_t st);

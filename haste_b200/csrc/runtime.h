@@ -20,7 +20,8 @@ void dependent_launch_scope(int on);
 // Test hook: tile index at which the next debug step withholds one barrier arrival (-1 = none); reading clears it.
 int take_stall_tile();
 
-// 2-D bf16 tensor map [outer][inner] with the 128-byte swizzle, zero fill outside the tensor.
+// 2-D bf16 tensor map [outer][inner], zero fill outside the tensor; the swizzle is that of the box's row: 128 bytes for a
+// box of 64 columns, 64 bytes for 32.
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes, uint32_t box_inner,
                       uint32_t box_outer);
 

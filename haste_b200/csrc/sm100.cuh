@@ -255,6 +255,17 @@ __device__ __forceinline__ uint64_t make_sdesc(uint32_t saddr, uint32_t lbo_byte
   d |= 2ull << 61;
   return d;
 }
+// Same, 64-byte swizzle (layout type 4): rows of 64 bytes (32 bf16), 16-byte chunk index XORed with ((row >> 1) & 3), 8-row
+// groups 512 B apart; for an MN-major operand LBO is the distance between 32-element blocks along M/N.
+__device__ __forceinline__ uint64_t make_sdesc64(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
+  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
+  d |= 1ull << 46;
+  d |= 4ull << 61;
+  return d;
+}
 // Same, without swizzle (layout type 0), for a K-major operand: 8 rows x 16 bytes form one contiguous 128-byte core
 // matrix; the second 16-byte chunk along K (a K = 16 step of bf16 has two) lies lbo_bytes further, the next 8 rows
 // sbo_bytes further.

@@ -45,17 +45,31 @@ def transpose_bf16(x):
     return xt
 
 
-def forward(loc, xt, w, bias, G):
-    """z [B, L] (a view of a [B, ceil8(L)] buffer, like the reference's narrow())."""
+def transpose_padded(x):
+    """x^T as [D, ceil8(B)], zeros right of column B: 16-byte rows for the tensor maps whatever B is.  Functions below
+    that take ``B`` accept it as ``xt``."""
+    _req(x, "x", torch.bfloat16)
+    B, D = x.shape
+    ldx = (B + 7) // 8 * 8
+    xt = torch.empty(D, ldx, dtype=torch.bfloat16, device=x.device)
+    with torch.cuda.device(x.device):
+        check(lib.haste_transpose_bf16_ldx(_ptr(x), _ptr(xt), B, D, ldx, _stream(x)), "transpose_bf16")
+    return xt
+
+
+def forward(loc, xt, w, bias, G, B=None):
+    """z [B, L] (a view of a [B, ceil8(L)] buffer, like the reference's narrow()).  ``B``: batch size when ``xt`` has
+    padded rows (``transpose_padded``)."""
     _req(loc, "locations", torch.int32); _req(xt, "features", torch.bfloat16); _req(w, "weights", torch.bfloat16)
     if bias is not None:
         _req(bias, "bias", torch.bfloat16)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = ldx if B is None else B
     L, F = w.shape
     ldz = (L + 7) // 8 * 8
     z = torch.empty(B, ldz, dtype=torch.bfloat16, device=xt.device)
     with torch.cuda.device(xt.device):
-        check(lib.haste_ffi_forward(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(z), B, D, F, L, G, ldz, _stream(xt)),
+        check(lib.haste_ffi_forward_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(z), B, D, F, L, G, ldz, ldz, ldx, _stream(xt)),
               "ffi_forward")
     return z.narrow(1, 0, L)
 
@@ -86,10 +100,11 @@ def _rows(dy, L):
     return dy, dy.stride(0)
 
 
-def backward_features(xt, w, loc, dy, G):
-    """dxt fp32 [D,B]."""
+def backward_features(xt, w, loc, dy, G, B=None):
+    """dxt fp32 [D,B].  ``B`` as in ``forward``."""
     _req(loc, "locations", torch.int32); _req(w, "weights", torch.bfloat16)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = ldx if B is None else B
     L, F = w.shape
     dy, ldy = _rows(dy, L)
     dxt = torch.empty(D, B, dtype=torch.float32, device=w.device)
@@ -99,24 +114,27 @@ def backward_features(xt, w, loc, dy, G):
     return dxt
 
 
-def backward_weights(xt, w, loc, dy, G, want_dbias=False):
-    """dw bf16 [L,F] (and dbias bf16 [L] when asked)."""
+def backward_weights(xt, w, loc, dy, G, want_dbias=False, B=None):
+    """dw bf16 [L,F] (and dbias bf16 [L] when asked).  ``B`` as in ``forward``."""
     _req(loc, "locations", torch.int32); _req(xt, "features", torch.bfloat16)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = ldx if B is None else B
     L, F = w.shape
     dy, ldy = _rows(dy, L)
     dw = torch.empty(L, F, dtype=torch.bfloat16, device=xt.device)
     db = torch.empty(L, dtype=torch.bfloat16, device=xt.device) if want_dbias else None
     with torch.cuda.device(xt.device):
-        check(lib.haste_ffi_backward_weights(_ptr(xt), _ptr(loc), _ptr(dy), _ptr(dw), _ptr(db), B, D, F, L, G, ldy, _stream(xt)),
+        check(lib.haste_ffi_backward_weights_ldx(_ptr(xt), _ptr(loc), _ptr(dy), _ptr(dw), _ptr(db), B, D, F, L, G, ldy, ldx, _stream(xt)),
               "ffi_backward_weights")
     return (dw, db) if want_dbias else dw
 
 
-def backward_both(xt, w, loc, dy, G, want_dbias=True):
-    """(dxt fp32 [D,B], dw bf16 [L,F], dbias bf16 [L] or None) from one pass over dy where the shape allows."""
+def backward_both(xt, w, loc, dy, G, want_dbias=True, B=None):
+    """(dxt fp32 [D,B], dw bf16 [L,F], dbias bf16 [L] or None) from one pass over dy where the shape allows.  ``B`` as
+    in ``forward``."""
     _req(loc, "locations", torch.int32); _req(xt, "features", torch.bfloat16); _req(w, "weights", torch.bfloat16)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = ldx if B is None else B
     L, F = w.shape
     dy, ldy = _rows(dy, L)
     dev = xt.device
@@ -124,8 +142,8 @@ def backward_both(xt, w, loc, dy, G, want_dbias=True):
         dxt = torch.empty(D, B, dtype=torch.float32, device=dev)
         dw = torch.empty(L, F, dtype=torch.bfloat16, device=dev)
         db = torch.empty(L, dtype=torch.bfloat16, device=dev) if want_dbias else None
-        check(lib.haste_ffi_backward(_ptr(xt), _ptr(w), _ptr(loc), _ptr(dy), _ptr(dxt), _ptr(dw), _ptr(db), B, D, F, L, G, ldy,
-                                     _lib.F_ZERO_DXT, _stream(xt)), "ffi_backward")
+        check(lib.haste_ffi_backward_ldx(_ptr(xt), _ptr(w), _ptr(loc), _ptr(dy), _ptr(dxt), _ptr(dw), _ptr(db), B, D, F, L, G, ldy,
+                                         _lib.F_ZERO_DXT, ldx, _stream(xt)), "ffi_backward")
     return dxt, dw, db
 
 
@@ -181,27 +199,28 @@ def train_step_on(stream_handle, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_en
 
 
 def train_step(loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, G, label0, loss_kind, grad_scale, lr, wd, mu,
-               seed, step, flags):
+               seed, step, flags, B=None):
     _req(loc, "locations", torch.int32); _req(xt, "features", torch.bfloat16); _req(w, "weights", torch.bfloat16)
     _req(dxt, "dxt", torch.float32)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = ldx if B is None else B
     L, F = w.shape
     with torch.cuda.device(xt.device):
-        check(lib.haste_ffi_train_step(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b), _ptr(tgt_ptr),
-                                       _ptr(tgt_ent), _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd,
-                                       mu, seed, step, flags, _stream(xt)), "ffi_train_step")
+        check(lib.haste_ffi_train_step_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b), _ptr(tgt_ptr),
+                                           _ptr(tgt_ent), _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd,
+                                           mu, seed, step, flags, ldx, _stream(xt)), "ffi_train_step")
 
 
 def step(x, coo, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, G, label0, loss_kind, grad_scale, lr, wd, mu, seed, step_no,
          flags):
     """Preparation + fused step in one library call (the per-step path of ``FusedFFIShard.step``: argument checks are
-    the caller's, done once when the buffers are created)."""
+    the caller's, done once when the buffers are created).  ``xt``: work buffer [D, ldx], ldx >= B."""
     B, D = x.shape
     L, F = w.shape
     with torch.cuda.device(x.device):
-        check(lib.haste_ffi_step(_ptr(x), _ptr(coo), coo.shape[0], _ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b),
+        check(lib.haste_ffi_step_ldx(_ptr(x), _ptr(coo), coo.shape[0], _ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b),
                                  _ptr(tgt_ptr), _ptr(tgt_ent), _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd,
-                                 mu, seed, step_no, flags, _stream(x)), "ffi_step")
+                                 mu, seed, step_no, flags, xt.shape[1], _stream(x)), "ffi_step")
 
 
 def train_step_dbg(loc, xt, w, bias, tgt_ptr, tgt_ent, dxt, loss, G, label0, loss_kind, grad_scale, lr, wd, seed, step, flags):
@@ -308,16 +327,18 @@ def rewire_ex(w, loc, mom_w, D, G, group0, score_mode, prune_mode, threshold, n_
 
 
 def topk(loc, xt, w, bias, zbuf, groups_per_chunk, k, G, label0, vals, idx):
-    """Chunked forward + running top-k of the whole layer in one library call (``zbuf``: bf16 [B, >= groups_per_chunk * G])."""
+    """Chunked forward + running top-k of the whole layer in one library call (``zbuf``: bf16 [B, >= groups_per_chunk * G];
+    ``xt`` may have padded rows: the batch size is that of ``vals``)."""
     _req(loc, "locations", torch.int32); _req(xt, "features", torch.bfloat16); _req(w, "weights", torch.bfloat16)
     _req(zbuf, "logit buffer", torch.bfloat16); _req(vals, "values", torch.float32); _req(idx, "labels", torch.int32)
     if bias is not None:
         _req(bias, "bias", torch.bfloat16)
-    D, B = xt.shape
+    D, ldx = xt.shape
+    B = vals.shape[0]
     L, F = w.shape
     with torch.cuda.device(xt.device):
-        check(lib.haste_ffi_topk(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(zbuf), zbuf.stride(0), B, D, F, L, G, groups_per_chunk, k,
-                                 label0, _ptr(vals), _ptr(idx), _stream(xt)), "ffi_topk")
+        check(lib.haste_ffi_topk_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(zbuf), zbuf.stride(0), B, D, F, L, G, groups_per_chunk, k,
+                                 label0, _ptr(vals), _ptr(idx), ldx, _stream(xt)), "ffi_topk")
 
 
 def topk_update(z, C, col0, vals, idx):

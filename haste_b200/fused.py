@@ -126,10 +126,14 @@ class FusedFFIShard:
 
     def step_xt(self, xt, targets, dxt=None, want_loss=True):
         """One step given the transposed features [D,B] (bf16).  Returns (dxt fp32 [D,B], loss fp32 [1] or None)."""
-        D, B = xt.shape
+        return self._step_xt(xt, xt.shape[1], targets, dxt, want_loss)
+
+    def _step_xt(self, xt, B, targets, dxt, want_loss):
+        D = xt.shape[0]
         if dxt is None:
             if self._dxt is None or self._dxt.shape != (D, B):
                 self._dxt = torch.empty(D, B, dtype=torch.float32, device=xt.device)
+                self._xt = None
             dxt = self._dxt
         self.bucket_targets(targets)
         if want_loss:
@@ -138,7 +142,7 @@ class FusedFFIShard:
         flags = _ffi.make_flags(sr=self.sr, contract=self.contract, rng=self.rng, zero_dxt=True, loss=want_loss)
         _ffi.train_step(self.loc, xt, self.w, self.bias, self.mom_w, self.mom_b, self.tgt_ptr, self.tgt_ent, dxt,
                         self.loss_buf if want_loss else None, self.G, self.label0, self.loss_kind, self.grad_scale, self.lr,
-                        self.wd, self.mu, seed, step, flags)
+                        self.wd, self.mu, seed, step, flags, B=B)
         self.steps += 1
         return dxt, (self.loss_buf if want_loss else None)
 
@@ -147,10 +151,11 @@ class FusedFFIShard:
         bucketing) and one fused-step launch."""
         B, D = x.shape
         if self.NG * 4 > 200 * 1024:                       # too many groups for the single-block bucketing
-            return self.step_xt(_ffi.transpose_bf16(x), targets, want_loss=want_loss)
-        if self._dxt is None or self._dxt.shape != (D, B):
+            return self._step_xt(_ffi.transpose_padded(x), B, targets, None, want_loss)
+        if self._dxt is None or self._dxt.shape != (D, B) or self._xt is None:
             self._dxt = torch.empty(D, B, dtype=torch.float32, device=x.device)
-            self._xt = torch.empty(D, B, dtype=torch.bfloat16, device=x.device)
+            # rows padded to 16 bytes: the tcgen05 kernel's tensor map then serves every batch size
+            self._xt = torch.empty(D, (B + 7) // 8 * 8, dtype=torch.bfloat16, device=x.device)
         if targets.shape[0] > self.tgt_ent.numel():
             self.tgt_ent = torch.zeros(int(targets.shape[0] * 1.5) + 1, dtype=torch.int32, device=targets.device)
         if not (x.is_cuda and targets.is_cuda) or x.dtype != torch.bfloat16 or targets.dtype != torch.int32 or not x.is_contiguous() \

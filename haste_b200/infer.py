@@ -30,7 +30,7 @@ def ffi_topk(group_locations, weights, bias, features, k, group_size, *, groups_
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         per_group = B * G * 2
         groups_per_chunk = max(sms, (64 << 20) // per_group // sms * sms)
-    xt = _ffi.transpose_bf16(features)
+    xt = _ffi.transpose_padded(features)
     vals = torch.full((B, k), float("-inf"), dtype=torch.float32, device=dev)
     idx = torch.full((B, k), -1, dtype=torch.int32, device=dev)
     # one library call walks the chunks (forward kernel, then the running top-k kernel, per chunk) on the current stream

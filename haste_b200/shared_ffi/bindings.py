@@ -15,11 +15,11 @@ class GroupFFIMulFunction(torch.autograd.Function):
         # (the reference's fp32 kernels silently compute in fp16, which is not imitated).
         ctx.in_dtype = features.dtype
         feats = features if features.dtype == torch.bfloat16 else features.to(torch.bfloat16)
-        features_t = _ffi.transpose_bf16(feats.contiguous())
+        features_t = _ffi.transpose_padded(feats.contiguous())
         ctx.save_for_backward(features_t, weights, group_locations)
-        ctx.gsize = int(gsize)
+        ctx.gsize, ctx.batch = int(gsize), feats.shape[0]
         ctx.use_bias = bias is not None
-        return _ffi.forward(group_locations, features_t, weights, bias, int(gsize))
+        return _ffi.forward(group_locations, features_t, weights, bias, int(gsize), B=ctx.batch)
 
     @staticmethod
     @torch.amp.custom_bwd(device_type="cuda")
@@ -34,20 +34,20 @@ class GroupFFIMulFunction(torch.autograd.Function):
         if need_x and need_w:
             # both gradients from one pass over grad_output
             dxt, weight_gradient, bias_gradient = _ffi.backward_both(features_t, weights, group_locations, grad_output, gsize,
-                                                                     want_dbias=bool(need_b))
+                                                                     want_dbias=bool(need_b), B=ctx.batch)
             input_gradient = _ffi.dxt_to_dx_sr(dxt, 123)
             if ctx.in_dtype != torch.bfloat16:
                 input_gradient = input_gradient.to(ctx.in_dtype)
             return input_gradient, weight_gradient, None, bias_gradient, None
         if need_x:
-            dxt = _ffi.backward_features(features_t, weights, group_locations, grad_output, gsize)
+            dxt = _ffi.backward_features(features_t, weights, group_locations, grad_output, gsize, B=ctx.batch)
             # bindings.py:44-50 of the reference: transpose, then stochastic rounding with the fixed seed 123
             input_gradient = _ffi.dxt_to_dx_sr(dxt, 123)
             if ctx.in_dtype != torch.bfloat16:
                 input_gradient = input_gradient.to(ctx.in_dtype)
         if need_w or need_b:
             weight_gradient, bias_gradient = _ffi.backward_weights(features_t, weights, group_locations, grad_output, gsize,
-                                                                   want_dbias=True)
+                                                                   want_dbias=True, B=ctx.batch)
             if not need_b:
                 bias_gradient = None
         return input_gradient, weight_gradient, None, bias_gradient, None

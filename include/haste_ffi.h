@@ -88,8 +88,8 @@ int haste_ffi_backward_weights(const void* xt, const int32_t* loc, const void* d
                                haste_stream_t stream);
 
 /* Both gradients of the autograd backward from one pass over dy: dxt as haste_ffi_backward_features, dw / dbias
- * as haste_ffi_backward_weights (dbias may be NULL).  For (G=128, F=64) and (G=64, F=128) with B % 8 == 0 one
- * tcgen05 kernel reads dy once; its rows need no alignment beyond that of a bf16 (a contiguous [B, L] gradient
+ * as haste_ffi_backward_weights (dbias may be NULL).  For (G=128, F=64) and (G=64, F=128) one
+ * tcgen05 kernel reads dy once (xt rows at a stride that is a multiple of 8); its rows need no alignment beyond that of a bf16 (a contiguous [B, L] gradient
  * with odd L is read in place) and whatever lies in columns L..ldy-1 is ignored.  Otherwise the two warp-mma
  * kernels run back to back.  flags: HASTE_F_ZERO_DXT.
  * Replaces the pair of calls at shared_ffi/bindings.py:44 and :52. */
@@ -306,6 +306,35 @@ int haste_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t 
 int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void* bias, void* zbuf, int64_t ldz, int64_t B,
                    int64_t D, int64_t F, int64_t L, int64_t G, int64_t groups_per_chunk, int32_t k, int64_t label0,
                    float* vals, int32_t* idx, haste_stream_t stream);
+
+/* The entry points above that take the transposed features, with a row stride: xt is [D, ldxt], ldxt >= B.  The tensor
+ * maps of the tcgen05 kernels need 16-byte aligned rows, so a batch whose size is not a multiple of 8 reaches them with
+ * ldxt = B rounded up to 8.  haste_transpose_bf16_ldx and haste_ffi_step_ldx write zeros into columns B..ldxt-1; the
+ * other calls need them to be zero.  dxt stays [D, B].  haste_ffi_forward_ldx takes zcols as haste_ffi_forward_into
+ * does.  (No counterpart in the reference: its kernels take [D, B].) */
+int haste_transpose_bf16_ldx(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream);
+int haste_ffi_forward_ldx(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z,
+                          int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t zcols,
+                          int64_t ldxt, haste_stream_t stream);
+int haste_ffi_backward_weights_ldx(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias,
+                                   int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy,
+                                   int64_t ldxt, haste_stream_t stream);
+int haste_ffi_backward_ldx(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias,
+                           int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, uint32_t flags,
+                           int64_t ldxt, haste_stream_t stream);
+int haste_ffi_train_step_ldx(const int32_t* loc, const void* xt, void* w, void* bias, float* mom_w, float* mom_b,
+                             const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
+                             int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t label0, int32_t loss_kind,
+                             float grad_scale, float lr, float wd, float mu, uint64_t seed, uint32_t step, uint32_t flags,
+                             int64_t ldxt, haste_stream_t stream);
+int haste_ffi_step_ldx(const void* x, const int32_t* coo, int64_t nnz, const int32_t* loc, void* xt, void* w, void* bias,
+                       float* mom_w, float* mom_b, int32_t* tgt_ptr, uint32_t* tgt_ent, float* dxt, float* loss,
+                       int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t label0, int32_t loss_kind,
+                       float grad_scale, float lr, float wd, float mu, uint64_t seed, uint32_t step, uint32_t flags,
+                       int64_t ldxt, haste_stream_t stream);
+int haste_ffi_topk_ldx(const int32_t* loc, const void* xt, const void* w, const void* bias, void* zbuf, int64_t ldz, int64_t B,
+                       int64_t D, int64_t F, int64_t L, int64_t G, int64_t groups_per_chunk, int32_t k, int64_t label0,
+                       float* vals, int32_t* idx, int64_t ldxt, haste_stream_t stream);
 
 /* Rate probes (measurement only; timed by the benchmark's auxiliary mode; no counterpart in the reference).  Each
  * isolates one access pattern of the fused train step at the step's own sizes:

@@ -1,0 +1,84 @@
+"""GPU parity tests of the tcgen05 kernels at the layer shapes whose tiles hold 64 labels or two label groups, at batch
+sizes that are not multiples of 8 (padded rows of xt).  Tolerances: bf16 inputs, fp32
+accumulation, bf16 logits and loss gradients — rel 1e-2 / abs 1e-3 of the magnitude, as for the other shapes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from oracle import ffi_oracle as fo
+
+# (G, F, L): one tile, an odd number of groups (the last tile of a pair holds one), ragged last groups, more tiles than SMs
+LAYERS = [(32, 32, 40), (32, 32, 32 * 401 + 7), (32, 64, 32 * 7), (32, 64, 32 * 310 + 1), (64, 64, 64 * 160 + 33), (64, 64, 8),
+          (128, 64, 128 * 5 + 3), (64, 128, 64 * 9 + 1)]
+
+
+def _close(got, want, what, rel=1e-2):
+    got, want = got.float().cpu(), want.float().cpu()
+    bad = (got - want).abs() > 1e-3 * max(1.0, float(want.abs().max())) + rel * want.abs()
+    assert not bad.any(), f"{what}: {int(bad.sum())}/{bad.numel()} outside tolerance, max err {float((got - want).abs().max())}"
+
+
+@pytest.mark.parametrize("B", [1, 64, 135, 333])
+@pytest.mark.parametrize("layer", LAYERS, ids=[f"G{g}F{f}L{l}" for g, f, l in LAYERS])
+def test_forward_and_both_gradients(layer, B):
+    from haste_b200 import ffi
+    G, F, L = layer
+    D = 200
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=B + L, x_kind="normal", bias_zero=False)
+    dev = {k: v.cuda() for k, v in inp.items()}
+    xt = ffi.transpose_padded(dev["X"])
+    assert torch.equal(xt[:, :B].cpu(), inp["X"].t()) and not xt[:, B:].any()
+    z = ffi.forward(dev["loc"], xt, dev["W"], dev["bias"], G, B=B)
+    _close(z, fo.forward(inp["loc"], inp["X"], inp["W"], inp["bias"], G, round_bf16=False), "logits")
+    dY = (torch.randn(B, L, generator=torch.Generator().manual_seed(3)) * 0.5).to(torch.bfloat16)
+    want_x, want_w = fo.backward_features(inp["loc"], inp["W"], dY, G, D), fo.backward_weights(inp["loc"], inp["X"], dY, G, L, round_bf16=False)
+    dxt, dw, db = ffi.backward_both(xt, dev["W"], dev["loc"], dY.cuda(), G, B=B)
+    for got_x, got_w, got_b in ((dxt, dw, db), (ffi.backward_features(xt, dev["W"], dev["loc"], dY.cuda(), G, B=B),
+                                                *ffi.backward_weights(xt, dev["W"], dev["loc"], dY.cuda(), G, want_dbias=True, B=B))):
+        _close(got_x, want_x, "dXt")
+        _close(got_w, want_w, "dW")
+        _close(got_b, dY.float().sum(0), "dbias")
+
+
+@pytest.mark.parametrize("B", [8, 100, 333])
+@pytest.mark.parametrize("loss", ["bce", "squared_hinge"])
+@pytest.mark.parametrize("layer", LAYERS, ids=[f"G{g}F{f}L{l}" for g, f, l in LAYERS])
+def test_step(layer, loss, B):
+    """avg_pos 40 on few labels fills the tiles' target bitmaps, on many labels most groups take the entry list."""
+    from haste_b200.fused import FusedFFIShard
+    G, F, L = layer
+    D, scale, lr, wd = 264, 0.5, 0.05, 1e-4
+    inp = fo.make_inputs(B, D, L, F, G, min(40, max(1, L // 10)), 1.1, seed=B + L, x_kind="normal", bias_zero=False)
+    kind = fo.LOSS_SQHINGE if loss == "squared_hinge" else fo.LOSS_BCE
+    for mu, rng in ((0.0, "packed"), (0.0, "reference"), (0.9, "packed")):
+        sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss=loss, lr=lr, weight_decay=wd,
+                           momentum=mu, seed=42, rng=rng, grad_scale=scale)
+        dxt, loss_dev = sh.step(inp["X"].cuda(), inp["targets"].cuda())
+        ref = fo.train_step(inp["loc"], inp["X"], inp["W"], inp["bias"], inp["targets"], G, kind, lr, wd, 42, grad_scale=scale, rng_mode=rng)
+        assert abs(float(loss_dev) - ref["loss"]) <= 2e-3 * abs(ref["loss"]) + 1e-3
+        _close(dxt, ref["dXt"], "dXt")
+        if mu == 0.0:
+            same = (fo._bf16_to_bits(sh.w.cpu()) == fo._bf16_to_bits(ref["W_new"])).mean()
+            assert same >= 0.95, f"{same:.3f} of the weights match bit for bit"
+            _close(sh.bias, ref["bias_new"], "bias")
+        else:
+            _close(sh.mom_w, ref["dW"].float() + wd * inp["W"].float(), "momentum")
+            _close(sh.mom_b, ref["dbias"].float() + wd * inp["bias"].float(), "bias momentum")
+            _close(sh.w, inp["W"].float() - lr * sh.mom_w.cpu(), "weights")
+
+
+@pytest.mark.parametrize("layer", [(32, 32, 32 * 5), (32, 64, 32 * 5), (64, 64, 64 * 3), (128, 64, 128 * 3), (64, 128, 64 * 3)])
+def test_step_bce_gradient_of_very_negative_logits(layer):
+    """Logits around -12: the gradient is sigmoid(z) = 6e-6 and its sum over the batch has to be right to bf16, which an
+    absolute error of the sigmoid would destroy (batch 100: the shapes and sizes that compute it with exp)."""
+    from haste_b200.fused import FusedFFIShard
+    G, F, L = layer
+    B, D = 100, 264
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=5, x_kind="l2norm", bias_zero=True)
+    inp["bias"] -= 12.0
+    sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss="bce", lr=0.0, momentum=0.9, seed=1)
+    sh.step(inp["X"].cuda(), torch.zeros(0, 2, dtype=torch.int32, device="cuda"))
+    z = fo.forward(inp["loc"], inp["X"], inp["W"], inp["bias"], G).double()
+    want = torch.sigmoid(z).sum(0)
+    assert ((sh.mom_b.cpu().double() - want).abs() <= 2 ** -7 * want).all()          # two bf16 roundings of dY and its sum
