@@ -57,6 +57,8 @@ SIGNATURES = {
     "haste_ffi_step_ldx": [P, P, I64, P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I32, F32, F32, F32, F32, U64, U32, U32,
                            I64, P],
     "haste_ffi_topk_ldx": [P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, I32, I64, P, P, I64, P],
+    "haste_ffi_topk_fused_scratch": [I64, I64, I64, I64, I64, I32],
+    "haste_ffi_topk_fused": [P, P, P, P, P, I64, I64, I64, I64, I64, I64, I32, I64, P, P, P],
     "haste_ffi_check_locations": [P, I64, I64, P],
     "haste_ffi_set_max_ctas": [I32],
     "haste_poll_status": [],
@@ -75,6 +77,7 @@ for _name, _args in SIGNATURES.items():
 lib.haste_last_error_string.restype = c_char_p
 lib.haste_last_error_string.argtypes = []
 lib.haste_version.restype = c_int
+lib.haste_ffi_topk_fused_scratch.restype = I64          # bytes, not a status
 lib.haste_version.argtypes = []
 
 # status codes and flags (include/haste_ffi.h)

@@ -439,6 +439,25 @@ int haste_ffi_topk_ldx(const int32_t* loc, const void* xt, const void* w, const 
   return HASTE_OK;
 }
 
+int64_t haste_ffi_topk_fused_scratch(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k) {
+  if (k < 1 || k > 128 || validate_shape("haste_ffi_topk_fused_scratch", B, D, F, L, G) != HASTE_OK) return 0;
+  return topk_fused_scratch_bytes(B, D, F, L, G, k);
+}
+
+int haste_ffi_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t scratch_bytes, int64_t B,
+                         int64_t D, int64_t F, int64_t L, int64_t G, int32_t k, int64_t label0, float* vals, int32_t* idx,
+                         haste_stream_t stream) {
+  const char* who = "haste_ffi_topk_fused";
+  REQUIRE_PTR(loc, who); REQUIRE_PTR(x, who); REQUIRE_PTR(w, who); REQUIRE_PTR(scratch, who); REQUIRE_PTR(vals, who); REQUIRE_PTR(idx, who);
+  REQUIRE_ALIGNED(loc, who); REQUIRE_ALIGNED(w, who); REQUIRE_ALIGNED(scratch, who);
+  if (int rc = validate_shape(who, B, D, F, L, G)) return rc;
+  if (k < 1 || k > 128) return fail(HASTE_ERR_UNSUPPORTED, "%s: k=%d outside [1,128]", who, k);
+  if (label0 < 0 || label0 + L >= (1ll << 31)) return fail(HASTE_ERR_UNSUPPORTED, "%s: label ids must fit in int32", who);
+  const int64_t need = topk_fused_scratch_bytes(B, D, F, L, G, k);
+  if (need > 0 && scratch_bytes < need) return fail(HASTE_ERR_BAD_ARG, "%s: %lld bytes of scratch, %lld needed", who, (long long)scratch_bytes, (long long)need);
+  return launch_topk_fused(loc, x, w, bias, scratch, B, D, F, L, G, k, label0, vals, idx, static_cast<cudaStream_t>(stream));
+}
+
 int haste_ffi_check_locations(const int32_t* loc, int64_t n, int64_t D, haste_stream_t stream) {
   const char* who = "haste_ffi_check_locations";
   REQUIRE_PTR(loc, who);

@@ -76,6 +76,21 @@ __device__ __forceinline__ uint16_t rn_bf16_bits(float v) {
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float(static_cast<uint32_t>(b) << 16); }
 __device__ __forceinline__ float round_to_bf16_f(float v) { return bf16_bits_to_float(rn_bf16_bits(v)); }
 
+// ---------------------------------------------------------------- top-k keys
+// Key of a (logit, label) pair: larger logits first, among equal logits the lower label id.  Keys of one row are
+// distinct; 0 means "nothing" (no real pair has it).  A logit that compares equal to another has the same upper half
+// (-0 counts as +0).
+__device__ __forceinline__ unsigned long long topk_key(float v, uint32_t label) {
+  const uint32_t u = __float_as_uint(v == 0.f ? 0.f : v);
+  const uint32_t o = u ^ ((u >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+  return (static_cast<unsigned long long>(o) << 32) | (0xFFFFFFFFu - label);
+}
+__device__ __forceinline__ float topk_key_value(unsigned long long key) {
+  const uint32_t o = static_cast<uint32_t>(key >> 32);
+  return __uint_as_float(o ^ ((o >> 31) ? 0x80000000u : 0xFFFFFFFFu));
+}
+__device__ __forceinline__ int topk_key_label(unsigned long long key) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(key)); }
+
 // ---------------------------------------------------------------- SGD arithmetic (fp32)
 // sr_triton.py:140-158.  CONTRACT = fused multiply-add (what the compiled Triton kernel emits with
 // fp fusion on); otherwise multiply and add are rounded separately.

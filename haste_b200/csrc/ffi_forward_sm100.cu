@@ -14,6 +14,13 @@
 // columns, and the up to 7 columns left over are written with ordinary 2-byte stores).  Warp roles (416 threads): warps 0, 2, 3, 12 produce, warp 1 issues the MMAs,
 // warps 4-11 drain the accumulator: TMEM -> bf16 -> staging tile; one thread issues the store.
 // All waits are bounded (see mbar_wait).
+//
+// The TOPK instantiations write no logits: the epilogue warps compare each logit (rounded to bf16, as it would have been
+// stored) with the k-th best value its row had before the launch and keep the few that beat it — expected k times the
+// ratio of labels in this launch to labels before it — as keys for the merge kernel in topk.cu.  A maximum tree over 16
+// packed logits decides per chunk whether anything passed; what did is collected in a list per warp in the shared
+// memory the staging tiles would use, and flushed 32 entries at a time, so that the latency of the atomics on the
+// rows' counters is paid once per flush and not once per candidate.
 #include "common.cuh"
 #include "launchers.h"
 #include "runtime.h"
@@ -71,14 +78,23 @@ struct FwdArgs {
   int64_t B, L, ldz, zw;
   int D, NG, NGR;      // NG: tiles of G labels; NGR: label groups
   long long wait_limit;
+  // TOPK
+  const float* thr;            // [B] current k-th best value of every row (-inf: none yet)
+  unsigned long long* cand;    // [B][cap] keys of the logits that beat it
+  int* cnt;                    // [B] number of them, also beyond cap
+  int cap, label0;
 };
 
+__device__ __forceinline__ uint32_t max2(uint32_t x, uint32_t y) {      // a NaN loses against a number
+  const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int GG_, int FF_, int P_>
+template <int GG_, int FF_, int P_, bool TOPK>
 __global__ void __launch_bounds__(Cfg<GG_, FF_, P_>::NTHREADS, 1)
 ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
                          const __grid_constant__ CUtensorMap tm_z) {
@@ -258,6 +274,76 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
     const int row = q * 32 + lane;
     const bool storer = (ep == 0 && lane == 0);
     int it = 0;
+    if constexpr (TOPK) {
+      constexpr int CAPW = 2 * C::CSTAGE / C::N_EPI / 8;     // entries of this warp's list
+      static_assert(CAPW >= 16 * 32, "one chunk's logits fit an empty list");
+      uint2* list = reinterpret_cast<uint2*>(sm + C::OFF_C) + ep * CAPW;     // .x label, .y bf16 logit << 16 | batch row
+      int count = 0;                                         // warp-uniform
+      auto flush = [&]() {
+        __syncwarp();
+        for (int i = lane; i < count; i += 32) {
+          const uint2 e = list[i];
+          const int b = static_cast<int>(e.y & 0xFFFFu);
+          const int slot = atomicAdd(a.cnt + b, 1);
+          if (slot < a.cap) a.cand[static_cast<int64_t>(b) * a.cap + slot] = topk_key(__uint_as_float(e.y & 0xFFFF0000u), e.x);
+        }
+        count = 0;
+        __syncwarp();
+      };
+      for (int gi = 0; gi < n_my_groups; ++gi) {
+        const int l0 = (blockIdx.x + gi * gridDim.x) * G;
+        const int rows_real = static_cast<int>(imin64(G, a.L - l0));
+        for (int t = 0; t < T; ++t, ++it) {
+          const int zs = it & 1;
+          const int b = t * BT + row;
+          const float thr = b < a.B ? __ldg(a.thr + b) : INFINITY;       // rows beyond the batch never pass
+          const bool ok = mbar_wait(bar(C::B_ZFULL + zs), (it >> 1) & 1, abort_flag, a.err, 27, WL);
+          tc_fence_after();
+          const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + zs * G + h * C::EC;
+#pragma unroll 1
+          for (int c16 = 0; c16 < C::EC; c16 += 16) {
+            uint32_t r[16];
+            __syncwarp();
+            tmem_ld16(ta + c16, r);
+            tmem_ld_wait();
+            uint32_t p[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) p[x] = pack2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
+            const uint32_t m = max2(max2(max2(p[0], p[1]), max2(p[2], p[3])), max2(max2(p[4], p[5]), max2(p[6], p[7])));
+            const float best = fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
+            if (!__any_sync(0xffffffffu, best > thr)) continue;
+            const int col0 = h * C::EC + c16, nvalid = rows_real - col0;     // columns of this chunk that are real labels
+            uint32_t hit = 0u;
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              if (__uint_as_float(p[x] << 16) > thr) hit |= 1u << (2 * x);
+              if (__uint_as_float(p[x] & 0xFFFF0000u) > thr) hit |= 2u << (2 * x);
+            }
+            if (nvalid < 16) hit &= nvalid <= 0 ? 0u : (1u << nvalid) - 1u;
+            if (!ok || *abort_flag) hit = 0u;
+            const int mine = __popc(hit);
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            if (count + total > CAPW) flush();
+            int pos = count + incl - mine;
+#pragma unroll
+            for (int x = 0; x < 16; ++x) {                   // registers are indexed by constants only
+              if (hit & (1u << x)) {
+                const uint32_t bits = (x & 1) ? (p[x >> 1] & 0xFFFF0000u) : (p[x >> 1] << 16);
+                list[pos++] = make_uint2(static_cast<uint32_t>(a.label0 + l0 + col0 + x), bits | static_cast<uint32_t>(b));
+              }
+            }
+            count += total;
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
+        }
+      }
+      flush();
+    } else {
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = blockIdx.x + gi * gridDim.x;
       const int l0 = g * G;
@@ -318,6 +404,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
       }
     }
     if (storer) bulk_wait<0>();
+    }
   }
 
   tc_fence_before();
@@ -327,7 +414,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
 
 template <int GG_, int FF_, int P_>
 static int launch_shape(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t L,
-                        int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
+                        int64_t ldz, int64_t zw, int64_t ldxt, const TopkFilter* tk, cudaStream_t st) {
   using C = Cfg<GG_, FF_, P_>;
   if (int rc = report_pending_status("tcgen05 forward")) return rc;
   int* err_dev = nullptr;
@@ -337,18 +424,21 @@ static int launch_shape(const int32_t* loc, const void* xt, const void* w, const
   a.B = B; a.L = L; a.ldz = ldz; a.zw = zw; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::G - 1) / C::G);
   a.NGR = static_cast<int>((L + C::GG - 1) / C::GG);
   a.wait_limit = wait_limit_cycles();
+  a.thr = nullptr; a.cand = nullptr; a.cnt = nullptr; a.cap = 0; a.label0 = 0;
+  if (tk) { a.thr = tk->thr; a.cand = tk->cand; a.cnt = tk->cnt; a.cap = tk->cap; a.label0 = tk->label0; }
   CUtensorMap tm_x, tm_w, tm_z;
   if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc;
   if (int rc = make_tmap_bf16_2d(&tm_w, w, static_cast<uint64_t>(C::FF), static_cast<uint64_t>(L), static_cast<uint64_t>(C::FF) * 2, C::FF == 32 ? 32 : 64, C::G)) return rc;
   // the store clips at the writable width, in whole 16-byte chunks (columns L..zw-1 of the last group receive the
   // zeros its absent weight rows produce); the kernel writes the remaining zw % 8 columns itself
-  if (zw < 8) return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: writable width below 8 columns");
-  if (int rc = make_tmap_bf16_2d(&tm_z, z, static_cast<uint64_t>(zw & ~int64_t(7)), static_cast<uint64_t>(B), static_cast<uint64_t>(ldz) * 2, 64, C::BT)) return rc;
+  if (tk) tm_z = tm_w;                          // not used
+  else if (zw < 8) return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: writable width below 8 columns");
+  else if (int rc = make_tmap_bf16_2d(&tm_z, z, static_cast<uint64_t>(zw & ~int64_t(7)), static_cast<uint64_t>(B), static_cast<uint64_t>(ldz) * 2, 64, C::BT)) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = a.NG < sms ? a.NG : sms;
-  auto k = ffi_forward_sm100_kernel<GG_, FF_, P_>;
+  auto k = tk ? ffi_forward_sm100_kernel<GG_, FF_, P_, true> : ffi_forward_sm100_kernel<GG_, FF_, P_, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   k<<<grid, C::NTHREADS, C::SMEM_BYTES, st>>>(a, tm_x, tm_w, tm_z);
@@ -366,12 +456,23 @@ bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64
 
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
                          int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
-  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
-  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
-  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
-  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
-  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, st);
+  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
+  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
+  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
+  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
+  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
   return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
+}
+
+int launch_topk_filter_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, int64_t B, int64_t D, int64_t F, int64_t L,
+                             int64_t G, int64_t ldxt, const TopkFilter& tk, cudaStream_t st) {
+  if (B > 65536) return fail(HASTE_ERR_UNSUPPORTED, "top-k filter: batch %lld too large", (long long)B);      // 16 bits of a list entry
+  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  return fail(HASTE_ERR_UNSUPPORTED, "top-k filter: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }
 
 }  // namespace haste

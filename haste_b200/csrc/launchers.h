@@ -26,6 +26,15 @@ int launch_forward(const int32_t* loc, const void* xt, const void* w, const void
 bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t ldxt);
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
                          int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st);
+// Forward whose epilogue keeps only the logits above thr[b], as keys in cand[b][0 .. cap) (cnt[b] counts them all).
+struct TopkFilter {
+  const float* thr;
+  unsigned long long* cand;
+  int* cnt;
+  int cap, label0;
+};
+int launch_topk_filter_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, int64_t B, int64_t D, int64_t F, int64_t L,
+                             int64_t G, int64_t ldxt, const TopkFilter& tk, cudaStream_t st);
 int launch_bwd_features(const void* w, const int32_t* loc, const void* dy, float* dxt, int64_t B, int64_t D, int64_t F, int64_t L,
                         int64_t G, int64_t ldy, cudaStream_t st);
 int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void* dw, void* dbias, const UpdateArgs* upd, int64_t B,
@@ -72,6 +81,10 @@ int launch_backward_sm100(const void* xt, const void* w, const int32_t* loc, con
                           const UpdateArgs* upd, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldy, int64_t ldxt, cudaStream_t st);
 int launch_pad_rows(const void* src, int64_t ld_src, void* dst, int64_t ld_dst, int64_t rows, int64_t cols, cudaStream_t st);
 int launch_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t col0, int k, float* vals, int32_t* idx, cudaStream_t st);
+// Whole top-k of a layer, filtered (topk.cu); scratch: topk_fused_scratch_bytes bytes, 0 = this shape takes the chunked path.
+int64_t topk_fused_scratch_bytes(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k);
+int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t B, int64_t D, int64_t F, int64_t L,
+                      int64_t G, int k, int64_t label0, float* vals, int32_t* idx, cudaStream_t st);
 int launch_check_loc(const int32_t* loc, int64_t n, int64_t D, cudaStream_t st);
 // score_mode 0 mean / 1 max; prune_mode 0 threshold / 1 per-group fraction / 2 global fraction (n_prune is then the
 // layer-wide count and scratch holds HASTE_REWIRE_SCRATCH_WORDS(NG, F) words)

@@ -134,4 +134,391 @@ int launch_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t
   return check_launch("topk_update_kernel");
 }
 
+
+// ================================================================ whole top-k with a filtered forward
+// The chunked path above writes every logit to L2 and reads it back once (670 K labels, 512 rows: 686 MB each way).  Here
+// only a first chunk of TF_FIRST labels is stored; its k-th best logit is a threshold that all but k * (labels of the
+// launch / labels before it) of the remaining logits fail, so the forward's epilogue filters them in registers
+// (TOPK instantiations of the tcgen05 forward) and a merge kernel folds the survivors in.  Each launch covers TF_GROW
+// times the labels seen before it: for random label order that is TF_GROW * k candidates a row, against a list of
+// TF_CAP.  A row whose list overflows (labels laid out so that later ones are systematically better for it) is computed
+// again by the merge kernel on the CUDA cores: slower, the same result up to the order of the fp32 sums.
+constexpr int TF_THREADS = 256;
+constexpr int64_t TF_FIRST = 16384, TF_GROW = 8;
+constexpr int TF_CAP = 8192;
+typedef unsigned long long u64;
+
+// The keys that can be among the k best of n: all that are not below the k-th largest of the threads' maxima (a key below
+// it has k better ones).  key(i) for i < n, 0 = no entry; non-zero keys are distinct.  At most k * ceil(n / NT) pass.
+// Returns their number; all threads call it, and it ends with a barrier.
+template <int NT, class KEY>
+__device__ __forceinline__ int keep_candidates(KEY key, int n, int k, u64* out, u64* s_max, u64* s_tau, int* s_n) {
+  const int tid = threadIdx.x;
+  u64 m = 0;
+#pragma unroll 4
+  for (int i = tid; i < n; i += NT) { const u64 v = key(i); m = v > m ? v : m; }
+  s_max[tid] = m;
+  if (tid == 0) { *s_tau = 0; *s_n = 0; }
+  __syncthreads();
+  int rank = 0;
+#pragma unroll 8
+  for (int j = 0; j < NT; ++j) rank += s_max[j] > m;
+  if (m != 0 && rank == k - 1) *s_tau = m;
+  __syncthreads();
+  const u64 tau = *s_tau;
+#pragma unroll 4
+  for (int i = tid; i < n; i += NT) {
+    const u64 v = key(i);
+    if (v != 0 && v >= tau) out[atomicAdd(s_n, 1)] = v;
+  }
+  __syncthreads();
+  return *s_n;
+}
+static int64_t keep_bound(int64_t n, int k, int nt) { return static_cast<int64_t>(k) * ((n + nt - 1) / nt); }
+
+// The k best of keys[0..s) in order, to vals / idx (label ids as in the keys; -inf / -1 where there are fewer); returns
+// nothing, writes *thr = the k-th value when thr != NULL.
+template <int NT>
+__device__ __forceinline__ void write_best(const u64* keys, int s, int k, float* vals, int32_t* idx, float* thr) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < k; i += NT)
+    if (i >= s) { vals[i] = -INFINITY; idx[i] = -1; }
+  if (tid == 0 && thr != nullptr && s < k) *thr = -INFINITY;
+  for (int i = tid; i < s; i += NT) {
+    const u64 v = keys[i];
+    int rank = 0;
+#pragma unroll 4
+    for (int j = 0; j < s; ++j) rank += keys[j] > v;
+    if (rank < k) {
+      vals[rank] = topk_key_value(v);
+      idx[rank] = topk_key_label(v);
+      if (thr != nullptr && rank == k - 1) *thr = topk_key_value(v);
+    }
+  }
+}
+__device__ __forceinline__ u64 logit_key(uint16_t bits, uint32_t label) {
+  const float v = bf16_bits_to_float(bits);
+  return v > -INFINITY ? topk_key(v, label) : 0ull;                 // -inf and NaN are never selected
+}
+
+// First chunk: the k best of z[b, 0..C), labels col0 + c; also the row's threshold and its empty candidate list.
+__global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* __restrict__ z, int64_t ldz, int C, uint32_t col0, int k,
+                                                                float* __restrict__ vals, int32_t* __restrict__ idx, float* __restrict__ thr,
+                                                                int* __restrict__ cnt) {
+  extern __shared__ __align__(16) u64 kept[];
+  __shared__ u64 s_max[TF_THREADS], s_tau;
+  __shared__ int s_n;
+  const int64_t b = blockIdx.x;
+  const uint16_t* zr = z + b * ldz;
+  const int s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], col0 + i); }, C, k, kept, s_max, &s_tau, &s_n);
+  write_best<TF_THREADS>(kept, s, k, vals + b * k, idx + b * k, thr + b);
+  if (threadIdx.x == 0) cnt[b] = 0;
+}
+
+// Merge: the row's kept list and its candidates -> kept list, threshold; the candidate list is emptied.
+constexpr int TM_LIST = 2048 + TF_THREADS;          // recomputation: running list ...
+constexpr int TM_KEEP = TK_KMAX * ((TM_LIST + TF_THREADS - 1) / TF_THREADS);      // ... and what a compaction of it can keep
+constexpr int TM_KEYS = TK_KMAX * ((TF_CAP + TK_KMAX + TF_THREADS - 1) / TF_THREADS);
+static_assert(TM_LIST + TM_KEEP <= TM_KEYS, "the recomputation works inside the merge's buffer");
+
+struct TopkMergeArgs {
+  const int32_t* loc;
+  const uint16_t *xt, *w, *bias;                    // of the launch's labels
+  const u64* cand;
+  float *vals, *thr;
+  int32_t* idx;
+  int* cnt;
+  int64_t L, ldxt;
+  int D, F, G, k;
+  uint32_t label0;
+};
+
+__global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a) {
+  __shared__ __align__(16) u64 keys[TM_KEYS];
+  __shared__ u64 s_max[TF_THREADS], s_tau;
+  __shared__ int s_n, s_list;
+  const int tid = threadIdx.x, k = a.k;
+  const int64_t b = blockIdx.x;
+  float* vals = a.vals + b * k;
+  int32_t* idx = a.idx + b * k;
+  const int n = a.cnt[b];
+  if (n == 0) return;                               // uniform: nothing beat the kept list
+  auto kept = [&](int i) { const int id = idx[i]; return id < 0 ? 0ull : topk_key(vals[i], static_cast<uint32_t>(id)); };
+  int s;
+  if (n <= TF_CAP) {
+    const u64* c = a.cand + b * TF_CAP;
+    s = keep_candidates<TF_THREADS>([&](int i) { return i < n ? c[i] : kept(i - n); }, n + k, k, keys, s_max, &s_tau, &s_n);
+  } else {
+    // every logit of the launch again: 256 threads take 256 / G groups at a time, one label each
+    __shared__ float xs[TF_THREADS / 16][128];      // gathered features of these groups
+    u64* best = keys + TM_LIST;
+    if (tid == 0) s_list = k;
+    if (tid < k) keys[tid] = kept(tid);
+    float thr = a.thr[b];
+    __syncthreads();
+    const int per = TF_THREADS / a.G, gl = tid / a.G, r = tid % a.G;
+    const int64_t NG = (a.L + a.G - 1) / a.G;
+    for (int64_t g0 = 0; g0 < NG; g0 += per) {
+      for (int i = tid; i < per * a.F; i += TF_THREADS) {
+        const int64_t g = g0 + i / a.F;
+        float v = 0.f;
+        if (g < NG) {
+          const int d = min(max(__ldg(a.loc + g * a.F + i % a.F), 0), a.D - 1);
+          v = bf16_bits_to_float(__ldg(a.xt + static_cast<int64_t>(d) * a.ldxt + b));
+        }
+        xs[i / a.F][i % a.F] = v;
+      }
+      __syncthreads();
+      const int64_t l = (g0 + gl) * a.G + r;
+      if (l < a.L) {
+        float acc = 0.f;
+        const uint4* wr = reinterpret_cast<const uint4*>(a.w + l * a.F);
+        for (int c = 0; c < a.F / 8; ++c) {
+          const uint4 v = __ldg(wr + c);
+          const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc = fmaf(__uint_as_float(w4[j] << 16), xs[gl][c * 8 + 2 * j], acc);
+            acc = fmaf(__uint_as_float(w4[j] & 0xFFFF0000u), xs[gl][c * 8 + 2 * j + 1], acc);
+          }
+        }
+        if (a.bias != nullptr) acc += bf16_bits_to_float(a.bias[l]);
+        const float z = round_to_bf16_f(acc);
+        if (z > thr) keys[atomicAdd(&s_list, 1)] = topk_key(z, a.label0 + static_cast<uint32_t>(l));
+      }
+      __syncthreads();
+      if (s_list > TM_LIST - TF_THREADS) {          // uniform; room for one more round of labels is kept
+        const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, best, s_max, &s_tau, &s_n);
+        for (int i = tid; i < m; i += TF_THREADS) {
+          int rank = 0;
+          for (int j = 0; j < m; ++j) rank += best[j] > best[i];
+          if (rank < k) { keys[rank] = best[i]; if (rank == k - 1) s_max[0] = best[i]; }
+        }
+        if (tid == 0) s_list = min(m, k);
+        __syncthreads();
+        if (m >= k) thr = topk_key_value(s_max[0]);
+        __syncthreads();
+      }
+    }
+    const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, best, s_max, &s_tau, &s_n);
+    for (int i = tid; i < m; i += TF_THREADS) keys[i] = best[i];
+    __syncthreads();
+    s = m;
+  }
+  __syncthreads();
+  write_best<TF_THREADS>(keys, s, k, vals, idx, a.thr + b);
+  if (tid == 0) a.cnt[b] = 0;
+}
+
+// ================================================================ a few rows: bandwidth-bound product on the CUDA cores
+// With up to TS_ROWS batch rows the layer is one read of the weights, and a 128-row tensor-core tile is nearly all padding.
+// Grid: segments of whole label groups, at least two per SM where the layer is large enough.  A warp takes TS_UNIT label
+// rows at a time: lane = (row of the load, 16-byte chunk), the gathered features of its 8 slots in registers, all loads of
+// the unit issued before the first product.  The segment's logits stay in shared memory, where the block picks the
+// k best of every batch row; topk_parts_kernel merges the segments.
+constexpr int TS_ROWS = 8, TS_UNIT = 16, TS_THREADS = 256, TS_SEG = 4096, TS_MERGE = 1024;
+
+template <int F, int NB>
+__global__ void __launch_bounds__(TS_THREADS) topk_rows_kernel(const int32_t* __restrict__ loc, const uint16_t* __restrict__ x,
+                                                               const uint16_t* __restrict__ w, const uint16_t* __restrict__ bias, int B, int D,
+                                                               int64_t L, int G, int seg, int k, uint32_t label0, u64* __restrict__ part) {
+  constexpr int LPR = F / 8, RPL = 32 / LPR, NLD = TS_UNIT / RPL > 0 ? TS_UNIT / RPL : 1;
+  static_assert(RPL <= TS_UNIT && TS_UNIT % RPL == 0, "whole loads");
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ u64 s_max[TS_THREADS], s_tau;
+  __shared__ int s_n;
+  uint16_t* xs = reinterpret_cast<uint16_t*>(smem);                        // [NB][D]
+  uint16_t* zs = xs + (static_cast<int64_t>(NB) * D + 7) / 8 * 8;          // [NB][seg]
+  u64* kept = reinterpret_cast<u64*>(zs + NB * seg);                       // seg % 16 == 0
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t l_beg = static_cast<int64_t>(blockIdx.x) * seg;
+  const int n_lab = static_cast<int>(imin64(seg, L - l_beg));
+  for (int i = tid; i < NB * D; i += TS_THREADS) xs[i] = i < B * D ? x[i] : uint16_t(0);
+  __syncthreads();
+  const int c = lane % LPR, rl = lane / LPR;
+  for (int u0 = warp * TS_UNIT; u0 < n_lab; u0 += TS_THREADS / 32 * TS_UNIT) {
+    const int64_t l0 = l_beg + u0;                                         // TS_UNIT divides every group size: one group per unit
+    uint4 wv[NLD];
+#pragma unroll
+    for (int j = 0; j < NLD; ++j) {
+      const int64_t l = l0 + j * RPL + rl;
+      wv[j] = l < L ? __ldg(reinterpret_cast<const uint4*>(w + l * F) + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const int4* lp = reinterpret_cast<const int4*>(loc + (l0 / G) * F + c * 8);
+    const int4 i0 = __ldg(lp), i1 = __ldg(lp + 1);
+    const int id[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+    float xf[NB][8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int d = min(max(id[j], 0), D - 1);
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) xf[nb][j] = bf16_bits_to_float(xs[nb * D + d]);
+    }
+#pragma unroll
+    for (int j = 0; j < NLD; ++j) {
+      const uint32_t w4[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w};
+      const int64_t l = l0 + j * RPL + rl;
+      const float bv = (bias != nullptr && l < L) ? bf16_bits_to_float(__ldg(bias + l)) : 0.f;
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        float acc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          acc = fmaf(__uint_as_float(w4[e] << 16), xf[nb][2 * e], acc);
+          acc = fmaf(__uint_as_float(w4[e] & 0xFFFF0000u), xf[nb][2 * e + 1], acc);
+        }
+#pragma unroll
+        for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (c == 0 && u0 + j * RPL + rl < n_lab) zs[nb * seg + u0 + j * RPL + rl] = rn_bf16_bits(acc + bv);
+      }
+    }
+  }
+  __syncthreads();
+  for (int b = 0; b < B; ++b) {
+    const uint16_t* zb = zs + b * seg;
+    const int s = keep_candidates<TS_THREADS>([&](int i) { return logit_key(zb[i], label0 + static_cast<uint32_t>(l_beg + i)); }, n_lab, k, kept,
+                                              s_max, &s_tau, &s_n);
+    u64* out = part + (static_cast<int64_t>(b) * gridDim.x + blockIdx.x) * k;
+    for (int i = tid; i < k; i += TS_THREADS)
+      if (i >= s) out[i] = 0ull;
+    for (int i = tid; i < s; i += TS_THREADS) {
+      const u64 v = kept[i];
+      int rank = 0;
+      for (int j = 0; j < s; ++j) rank += kept[j] > v;
+      if (rank < k) out[rank] = v;
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(TS_MERGE) topk_parts_kernel(const u64* __restrict__ part, int n, int k, float* __restrict__ vals,
+                                                              int32_t* __restrict__ idx) {
+  extern __shared__ __align__(16) u64 kept[];
+  __shared__ u64 s_max[TS_MERGE], s_tau;
+  __shared__ int s_n;
+  const int64_t b = blockIdx.x;
+  const u64* p = part + b * n;
+  const int s = keep_candidates<TS_MERGE>([&](int i) { return p[i]; }, n, k, kept, s_max, &s_tau, &s_n);
+  write_best<TS_MERGE>(kept, s, k, vals + b * k, idx + b * k, nullptr);
+}
+
+// ---------------------------------------------------------------- host side
+// Segment length of the few-rows kernel: whole groups, two blocks per SM, at most TS_SEG labels.
+static int64_t rows_seg(int64_t L, int64_t G) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t NG = (L + G - 1) / G;
+  int64_t gps = (NG + 2 * sms - 1) / (2 * sms);
+  if (gps * G > TS_SEG) gps = TS_SEG / G;
+  return gps * G;
+}
+static int64_t round16(int64_t v) { return (v + 15) / 16 * 16; }
+static int pow2_rows(int64_t B) { return B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8; }
+static size_t rows_smem(int64_t B, int64_t D, int64_t seg, int k) {
+  const int64_t nb = pow2_rows(B);
+  return static_cast<size_t>((nb * D + 7) / 8 * 16 + nb * seg * 2 + keep_bound(seg, k, TS_THREADS) * 8);
+}
+// Which path: 0 the chunked one (above), 1 few rows, 2 filtered forward.
+// Few rows up to TS_ROWS: the filtered forward reads the same weights but pays five launches and a 128-row tile.
+static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
+  if (B <= TS_ROWS && (F == 16 || F == 32 || F == 64 || F == 128)) {
+    const int64_t seg = rows_seg(L, G), parts = (L + seg - 1) / seg;
+    if (rows_smem(B, D, seg, k) <= 200 * 1024 && keep_bound(parts * k, k, TS_MERGE) * 8 <= 200 * 1024) return 1;
+  }
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 64 || F == 32));
+  if (shape && B <= 65536 && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
+  return 0;
+}
+
+// Scratch of the filtered path, in bytes from a 16-byte aligned base: xt | logits of the first chunk | candidates | thresholds | counters
+struct FusedScratch { int64_t xt, z, cand, thr, cnt, total; };
+static FusedScratch fused_layout(int64_t B, int64_t D, int64_t L, int64_t G) {
+  const int64_t ldxt = (B + 7) / 8 * 8, first = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
+  FusedScratch s;
+  s.xt = 0;
+  s.z = round16(s.xt + D * ldxt * 2);
+  s.cand = round16(s.z + B * first * 2);
+  s.thr = s.cand + (L > first ? B * TF_CAP * 8 : 0);
+  s.cnt = round16(s.thr + B * 4);
+  s.total = round16(s.cnt + B * 4);
+  return s;
+}
+int64_t topk_fused_scratch_bytes(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
+  switch (topk_route(B, D, F, L, G, k)) {
+    case 1: { const int64_t seg = rows_seg(L, G); return B * ((L + seg - 1) / seg) * k * 8; }
+    case 2: return fused_layout(B, D, L, G).total;
+    default: return 0;
+  }
+}
+
+template <class K>
+static int allow_smem(K kernel, size_t bytes) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(e));
+  return HASTE_OK;
+}
+
+int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t B, int64_t D, int64_t F, int64_t L,
+                      int64_t G, int k, int64_t label0, float* vals, int32_t* idx, cudaStream_t st) {
+  const int route = topk_route(B, D, F, L, G, k);
+  if (route == 1) {
+    const int64_t seg = rows_seg(L, G), parts = (L + seg - 1) / seg;
+    const size_t sm = rows_smem(B, D, seg, k);
+    u64* part = static_cast<u64*>(scratch);
+#define HASTE_TOPK_ROWS(F_, NB_)                                                                                             \
+  {                                                                                                                          \
+    auto kern = topk_rows_kernel<F_, NB_>;                                                                                   \
+    if (int rc = allow_smem(kern, sm)) return rc;                                                                            \
+    kern<<<static_cast<unsigned>(parts), TS_THREADS, sm, st>>>(loc, (const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)bias, int(B), int(D), L, \
+                                                               int(G), int(seg), k, static_cast<uint32_t>(label0), part);    \
+  }
+#define HASTE_TOPK_ROWS_NB(F_)                                                                                               \
+  { switch (pow2_rows(B)) { case 1: HASTE_TOPK_ROWS(F_, 1) break; case 2: HASTE_TOPK_ROWS(F_, 2) break; case 4: HASTE_TOPK_ROWS(F_, 4) break; \
+                            default: HASTE_TOPK_ROWS(F_, 8) } }
+    if (F == 16) HASTE_TOPK_ROWS_NB(16) else if (F == 32) HASTE_TOPK_ROWS_NB(32) else if (F == 64) HASTE_TOPK_ROWS_NB(64) else HASTE_TOPK_ROWS_NB(128)
+#undef HASTE_TOPK_ROWS_NB
+#undef HASTE_TOPK_ROWS
+    if (int rc = check_launch("topk_rows_kernel")) return rc;
+    const size_t sm2 = static_cast<size_t>(keep_bound(parts * k, k, TS_MERGE)) * 8;
+    if (int rc = allow_smem(topk_parts_kernel, sm2)) return rc;
+    topk_parts_kernel<<<static_cast<unsigned>(B), TS_MERGE, sm2, st>>>(part, int(parts * k), k, vals, idx);
+    return check_launch("topk_parts_kernel");
+  }
+  if (route != 2) return fail(HASTE_ERR_UNSUPPORTED, "top-k: group size %lld, fan-in %lld, batch %lld take the chunked call", (long long)G, (long long)F, (long long)B);
+  const FusedScratch fs = fused_layout(B, D, L, G);
+  char* base = static_cast<char*>(scratch);
+  const int64_t ldxt = (B + 7) / 8 * 8;
+  void* xt = base + fs.xt;
+  uint16_t* z = reinterpret_cast<uint16_t*>(base + fs.z);
+  float* thr = reinterpret_cast<float*>(base + fs.thr);
+  int* cnt = reinterpret_cast<int*>(base + fs.cnt);
+  u64* cand = reinterpret_cast<u64*>(base + fs.cand);
+  const char* wb = static_cast<const char*>(w);
+  const char* bb = static_cast<const char*>(bias);
+  if (int rc = launch_transpose(x, xt, B, D, ldxt, st)) return rc;
+  const int64_t ldz = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
+  const int64_t first = imin64(ldz, L);
+  if (int rc = launch_forward(loc, xt, w, bias, z, B, D, F, first, G, ldz, (first + 7) / 8 * 8, ldxt, st)) return rc;
+  const size_t sm = static_cast<size_t>(keep_bound(first, k, TF_THREADS)) * 8;
+  if (int rc = allow_smem(topk_first_kernel, sm)) return rc;
+  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, sm, st>>>(z, ldz, int(first), static_cast<uint32_t>(label0), k, vals, idx, thr, cnt);
+  if (int rc = check_launch("topk_first_kernel")) return rc;
+  for (int64_t l0 = first; l0 < L;) {
+    const int64_t n = imin64(TF_GROW * l0, L - l0), g0 = l0 / G;          // first is a multiple of G when there is more, so l0 always is
+    TopkFilter tk{thr, cand, cnt, TF_CAP, static_cast<int>(label0 + l0)};
+    const void* w0 = wb + l0 * F * 2;
+    const void* b0 = bb ? bb + l0 * 2 : nullptr;
+    if (int rc = launch_topk_filter_sm100(loc + g0 * F, xt, w0, b0, B, D, F, n, G, ldxt, tk, st)) return rc;
+    TopkMergeArgs a;
+    a.loc = loc + g0 * F; a.xt = static_cast<const uint16_t*>(xt); a.w = static_cast<const uint16_t*>(w0); a.bias = static_cast<const uint16_t*>(b0);
+    a.cand = cand; a.vals = vals; a.thr = thr; a.idx = idx; a.cnt = cnt; a.L = n; a.ldxt = ldxt;
+    a.D = int(D); a.F = int(F); a.G = int(G); a.k = k; a.label0 = static_cast<uint32_t>(label0 + l0);
+    topk_merge_kernel<<<static_cast<unsigned>(B), TF_THREADS, 0, st>>>(a);
+    if (int rc = check_launch("topk_merge_kernel")) return rc;
+    l0 += n;
+  }
+  return HASTE_OK;
+}
+
 }  // namespace haste

@@ -341,6 +341,26 @@ def topk(loc, xt, w, bias, zbuf, groups_per_chunk, k, G, label0, vals, idx):
                                  label0, _ptr(vals), _ptr(idx), ldx, _stream(xt)), "ffi_topk")
 
 
+def topk_fused(loc, x, w, bias, k, G, label0):
+    """Top-k straight from features [B, D] in one library call: (values fp32 [B, k], labels int32 [B, k]), or None for
+    the shapes that take ``topk``."""
+    _req(loc, "locations", torch.int32); _req(x, "x", torch.bfloat16); _req(w, "weights", torch.bfloat16)
+    if bias is not None:
+        _req(bias, "bias", torch.bfloat16)
+    B, D = x.shape
+    L, F = w.shape
+    with torch.cuda.device(x.device):
+        n = lib.haste_ffi_topk_fused_scratch(B, D, F, L, G, k)
+        if n == 0 or _ptr(loc) % 16 or _ptr(w) % 16:
+            return None
+        scratch = torch.empty(n, dtype=torch.uint8, device=x.device)
+        vals = torch.empty(B, k, dtype=torch.float32, device=x.device)
+        idx = torch.empty(B, k, dtype=torch.int32, device=x.device)
+        check(lib.haste_ffi_topk_fused(_ptr(loc), _ptr(x), _ptr(w), _ptr(bias), _ptr(scratch), n, B, D, F, L, G, k, label0, _ptr(vals),
+                                       _ptr(idx), _stream(x)), "ffi_topk_fused")
+    return vals, idx
+
+
 def topk_update(z, C, col0, vals, idx):
     """Fold logits z[:, :C] (labels col0..col0+C-1) into the running top-k state (vals fp32 [B,k], idx int32 [B,k])."""
     _req(z, "logits", torch.bfloat16, contiguous=False); _req(vals, "vals", torch.float32); _req(idx, "idx", torch.int32)

@@ -26,6 +26,9 @@ def ffi_topk(group_locations, weights, bias, features, k, group_size, *, groups_
     NG = (L + G - 1) // G
     dev = features.device
     if groups_per_chunk is None:
+        best = _ffi.topk_fused(group_locations, features, weights, bias, k, G, label0)
+        if best is not None:
+            return best
         # about 64 MB of logits per chunk (well inside the 126 MB L2), in whole waves of one group per SM
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         per_group = B * G * 2

@@ -307,6 +307,16 @@ int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void
                    int64_t D, int64_t F, int64_t L, int64_t G, int64_t groups_per_chunk, int32_t k, int64_t label0,
                    float* vals, int32_t* idx, haste_stream_t stream);
 
+/* The same top-k without a chunk loop over stored logits, straight from the features x bf16 [B,D]: for few rows one
+ * weight-streaming kernel and a merge; otherwise the logits of a first chunk set a threshold per row, and the forward
+ * kernels of the remaining labels keep only what beats it.  vals / idx are outputs (no start values).  `scratch`: 16-byte
+ * aligned, haste_ffi_topk_fused_scratch(...) bytes; that function returns 0 for shapes that need haste_ffi_topk (and for
+ * invalid ones).  Results as haste_ffi_topk up to the order of the fp32 sums of a logit. */
+int64_t haste_ffi_topk_fused_scratch(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k);
+int haste_ffi_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t scratch_bytes,
+                         int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k, int64_t label0,
+                         float* vals, int32_t* idx, haste_stream_t stream);
+
 /* The entry points above that take the transposed features, with a row stride: xt is [D, ldxt], ldxt >= B.  The tensor
  * maps of the tcgen05 kernels need 16-byte aligned rows, so a batch whose size is not a multiple of 8 reaches them with
  * ldxt = B rounded up to 8.  haste_transpose_bf16_ldx and haste_ffi_step_ldx write zeros into columns B..ldxt-1; the

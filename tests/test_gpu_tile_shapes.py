@@ -1,5 +1,5 @@
 """GPU parity tests of the tcgen05 kernels at the layer shapes whose tiles hold 64 labels or two label groups, at batch
-sizes that are not multiples of 8 (padded rows of xt).  Tolerances: bf16 inputs, fp32
+sizes that are not multiples of 8 (padded rows of xt), and of the filtered top-k.  Tolerances: bf16 inputs, fp32
 accumulation, bf16 logits and loss gradients — rel 1e-2 / abs 1e-3 of the magnitude, as for the other shapes."""
 import pytest
 import torch
@@ -82,3 +82,73 @@ def test_step_bce_gradient_of_very_negative_logits(layer):
     z = fo.forward(inp["loc"], inp["X"], inp["W"], inp["bias"], G).double()
     want = torch.sigmoid(z).sum(0)
     assert ((sh.mom_b.cpu().double() - want).abs() <= 2 ** -7 * want).all()          # two bf16 roundings of dY and its sum
+
+
+# ------------------------------------------------------------------------------------------------ filtered top-k
+def _check_topk(vals, idx, z, k, label0):
+    """Against the full logits z (float, -inf and NaN never selected): values, and ids that are distinct, point at a logit
+    of their value and stand in label order among equal values.  A logit may be the bf16 neighbour of z's (fp32 sum in
+    another order)."""
+    L = z.shape[1]
+    z = torch.where(torch.isnan(z), torch.full_like(z, float("-inf")), z)
+    want = torch.topk(z, min(k, L), dim=1).values
+    got = vals[:, :want.shape[1]]
+    none = torch.isinf(want) & (want < 0)
+    assert torch.equal(torch.isinf(got) & (got < 0), none)
+    assert (idx[:, :want.shape[1]][none] == -1).all() and (idx[:, want.shape[1]:] == -1).all() and torch.isinf(vals[:, want.shape[1]:]).all()
+    ok = ~none
+    if none.all():
+        return
+    near = (got - want).abs() <= 2 ** -7 * want.abs() + 1e-6
+    assert near[ok].all() and (got == want)[ok].float().mean() >= 0.99
+    ids = (idx[:, :want.shape[1]].long() - label0)
+    assert ((ids >= 0) & (ids < L))[ok].all()
+    at = torch.gather(z, 1, ids.clamp(0, L - 1))
+    assert ((at - got).abs() <= 2 ** -7 * got.abs() + 1e-6)[ok].all() and (at == got)[ok].float().mean() >= 0.99
+    for r, o in zip(ids.cpu(), ok.cpu()):
+        assert len(set(r[o].tolist())) == int(o.sum())
+    eq = (got[:, 1:] == got[:, :-1]) & ok[:, 1:]
+    assert (ids[:, 1:] > ids[:, :-1])[eq].all()
+
+
+@pytest.mark.parametrize("cfg", [
+    dict(B=1, L=131073, F=128, G=64, k=5), dict(B=1, L=40, F=16, G=16, k=128), dict(B=3, L=5000, F=32, G=32, k=100),
+    dict(B=8, L=70001, F=64, G=128, k=50), dict(B=7, L=300007, F=32, G=32, k=128),
+    dict(B=9, L=16385, F=32, G=32, k=10), dict(B=40, L=160001, F=32, G=32, k=100), dict(B=200, L=40003, F=64, G=128, k=100),
+    dict(B=130, L=30000, F=128, G=64, k=1), dict(B=17, L=20011, F=64, G=64, k=128), dict(B=16, L=20011, F=64, G=32, k=7),
+], ids=lambda c: "-".join(f"{n}{v}" for n, v in c.items()))
+def test_topk_fused(cfg):
+    from haste_b200 import ffi
+    from haste_b200.infer import ffi_topk
+    B, L, F, G, k, D = cfg["B"], cfg["L"], cfg["F"], cfg["G"], cfg["k"], 256
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=11, x_kind="normal", bias_zero=False)
+    dev = {n: v.cuda() for n, v in inp.items()}
+    vals, idx = ffi_topk(dev["loc"], dev["W"], dev["bias"], dev["X"], k, G, label0=5)
+    z = ffi.forward(dev["loc"], ffi.transpose_padded(dev["X"]), dev["W"], dev["bias"], G, B=B).float()
+    _check_topk(vals, idx, z, k, 5)
+
+
+@pytest.mark.parametrize("kind", ["ascending", "equal", "masked", "none"])
+@pytest.mark.parametrize("B", [2, 16])
+def test_topk_fused_unusual_logits(kind, B):
+    """ascending: every later label beats all earlier ones, so the candidate lists overflow and the rows are computed
+    again; equal: only the label id decides; masked: -inf and NaN biases are never selected; none: nothing is."""
+    from haste_b200 import ffi
+    from haste_b200.infer import ffi_topk
+    D, L, F, G, k = 128, 16384 + 12007, 64, 64, 100
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=12, x_kind="normal", bias_zero=True)
+    if kind == "ascending":
+        inp["bias"] = (torch.arange(L) / 64.0).to(torch.bfloat16)
+    elif kind == "equal":
+        inp["W"].zero_()
+    elif kind == "masked":
+        inp["bias"][::3] = float("-inf")
+        inp["bias"][1::3] = float("nan")
+    else:
+        inp["bias"][:] = float("-inf")
+    dev = {n: v.cuda() for n, v in inp.items()}
+    vals, idx = ffi_topk(dev["loc"], dev["W"], dev["bias"], dev["X"], k, G)
+    z = ffi.forward(dev["loc"], ffi.transpose_padded(dev["X"]), dev["W"], dev["bias"], G, B=B).float()
+    _check_topk(vals, idx, z, k, 0)
+    if kind == "equal":
+        assert torch.equal(idx.cpu(), torch.arange(k, dtype=torch.int32).expand(B, k))
