@@ -1,5 +1,5 @@
-// Unfused backward of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size, fan-in) = (128, 64), (64, 128), (64, 64)
-// and, with two consecutive groups per tile, (32, 64) and (32, 32): one pass over dY [B, ldy] produces both gradients of the autograd surface,
+// Unfused backward of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size, fan-in) = (128, 64), (64, 128), (64, 64),
+// (32, 128) (label columns 32-63 of its tiles are zeros) and, with two consecutive groups per tile, (32, 64) and (32, 32): one pass over dY [B, ldy] produces both gradients of the autograd surface,
 //     dxt[loc[g,k], b] += sum_{l in g} w[l,k] * dy[b,l]          (fp32, reduced into dxt with red.global.add)
 //     dw [l, k]         = sum_b dy[b,l] * xt[loc[g,k], b]          (bf16, round to nearest)
 //     dbias[l]          = sum_b dy[b,l]                            (bf16; via a row of ones under the X tile)
@@ -33,7 +33,8 @@ using namespace sm100;
 template <int GG_, int FF_, int P_>
 struct Cfg {
   static constexpr int GG = GG_, FF = FF_, P = P_;     // label group, fan-in, groups per tile
-  static constexpr int G = P * GG, F = P * FF, BT = 128;
+  static constexpr int LS = P * GG;                    // labels of a tile
+  static constexpr int G = LS < 64 ? 64 : LS, F = P * FF, BT = 128;      // label columns (M of the dW accumulator: at least 64) and slots
   static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)), "tile shapes with a tcgen05 backward");
   static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
   static constexpr int WROW = FF == 32 ? 64 : 128;    // bytes of one swizzled row of a W block
@@ -47,7 +48,7 @@ struct Cfg {
   static constexpr int XBLK = FR * 128, XSTAGE = 2 * XBLK;
   static constexpr int NWB = FF == 32 ? 1 : FF / 64, WBLK = G * WROW, WSTAGE = NWB * WBLK;
   static constexpr int NYB = G / 64, YBLK = BT * 128, YSTAGE = NYB * YBLK;
-  static constexpr int NCH = G / 8;                   // 16-byte chunks of a row slice
+  static constexpr int NCH = LS / 8;                  // 16-byte chunks of a row slice
   static constexpr int YSIDE = BT * 16;               // one more aligned chunk per row (the tail of a misaligned slice)
   static constexpr int OFF_X = 0;
   static constexpr int OFF_W = OFF_X + NXS * XSTAGE;
@@ -86,7 +87,7 @@ struct BwdArgs {
   __nv_bfloat16* dbias;
   int* err;
   int64_t B, L, ldy;
-  int D, NG, NGR;      // NG: tiles of G labels; NGR: label groups
+  int D, NG, NGR;      // NG: tiles of LS labels; NGR: label groups
   long long wait_limit;
 };
 
@@ -104,7 +105,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
   static_assert(DX || DW, "nothing to compute");
   static_assert(!UPD || DW, "the update consumes the weight gradient");
   using C = Cfg<GG_, FF_, P_>;
-  constexpr int GG = C::GG, FF = C::FF, P = C::P;
+  constexpr int GG = C::GG, FF = C::FF, P = C::P, LS = C::LS;
   constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX, NDW = C::NDW;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE, NCH = C::NCH;
   extern __shared__ uint8_t smem_raw[];
@@ -137,6 +138,10 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     const uint32_t v = (row == 0) ? 0x3F803F80u : 0u;
     *reinterpret_cast<uint4*>(sm + C::OFF_X + blk * XBLK + (F + row) * 128 + chunk * 16) = make_uint4(v, v, v, v);
   }
+  if (LS < G) {       // the label columns that no tile of this shape has: zeros, never written again
+    for (int i = tid; i < NYS * BT * 8; i += C::NTHREADS)
+      if ((i & 7) >= NCH) *reinterpret_cast<uint4*>(sm + C::OFF_Y + (i >> 10) * YSTAGE + ((i >> 3) & 127) * 128 + (((i & 7) ^ ((i >> 3) & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+  }
   fence_proxy_async();
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TM_COLS);
@@ -159,7 +164,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int ws = gi & 1;
-      const int64_t l0 = static_cast<int64_t>(g) * G;
+      const int64_t l0 = static_cast<int64_t>(g) * LS;
       const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
       int locv[F / 32];
 #pragma unroll
@@ -238,11 +243,11 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         cp_async_wait<LAG - 1>();                      // this lane's copies of tile it - LAG have landed (groups 0 .. it-1 are committed)
         __syncwarp();                                  // ... and so have the other lanes'
         const int jt = it - LAG, ys = jt % NYS;
-        const int64_t l0 = static_cast<int64_t>(group_of(gi_p)) * G;
+        const int64_t l0 = static_cast<int64_t>(group_of(gi_p)) * LS;
         const int64_t b0 = static_cast<int64_t>(t_p) * BT;
         // all rows of this warp start at the same offset inside a 16-byte granule
         const uint32_t sh = static_cast<uint32_t>((dy_base + 2ull * static_cast<uint64_t>((b0 + k) * a.ldy + l0)) & 15u);
-        const bool mask_cols = l0 + G > a.L;
+        const bool mask_cols = l0 + LS > a.L;
         if ((sh != 0 || mask_cols) && !*abort_flag) {
           const uint32_t wo = sh >> 2, hb = (sh & 2u) << 3;     // whole words, then 0 or 16 bits
           uint8_t* yb = sm + C::OFF_Y + ys * YSTAGE;
@@ -256,7 +261,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
             for (int blk = 0; blk < C::NYB; ++blk) {           // ascending: chunk 8 is read (as a neighbour) before it is rewritten
               const int cj = blk * 8 + c;
               uint8_t* p = yb + blk * YBLK + r * 128 + ((c ^ (r & 7)) << 4);
-              const uint8_t* pn = (cj + 1 == NCH) ? yside + r * 16
+              // (a chunk no label has: nothing is read beyond the tile, nothing is written)
+              const uint8_t* pn = cj >= NCH ? p : (cj + 1 == NCH) ? yside + r * 16
                                                   : yb + ((cj + 1) >> 3) * YBLK + r * 128 + ((((cj + 1) & 7) ^ (r & 7)) << 4);
               const uint4 v0 = *reinterpret_cast<const uint4*>(p);
               const uint4 v1 = *reinterpret_cast<const uint4*>(pn);
@@ -279,7 +285,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
                   o.w = nv == 7 ? (o.w & 0xFFFFu) : 0u;
                 }
               }
-              *reinterpret_cast<uint4*>(p) = o;
+              if (cj < NCH) *reinterpret_cast<uint4*>(p) = o;
             }
           }
         }
@@ -293,7 +299,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         const bool ok = mbar_wait(bar(C::B_YEMPTY + ys), ((it / NYS) & 1) ^ 1, abort_flag, a.err, 33, WL, 100);
         __syncwarp();
         if (ok && !*abort_flag) {
-          const int64_t l0 = static_cast<int64_t>(group_of(gi_i)) * G;
+          const int64_t l0 = static_cast<int64_t>(group_of(gi_i)) * LS;
           const int64_t b0 = static_cast<int64_t>(t_i) * BT;
           const uint32_t yb = sbase + C::OFF_Y + ys * YSTAGE, yside = sbase + C::OFF_YSIDE + ys * C::YSIDE;
 #pragma unroll
@@ -452,12 +458,12 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int dws = gi % NDW;
-      const int64_t l0 = static_cast<int64_t>(g) * G;
-      const int rows_real = static_cast<int>(imin64(G, a.L - l0));
+      const int64_t l0 = static_cast<int64_t>(g) * LS;
+      const int rows_real = static_cast<int>(imin64(LS, a.L - l0));
       mbar_wait(bar(C::B_DWFULL + dws), (gi / NDW) & 1, abort_flag, a.err, 42, WL);
       tc_fence_after();
       const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW + dws * FR;
-      const uint32_t tg = ta + (q * C::ROWS_PER_Q) / GG * FF;      // the columns of this quarter's group: its block on the diagonal
+      const uint32_t tg = ta + (P == 1 ? 0 : (q * C::ROWS_PER_Q) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
       const bool do_row = row < rows_real && !*abort_flag;
       const int64_t l = l0 + row, gl = u.label0 + l;
       const bool fast = UPD && u.mom_w == nullptr && (u.flags & HASTE_F_SR) && (u.flags & HASTE_F_CONTRACT);
@@ -569,7 +575,7 @@ static int launch_shape(const void* xt, const void* w, const int32_t* loc, const
   BwdArgs a;
   a.loc = loc; a.dy = static_cast<const __nv_bfloat16*>(dy); a.dxt = dxt; a.dw = static_cast<__nv_bfloat16*>(dw);
   a.dbias = static_cast<__nv_bfloat16*>(dbias); a.err = err_dev;
-  a.B = B; a.L = L; a.ldy = ldy; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::G - 1) / C::G);
+  a.B = B; a.L = L; a.ldy = ldy; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::LS - 1) / C::LS);
   a.NGR = static_cast<int>((L + C::GG - 1) / C::GG);
   a.wait_limit = wait_limit_cycles();
   UpdateArgs u{};
@@ -609,7 +615,7 @@ bool backward_sm100_supported(const void* xt, const void* w, const void* dy, con
                               int64_t G, int64_t ldxt) {
   // tensor maps need 16-byte aligned bases and row strides; dxt row offsets and tile coordinates are 32-bit; dy only
   // needs its natural 2-byte alignment
-  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 64 || F == 32));
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
   return shape && (xt == nullptr || (ldxt % 8) == 0) && aligned16(xt) && aligned16(w) && aligned16(dw) &&
          (reinterpret_cast<uintptr_t>(dy) & 1u) == 0 && D * B < (int64_t(1) << 32) && L < (int64_t(1) << 31) && ldxt < (int64_t(1) << 31);
 }
@@ -622,6 +628,7 @@ int launch_backward_sm100(const void* xt, const void* w, const int32_t* loc, con
   if (G == 64 && F == 128) return b100::launch_shape<64, 128, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
   if (G == 64 && F == 64) return b100::launch_shape<64, 64, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
   if (G == 32 && F == 64) return b100::launch_shape<32, 64, 2>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
+  if (G == 32 && F == 128) return b100::launch_shape<32, 128, 1>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
   if (G == 32 && F == 32) return b100::launch_shape<32, 32, 2>(xt, w, loc, dy, dxt, dw, dbias, upd, B, D, L, ldy, ldxt, st);
   return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 backward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }

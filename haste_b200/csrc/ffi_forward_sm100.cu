@@ -1,5 +1,5 @@
 // Forward gather-GEMM of the FFI layer on tcgen05 / TMEM, for the layer shapes (group size, fan-in) = (128, 64), (64, 128),
-// (64, 64), and, with two consecutive groups per tile, (32, 64) and (32, 32):
+// (64, 64), (32, 128) and, with two consecutive groups per tile, (32, 64) and (32, 32):
 //     z[b, l] = sum_k xt[loc[l/G, k], b] * w[l, k] + bias[l]        (bf16 in, fp32 accumulate, bf16 out)
 // This is the unfused forward of the autograd surface: it has to write the [B, L] logits, so it is bound by
 // that HBM write (2*B*L bytes), not by the tensor pipe.
@@ -34,7 +34,7 @@ template <int GG_, int FF_, int P_>
 struct Cfg {
   static constexpr int GG = GG_, FF = FF_, P = P_;     // label group, fan-in, groups per tile
   static constexpr int G = P * GG, F = P * FF, BT = 128;
-  static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)), "tile shapes with a tcgen05 forward");
+  static_assert((G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && F == 128), "tile shapes with a tcgen05 forward");
   static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
   static constexpr int WROW = FF == 32 ? 64 : 128;    // bytes of one swizzled row of a W block
   static constexpr int FR = F + 16;                   // rows of an X block: F gathered rows, one row of ones, 15 zero rows
@@ -44,7 +44,8 @@ struct Cfg {
   static constexpr int NWB = FF == 32 ? 1 : FF / 64;  // blocks of a W stage (64 slots each, 32 at fan-in 32)
   static constexpr int WBLK = G * WROW;
   static constexpr int WSTAGE = NWB * WBLK;
-  static constexpr int NCB = G / 64;                  // 64-label blocks of a staging tile
+  static constexpr int CROW = G == 32 ? 64 : 128;     // bytes of one swizzled row of a staging block
+  static constexpr int NCB = G == 32 ? 1 : G / 64;    // blocks of a staging tile (64 labels each, 32 at G = 32)
   static constexpr int CBLK = BT * 128;
   static constexpr int CSTAGE = NCB * CBLK;
   static constexpr int BTILE = G * 32;                // bias tile: G rows x 16 bf16, no swizzle
@@ -68,6 +69,11 @@ struct Cfg {
   static constexpr int W_EPI = 4, W_XP = W_EPI + N_EPI;
   static constexpr int NTHREADS = (W_XP + 1) * 32;
   static constexpr uint32_t TM_COLS = 2 * G;          // two accumulator stages
+  // byte offset of 16-byte chunk c (8 labels) of batch row `row` in a staging tile: as the tensor map's swizzle expects it
+  __device__ static __forceinline__ int c_chunk(int row, int c) {
+    if (G == 32) return row * 64 + ((c ^ ((row >> 1) & 3)) << 4);
+    return (c >> 3) * CBLK + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+  }
 };
 
 struct FwdArgs {
@@ -355,8 +361,8 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
         // the store that last read this staging buffer (two tiles ago) has finished reading: the storing thread
         // waited for that before it arrived here
         named_bar_sync(1, C::N_EPI * 32);
-        uint8_t* crow = sm + C::OFF_C + zs * C::CSTAGE + (G == 128 ? h * C::CBLK : 0) + row * 128;
-        const int chunk0 = (G == 128) ? 0 : h * (C::EC / 8);
+        uint8_t* cst = sm + C::OFF_C + zs * C::CSTAGE;
+        const int chunk0 = h * (C::EC / 8);
 #pragma unroll 1
         for (int c16 = 0; c16 < C::EC; c16 += 16) {
           uint32_t r[16];
@@ -369,8 +375,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
                                        pack2(__uint_as_float(r[e8 + 2]), __uint_as_float(r[e8 + 3])),
                                        pack2(__uint_as_float(r[e8 + 4]), __uint_as_float(r[e8 + 5])),
                                        pack2(__uint_as_float(r[e8 + 6]), __uint_as_float(r[e8 + 7])));
-            const int chunk = chunk0 + ((c16 + e8) >> 3);         // 0..7 inside the 128-byte row
-            *reinterpret_cast<uint4*>(crow + ((chunk ^ (row & 7)) << 4)) = v;
+            *reinterpret_cast<uint4*>(cst + C::c_chunk(row, chunk0 + ((c16 + e8) >> 3))) = v;
           }
         }
         tc_fence_before();
@@ -393,8 +398,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
         const int tail0 = static_cast<int>(a.zw & ~int64_t(7)), tail_n = static_cast<int>(a.zw - tail0);
         if (tail_n > 0 && h == 0 && tail0 >= l0 && tail0 < l0 + G && ok && !*abort_flag && t * BT + row < a.B) {
           const int tc = (tail0 - l0) >> 3;                   // chunk index inside the group's row
-          const uint4 v = *reinterpret_cast<const uint4*>(sm + C::OFF_C + zs * C::CSTAGE + (tc >> 3) * C::CBLK + row * 128 +
-                                                          (((tc & 7) ^ (row & 7)) << 4));
+          const uint4 v = *reinterpret_cast<const uint4*>(sm + C::OFF_C + zs * C::CSTAGE + C::c_chunk(row, tc));
           const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
           uint16_t* dst = reinterpret_cast<uint16_t*>(a.z) + (static_cast<int64_t>(t) * BT + row) * a.ldz + tail0;
 #pragma unroll
@@ -433,7 +437,7 @@ static int launch_shape(const int32_t* loc, const void* xt, const void* w, const
   // zeros its absent weight rows produce); the kernel writes the remaining zw % 8 columns itself
   if (tk) tm_z = tm_w;                          // not used
   else if (zw < 8) return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: writable width below 8 columns");
-  else if (int rc = make_tmap_bf16_2d(&tm_z, z, static_cast<uint64_t>(zw & ~int64_t(7)), static_cast<uint64_t>(B), static_cast<uint64_t>(ldz) * 2, 64, C::BT)) return rc;
+  else if (int rc = make_tmap_bf16_2d(&tm_z, z, static_cast<uint64_t>(zw & ~int64_t(7)), static_cast<uint64_t>(B), static_cast<uint64_t>(ldz) * 2, C::G == 32 ? 32 : 64, C::BT)) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -449,7 +453,7 @@ static int launch_shape(const int32_t* loc, const void* xt, const void* w, const
 
 bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t ldxt) {
   // tensor maps need 16-byte aligned bases and row strides; coordinates are 32-bit
-  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 64 || F == 32));
+  const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
   return shape && (ldxt % 8) == 0 && (ldz % 8) == 0 && aligned16(z) && aligned16(xt) &&
          aligned16(w) && L < (int64_t(1) << 31) && ldxt < (int64_t(1) << 31);
 }
@@ -460,6 +464,7 @@ int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, cons
   if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
   if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
   if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
+  if (G == 32 && F == 128) return f100::launch_shape<32, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
   if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
   return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }
@@ -471,6 +476,7 @@ int launch_topk_filter_sm100(const int32_t* loc, const void* xt, const void* w, 
   if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
   if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
   if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
+  if (G == 32 && F == 128) return f100::launch_shape<32, 128, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
   if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
   return fail(HASTE_ERR_UNSUPPORTED, "top-k filter: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
 }

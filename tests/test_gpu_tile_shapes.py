@@ -10,7 +10,7 @@ from oracle import ffi_oracle as fo
 
 # (G, F, L): one tile, an odd number of groups (the last tile of a pair holds one), ragged last groups, more tiles than SMs
 LAYERS = [(32, 32, 40), (32, 32, 32 * 401 + 7), (32, 64, 32 * 7), (32, 64, 32 * 310 + 1), (64, 64, 64 * 160 + 33), (64, 64, 8),
-          (128, 64, 128 * 5 + 3), (64, 128, 64 * 9 + 1)]
+          (32, 128, 32 * 160 + 9), (32, 128, 17), (128, 64, 128 * 5 + 3), (64, 128, 64 * 9 + 1)]
 
 
 def _close(got, want, what, rel=1e-2):
@@ -68,7 +68,7 @@ def test_step(layer, loss, B):
             _close(sh.w, inp["W"].float() - lr * sh.mom_w.cpu(), "weights")
 
 
-@pytest.mark.parametrize("layer", [(32, 32, 32 * 5), (32, 64, 32 * 5), (64, 64, 64 * 3), (128, 64, 128 * 3), (64, 128, 64 * 3)])
+@pytest.mark.parametrize("layer", [(32, 32, 32 * 5), (32, 64, 32 * 5), (32, 128, 32 * 5), (64, 64, 64 * 3), (128, 64, 128 * 3), (64, 128, 64 * 3)])
 def test_step_bce_gradient_of_very_negative_logits(layer):
     """Logits around -12: the gradient is sigmoid(z) = 6e-6 and its sum over the batch has to be right to bf16, which an
     absolute error of the sigmoid would destroy (batch 100: the shapes and sizes that compute it with exp)."""
@@ -115,7 +115,7 @@ def _check_topk(vals, idx, z, k, label0):
     dict(B=1, L=131073, F=128, G=64, k=5), dict(B=1, L=40, F=16, G=16, k=128), dict(B=3, L=5000, F=32, G=32, k=100),
     dict(B=8, L=70001, F=64, G=128, k=50), dict(B=7, L=300007, F=32, G=32, k=128),
     dict(B=9, L=16385, F=32, G=32, k=10), dict(B=40, L=160001, F=32, G=32, k=100), dict(B=200, L=40003, F=64, G=128, k=100),
-    dict(B=130, L=30000, F=128, G=64, k=1), dict(B=17, L=20011, F=64, G=64, k=128), dict(B=16, L=20011, F=64, G=32, k=7),
+    dict(B=130, L=30000, F=128, G=64, k=1), dict(B=17, L=20011, F=64, G=64, k=128), dict(B=16, L=20011, F=64, G=32, k=7), dict(B=16, L=20011, F=128, G=32, k=20),
 ], ids=lambda c: "-".join(f"{n}{v}" for n, v in c.items()))
 def test_topk_fused(cfg):
     from haste_b200 import ffi
