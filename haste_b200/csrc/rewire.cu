@@ -49,9 +49,11 @@ __device__ __forceinline__ float regrow_value(uint64_t seed, uint32_t step, int6
 __device__ __forceinline__ float slot_score(const uint16_t* tile, int rows, int F, int k, int score_mode) {
   float acc = 0.f;
   if (score_mode == 0) {
+#pragma unroll 8
     for (int r = 0; r < rows; ++r) acc = __fadd_rn(acc, fabsf(bf16_bits_to_float(tile[r * F + k])));
     return __fdiv_rn(acc, static_cast<float>(rows));
   }
+#pragma unroll 8
   for (int r = 0; r < rows; ++r) acc = fmaxf(acc, fabsf(bf16_bits_to_float(tile[r * F + k])));
   return acc;
 }
@@ -157,6 +159,11 @@ __global__ void __launch_bounds__(SEL_THREADS) select_scan_kernel(uint32_t* __re
   for (int g = lo; g < hi; ++g) { const int c = static_cast<int>(eq[g]); eq[g] = static_cast<uint32_t>(run); run += c; }
 }
 
+// One block per label group; the group's weights are read once into shared memory and written once, in 16-byte pieces.
+// What bounds it is the chain of small steps between the two (score, rank, draw, sort), so each is kept short: 'unused' draws
+// are resolved by one warp that holds the whole index row in registers (one vote per draw, no block barrier; the first
+// draw of every pruned slot is computed in parallel beforehand), and re-initialisation and column permutation happen while
+// the weights are written out (a thread keeps the sources of its 8 columns in registers for all its rows).
 __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __restrict__ w, int32_t* __restrict__ loc, float* __restrict__ mom,
                                                                 int D, int F, int64_t L, int G, int64_t group0, int score_mode, int prune_mode,
                                                                 float threshold, int n_prune, const uint32_t* __restrict__ sel,
@@ -168,23 +175,24 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
   float* score = reinterpret_cast<float*>(smem + size_t(G) * F * 2);  // [F]
   int* cur = reinterpret_cast<int*>(score + F);                       // [F] index row being edited
   int* pruned = cur + F;                                              // [F]
-  int* src_of = pruned + F;                                           // [F] output position -> source slot
+  int* src_of = pruned + F;                                           // [F] output position -> source slot, or ~slot when its column is re-initialised
   const int tid = threadIdx.x;
   const int64_t g = blockIdx.x;
   const int64_t l0 = g * G;
   const int rows = static_cast<int>(imin64(G, L - l0));
   uint16_t* wg = w + l0 * F;
 
+#pragma unroll 4
   for (int i = tid; i < rows * F / 8; i += RW_THREADS)
     reinterpret_cast<uint4*>(tile)[i] = reinterpret_cast<const uint4*>(wg)[i];
-  if (tid < F) cur[tid] = loc[g * F + tid];
+  int mine = tid < F ? loc[g * F + tid] : 0;                          // this thread's slot of the index row
   __syncthreads();
 
-  if (tid < F) score[tid] = slot_score(tile, rows, F, tid, score_mode);
+  const float s = tid < F ? slot_score(tile, rows, F, tid, score_mode) : 0.f;
+  if (tid < F) score[tid] = s;
   __syncthreads();
+  int p = 0;
   if (tid < F) {
-    int p;
-    const float s = score[tid];
     if (prune_mode == 0) {
       p = s < threshold;
     } else if (prune_mode == 2) {
@@ -200,77 +208,111 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
       }
     } else {
       int rank = 0;
-      for (int j = 0; j < F; ++j) {
-        const float sj = score[j];
-        rank += (sj < s) || (sj == s && j < tid);
+      const float4* s4 = reinterpret_cast<const float4*>(score);
+#pragma unroll 4
+      for (int j = 0; j < F; j += 4) {
+        const float4 v = s4[j >> 2];
+        rank += (v.x < s || (v.x == s && j < tid)) + (v.y < s || (v.y == s && j + 1 < tid)) + (v.z < s || (v.z == s && j + 2 < tid)) +
+                (v.w < s || (v.w == s && j + 3 < tid));
       }
       p = rank < n_prune;
     }
-    pruned[tid] = p;
   }
-  __syncthreads();
-  int n_pruned = 0;
-  for (int k = 0; k < F; ++k) n_pruned += pruned[k];
+  const int n_pruned = __syncthreads_count(p);
   if (n_pruned == 0 && !regroup) return;
 
-  // ---- regrow
-  if (regrow_mode == 0) {
-    if (tid < F && pruned[tid]) cur[tid] = regrow_index(seed, step, group0 + g, tid, 0, D);
-    __syncthreads();
-  } else {
+  // ---- regrow: the first draw of every pruned slot
+  if (p) mine = regrow_index(seed, step, group0 + g, tid, 0, D);
+  if (tid < F) { cur[tid] = mine; pruned[tid] = p; }
+  __syncthreads();
+  if (regrow_mode != 0 && n_pruned != 0) {
     // 'unused': slots are served in ascending order; a candidate is rejected while any live slot of
     // the row (kept, or already re-grown) holds the same index.  After 64 rejections the search walks
     // upward from the last candidate, which ends within F+1 steps because at most F indices are taken.
-    int live = (tid < F) ? !pruned[tid] : 0;
-    for (int k = 0; k < F; ++k) {
-      if (!pruned[k]) continue;                       // uniform: read from shared memory
-      int v = 0;
-      bool found = false;
-      for (int t = 0; t < 64 && !found; ++t) {
-        v = regrow_index(seed, step, group0 + g, k, t, D);
-        const int clash = __syncthreads_or(live && cur[tid < F ? tid : 0] == v);
-        found = !clash;
+    if (tid < 32) {
+      constexpr int PER = 128 / 32;                     // F <= 128
+      int draw[PER], held[PER];                         // held: this lane's live indices (-1: none, never equal to a candidate)
+      bool pr[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int k = tid + 32 * i;
+        pr[i] = k < F && pruned[k];
+        draw[i] = k < F ? cur[k] : -1;
+        held[i] = pr[i] || k >= F ? -1 : draw[i];
       }
-      for (int t = 0; t <= F && !found; ++t) {
-        v = (v + 1) % D;
-        const int clash = __syncthreads_or(live && cur[tid < F ? tid : 0] == v);
-        found = !clash;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        for (unsigned todo = __ballot_sync(0xffffffffu, pr[i]); todo != 0u; todo &= todo - 1u) {
+          const int who = __ffs(todo) - 1, k = who + 32 * i;
+          auto clashes = [&](int v) {
+            bool c = false;
+#pragma unroll
+            for (int x = 0; x < PER; ++x) c |= held[x] == v;
+            return __any_sync(0xffffffffu, c) != 0;
+          };
+          int v = __shfl_sync(0xffffffffu, draw[i], who);
+          bool clash = clashes(v);
+          for (int t = 1; t < 64 && clash; ++t) {
+            v = regrow_index(seed, step, group0 + g, k, t, D);
+            clash = clashes(v);
+          }
+          for (int t = 0; t <= F && clash; ++t) {
+            v = (v + 1) % D;
+            clash = clashes(v);
+          }
+          if (tid == who) held[i] = v;
+        }
       }
-      if (tid == k) { cur[k] = v; live = 1; }
-      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (pr[i]) cur[tid + 32 * i] = held[i];
     }
+    __syncthreads();
   }
 
-  // ---- re-initialise pruned columns (all real rows of the group)
-  for (int i = tid; i < rows * F; i += RW_THREADS) {
-    const int r = i / F, k = i - r * F;
-    if (pruned[k]) {
-      uint16_t v = 0;
-      if (init_mode == 1) v = rn_bf16_bits(regrow_value(seed, step, group0 * G + l0 + r, k, bound));
-      tile[i] = v;
-    }
-  }
   // ---- regroup: stable sort of the index row, columns follow
   if (tid < F) {
     int pos = tid;
+    mine = cur[tid];
     if (regroup) {
       pos = 0;
-      const int64_t key = static_cast<int64_t>(cur[tid]) * 256 + tid;
-      for (int j = 0; j < F; ++j) pos += (static_cast<int64_t>(cur[j]) * 256 + j) < key;
+      const int4* c4 = reinterpret_cast<const int4*>(cur);
+#pragma unroll 4
+      for (int j = 0; j < F; j += 4) {
+        const int4 v = c4[j >> 2];
+        pos += (v.x < mine || (v.x == mine && j < tid)) + (v.y < mine || (v.y == mine && j + 1 < tid)) +
+               (v.z < mine || (v.z == mine && j + 2 < tid)) + (v.w < mine || (v.w == mine && j + 3 < tid));
+      }
     }
-    src_of[pos] = tid;
+    src_of[pos] = p ? ~tid : tid;
+    loc[g * F + pos] = mine;
   }
   __syncthreads();
-  if (tid < F) loc[g * F + tid] = cur[src_of[tid]];
-  for (int i = tid; i < rows * F; i += RW_THREADS) {
-    const int r = i / F, p = i - r * F;
-    wg[i] = tile[r * F + src_of[p]];
+  // ---- columns out: permuted, the pruned ones re-initialised (all real rows of the group)
+  const int chunks = F >> 3, rows_per = RW_THREADS / chunks;
+  if (tid < rows_per * chunks) {
+    const int c = tid % chunks;
+    int src[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) src[j] = src_of[c * 8 + j];
+#pragma unroll 2
+    for (int r = tid / chunks; r < rows; r += rows_per) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint32_t v = 0u;
+        if (src[j] >= 0) v = tile[r * F + src[j]];
+        else if (init_mode == 1) v = rn_bf16_bits(regrow_value(seed, step, group0 * G + l0 + r, ~src[j], bound));
+        if (j & 1) o[j >> 1] |= v << 16; else o[j >> 1] = v;
+      }
+      *reinterpret_cast<uint4*>(wg + static_cast<int64_t>(r) * F + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
   }
   if (mom != nullptr) {
     float* mg = mom + l0 * F;
     for (int r = 0; r < rows; ++r) {
       float v = 0.f;
-      if (tid < F) { const int s = src_of[tid]; v = pruned[s] ? 0.f : mg[r * F + s]; }
+      if (tid < F) { const int sl = src_of[tid]; v = sl < 0 ? 0.f : mg[r * F + sl]; }
       __syncthreads();
       if (tid < F) mg[r * F + tid] = v;
     }
