@@ -27,39 +27,50 @@ __global__ void __launch_bounds__(256) sr_round_kernel(const float* __restrict__
 // ---------------------------------------------------------------- SGD + SR on [rows, cols]
 // One thread owns 8 consecutive columns of one row when cols % 8 == 0 (one Philox call in the packed
 // stream, one 16-byte weight access), else one element.
+// The reference stream is bound by its integer work, one Philox4x32-10 per weight, so nothing else may cost per element: the
+// stream, momentum and rounding are template parameters, and the reference stream needs no row index, its counter being the
+// flat element index, of which only the lower 32 bits count.
+enum { SGD_RN = 0, SGD_REFERENCE = 1, SGD_PACKED = 2 };
+template <int RNG, bool MOM, bool CONTRACT>
 __global__ void __launch_bounds__(256) sgd_sr_vec8_kernel(uint16_t* __restrict__ w, const uint16_t* __restrict__ g, float* __restrict__ m,
-                                                          int64_t rows, int cols, int64_t row0, float lr, float wd, float mu,
-                                                          uint64_t seed, uint32_t step, uint32_t flags) {
-  const int c8n = cols >> 3;
-  const int64_t n8 = rows * c8n;
+                                                          int64_t n8, uint32_t c8n, int64_t row0, int64_t flat0, float lr, float wd, float mu,
+                                                          uint64_t seed, uint32_t step) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8; i += stride) {
-    const int64_t r = i / c8n;
-    const int c8 = static_cast<int>(i - r * c8n);
-    const int64_t off = r * cols + c8 * 8;
-    uint4 wv = *reinterpret_cast<const uint4*>(w + off);
+    const int64_t off = i * 8;
+    const uint4 wv = *reinterpret_cast<const uint4*>(w + off);
     const uint4 gv = __ldg(reinterpret_cast<const uint4*>(g + off));
-    uint32_t* wp = reinterpret_cast<uint32_t*>(&wv);
-    const uint32_t* gp = reinterpret_cast<const uint32_t*>(&gv);
+    const uint32_t wp[4] = {wv.x, wv.y, wv.z, wv.w}, gp[4] = {gv.x, gv.y, gv.z, gv.w};
     float mv[8];
-    if (m) {
+    if (MOM) {
       const float4 a = *reinterpret_cast<const float4*>(m + off), b = *reinterpret_cast<const float4*>(m + off + 4);
       mv[0] = a.x; mv[1] = a.y; mv[2] = a.z; mv[3] = a.w; mv[4] = b.x; mv[5] = b.y; mv[6] = b.z; mv[7] = b.w;
     }
-    uint4 rp = make_uint4(0, 0, 0, 0);
-    const bool sr = flags & HASTE_F_SR, packed = flags & HASTE_F_RNG_PACKED;
-    if (sr && packed) rp = rand_packed8(seed, step, row0 + r, c8);
+    uint32_t rnd[4] = {0u, 0u, 0u, 0u};                 // 8 x 16 random bits, two per word
+    if (RNG == SGD_PACKED) {
+      int64_t r;
+      uint32_t c8;
+      if (n8 < (int64_t(1) << 32)) { const uint32_t i32 = static_cast<uint32_t>(i), q = i32 / c8n; r = q; c8 = i32 - q * c8n; }
+      else { r = i / c8n; c8 = static_cast<uint32_t>(i - r * c8n); }
+      const uint4 rp = rand_packed8(seed, step, row0 + r, static_cast<int>(c8));
+      rnd[0] = rp.x; rnd[1] = rp.y; rnd[2] = rp.z; rnd[3] = rp.w;
+    } else if (RNG == SGD_REFERENCE) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint32_t r16 = 0;
-      if (sr) r16 = packed ? unpack16(rp, j) : rand16_reference(seed, (row0 + r) * cols + c8 * 8 + j);
-      const uint16_t wb = (wp[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-      const uint16_t gb = (gp[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-      const uint16_t nb = sgd_update_bits(wb, bf16_bits_to_float(gb), m ? &mv[j] : nullptr, lr, wd, mu, flags, r16);
-      wp[j >> 1] = (j & 1) ? ((wp[j >> 1] & 0xFFFFu) | (uint32_t(nb) << 16)) : ((wp[j >> 1] & 0xFFFF0000u) | nb);
+      for (int p = 0; p < 4; ++p)
+        rnd[p] = rand16_reference(seed, flat0 + off + 2 * p) | (rand16_reference(seed, flat0 + off + 2 * p + 1) << 16);
     }
-    *reinterpret_cast<uint4*>(w + off) = wv;
-    if (m) {
+    uint32_t o[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const float g0 = __uint_as_float(gp[p] << 16), g1 = __uint_as_float(gp[p] & 0xFFFF0000u);
+      const float w0 = __uint_as_float(wp[p] << 16), w1 = __uint_as_float(wp[p] & 0xFFFF0000u);
+      const float n0 = sgd_math<CONTRACT>(w0, g0, MOM ? &mv[2 * p] : nullptr, lr, wd, mu);
+      const float n1 = sgd_math<CONTRACT>(w1, g1, MOM ? &mv[2 * p + 1] : nullptr, lr, wd, mu);
+      if (RNG == SGD_RN) o[p] = rn_bf16_bits(n0) | (static_cast<uint32_t>(rn_bf16_bits(n1)) << 16);
+      else o[p] = __byte_perm(__float_as_uint(n0) + (rnd[p] & 0xFFFFu), __float_as_uint(n1) + (rnd[p] >> 16), 0x7632);   // the high halves
+    }
+    *reinterpret_cast<uint4*>(w + off) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (MOM) {
       *reinterpret_cast<float4*>(m + off) = make_float4(mv[0], mv[1], mv[2], mv[3]);
       *reinterpret_cast<float4*>(m + off + 4) = make_float4(mv[4], mv[5], mv[6], mv[7]);
     }
@@ -357,10 +368,20 @@ int launch_sgd_sr(void* w, const void* g, float* m, int64_t rows, int64_t cols, 
                   uint64_t seed, uint32_t step, uint32_t flags, cudaStream_t st) {
   if (rows * cols == 0) return HASTE_OK;
   const bool vec = (cols % 8 == 0) && aligned16(w) && aligned16(g) && (m == nullptr || aligned16(m));
-  if (vec)
-    sgd_sr_vec8_kernel<<<grid_for(rows * cols / 8, 256), 256, 0, st>>>((uint16_t*)w, (const uint16_t*)g, m, rows, int(cols), row0, lr, wd,
-                                                                       mu, seed, step, flags);
-  else
+  if (vec) {
+    const int rng = !(flags & HASTE_F_SR) ? SGD_RN : (flags & HASTE_F_RNG_PACKED) ? SGD_PACKED : SGD_REFERENCE;
+    const bool contract = flags & HASTE_F_CONTRACT;
+    const int64_t n8 = rows * cols / 8;
+#define HASTE_SGD(RNG, MOM, CON)                                                                                                          \
+  sgd_sr_vec8_kernel<RNG, MOM, CON><<<grid_for(n8, 256), 256, 0, st>>>((uint16_t*)w, (const uint16_t*)g, m, n8, static_cast<uint32_t>(cols / 8), \
+                                                                       row0, row0 * cols, lr, wd, mu, seed, step)
+#define HASTE_SGD_RNG(MOM, CON)                                                                                       \
+  { if (rng == SGD_PACKED) HASTE_SGD(SGD_PACKED, MOM, CON); else if (rng == SGD_REFERENCE) HASTE_SGD(SGD_REFERENCE, MOM, CON); else HASTE_SGD(SGD_RN, MOM, CON); }
+    if (m != nullptr) { if (contract) HASTE_SGD_RNG(true, true) else HASTE_SGD_RNG(true, false) }
+    else { if (contract) HASTE_SGD_RNG(false, true) else HASTE_SGD_RNG(false, false) }
+#undef HASTE_SGD_RNG
+#undef HASTE_SGD
+  } else
     sgd_sr_scalar_kernel<<<grid_for(rows * cols, 256), 256, 0, st>>>((uint16_t*)w, (const uint16_t*)g, m, rows, int(cols), row0, lr, wd,
                                                                      mu, seed, step, flags);
   return check_launch("sgd_sr_kernel");
