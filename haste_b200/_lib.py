@@ -49,6 +49,8 @@ SIGNATURES = {
     "haste_topk_update": [P, I64, I64, I64, I64, I32, P, P, P],
     "haste_ffi_topk": [P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, I32, I64, P, P, P],
     "haste_transpose_bf16_ldx": [P, P, I64, I64, I64, P],
+    "haste_transpose_f32_ldx": [P, P, I64, I64, I64, P],
+    "haste_dxt_to_dx_sr_f32": [P, P, I64, I64, U64, P],
     "haste_ffi_forward_ldx": [P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, I64, P],
     "haste_ffi_backward_weights_ldx": [P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, P],
     "haste_ffi_backward_ldx": [P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, U32, I64, P],

@@ -312,7 +312,22 @@ int haste_dxt_to_dx_sr(const float* dxt, void* dx, int64_t B, int64_t D, uint64_
   const char* who = "haste_dxt_to_dx_sr";
   REQUIRE_PTR(dxt, who); REQUIRE_PTR(dx, who);
   if (B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad shape", who);
-  return launch_dxt_to_dx(dxt, dx, B, D, seed, static_cast<cudaStream_t>(stream));
+  return launch_dxt_to_dx(dxt, dx, B, D, seed, false, static_cast<cudaStream_t>(stream));
+}
+
+int haste_dxt_to_dx_sr_f32(const float* dxt, float* dx, int64_t B, int64_t D, uint64_t seed, haste_stream_t stream) {
+  const char* who = "haste_dxt_to_dx_sr_f32";
+  REQUIRE_PTR(dxt, who); REQUIRE_PTR(dx, who);
+  if (B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad shape", who);
+  return launch_dxt_to_dx(dxt, dx, B, D, seed, true, static_cast<cudaStream_t>(stream));
+}
+
+int haste_transpose_f32_ldx(const float* x, void* xt, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream) {
+  const char* who = "haste_transpose_f32_ldx";
+  if (int rc = check_ldxt(who, B, ldxt)) return rc;
+  REQUIRE_PTR(x, who); REQUIRE_PTR(xt, who);
+  if (B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad shape", who);
+  return launch_transpose(x, xt, B, D, ldxt, true, static_cast<cudaStream_t>(stream));
 }
 
 int haste_transpose_bf16(const void* x, void* xt, int64_t B, int64_t D, haste_stream_t stream) {
@@ -324,7 +339,7 @@ int haste_transpose_bf16_ldx(const void* x, void* xt, int64_t B, int64_t D, int6
   if (int rc = check_ldxt(who, B, ldxt)) return rc;
   REQUIRE_PTR(x, who); REQUIRE_PTR(xt, who);
   if (B < 1 || D < 1) return fail(HASTE_ERR_BAD_ARG, "%s: bad shape", who);
-  return launch_transpose(x, xt, B, D, ldxt, static_cast<cudaStream_t>(stream));
+  return launch_transpose(x, xt, B, D, ldxt, false, static_cast<cudaStream_t>(stream));
 }
 
 int haste_ffi_rewire(void* w, int32_t* loc, float* mom_w, int64_t D, int64_t F, int64_t L, int64_t G, int64_t group0, int32_t prune_mode,

@@ -94,7 +94,9 @@ __global__ void __launch_bounds__(256) sgd_sr_scalar_kernel(uint16_t* __restrict
 }
 
 // ---------------------------------------------------------------- dxt [D,B] fp32 -> dx [B,D] bf16 (SR)
-__global__ void __launch_bounds__(256) dxt_to_dx_sr_kernel(const float* __restrict__ dxt, uint16_t* __restrict__ dx, int64_t B, int64_t D,
+// (F32: the rounded value is stored as fp32, for a caller whose activations are fp32 — the cast would be one more pass)
+template <bool F32>
+__global__ void __launch_bounds__(256) dxt_to_dx_sr_kernel(const float* __restrict__ dxt, void* __restrict__ dx, int64_t B, int64_t D,
                                                            uint64_t seed) {
   __shared__ float tile[32][33];
   const int64_t d0 = static_cast<int64_t>(blockIdx.x) * 32, b0 = static_cast<int64_t>(blockIdx.y) * 32;
@@ -108,18 +110,23 @@ __global__ void __launch_bounds__(256) dxt_to_dx_sr_kernel(const float* __restri
     const int64_t b = b0 + j, d = d0 + tx;
     if (b < B && d < D) {
       const int64_t flat = b * D + d;
-      dx[flat] = sr_bf16_bits(tile[tx][j], rand16_reference(seed, flat));
+      const uint16_t v = sr_bf16_bits(tile[tx][j], rand16_reference(seed, flat));
+      if (F32) static_cast<float*>(dx)[flat] = bf16_bits_to_float(v); else static_cast<uint16_t*>(dx)[flat] = v;
     }
   }
 }
 
-__global__ void __launch_bounds__(256) transpose_bf16_kernel(const uint16_t* __restrict__ x, uint16_t* __restrict__ xt, int64_t B, int64_t D, int64_t ldxt) {
+// (fp32 features are rounded to bf16, nearest even, on the way)
+__device__ __forceinline__ uint16_t as_bf16_bits(uint16_t v) { return v; }
+__device__ __forceinline__ uint16_t as_bf16_bits(float v) { return rn_bf16_bits(v); }
+template <class X>
+__global__ void __launch_bounds__(256) transpose_bf16_kernel(const X* __restrict__ x, uint16_t* __restrict__ xt, int64_t B, int64_t D, int64_t ldxt) {
   __shared__ uint16_t tile[32][34];
   const int64_t d0 = static_cast<int64_t>(blockIdx.x) * 32, b0 = static_cast<int64_t>(blockIdx.y) * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int j = ty; j < 32; j += 8) {
     const int64_t b = b0 + j, d = d0 + tx;
-    tile[j][tx] = (b < B && d < D) ? x[b * D + d] : uint16_t(0);
+    tile[j][tx] = (b < B && d < D) ? as_bf16_bits(x[b * D + d]) : uint16_t(0);
   }
   __syncthreads();
   for (int j = ty; j < 32; j += 8) {
@@ -387,15 +394,16 @@ int launch_sgd_sr(void* w, const void* g, float* m, int64_t rows, int64_t cols, 
   return check_launch("sgd_sr_kernel");
 }
 
-int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t seed, cudaStream_t st) {
+int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t seed, bool f32, cudaStream_t st) {
   dim3 grid(static_cast<unsigned>((D + 31) / 32), static_cast<unsigned>((B + 31) / 32));
-  dxt_to_dx_sr_kernel<<<grid, 256, 0, st>>>(dxt, (uint16_t*)dx, B, D, seed);
+  (f32 ? dxt_to_dx_sr_kernel<true> : dxt_to_dx_sr_kernel<false>)<<<grid, 256, 0, st>>>(dxt, dx, B, D, seed);
   return check_launch("dxt_to_dx_sr_kernel");
 }
 
-int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st) {
+int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, bool f32, cudaStream_t st) {
   dim3 grid(static_cast<unsigned>((D + 31) / 32), static_cast<unsigned>((ldxt + 31) / 32));
-  transpose_bf16_kernel<<<grid, 256, 0, st>>>((const uint16_t*)x, (uint16_t*)xt, B, D, ldxt);
+  if (f32) transpose_bf16_kernel<<<grid, 256, 0, st>>>((const float*)x, (uint16_t*)xt, B, D, ldxt);
+  else transpose_bf16_kernel<<<grid, 256, 0, st>>>((const uint16_t*)x, (uint16_t*)xt, B, D, ldxt);
   return check_launch("transpose_bf16_kernel");
 }
 

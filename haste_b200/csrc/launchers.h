@@ -67,8 +67,10 @@ int launch_train_step(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
 int launch_sr_round(const float* x, void* out, int64_t n, uint64_t seed, cudaStream_t st);
 int launch_sgd_sr(void* w, const void* g, float* m, int64_t rows, int64_t cols, int64_t row0, float lr, float wd, float mu, uint64_t seed,
                   uint32_t step, uint32_t flags, cudaStream_t st);
-int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t seed, cudaStream_t st);
-int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, cudaStream_t st);
+// f32: dx receives the rounded values as fp32
+int launch_dxt_to_dx(const float* dxt, void* dx, int64_t B, int64_t D, uint64_t seed, bool f32, cudaStream_t st);
+// f32: x is fp32, rounded to bf16 on the way
+int launch_transpose(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, bool f32, cudaStream_t st);
 int launch_targets_bucket(const int32_t* coo, int64_t nnz, int64_t label0, int64_t L, int64_t G, int32_t* ptr, uint32_t* ent,
                           int32_t* scratch, cudaStream_t st);
 int launch_targets_bucket_noalloc(const int32_t* coo, int64_t nnz, int64_t label0, int64_t L, int64_t G, int32_t* ptr, uint32_t* ent,

@@ -496,7 +496,7 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
   u64* cand = reinterpret_cast<u64*>(base + fs.cand);
   const char* wb = static_cast<const char*>(w);
   const char* bb = static_cast<const char*>(bias);
-  if (int rc = launch_transpose(x, xt, B, D, ldxt, st)) return rc;
+  if (int rc = launch_transpose(x, xt, B, D, ldxt, false, st)) return rc;
   const int64_t ldz = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
   const int64_t first = imin64(ldz, L);
   if (int rc = launch_forward(loc, xt, w, bias, z, B, D, F, first, G, ldz, (first + 7) / 8 * 8, ldxt, st)) return rc;

@@ -45,15 +45,15 @@ def transpose_bf16(x):
     return xt
 
 
-def transpose_padded(x):
-    """x^T as [D, ceil8(B)], zeros right of column B: 16-byte rows for the tensor maps whatever B is.  Functions below
-    that take ``B`` accept it as ``xt``."""
-    _req(x, "x", torch.bfloat16)
+def transpose_padded(x, f32=False):
+    """x^T in bf16 as [D, ceil8(B)], zeros right of column B: 16-byte rows for the tensor maps whatever B is.  Functions
+    below that take ``B`` accept it as ``xt``.  ``f32``: x is fp32 and is rounded on the way."""
+    _req(x, "x", torch.float32 if f32 else torch.bfloat16)
     B, D = x.shape
     ldx = (B + 7) // 8 * 8
     xt = torch.empty(D, ldx, dtype=torch.bfloat16, device=x.device)
     with torch.cuda.device(x.device):
-        check(lib.haste_transpose_bf16_ldx(_ptr(x), _ptr(xt), B, D, ldx, _stream(x)), "transpose_bf16")
+        check((lib.haste_transpose_f32_ldx if f32 else lib.haste_transpose_bf16_ldx)(_ptr(x), _ptr(xt), B, D, ldx, _stream(x)), "transpose_bf16")
     return xt
 
 
@@ -254,12 +254,13 @@ def sgd_sr_update(w, grad, mom, row0, lr, wd, mu, seed, step, flags):
               "sgd_sr_update")
 
 
-def dxt_to_dx_sr(dxt, seed=123):
+def dxt_to_dx_sr(dxt, seed=123, dtype=torch.bfloat16):
+    """dx [B, D]: the transpose, stochastically rounded to bf16 (``dtype`` torch.float32: the same values as fp32)."""
     _req(dxt, "dxt", torch.float32)
     D, B = dxt.shape
-    dx = torch.empty(B, D, dtype=torch.bfloat16, device=dxt.device)
+    dx = torch.empty(B, D, dtype=dtype, device=dxt.device)
     with torch.cuda.device(dxt.device):
-        check(lib.haste_dxt_to_dx_sr(_ptr(dxt), _ptr(dx), B, D, seed, _stream(dxt)), "dxt_to_dx_sr")
+        check((lib.haste_dxt_to_dx_sr_f32 if dtype == torch.float32 else lib.haste_dxt_to_dx_sr)(_ptr(dxt), _ptr(dx), B, D, seed, _stream(dxt)), "dxt_to_dx_sr")
     return dx
 
 

@@ -6,6 +6,12 @@ import torch
 from .. import ffi as _ffi
 
 
+def _input_gradient(dxt, dtype):
+    if dtype in (torch.bfloat16, torch.float32):
+        return _ffi.dxt_to_dx_sr(dxt, 123, dtype)
+    return _ffi.dxt_to_dx_sr(dxt, 123).to(dtype)
+
+
 class GroupFFIMulFunction(torch.autograd.Function):
     @staticmethod
     @torch.amp.custom_fwd(device_type="cuda")
@@ -14,8 +20,8 @@ class GroupFFIMulFunction(torch.autograd.Function):
         # The kernels compute in bf16 with fp32 accumulation; fp32 activations are cast at the boundary
         # (the reference's fp32 kernels silently compute in fp16, which is not imitated).
         ctx.in_dtype = features.dtype
-        feats = features if features.dtype == torch.bfloat16 else features.to(torch.bfloat16)
-        features_t = _ffi.transpose_padded(feats.contiguous())
+        feats = features if features.dtype in (torch.bfloat16, torch.float32) else features.to(torch.bfloat16)
+        features_t = _ffi.transpose_padded(feats.contiguous(), f32=feats.dtype == torch.float32)
         ctx.save_for_backward(features_t, weights, group_locations)
         ctx.gsize, ctx.batch = int(gsize), feats.shape[0]
         ctx.use_bias = bias is not None
@@ -35,16 +41,11 @@ class GroupFFIMulFunction(torch.autograd.Function):
             # both gradients from one pass over grad_output
             dxt, weight_gradient, bias_gradient = _ffi.backward_both(features_t, weights, group_locations, grad_output, gsize,
                                                                      want_dbias=bool(need_b), B=ctx.batch)
-            input_gradient = _ffi.dxt_to_dx_sr(dxt, 123)
-            if ctx.in_dtype != torch.bfloat16:
-                input_gradient = input_gradient.to(ctx.in_dtype)
-            return input_gradient, weight_gradient, None, bias_gradient, None
+            return _input_gradient(dxt, ctx.in_dtype), weight_gradient, None, bias_gradient, None
         if need_x:
             dxt = _ffi.backward_features(features_t, weights, group_locations, grad_output, gsize, B=ctx.batch)
             # bindings.py:44-50 of the reference: transpose, then stochastic rounding with the fixed seed 123
-            input_gradient = _ffi.dxt_to_dx_sr(dxt, 123)
-            if ctx.in_dtype != torch.bfloat16:
-                input_gradient = input_gradient.to(ctx.in_dtype)
+            input_gradient = _input_gradient(dxt, ctx.in_dtype)
         if need_w or need_b:
             weight_gradient, bias_gradient = _ffi.backward_weights(features_t, weights, group_locations, grad_output, gsize,
                                                                    want_dbias=True, B=ctx.batch)

@@ -323,6 +323,10 @@ int haste_ffi_topk_fused(const int32_t* loc, const void* x, const void* w, const
  * other calls need them to be zero.  dxt stays [D, B].  haste_ffi_forward_ldx takes zcols as haste_ffi_forward_into
  * does.  (No counterpart in the reference: its kernels take [D, B].) */
 int haste_transpose_bf16_ldx(const void* x, void* xt, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream);
+/* fp32 activations: x fp32 [B,D] rounded to bf16 (nearest even) while it is transposed, and the dX tail with its rounded
+ * values stored as fp32 — the casts of the two calls above without a pass of their own. */
+int haste_transpose_f32_ldx(const float* x, void* xt, int64_t B, int64_t D, int64_t ldxt, haste_stream_t stream);
+int haste_dxt_to_dx_sr_f32(const float* dxt, float* dx, int64_t B, int64_t D, uint64_t seed, haste_stream_t stream);
 int haste_ffi_forward_ldx(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z,
                           int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t zcols,
                           int64_t ldxt, haste_stream_t stream);

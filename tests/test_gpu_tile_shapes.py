@@ -84,6 +84,17 @@ def test_step_bce_gradient_of_very_negative_logits(layer):
     assert ((sh.mom_b.cpu().double() - want).abs() <= 2 ** -7 * want).all()          # two bf16 roundings of dY and its sum
 
 
+@pytest.mark.parametrize("B,D", [(1, 1), (33, 70), (64, 768)])
+def test_fp32_activations_are_cast_on_the_way(B, D):
+    from haste_b200 import ffi
+    x = torch.randn(B, D, generator=torch.Generator().manual_seed(1)).cuda()
+    assert torch.equal(ffi.transpose_padded(x, f32=True), ffi.transpose_padded(x.to(torch.bfloat16)))
+    dxt = x.t().contiguous()
+    assert torch.equal(ffi.dxt_to_dx_sr(dxt, 7, torch.float32), ffi.dxt_to_dx_sr(dxt, 7).float())
+    with pytest.raises(RuntimeError):
+        ffi.transpose_padded(x)
+
+
 # ------------------------------------------------------------------------------------------------ filtered top-k
 def _check_topk(vals, idx, z, k, label0):
     """Against the full logits z (float, -inf and NaN never selected): values, and ids that are distinct, point at a logit
