@@ -153,6 +153,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2_relu(float lo, float hi) {
   asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
+// Two fp32 operations in one instruction (the loss epilogue and with it the kernel is bound by instruction issue): each half
+// is rounded as the scalar operation rounds.  PAIRED = false: two scalar instructions.
+struct F2 { float x, y; };
+template <bool PAIRED>
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  if (!PAIRED) return {fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)};
+  F2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\tfma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 // v rounded to bf16 (nearest even), returned as fp32: converting (v, 0) to a bf16x2 word puts bf16(v) in the
 // upper half over a zero lower half, which is the fp32 image of the rounded value — no unpacking needed.
 __device__ __forceinline__ float round_bf16_as_f32(float v) {
@@ -181,6 +192,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE;
   constexpr int N_EA = C::N_EA, N_EB = C::N_EB, N_UP = C::N_UP, EA_COLS = C::EA_COLS, UPS = C::UPS;
+  // Paired fp32 instructions: 670 K labels, hinge, 266 -> 260 us; no gain for BCE, whose loop waits for the MUFU (2.8 M labels: 2,234
+  // against 2,243 us), and a loss at 128 slots (501 K labels: 352 against 364 us), where 64 registers per thread spill.
+  constexpr bool PAIRED = LOSS == HASTE_LOSS_SQHINGE && F == 64;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
 
   extern __shared__ uint8_t smem_raw[];
@@ -560,6 +574,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           if (!general) {
             float bce_prod = 1.f;
             float fl[4] = {0.f, 0.f, 0.f, 0.f};        // partial sums: no serial dependency through one accumulator
+            F2 fh[2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll
             for (int e8 = 0; e8 < CH; e8 += 8) {
               uint4 pk;
@@ -570,9 +585,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 // (1 + z) * 2s.  The max is left to the bf16 conversion.  The loss term max(0,1+z)^2 is accumulated
                 // as (x + |x|)^2 = (2 max(0,x))^2 and rescaled by 1/(4s)^2 once per tile.
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  x[i] = fmaf(gs2, round_bf16_as_f32(__uint_as_float(r[e8 + i])), gs2);   // logits are rounded to bf16 first, as the unfused forward stores them
-                  if (WITH_LOSS) { const float m2 = x[i] + fabsf(x[i]); fl[i & 3] = fmaf(m2, m2, fl[i & 3]); }
+                for (int i = 0; i < 8; i += 2) {
+                  // logits are rounded to bf16 first, as the unfused forward stores them
+                  const F2 z2 = {round_bf16_as_f32(__uint_as_float(r[e8 + i])), round_bf16_as_f32(__uint_as_float(r[e8 + i + 1]))};
+                  const F2 x2 = fma2<PAIRED>({gs2, gs2}, z2, {gs2, gs2});
+                  x[i] = x2.x; x[i + 1] = x2.y;
+                  if (WITH_LOSS) { const F2 m2 = {x2.x + fabsf(x2.x), x2.y + fabsf(x2.y)}; fh[(i >> 1) & 1] = fma2<PAIRED>(m2, m2, fh[(i >> 1) & 1]); }
                 }
                 pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
               } else if (LOSS == LOSS_BCE_EXP) {
@@ -603,7 +621,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             }
             if (WITH_LOSS) {
               if (LOSS != HASTE_LOSS_SQHINGE) { fast_loss += __log2f(bce_prod); tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]); }
-              else fast_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
+              else fast_loss += (fh[0].x + fh[0].y) + (fh[1].x + fh[1].y);
             }
           } else {
             const int nvalid = rows_real - (col0 + c16);           // columns of this chunk that are real labels
@@ -844,9 +862,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             for (int p = 0; p < NSL / 2; ++p) {
               const float g0 = __uint_as_float(g8[p] << 16), g1 = __uint_as_float(g8[p] & 0xFFFF0000u);
               const float w0 = __uint_as_float(w8[p] << 16), w1 = __uint_as_float(w8[p] & 0xFFFF0000u);
-              const float n0 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w0, g0), w0), n1 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w1, g1), w1);
+              const F2 wv = {w0, w1}, nv = fma2<PAIRED>({-u.lr, -u.lr}, fma2<PAIRED>({u.wd, u.wd}, wv, {g0, g1}), wv);
               const uint32_t rr = rnd[p];
-              const uint32_t s0b = __float_as_uint(n0) + (rr & 0xFFFFu), s1b = __float_as_uint(n1) + (rr >> 16);
+              const uint32_t s0b = __float_as_uint(nv.x) + (rr & 0xFFFFu), s1b = __float_as_uint(nv.y) + (rr >> 16);
               ob[p] = __byte_perm(s0b, s1b, 0x7632);              // high halves: s0b -> low 16 bits, s1b -> high 16 bits
             }
           } else {
