@@ -148,22 +148,28 @@ constexpr int64_t TF_FIRST = 16384, TF_GROW = 8;
 constexpr int TF_CAP = 8192;
 typedef unsigned long long u64;
 
-// The keys that can be among the k best of n: all that are not below the k-th largest of the threads' maxima (a key below
-// it has k better ones).  key(i) for i < n, 0 = no entry; non-zero keys are distinct.  At most k * ceil(n / NT) pass.
-// Returns their number; all threads call it, and it ends with a barrier.
+// The keys that can be among the k best of n: all that are not below the k-th largest of the maxima of NT / lanes groups of
+// `lanes` threads (a key below it has k better ones).  key(i) for i < n, 0 = no entry; non-zero keys are distinct.  At most
+// k * ceil(n / NT) * lanes pass.  Ranking the maxima takes NT / lanes steps of every thread, so a small k takes few groups
+// (keep_lanes).  Returns the number kept; all threads call it, and it ends with a barrier.
 template <int NT, class KEY>
-__device__ __forceinline__ int keep_candidates(KEY key, int n, int k, u64* out, u64* s_max, u64* s_tau, int* s_n) {
+__device__ __forceinline__ int keep_candidates(KEY key, int n, int k, int lanes, u64* out, u64* s_max, u64* s_tau, int* s_n) {
   const int tid = threadIdx.x;
   u64 m = 0;
 #pragma unroll 4
   for (int i = tid; i < n; i += NT) { const u64 v = key(i); m = v > m ? v : m; }
-  s_max[tid] = m;
+  for (int o = 1; o < lanes; o <<= 1) { const u64 v = __shfl_xor_sync(0xffffffffu, m, o); m = v > m ? v : m; }
+  const int groups = NT / lanes;
+  if (tid % lanes == 0) s_max[tid / lanes] = m;
   if (tid == 0) { *s_tau = 0; *s_n = 0; }
   __syncthreads();
-  int rank = 0;
+  if (tid < groups) {
+    const u64 mine = s_max[tid];
+    int rank = 0;
 #pragma unroll 8
-  for (int j = 0; j < NT; ++j) rank += s_max[j] > m;
-  if (m != 0 && rank == k - 1) *s_tau = m;
+    for (int j = 0; j < groups; ++j) rank += s_max[j] > mine;
+    if (mine != 0 && rank == k - 1) *s_tau = mine;
+  }
   __syncthreads();
   const u64 tau = *s_tau;
 #pragma unroll 4
@@ -174,7 +180,13 @@ __device__ __forceinline__ int keep_candidates(KEY key, int n, int k, u64* out, 
   __syncthreads();
   return *s_n;
 }
-static int64_t keep_bound(int64_t n, int k, int nt) { return static_cast<int64_t>(k) * ((n + nt - 1) / nt); }
+// Threads per group: the most (a power of two up to a warp) that leave 2k groups and keep the bound on what passes small.
+static int keep_lanes(int64_t n, int k, int nt) {
+  int lanes = 1;
+  while (lanes < 32 && nt / (2 * lanes) >= (2 * k > 32 ? 2 * k : 32) && static_cast<int64_t>(k) * ((n + nt - 1) / nt) * 2 * lanes <= 2048) lanes *= 2;
+  return lanes;
+}
+static int64_t keep_bound(int64_t n, int k, int nt) { return static_cast<int64_t>(k) * ((n + nt - 1) / nt) * keep_lanes(n, k, nt); }
 
 // The k best of keys[0..s) in order, to vals / idx (label ids as in the keys; -inf / -1 where there are fewer); returns
 // nothing, writes *thr = the k-th value when thr != NULL.
@@ -201,18 +213,74 @@ __device__ __forceinline__ u64 logit_key(uint16_t bits, uint32_t label) {
   return v > -INFINITY ? topk_key(v, label) : 0ull;                 // -inf and NaN are never selected
 }
 
-// First chunk: the k best of z[b, 0..C), labels col0 + c; also the row's threshold and its empty candidate list.
+// First chunk: the k best of z[b, 0..C), labels col0 + c; also the row's threshold and its empty candidate list.  Rows are
+// 16-byte aligned and their length is that of whole chunks (the forward writes zeros past C, which are masked here).
+// The threads' maxima are found on packed bf16 pairs, eight logits per load; equal logits around the k-th maximum may let more
+// through than the list holds, and then the keys decide (which order equal logits by label).
+// The kernel with keys throughout took 33 us for 512 rows.
+__device__ __forceinline__ uint32_t max2u(uint32_t x, uint32_t y) {          // a NaN loses against a number
+  const __nv_bfloat162 v = __hmax2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float max8(const uint4& v) {
+  const uint32_t m = max2u(max2u(v.x, v.y), max2u(v.z, v.w));
+  return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
+}
 __global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* __restrict__ z, int64_t ldz, int C, uint32_t col0, int k,
-                                                                float* __restrict__ vals, int32_t* __restrict__ idx, float* __restrict__ thr,
-                                                                int* __restrict__ cnt) {
+                                                                int cap, float* __restrict__ vals, int32_t* __restrict__ idx,
+                                                                float* __restrict__ thr, int* __restrict__ cnt) {
   extern __shared__ __align__(16) u64 kept[];
   __shared__ u64 s_max[TF_THREADS], s_tau;
+  __shared__ __align__(16) float s_val[TF_THREADS];
+  __shared__ float s_cut;
   __shared__ int s_n;
+  const int tid = threadIdx.x;
   const int64_t b = blockIdx.x;
   const uint16_t* zr = z + b * ldz;
-  const int s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], col0 + i); }, C, k, kept, s_max, &s_tau, &s_n);
+  const uint4* z4 = reinterpret_cast<const uint4*>(zr);
+  const int whole = C >> 3;                                                  // chunks without a masked column
+  float m = -INFINITY;
+#pragma unroll 4
+  for (int c = tid; c < whole; c += TF_THREADS) m = fmaxf(m, max8(z4[c]));   // fmaxf drops a NaN
+  for (int c = whole * 8 + tid; c < C; c += TF_THREADS) m = fmaxf(m, bf16_bits_to_float(zr[c]));
+  s_val[tid] = m;
+  if (tid == 0) { s_cut = -INFINITY; s_n = 0; }
+  __syncthreads();
+  int rank = 0;
+#pragma unroll 8
+  for (int j = 0; j < TF_THREADS; j += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(s_val + j);
+    rank += (v.x > m || (v.x == m && j < tid)) + (v.y > m || (v.y == m && j + 1 < tid)) + (v.z > m || (v.z == m && j + 2 < tid)) +
+            (v.w > m || (v.w == m && j + 3 < tid));
+  }
+  if (rank == k - 1) s_cut = m;
+  __syncthreads();
+  const float cut = s_cut;
+  auto take = [&](uint16_t bits, int c) {
+    const float v = bf16_bits_to_float(bits);
+    if (v >= cut && v > -INFINITY) {
+      const int slot = atomicAdd(&s_n, 1);
+      if (slot < cap) kept[slot] = topk_key(v, col0 + static_cast<uint32_t>(c));
+    }
+  };
+#pragma unroll 4
+  for (int c = tid; c < whole; c += TF_THREADS) {
+    const uint4 v = z4[c];
+    if (max8(v) >= cut) {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) take(static_cast<uint16_t>(w[e >> 1] >> ((e & 1) * 16)), c * 8 + e);
+    }
+  }
+  for (int c = whole * 8 + tid; c < C; c += TF_THREADS) take(zr[c], c);
+  __syncthreads();
+  int s = s_n;
+  if (s > cap) {                                                             // uniform
+    __syncthreads();
+    s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], col0 + static_cast<uint32_t>(i)); }, C, k, 1, kept, s_max, &s_tau, &s_n);
+  }
   write_best<TF_THREADS>(kept, s, k, vals + b * k, idx + b * k, thr + b);
-  if (threadIdx.x == 0) cnt[b] = 0;
+  if (tid == 0) cnt[b] = 0;
 }
 
 // Merge: the row's kept list and its candidates -> kept list, threshold; the candidate list is emptied.
@@ -247,7 +315,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
   int s;
   if (n <= TF_CAP) {
     const u64* c = a.cand + b * TF_CAP;
-    s = keep_candidates<TF_THREADS>([&](int i) { return i < n ? c[i] : kept(i - n); }, n + k, k, keys, s_max, &s_tau, &s_n);
+    s = keep_candidates<TF_THREADS>([&](int i) { return i < n ? c[i] : kept(i - n); }, n + k, k, 1, keys, s_max, &s_tau, &s_n);
   } else {
     // every logit of the launch again: 256 threads take 256 / G groups at a time, one label each
     __shared__ float xs[TF_THREADS / 16][128];      // gathered features of these groups
@@ -288,7 +356,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
       }
       __syncthreads();
       if (s_list > TM_LIST - TF_THREADS) {          // uniform; room for one more round of labels is kept
-        const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, best, s_max, &s_tau, &s_n);
+        const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, 1, best, s_max, &s_tau, &s_n);
         for (int i = tid; i < m; i += TF_THREADS) {
           int rank = 0;
           for (int j = 0; j < m; ++j) rank += best[j] > best[i];
@@ -300,7 +368,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
         __syncthreads();
       }
     }
-    const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, best, s_max, &s_tau, &s_n);
+    const int m = keep_candidates<TF_THREADS>([&](int i) { return keys[i]; }, s_list, k, 1, best, s_max, &s_tau, &s_n);
     for (int i = tid; i < m; i += TF_THREADS) keys[i] = best[i];
     __syncthreads();
     s = m;
@@ -321,7 +389,7 @@ constexpr int TS_ROWS = 8, TS_UNIT = 16, TS_THREADS = 256, TS_SEG = 4096, TS_MER
 template <int F, int NB>
 __global__ void __launch_bounds__(TS_THREADS) topk_rows_kernel(const int32_t* __restrict__ loc, const uint16_t* __restrict__ x,
                                                                const uint16_t* __restrict__ w, const uint16_t* __restrict__ bias, int B, int D,
-                                                               int64_t L, int G, int seg, int k, uint32_t label0, u64* __restrict__ part) {
+                                                               int64_t L, int G, int seg, int k, uint32_t label0, int lanes, u64* __restrict__ part) {
   constexpr int LPR = F / 8, RPL = 32 / LPR, NLD = TS_UNIT / RPL > 0 ? TS_UNIT / RPL : 1;
   static_assert(RPL <= TS_UNIT && TS_UNIT % RPL == 0, "whole loads");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -376,7 +444,7 @@ __global__ void __launch_bounds__(TS_THREADS) topk_rows_kernel(const int32_t* __
   __syncthreads();
   for (int b = 0; b < B; ++b) {
     const uint16_t* zb = zs + b * seg;
-    const int s = keep_candidates<TS_THREADS>([&](int i) { return logit_key(zb[i], label0 + static_cast<uint32_t>(l_beg + i)); }, n_lab, k, kept,
+    const int s = keep_candidates<TS_THREADS>([&](int i) { return logit_key(zb[i], label0 + static_cast<uint32_t>(l_beg + i)); }, n_lab, k, lanes, kept,
                                               s_max, &s_tau, &s_n);
     u64* out = part + (static_cast<int64_t>(b) * gridDim.x + blockIdx.x) * k;
     for (int i = tid; i < k; i += TS_THREADS)
@@ -391,15 +459,16 @@ __global__ void __launch_bounds__(TS_THREADS) topk_rows_kernel(const int32_t* __
   }
 }
 
-__global__ void __launch_bounds__(TS_MERGE) topk_parts_kernel(const u64* __restrict__ part, int n, int k, float* __restrict__ vals,
-                                                              int32_t* __restrict__ idx) {
+template <int NT>
+__global__ void __launch_bounds__(NT) topk_parts_kernel(const u64* __restrict__ part, int n, int k, int lanes, float* __restrict__ vals,
+                                                        int32_t* __restrict__ idx) {
   extern __shared__ __align__(16) u64 kept[];
-  __shared__ u64 s_max[TS_MERGE], s_tau;
+  __shared__ u64 s_max[NT], s_tau;
   __shared__ int s_n;
   const int64_t b = blockIdx.x;
   const u64* p = part + b * n;
-  const int s = keep_candidates<TS_MERGE>([&](int i) { return p[i]; }, n, k, kept, s_max, &s_tau, &s_n);
-  write_best<TS_MERGE>(kept, s, k, vals + b * k, idx + b * k, nullptr);
+  const int s = keep_candidates<NT>([&](int i) { return p[i]; }, n, k, lanes, kept, s_max, &s_tau, &s_n);
+  write_best<NT>(kept, s, k, vals + b * k, idx + b * k, nullptr);
 }
 
 // ---------------------------------------------------------------- host side
@@ -424,7 +493,7 @@ static size_t rows_smem(int64_t B, int64_t D, int64_t seg, int k) {
 static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
   if (B <= TS_ROWS && (F == 16 || F == 32 || F == 64 || F == 128)) {
     const int64_t seg = rows_seg(L, G), parts = (L + seg - 1) / seg;
-    if (rows_smem(B, D, seg, k) <= 200 * 1024 && keep_bound(parts * k, k, TS_MERGE) * 8 <= 200 * 1024) return 1;
+    if (rows_smem(B, D, seg, k) <= 200 * 1024 && keep_bound(parts * k, k, parts * k <= 4096 ? TS_THREADS : TS_MERGE) * 8 <= 200 * 1024) return 1;
   }
   const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
   if (shape && B <= 65536 && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
@@ -471,7 +540,7 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
     auto kern = topk_rows_kernel<F_, NB_>;                                                                                   \
     if (int rc = allow_smem(kern, sm)) return rc;                                                                            \
     kern<<<static_cast<unsigned>(parts), TS_THREADS, sm, st>>>(loc, (const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)bias, int(B), int(D), L, \
-                                                               int(G), int(seg), k, static_cast<uint32_t>(label0), part);    \
+                                                               int(G), int(seg), k, static_cast<uint32_t>(label0), keep_lanes(seg, k, TS_THREADS), part);    \
   }
 #define HASTE_TOPK_ROWS_NB(F_)                                                                                               \
   { switch (pow2_rows(B)) { case 1: HASTE_TOPK_ROWS(F_, 1) break; case 2: HASTE_TOPK_ROWS(F_, 2) break; case 4: HASTE_TOPK_ROWS(F_, 4) break; \
@@ -480,9 +549,13 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
 #undef HASTE_TOPK_ROWS_NB
 #undef HASTE_TOPK_ROWS
     if (int rc = check_launch("topk_rows_kernel")) return rc;
-    const size_t sm2 = static_cast<size_t>(keep_bound(parts * k, k, TS_MERGE)) * 8;
-    if (int rc = allow_smem(topk_parts_kernel, sm2)) return rc;
-    topk_parts_kernel<<<static_cast<unsigned>(B), TS_MERGE, sm2, st>>>(part, int(parts * k), k, vals, idx);
+    // few keys: 256 threads (their barriers and ranks cost less); many: 1024, which also keep the bound on the candidates
+    const int64_t n = parts * k;
+    const int nt = n <= 4096 ? TS_THREADS : TS_MERGE;
+    auto merge = nt == TS_THREADS ? topk_parts_kernel<TS_THREADS> : topk_parts_kernel<TS_MERGE>;
+    const size_t sm2 = static_cast<size_t>(keep_bound(n, k, nt)) * 8;
+    if (int rc = allow_smem(merge, sm2)) return rc;
+    merge<<<static_cast<unsigned>(B), nt, sm2, st>>>(part, int(n), k, keep_lanes(n, k, nt), vals, idx);
     return check_launch("topk_parts_kernel");
   }
   if (route != 2) return fail(HASTE_ERR_UNSUPPORTED, "top-k: group size %lld, fan-in %lld, batch %lld take the chunked call", (long long)G, (long long)F, (long long)B);
@@ -500,9 +573,10 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
   const int64_t ldz = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
   const int64_t first = imin64(ldz, L);
   if (int rc = launch_forward(loc, xt, w, bias, z, B, D, F, first, G, ldz, (first + 7) / 8 * 8, ldxt, st)) return rc;
-  const size_t sm = static_cast<size_t>(keep_bound(first, k, TF_THREADS)) * 8;
+  const int cap = static_cast<int>(k * ((first + TF_THREADS - 1) / TF_THREADS));      // the bound of keep_candidates with single threads
+  const size_t sm = static_cast<size_t>(cap) * 8;
   if (int rc = allow_smem(topk_first_kernel, sm)) return rc;
-  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, sm, st>>>(z, ldz, int(first), static_cast<uint32_t>(label0), k, vals, idx, thr, cnt);
+  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, sm, st>>>(z, ldz, int(first), static_cast<uint32_t>(label0), k, cap, vals, idx, thr, cnt);
   if (int rc = check_launch("topk_first_kernel")) return rc;
   for (int64_t l0 = first; l0 < L;) {
     const int64_t n = imin64(TF_GROW * l0, L - l0), g0 = l0 / G;          // first is a multiple of G when there is more, so l0 always is
