@@ -3,6 +3,8 @@
 PyTorch is used for device memory and streams only.  Every function validates what the C side cannot
 see (device, dtype, contiguity) and raises RuntimeError otherwise.
 """
+import contextlib
+
 import torch
 
 from . import _lib
@@ -10,7 +12,16 @@ from ._lib import lib, check
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.device.index)
+
+
+_raw_stream = torch._C._cuda_getCurrentRawStream      # the cudaStream_t itself: no Stream object per call
+_STAY = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context with ``device`` current; nothing to enter when it is already (a call enters one for every launch)."""
+    return _STAY if torch.cuda.is_initialized() and torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
 
 
 def _req(t, name, dtype=None, contiguous=True):
@@ -40,7 +51,7 @@ def transpose_bf16(x):
     _req(x, "x", torch.bfloat16)
     B, D = x.shape
     xt = torch.empty(D, B, dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.haste_transpose_bf16(_ptr(x), _ptr(xt), B, D, _stream(x)), "transpose_bf16")
     return xt
 
@@ -52,7 +63,7 @@ def transpose_padded(x, f32=False):
     B, D = x.shape
     ldx = (B + 7) // 8 * 8
     xt = torch.empty(D, ldx, dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check((lib.haste_transpose_f32_ldx if f32 else lib.haste_transpose_bf16_ldx)(_ptr(x), _ptr(xt), B, D, ldx, _stream(x)), "transpose_bf16")
     return xt
 
@@ -68,7 +79,7 @@ def forward(loc, xt, w, bias, G, B=None):
     L, F = w.shape
     ldz = (L + 7) // 8 * 8
     z = torch.empty(B, ldz, dtype=torch.bfloat16, device=xt.device)
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_forward_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(z), B, D, F, L, G, ldz, ldz, ldx, _stream(xt)),
               "ffi_forward")
     return z.narrow(1, 0, L)
@@ -85,7 +96,7 @@ def forward_into(loc, xt, w, bias, G, out, col0):
     L, F = w.shape
     if out.dim() != 2 or out.shape[0] != B or out.stride(1) != 1 or col0 < 0 or col0 + L > out.shape[1]:
         raise RuntimeError(f"out must be [B={B}, >= {col0 + L}] with unit column stride")
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_forward_into(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), out.data_ptr() + 2 * col0, B, D, F, L, G,
                                          out.stride(0), L, _stream(xt)), "ffi_forward_into")
     return out
@@ -108,7 +119,7 @@ def backward_features(xt, w, loc, dy, G, B=None):
     L, F = w.shape
     dy, ldy = _rows(dy, L)
     dxt = torch.empty(D, B, dtype=torch.float32, device=w.device)
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         check(lib.haste_ffi_backward_features(_ptr(w), _ptr(loc), _ptr(dy), _ptr(dxt), B, D, F, L, G, ldy, _lib.F_ZERO_DXT,
                                               _stream(w)), "ffi_backward_features")
     return dxt
@@ -123,7 +134,7 @@ def backward_weights(xt, w, loc, dy, G, want_dbias=False, B=None):
     dy, ldy = _rows(dy, L)
     dw = torch.empty(L, F, dtype=torch.bfloat16, device=xt.device)
     db = torch.empty(L, dtype=torch.bfloat16, device=xt.device) if want_dbias else None
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_backward_weights_ldx(_ptr(xt), _ptr(loc), _ptr(dy), _ptr(dw), _ptr(db), B, D, F, L, G, ldy, ldx, _stream(xt)),
               "ffi_backward_weights")
     return (dw, db) if want_dbias else dw
@@ -138,7 +149,7 @@ def backward_both(xt, w, loc, dy, G, want_dbias=True, B=None):
     L, F = w.shape
     dy, ldy = _rows(dy, L)
     dev = xt.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         dxt = torch.empty(D, B, dtype=torch.float32, device=dev)
         dw = torch.empty(L, F, dtype=torch.bfloat16, device=dev)
         db = torch.empty(L, dtype=torch.bfloat16, device=dev) if want_dbias else None
@@ -152,7 +163,7 @@ def bww_sr_sgd(xt, loc, dy, w, bias, mom_w, mom_b, G, label0, lr, wd, mu, seed, 
     D, B = xt.shape
     L, F = w.shape
     dy, ldy = _rows(dy, L)
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_bww_sr_sgd(_ptr(xt), _ptr(loc), _ptr(dy), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b), B, D, F, L, G,
                                        ldy, label0, lr, wd, mu, seed, step, flags, _stream(xt)), "ffi_bww_sr_sgd")
 
@@ -163,7 +174,7 @@ def targets_bucket(coo, label0, L, G, tgt_ptr, tgt_ent, scratch):
     NG = (L + G - 1) // G
     if tgt_ptr.numel() < NG + 1 or scratch.numel() < NG or tgt_ent.numel() < nnz:
         raise RuntimeError("targets_bucket: output buffers too small")
-    with torch.cuda.device(coo.device):
+    with _on(coo.device):
         check(lib.haste_targets_bucket(_ptr(coo), nnz, label0, L, G, _ptr(tgt_ptr), _ptr(tgt_ent), _ptr(scratch), _stream(coo)),
               "targets_bucket")
 
@@ -175,7 +186,7 @@ def step_prepare(x, xt, dxt, loss, coo, label0, L, G, tgt_ptr, tgt_ent):
     nnz = coo.shape[0]
     if tgt_ent.numel() < nnz:
         raise RuntimeError("step_prepare: tgt_ent too small")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.haste_ffi_step_prepare(_ptr(x), _ptr(xt), _ptr(dxt), _ptr(loss), _ptr(coo), nnz, label0, L, G, _ptr(tgt_ptr),
                                          _ptr(tgt_ent), B, D, _stream(x)), "ffi_step_prepare")
 
@@ -205,7 +216,7 @@ def train_step(loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, G, l
     D, ldx = xt.shape
     B = ldx if B is None else B
     L, F = w.shape
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_train_step_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b), _ptr(tgt_ptr),
                                            _ptr(tgt_ent), _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd,
                                            mu, seed, step, flags, ldx, _stream(xt)), "ffi_train_step")
@@ -217,7 +228,7 @@ def step(x, coo, loc, xt, w, bias, mom_w, mom_b, tgt_ptr, tgt_ent, dxt, loss, G,
     the caller's, done once when the buffers are created).  ``xt``: work buffer [D, ldx], ldx >= B."""
     B, D = x.shape
     L, F = w.shape
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.haste_ffi_step_ldx(_ptr(x), _ptr(coo), coo.shape[0], _ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(mom_w), _ptr(mom_b),
                                  _ptr(tgt_ptr), _ptr(tgt_ent), _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd,
                                  mu, seed, step_no, flags, xt.shape[1], _stream(x)), "ffi_step")
@@ -231,7 +242,7 @@ def train_step_dbg(loc, xt, w, bias, tgt_ptr, tgt_ent, dxt, loss, G, label0, los
     z = torch.zeros(B, L, dtype=torch.bfloat16, device=xt.device)
     dw = torch.zeros(L, F, dtype=torch.bfloat16, device=xt.device)
     db = torch.zeros(L, dtype=torch.bfloat16, device=xt.device)
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_train_step_dbg(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), None, None, _ptr(tgt_ptr), _ptr(tgt_ent),
                                            _ptr(dxt), _ptr(loss), B, D, F, L, G, label0, loss_kind, grad_scale, lr, wd, 0.0, seed,
                                            step, flags, _ptr(z), L, _ptr(dw), _ptr(db) if bias is not None else None, _stream(xt)),
@@ -241,7 +252,7 @@ def train_step_dbg(loc, xt, w, bias, tgt_ptr, tgt_ent, dxt, loss, G, label0, los
 
 def sr_round(x, out, seed):
     _req(x, "x", torch.float32); _req(out, "output", torch.bfloat16)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         check(lib.haste_sr_round(_ptr(x), _ptr(out), x.numel(), seed, _stream(x)), "sr_round")
 
 
@@ -249,7 +260,7 @@ def sgd_sr_update(w, grad, mom, row0, lr, wd, mu, seed, step, flags):
     _req(w, "weights", torch.bfloat16); _req(grad, "gradient", torch.bfloat16)
     rows = w.shape[0] if w.dim() >= 1 else 1
     cols = w.numel() // max(rows, 1) if w.dim() >= 2 else 1
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         check(lib.haste_sgd_sr_update(_ptr(w), _ptr(grad), _ptr(mom), rows, cols, row0, lr, wd, mu, seed, step, flags, _stream(w)),
               "sgd_sr_update")
 
@@ -259,7 +270,7 @@ def dxt_to_dx_sr(dxt, seed=123, dtype=torch.bfloat16):
     _req(dxt, "dxt", torch.float32)
     D, B = dxt.shape
     dx = torch.empty(B, D, dtype=dtype, device=dxt.device)
-    with torch.cuda.device(dxt.device):
+    with _on(dxt.device):
         check((lib.haste_dxt_to_dx_sr_f32 if dtype == torch.float32 else lib.haste_dxt_to_dx_sr)(_ptr(dxt), _ptr(dx), B, D, seed, _stream(dxt)), "dxt_to_dx_sr")
     return dx
 
@@ -267,7 +278,7 @@ def dxt_to_dx_sr(dxt, seed=123, dtype=torch.bfloat16):
 def rewire(w, loc, mom_w, D, G, group0, prune_mode, threshold, n_prune, regrow_mode, init_mode, regroup, seed, step, changed=None):
     _req(w, "weights", torch.bfloat16); _req(loc, "group_locations", torch.int32)
     L, F = w.shape
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         check(lib.haste_ffi_rewire(_ptr(w), _ptr(loc), _ptr(mom_w), D, F, L, G, group0, prune_mode, float(threshold), int(n_prune),
                                    regrow_mode, init_mode, int(bool(regroup)), seed, step, _ptr(changed), _stream(w)), "ffi_rewire")
 
@@ -293,21 +304,21 @@ class LayerwideSelect:
         self.ties = self.scratch[hi + 2 * 65536 + 4:hi + 2 * 65536 + 5]
 
     def begin(self):
-        with torch.cuda.device(self.w.device):
+        with _on(self.w.device):
             check(lib.haste_ffi_rewire_select_begin(_ptr(self.w), self.F, self.L, self.G, self.score_mode, _ptr(self.scratch), _stream(self.w)),
                   "rewire_select_begin")
 
     def refine(self, k_layer):
-        with torch.cuda.device(self.w.device):
+        with _on(self.w.device):
             check(lib.haste_ffi_rewire_select_refine(self.F, self.L, self.G, int(k_layer), _ptr(self.scratch), _stream(self.w)), "rewire_select_refine")
 
     def finish(self):
-        with torch.cuda.device(self.w.device):
+        with _on(self.w.device):
             check(lib.haste_ffi_rewire_select_finish(self.F, self.L, self.G, _ptr(self.scratch), _stream(self.w)), "rewire_select_finish")
 
     def apply(self, loc, mom_w, D, group0, tie_base, regrow_mode, init_mode, regroup, seed, step, changed=None):
         _req(loc, "group_locations", torch.int32)
-        with torch.cuda.device(self.w.device):
+        with _on(self.w.device):
             check(lib.haste_ffi_rewire_prepared(_ptr(self.w), _ptr(loc), _ptr(mom_w), D, self.F, self.L, self.G, group0, self.score_mode,
                                                 int(tie_base), regrow_mode, init_mode, int(bool(regroup)), seed, step, _ptr(self.scratch),
                                                 _ptr(changed), _stream(self.w)), "rewire_prepared")
@@ -321,7 +332,7 @@ def rewire_ex(w, loc, mom_w, D, G, group0, score_mode, prune_mode, threshold, n_
     NG = (L + G - 1) // G
     if prune_mode == 2 and scratch is None:
         scratch = torch.empty(rewire_scratch_words(NG, F), dtype=torch.int32, device=w.device)
-    with torch.cuda.device(w.device):
+    with _on(w.device):
         check(lib.haste_ffi_rewire_ex(_ptr(w), _ptr(loc), _ptr(mom_w), D, F, L, G, group0, score_mode, prune_mode, float(threshold), int(n_prune),
                                       regrow_mode, init_mode, int(bool(regroup)), seed, step, _ptr(scratch), _ptr(changed), _stream(w)),
               "ffi_rewire_ex")
@@ -337,7 +348,7 @@ def topk(loc, xt, w, bias, zbuf, groups_per_chunk, k, G, label0, vals, idx):
     D, ldx = xt.shape
     B = vals.shape[0]
     L, F = w.shape
-    with torch.cuda.device(xt.device):
+    with _on(xt.device):
         check(lib.haste_ffi_topk_ldx(_ptr(loc), _ptr(xt), _ptr(w), _ptr(bias), _ptr(zbuf), zbuf.stride(0), B, D, F, L, G, groups_per_chunk, k,
                                  label0, _ptr(vals), _ptr(idx), ldx, _stream(xt)), "ffi_topk")
 
@@ -350,7 +361,7 @@ def topk_fused(loc, x, w, bias, k, G, label0):
         _req(bias, "bias", torch.bfloat16)
     B, D = x.shape
     L, F = w.shape
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         n = lib.haste_ffi_topk_fused_scratch(B, D, F, L, G, k)
         if n == 0 or _ptr(loc) % 16 or _ptr(w) % 16:
             return None
@@ -368,11 +379,11 @@ def topk_update(z, C, col0, vals, idx):
     if z.dim() != 2 or z.stride(1) != 1:
         raise RuntimeError("logits must be [B, C] with unit column stride")
     B, k = vals.shape
-    with torch.cuda.device(z.device):
+    with _on(z.device):
         check(lib.haste_topk_update(_ptr(z), z.stride(0), B, C, col0, k, _ptr(vals), _ptr(idx), _stream(z)), "topk_update")
 
 
 def check_locations(loc, D):
     _req(loc, "group_locations", torch.int32)
-    with torch.cuda.device(loc.device):
+    with _on(loc.device):
         check(lib.haste_ffi_check_locations(_ptr(loc), loc.numel(), D, _stream(loc)), "check_locations")
