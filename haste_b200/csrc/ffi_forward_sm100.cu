@@ -17,8 +17,8 @@
 //
 // The TOPK instantiations write no logits: the epilogue warps compare each logit (rounded to bf16, as it would have been
 // stored) with the k-th best value its row had before the launch and keep the few that beat it — expected k times the
-// ratio of labels in this launch to labels before it — as keys for the merge kernel in topk.cu.  A maximum tree over 16
-// packed logits decides per chunk whether anything passed; what did is collected in a list per warp in the shared
+// ratio of labels in this launch to labels before it — as keys for the merge kernel in topk.cu.  A maximum tree over 32
+// logits decides per chunk whether anything passed; what did is collected in a list per warp in the shared
 // memory the staging tiles would use, and flushed 32 entries at a time, so that the latency of the atomics on the
 // rows' counters is paid once per flush and not once per candidate.
 #include "common.cuh"
@@ -311,34 +311,38 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
           const bool ok = mbar_wait(bar(C::B_ZFULL + zs), (it >> 1) & 1, abort_flag, a.err, 27, WL);
           tc_fence_after();
           const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + zs * G + h * C::EC;
+          constexpr int CW = C::EC < 32 ? C::EC : 32;            // columns per TMEM load
 #pragma unroll 1
-          for (int c16 = 0; c16 < C::EC; c16 += 16) {
-            uint32_t r[16];
+          for (int c0 = 0; c0 < C::EC; c0 += CW) {
+            uint32_t r[CW];
             __syncwarp();
-            tmem_ld16(ta + c16, r);
+            tmem_ld(ta + c0, r);
             tmem_ld_wait();
-            uint32_t p[8];
+            uint32_t p[CW / 2], m[CW / 2];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) p[x] = pack2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
-            const uint32_t m = max2(max2(max2(p[0], p[1]), max2(p[2], p[3])), max2(max2(p[4], p[5]), max2(p[6], p[7])));
-            const float best = fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
+            for (int x = 0; x < CW / 2; ++x) m[x] = p[x] = pack2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
+#pragma unroll
+            for (int w = CW / 4; w > 0; w >>= 1)
+#pragma unroll
+              for (int x = 0; x < w; ++x) m[x] = max2(m[x], m[x + w]);
+            const float best = fmaxf(__uint_as_float(m[0] << 16), __uint_as_float(m[0] & 0xFFFF0000u));
             if (!__any_sync(0xffffffffu, best > thr)) continue;
-            const int col0 = h * C::EC + c16, nvalid = rows_real - col0;     // columns of this chunk that are real labels
+            const int col0 = h * C::EC + c0, nvalid = rows_real - col0;      // columns of this chunk that are real labels
             // bit x: column 2x (lower half of p[x]), bit 16 + x: column 2x + 1
             uint32_t hit = 0u;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) hit |= gt2_mask(p[x], thr2) & ((1u << x) | (0x10000u << x));
-            if (nvalid < 16) hit &= nvalid <= 0 ? 0u : ((1u << ((nvalid + 1) >> 1)) - 1u) | (((1u << (nvalid >> 1)) - 1u) << 16);
+            for (int x = 0; x < CW / 2; ++x) hit |= gt2_mask(p[x], thr2) & ((1u << x) | (0x10000u << x));
+            if (nvalid < CW) hit &= nvalid <= 0 ? 0u : ((1u << ((nvalid + 1) >> 1)) - 1u) | (((1u << (nvalid >> 1)) - 1u) << 16);
             if (!ok || *abort_flag) hit = 0u;
-            // One entry per lane and round; nearly always one round is enough.  (A prefix sum over the lanes' counts and
-            // sixteen predicated stores per lane took 181 us for 523 K labels and 512 rows; this takes the place of both.)
+            // One entry per lane and round; nearly always one round is enough.  (523 K labels, 512 rows: 148 us with 16-column
+            // loads; a prefix sum over the lanes' counts and sixteen predicated stores per lane in its place: 181 us.)
             for (unsigned any; (any = __ballot_sync(0xffffffffu, hit != 0u)) != 0u;) {
               if (count + 32 > CAPW) flush();
               if (hit != 0u) {
                 const int x = __ffs(hit) - 1;
                 uint32_t v = p[0];
 #pragma unroll
-                for (int y = 1; y < 8; ++y) v = (x & 15) == y ? p[y] : v;
+                for (int y = 1; y < CW / 2; ++y) v = (x & 15) == y ? p[y] : v;
                 const uint32_t bits = (x & 16) ? (v & 0xFFFF0000u) : (v << 16);
                 list[count + __popc(any & ((1u << lane) - 1u))] =
                     make_uint2(static_cast<uint32_t>(a.label0 + l0 + col0 + 2 * (x & 15) + (x >> 4)), bits | static_cast<uint32_t>(b));
