@@ -159,11 +159,25 @@ __global__ void __launch_bounds__(SEL_THREADS) select_scan_kernel(uint32_t* __re
   for (int g = lo; g < hi; ++g) { const int c = static_cast<int>(eq[g]); eq[g] = static_cast<uint32_t>(run); run += c; }
 }
 
+// Number of keys below `key` among n (n % 4 == 0, 16-byte aligned).
+__device__ __forceinline__ int rank_of(const uint32_t* keys, int n, uint32_t key) {
+  const uint4* k4 = reinterpret_cast<const uint4*>(keys);
+  int rank = 0;
+#pragma unroll 4
+  for (int j = 0; j < n; j += 4) {
+    const uint4 v = k4[j >> 2];
+    rank += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
+  }
+  return rank;
+}
+
 // One block per label group; the group's weights are read once into shared memory and written once, in 16-byte pieces.
 // What bounds it is the chain of small steps between the two (score, rank, draw, sort), so each is kept short: 'unused' draws
 // are resolved by one warp that holds the whole index row in registers (one vote per draw, no block barrier; the first
 // draw of every pruned slot is computed in parallel beforehand), and re-initialisation and column permutation happen while
-// the weights are written out (a thread keeps the sources of its 8 columns in registers for all its rows).
+// the weights are written out (a thread keeps the sources of its 8 columns in registers for all its rows).  501 K labels
+// (G=64, F=128): 302 us with block-wide rejection sampling and 2-byte stores, 153 us so, 105 us with one-integer ranks and masks
+// instead of branches per column (instruction issue was 70 % busy).
 __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __restrict__ w, int32_t* __restrict__ loc, float* __restrict__ mom,
                                                                 int D, int F, int64_t L, int G, int64_t group0, int score_mode, int prune_mode,
                                                                 float threshold, int n_prune, const uint32_t* __restrict__ sel,
@@ -186,6 +200,8 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
   for (int i = tid; i < rows * F / 8; i += RW_THREADS)
     reinterpret_cast<uint4*>(tile)[i] = reinterpret_cast<const uint4*>(wg)[i];
   int mine = tid < F ? loc[g * F + tid] : 0;                          // this thread's slot of the index row
+  __shared__ __align__(16) uint32_t key_s[RW_THREADS];
+  __shared__ uint32_t edge[2];
   __syncthreads();
 
   const float s = tid < F ? slot_score(tile, rows, F, tid, score_mode) : 0.f;
@@ -207,16 +223,26 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
         p = rank < static_cast<int64_t>(sel[1]);
       }
     } else {
-      int rank = 0;
-      const float4* s4 = reinterpret_cast<const float4*>(score);
-#pragma unroll 4
-      for (int j = 0; j < F; j += 4) {
-        const float4 v = s4[j >> 2];
-        rank += (v.x < s || (v.x == s && j < tid)) + (v.y < s || (v.y == s && j + 1 < tid)) + (v.z < s || (v.z == s && j + 2 < tid)) +
-                (v.w < s || (v.w == s && j + 3 < tid));
-      }
-      p = rank < n_prune;
+      p = -1;                                           // below
     }
+  }
+  if (prune_mode == 1) {
+    // Rank by one integer per slot, the score's upper 25 bits (scores are not negative) over the slot: two instructions a pair
+    // instead of five.  That decides unless the last slot pruned and the first one kept agree in those bits.
+    const uint32_t key = tid < F ? (__float_as_uint(s) & ~127u) | static_cast<uint32_t>(tid) : 0xFFFFFFFFu;
+    if (tid < F) key_s[tid] = key;
+    if (tid < 2) edge[tid] = tid;                       // distinct unless both are written below
+    const bool nan = __syncthreads_or(s != s) != 0;      // a NaN compares with nothing: the comparisons decide
+    const int rank = rank_of(key_s, F, key);
+    if (tid < F && n_prune > 0 && (rank == n_prune - 1 || rank == n_prune)) edge[rank - n_prune + 1] = key >> 7;
+    p = rank < n_prune;
+    __syncthreads();
+    if ((nan || (n_prune > 0 && n_prune < F && edge[0] == edge[1])) && tid < F) {
+      int exact = 0;
+      for (int j = 0; j < F; ++j) exact += score[j] < s || (score[j] == s && j < tid);
+      p = exact < n_prune;
+    }
+    if (tid >= F) p = 0;
   }
   const int n_pruned = __syncthreads_count(p);
   if (n_pruned == 0 && !regroup) return;
@@ -271,18 +297,19 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
   }
 
   // ---- regroup: stable sort of the index row, columns follow
+  if (tid < F) mine = cur[tid];
+  // index and slot in one integer where the indices allow it (anything else an index table may hold takes the long way)
+  const bool fits = __syncthreads_and(tid >= F || static_cast<uint32_t>(mine) < (1u << 24)) != 0;
+  const uint32_t order = (static_cast<uint32_t>(mine) << 7) | static_cast<uint32_t>(tid);
+  if (tid < F) key_s[tid] = order;
+  __syncthreads();
   if (tid < F) {
     int pos = tid;
-    mine = cur[tid];
-    if (regroup) {
+    if (regroup && fits) {
+      pos = rank_of(key_s, F, order);
+    } else if (regroup) {
       pos = 0;
-      const int4* c4 = reinterpret_cast<const int4*>(cur);
-#pragma unroll 4
-      for (int j = 0; j < F; j += 4) {
-        const int4 v = c4[j >> 2];
-        pos += (v.x < mine || (v.x == mine && j < tid)) + (v.y < mine || (v.y == mine && j + 1 < tid)) +
-               (v.z < mine || (v.z == mine && j + 2 < tid)) + (v.w < mine || (v.w == mine && j + 3 < tid));
-      }
+      for (int j = 0; j < F; ++j) pos += cur[j] < mine || (cur[j] == mine && j < tid);
     }
     src_of[pos] = p ? ~tid : tid;
     loc[g * F + pos] = mine;
@@ -292,18 +319,27 @@ __global__ void __launch_bounds__(RW_THREADS) ffi_rewire_kernel(uint16_t* __rest
   const int chunks = F >> 3, rows_per = RW_THREADS / chunks;
   if (tid < rows_per * chunks) {
     const int c = tid % chunks;
-    int src[8];
+    int src[8];                                         // source slot; a re-initialised column is masked away
+    uint32_t keep[4] = {0u, 0u, 0u, 0u};
+    int fresh = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) src[j] = src_of[c * 8 + j];
+    for (int j = 0; j < 8; ++j) {
+      src[j] = src_of[c * 8 + j];
+      if (src[j] >= 0) keep[j >> 1] |= 0xFFFFu << (16 * (j & 1));
+      else { src[j] = ~src[j]; fresh |= 1 << j; }
+    }
+    if (init_mode == 0) fresh = 0;
 #pragma unroll 2
     for (int r = tid / chunks; r < rows; r += rows_per) {
+      const uint16_t* row = tile + r * F;
       uint32_t o[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        uint32_t v = 0u;
-        if (src[j] >= 0) v = tile[r * F + src[j]];
-        else if (init_mode == 1) v = rn_bf16_bits(regrow_value(seed, step, group0 * G + l0 + r, ~src[j], bound));
-        if (j & 1) o[j >> 1] |= v << 16; else o[j >> 1] = v;
+      for (int j = 0; j < 4; ++j) o[j] = __byte_perm(row[src[2 * j]], row[src[2 * j + 1]], 0x5410) & keep[j];
+      if (fresh) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (fresh & (1 << j))
+            o[j >> 1] |= static_cast<uint32_t>(rn_bf16_bits(regrow_value(seed, step, group0 * G + l0 + r, src[j], bound))) << (16 * (j & 1));
       }
       *reinterpret_cast<uint4*>(wg + static_cast<int64_t>(r) * F + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     }

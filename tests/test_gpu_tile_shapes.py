@@ -95,6 +95,34 @@ def test_fp32_activations_are_cast_on_the_way(B, D):
         ffi.transpose_padded(x)
 
 
+@pytest.mark.parametrize("kind", ["near", "equal", "nan", "big_index"])
+def test_rewire_scores_that_one_integer_does_not_order(kind):
+    """Scores that agree in their upper 25 bits (near: they differ below; equal), NaN scores, and index tables with values
+    beyond 24 bits: the kernel then compares the scores and indices themselves."""
+    from haste_b200 import ffi
+    D, L, F, G, frac = 1 << (26 if kind == "big_index" else 9), 300, 64, 64, 0.3
+    gen = torch.Generator().manual_seed(3)
+    W = torch.full((L, F), 0.5, dtype=torch.bfloat16)
+    if kind == "near":
+        for l0 in range(0, L, G):
+            W[l0] = (2.0 ** -9 * (1 + torch.randperm(128, generator=gen)[:F] / 128.0)).to(torch.bfloat16)
+    elif kind == "nan":
+        W[::17, ::5] = float("nan")
+    elif kind == "big_index":
+        W = (torch.rand(L, F, generator=gen) - 0.5).to(torch.bfloat16)
+    NG = (L + G - 1) // G
+    loc0 = torch.randint(0, D, (NG, F), generator=gen, dtype=torch.int32)
+    w, loc = W.clone().cuda(), loc0.clone().cuda()
+    ffi.rewire(w, loc, None, D, G, 0, 1, 0.0, int(F * frac), 0, 0, True, 5, 1)
+    if kind == "nan":      # a NaN score compares with nothing, so its rank is 0 and its slot is pruned
+        want_zero = torch.stack([torch.isnan(W[g * G:(g + 1) * G].float()).any(0) for g in range(NG)])
+        zero = torch.stack([(w.cpu()[g * G:(g + 1) * G].float() == 0).all(0) for g in range(NG)])
+        assert not torch.isnan(w.float()).any() and (zero.sum(1) >= want_zero.sum(1)).all()
+        return
+    W1, loc1, _ = fo.rewire(W, loc0, G, D, "fraction", frac, None, init_mode="zero", regrow="replace", regroup=True, seed=5, step=1)
+    assert torch.equal(loc.cpu(), loc1) and torch.equal(w.cpu(), W1)
+
+
 # ------------------------------------------------------------------------------------------------ filtered top-k
 def _check_topk(vals, idx, z, k, label0):
     """Against the full logits z (float, -inf and NaN never selected): values, and ids that are distinct, point at a logit
