@@ -1,8 +1,8 @@
 // Grouped fixed-fan-in GEMM kernels on warp-level mma (m16n8k16 bf16, fp32 accumulate).
 //
-// These kernels serve every (G,F,B) shape: the forward, the backward entry points and the fused
-// step of the two benchmark layer shapes dispatch to the tcgen05 kernels, everything else (other
-// group sizes and fan-ins, batch sizes that are not multiples of 8, misaligned bases) runs here.
+// These kernels serve every (G,F,B) shape.  The layer shapes the tcgen05 kernels have tiles for ((128,64), (64,128), (64,64),
+// (32,64), (32,32), (32,128)) dispatch there when xt has 16-byte rows; everything else (other group sizes and fan-ins,
+// [D,B] features whose batch is not a multiple of 8, misaligned bases) runs here.
 // One device routine, warp_gemm_tn, serves all three products because the three
 // shared-memory tiles of a group can each play two roles without being transposed:
 //     Xs [F][BT]  gathered rows of xt (batch contiguous)

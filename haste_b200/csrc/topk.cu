@@ -496,7 +496,8 @@ static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int
     if (rows_smem(B, D, seg, k) <= 200 * 1024 && keep_bound(parts * k, k, parts * k <= 4096 ? TS_THREADS : TS_MERGE) * 8 <= 200 * 1024) return 1;
   }
   const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
-  if (shape && B <= 65536 && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
+  // (the candidate lists take 64 KiB a row: beyond a few thousand rows the chunked path needs less memory)
+  if (shape && B <= 8192 && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
   return 0;
 }
 
