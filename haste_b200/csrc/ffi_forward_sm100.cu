@@ -87,7 +87,7 @@ struct FwdArgs {
   // TOPK
   const float* thr;            // [B] current k-th best value of every row (-inf: none yet)
   unsigned long long* cand;    // [B][cap] keys of the logits that beat it
-  int* cnt;                    // [B] number of them, also beyond cap
+  int* cnt;                    // [B] number of them, also beyond cap; TopkFilter::CNT_STRIDE apart
   int cap, label0;
 };
 
@@ -291,11 +291,21 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
       int count = 0;                                         // warp-uniform
       auto flush = [&]() {
         __syncwarp();
-        for (int i = lane; i < count; i += 32) {
-          const uint2 e = list[i];
-          const int b = static_cast<int>(e.y & 0xFFFFu);
-          const int slot = atomicAdd(a.cnt + b, 1);
-          if (slot < a.cap) a.cand[static_cast<int64_t>(b) * a.cap + slot] = topk_key(__uint_as_float(e.y & 0xFFFF0000u), e.x);
+        for (int i0 = lane; i0 < count; i0 += 128) {         // four atomics per lane in flight
+          uint2 e[4];
+          int slot[4];
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            slot[x] = a.cap;
+            if (i0 + 32 * x < count) {
+              e[x] = list[i0 + 32 * x];
+              slot[x] = atomicAdd(a.cnt + static_cast<int64_t>(e[x].y & 0xFFFFu) * TopkFilter::CNT_STRIDE, 1);
+            }
+          }
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            if (slot[x] < a.cap)
+              a.cand[static_cast<int64_t>(e[x].y & 0xFFFFu) * a.cap + slot[x]] = topk_key(__uint_as_float(e[x].y & 0xFFFF0000u), e[x].x);
         }
         count = 0;
         __syncwarp();

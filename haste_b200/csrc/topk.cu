@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* 
     s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], col0 + static_cast<uint32_t>(i)); }, C, k, 1, kept, s_max, &s_tau, &s_n);
   }
   write_best<TF_THREADS>(kept, s, k, vals + b * k, idx + b * k, thr + b);
-  if (tid == 0) cnt[b] = 0;
+  if (tid == 0) cnt[b * TopkFilter::CNT_STRIDE] = 0;
 }
 
 // Merge: the row's kept list and its candidates -> kept list, threshold; the candidate list is emptied.
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
   const int64_t b = blockIdx.x;
   float* vals = a.vals + b * k;
   int32_t* idx = a.idx + b * k;
-  const int n = a.cnt[b];
+  const int n = a.cnt[b * TopkFilter::CNT_STRIDE];
   if (n == 0) return;                               // uniform: nothing beat the kept list
   auto kept = [&](int i) { const int id = idx[i]; return id < 0 ? 0ull : topk_key(vals[i], static_cast<uint32_t>(id)); };
   int s;
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
   }
   __syncthreads();
   write_best<TF_THREADS>(keys, s, k, vals, idx, a.thr + b);
-  if (tid == 0) a.cnt[b] = 0;
+  if (tid == 0) a.cnt[b * TopkFilter::CNT_STRIDE] = 0;
 }
 
 // ================================================================ a few rows: bandwidth-bound product on the CUDA cores
@@ -511,7 +511,7 @@ static FusedScratch fused_layout(int64_t B, int64_t D, int64_t L, int64_t G) {
   s.cand = round16(s.z + B * first * 2);
   s.thr = s.cand + (L > first ? B * TF_CAP * 8 : 0);
   s.cnt = round16(s.thr + B * 4);
-  s.total = round16(s.cnt + B * 4);
+  s.total = round16(s.cnt + B * 4 * TopkFilter::CNT_STRIDE);
   return s;
 }
 int64_t topk_fused_scratch_bytes(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
