@@ -545,7 +545,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_Z + zs * G + col0;
         const float gs2 = 2.f * gs;
         const float inv_gs2_sq = row_valid ? inv_4gs2_sq : 0.f;
-        const bool ragged = col0 + EA_COLS > rows_real;     // only the last tile of the layer can be ragged (and absent columns)
+        bool ragged = col0 + EA_COLS > rows_real;     // only the last tile of the layer can be ragged (and absent columns)
         float tile_loss = 0.f, fast_loss = 0.f;             // fast_loss: hinge (4s)^2-scaled squares, or BCE raw log2 terms
         const float hgs = 0.5f * gs;
         // 16 label columns per iteration.  Nearly every chunk has no positive label in the warp's 32 rows and no
@@ -554,6 +554,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         // (not unrolled: two iterations per loop body cost 27 % of the kernel's time, four 40 %, measured; moving the
         // general branch out of line, to shrink the loop instead, changed nothing)
         constexpr int CH = 16;                             // label columns per TMEM load
+        for (;;) {                                         // one pass; rarely a second (below)
 #pragma unroll 1
         for (int c16 = 0; c16 < EA_COLS; c16 += CH) {
           if (LS < G && col0 + c16 >= LS) {                // columns no tile of this shape has
@@ -589,31 +590,32 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   // logits are rounded to bf16 first, as the unfused forward stores them
                   const F2 z2 = {round_bf16_as_f32(__uint_as_float(r[e8 + i])), round_bf16_as_f32(__uint_as_float(r[e8 + i + 1]))};
                   const F2 x2 = fma2<PAIRED>({gs2, gs2}, z2, {gs2, gs2});
-                  x[i] = x2.x; x[i + 1] = x2.y;
+                  // (without the loss sum nothing would tell of a NaN: max drops it here)
+                  x[i] = WITH_LOSS ? x2.x : fmaxf(x2.x, 0.f); x[i + 1] = WITH_LOSS ? x2.y : fmaxf(x2.y, 0.f);
                   if (WITH_LOSS) { const F2 m2 = {x2.x + fabsf(x2.x), x2.y + fabsf(x2.y)}; fh[(i >> 1) & 1] = fma2<PAIRED>(m2, m2, fh[(i >> 1) & 1]); }
                 }
                 pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
               } else if (LOSS == LOSS_BCE_EXP) {
-                // dLoss/dz = s sigmoid(z) = s / (1 + e^-z); loss term softplus(z) = max(z,0) - ln(max(sigmoid, 1 - sigmoid)),
+                // dLoss/dz = s sigmoid(z) = s / (1 + e^-z); loss term softplus(z) = max(z,0) - ln(0.5 + |sigmoid - 0.5|),
                 // whose logarithm arguments lie in [0.5, 1] as below
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                   const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
                   const float sg = sigmoid_exp(zr);
                   x[i] = sg * gs;
-                  if (WITH_LOSS) { fl[i & 1] += zr; fl[2 + (i & 1)] += fabsf(zr); bce_prod *= fmaxf(sg, 1.f - sg); }
+                  if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bce_prod *= 0.5f + fabsf(sg - 0.5f); }
                 }
                 pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
               } else {
                 // dLoss/dz = s sigmoid(z) = s/2 + s/2 tanh(z/2) (one MUFU op, one fma); loss term softplus(z) =
-                // max(z,0) - ln(0.5 + 0.5 |tanh(z/2)|).  max(z,0) is summed as (z + |z|) / 2; the logarithm arguments
+                // max(z,0) - ln(0.5 + 0.5 |tanh(z/2)|).  The logarithm arguments
                 // lie in [0.5, 1], so the 16 of a chunk are multiplied together (>= 2^-16) and one log2 is taken.
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                   const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
                   const float th = tanh_approx(0.5f * zr);
                   x[i] = fmaf(hgs, th, hgs);
-                  if (WITH_LOSS) { fl[i & 1] += zr; fl[2 + (i & 1)] += fabsf(zr); bce_prod *= fmaf(0.5f, fabsf(th), 0.5f); }
+                  if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bce_prod *= fmaf(0.5f, fabsf(th), 0.5f); }
                 }
                 pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
               }
@@ -632,6 +634,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
               for (int i = 0; i < 8; ++i) {
                 const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
                 const uint32_t pos = (ym16 >> (e8 + i)) & 1u;
+                const float zs = __uint_as_float(__float_as_uint(zr) ^ (pos << 31));       // max(z,0) - y z = max(zs,0)
                 float gl, la;
                 if (LOSS == HASTE_LOSS_SQHINGE) {
                   // squared hinge with target sign s: dLoss/dz = -2 s max(0, 1 - s z); ns = -s is built from the target bit
@@ -643,14 +646,13 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   const float y = static_cast<float>(pos);
                   const float sg = sigmoid_exp(zr);
                   gl = (sg - y) * gs;
-                  la = 2.f * (fmaxf(zr, 0.f) - y * zr - 0.69314718f * __log2f(fmaxf(sg, 1.f - sg)));
+                  la = fmaxf(zs, 0.f) - 0.69314718f * __log2f(0.5f + fabsf(sg - 0.5f));
                 } else {
-                  // dLoss/dz = sigmoid(z) - y, loss = max(z,0) - y z - ln(0.5 + 0.5 |tanh(z/2)|); the factor 2 matches
-                  // the (z + |z|) sums of the other branch, halved once per tile
+                  // dLoss/dz = sigmoid(z) - y, loss = max(z,0) - y z - ln(0.5 + 0.5 |tanh(z/2)|)
                   const float y = static_cast<float>(pos);
                   const float th = tanh_approx(0.5f * zr);
                   gl = (fmaf(0.5f, th, 0.5f) - y) * gs;
-                  la = 2.f * (fmaxf(zr, 0.f) - y * zr - 0.69314718f * __log2f(fmaf(0.5f, fabsf(th), 0.5f)));
+                  la = fmaxf(zs, 0.f) - 0.69314718f * __log2f(fmaf(0.5f, fabsf(th), 0.5f));
                 }
                 if (e8 + i >= nvalid) { gl = 0.f; la = 0.f; }
                 if (WITH_LOSS) tile_loss += la;
@@ -666,14 +668,22 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             }
           }
         }
+        // Hinge: a logit that is infinite or NaN (a label masked by its bias) leaves x + |x| undefined, and in a row beyond the batch, where
+        // s = 0 and the logits are the biases, x itself.  Such a tile goes through the general branch, which has a value for it;
+        // so does one whose sum of squares overflows.  (max(x, 0) in place of x + |x| needs no second pass and took 1.6 % more
+        // of the 670 K step: 276.9 against 272.5 us; this way 274.3.  BCE sums max(z, 0): 2.8 M labels 2,310 against 2,320 us.)
+        if (LOSS != HASTE_LOSS_SQHINGE || !WITH_LOSS || DEBUG || ragged || !__any_sync(0xffffffffu, !(fast_loss < INFINITY))) break;
+        ragged = true;
+        tile_loss = fast_loss = 0.f;
+        }
         tc_fence_before();                             // this warp's part of the Z stage has been read
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
         if (WITH_LOSS && row_valid) {
-          // hinge: tile_loss holds plain squares, fast_loss (4s)^2-scaled ones; BCE: tile_loss holds twice the
+          // hinge: tile_loss holds plain squares, fast_loss (4s)^2-scaled ones; BCE: tile_loss holds the
           // max(z,0)-type terms, fast_loss raw log2 sums
           if (LOSS == HASTE_LOSS_SQHINGE) loss_acc += tile_loss + fast_loss * inv_gs2_sq;
-          else loss_acc += 0.5f * tile_loss - 0.69314718f * fast_loss;
+          else loss_acc += tile_loss - 0.69314718f * fast_loss;
         }
         fence_proxy_async();
         __syncwarp();

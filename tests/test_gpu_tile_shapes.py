@@ -191,3 +191,45 @@ def test_topk_fused_unusual_logits(kind, B):
     _check_topk(vals, idx, z, k, 0)
     if kind == "equal":
         assert torch.equal(idx.cpu(), torch.arange(k, dtype=torch.int32).expand(B, k))
+
+
+SHAPES = [(32, 32), (32, 64), (64, 64), (32, 128), (128, 64), (64, 128)]
+
+
+@pytest.mark.parametrize("mask", [float("-inf"), -3.0e38, -1.0e4])
+@pytest.mark.parametrize("B", [100, 128])
+@pytest.mark.parametrize("loss", ["bce", "squared_hinge"])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_step_with_masked_labels(G, F, loss, B, mask):
+    """A label masked by a very negative bias adds nothing to the loss and to dX and keeps its weights bit for bit, also where
+    the last batch tile has rows beyond the batch (their logits are the biases alone)."""
+    from haste_b200.fused import FusedFFIShard
+    D, L, scale = 264, 3 * G + 7, 0.5
+    inp = fo.make_inputs(B, D, L, F, G, 3, 1.1, seed=B + F, x_kind="normal", bias_zero=False)
+    masked = torch.zeros(L, dtype=torch.bool)
+    masked[::7] = True
+    targets = inp["targets"][~masked[inp["targets"][:, 1].long()]].contiguous()
+    z = fo.forward(inp["loc"], inp["X"], inp["W"], inp["bias"], G).double()
+    y = torch.zeros(B, L, dtype=torch.float64)
+    y[targets[:, 0].long(), targets[:, 1].long()] = 1.0
+    if loss == "bce":
+        term, dY = torch.nn.functional.softplus(z) - y * z, torch.sigmoid(z) - y
+    else:
+        s = 2.0 * y - 1.0
+        m = (1.0 - s * z).clamp_min(0.0)
+        term, dY = m * m, -2.0 * s * m
+    term[:, masked], dY[:, masked] = 0.0, 0.0
+    want_loss, dY = float(term.sum()) * scale, (dY * scale).to(torch.bfloat16)
+    bias = inp["bias"].clone()
+    bias[masked] = mask
+    want_x = fo.backward_features(inp["loc"], inp["W"], dY, G, D)
+    for with_loss in (True, False):
+        sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), bias.clone().cuda(), G, D, loss=loss, lr=0.05, seed=42, grad_scale=scale)
+        dxt, loss_dev = sh.step(inp["X"].cuda(), targets.cuda(), want_loss=with_loss)
+        # as test_step: the logits are bf16, some one rounding away from the oracle's
+        assert not with_loss or abs(float(loss_dev) - want_loss) <= 2e-3 * want_loss
+        _close(dxt, want_x, "dXt")
+        assert (fo._bf16_to_bits(sh.w.cpu()[masked]) == fo._bf16_to_bits(inp["W"][masked])).all()
+        if mask != float("-inf"):          # (an infinite bias does not survive an update: 0 * inf in the weight decay)
+            assert (fo._bf16_to_bits(sh.bias.cpu()[masked]) == fo._bf16_to_bits(bias[masked])).all()
+        assert not torch.equal(sh.w.cpu()[~masked], inp["W"][~masked])
