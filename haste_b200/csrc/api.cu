@@ -43,7 +43,10 @@ static bool train_step_sm100_supported(int64_t B, int64_t D, int64_t F, int64_t 
 int launch_train_step(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                       const UpdateArgs& u, int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int loss_kind, float grad_scale,
                       int64_t ldxt, cudaStream_t st, const StepDump* dump) {
-  if (train_step_sm100_supported(B, D, F, L, G, ldxt)) {
+  // The tcgen05 epilogue evaluates the hinge gradient as max(0, 2 s (1 + z)) and sums the squares of (4 s) (1 + z): s (grad_scale)
+  // has to be positive and its square far from the ends of fp32.  Its debug variant does neither.
+  const bool scale_ok = loss_kind != HASTE_LOSS_SQHINGE || dump != nullptr || (grad_scale >= 0x1p-40f && grad_scale <= 0x1p32f);
+  if (scale_ok && train_step_sm100_supported(B, D, F, L, G, ldxt)) {
     if (dump == nullptr && (G == 32 || (G == 64 && F == 64)))
       return launch_train_step_sm100_small(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, F, L, G, loss_kind, grad_scale, ldxt, g_max_ctas, st);
     if (G == 128) return launch_train_step_sm100_g128f64(loc, xt, tgt_ptr, tgt_ent, dxt, loss, u, B, D, L, loss_kind, grad_scale, ldxt, g_max_ctas, st, dump);

@@ -233,3 +233,19 @@ def test_step_with_masked_labels(G, F, loss, B, mask):
         if mask != float("-inf"):          # (an infinite bias does not survive an update: 0 * inf in the weight decay)
             assert (fo._bf16_to_bits(sh.bias.cpu()[masked]) == fo._bf16_to_bits(bias[masked])).all()
         assert not torch.equal(sh.w.cpu()[~masked], inp["W"][~masked])
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.5, 1e-22, 1e-9, 2.0 ** 40])
+@pytest.mark.parametrize("G,F", [(32, 32), (128, 64)])
+def test_hinge_step_with_any_gradient_scale(G, F, scale):
+    """The scale multiplies loss and gradients, also where its square leaves fp32 or it is not positive."""
+    from haste_b200.fused import FusedFFIShard
+    B, D, L = 100, 264, 3 * G + 7
+    inp = fo.make_inputs(B, D, L, F, G, 3, 1.1, seed=9, x_kind="normal", bias_zero=False)
+    ref = fo.train_step(inp["loc"], inp["X"], inp["W"], inp["bias"], inp["targets"], G, fo.LOSS_SQHINGE, 0.0, 0.0, 42)
+    sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss="squared_hinge", lr=0.0, seed=42,
+                       grad_scale=scale)
+    dxt, loss_dev = sh.step(inp["X"].cuda(), inp["targets"].cuda())
+    assert abs(float(loss_dev) - ref["loss"] * scale) <= 2e-3 * abs(ref["loss"] * scale)
+    want = ref["dXt"].double() * scale
+    assert float((dxt.cpu().double() - want).norm()) <= 1e-2 * float(want.norm())
