@@ -340,12 +340,11 @@ int launch_step_prepare(const void* x, void* xt, float* dxt, float* loss, const 
   const int64_t NG = (L + G - 1) / G;
   if (reinterpret_cast<uintptr_t>(coo) & 7) return fail(HASTE_ERR_BAD_ARG, "haste_ffi_step_prepare: the COO target pairs must start on an 8-byte boundary");
   const size_t sm = sizeof(int32_t) * static_cast<size_t>(NG);
-  if (sm > 200 * 1024) return fail(HASTE_ERR_TOO_LARGE, "haste_ffi_step_prepare: %lld label groups need more shared memory than one block has; "
+  if (sm > DYN_SMEM_MAX) return fail(HASTE_ERR_TOO_LARGE, "haste_ffi_step_prepare: %lld label groups need more shared memory than one block has; "
                                    "use haste_transpose_bf16 + haste_targets_bucket", (long long)NG);
   const bool vec = (ldxt % 8) == 0 && (D % 8) == 0 && aligned16(x) && aligned16(xt) && aligned16(dxt);
   auto k = vec ? step_prepare_kernel<true> : step_prepare_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  if (int rc = allow_dynamic_smem(k)) return rc;
   const int tiles_d = static_cast<int>(vec ? (D + 127) / 128 : (D + 31) / 32), tiles_b = static_cast<int>(vec ? (ldxt + 63) / 64 : (ldxt + 31) / 32);
   k<<<1 + tiles_d * tiles_b, PREP_THREADS, sm, st>>>((const uint16_t*)x, (uint16_t*)xt, dxt, loss, coo, nnz, label0, L, int(G), int(NG), ptr, ent, B, D,
                                                      ldxt, tiles_d);

@@ -489,13 +489,6 @@ static size_t step_smem(int G, int F) {
          size_t(BT) * (G + PAD) * 2;
 }
 
-template <class K>
-static int set_smem(K kernel, size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(e));
-  return HASTE_OK;
-}
-
 #define HASTE_DISPATCH_G(G, ...)                    \
   switch (G) {                                      \
     case 16: { constexpr int G_ = 16; __VA_ARGS__; } break;   \
@@ -518,7 +511,7 @@ int launch_forward(const int32_t* loc, const void* xt, const void* w, const void
   const size_t sm = fwd_smem(int(G), int(F));
   HASTE_DISPATCH_G(G, {
     auto k = ffi_forward_kernel<G_>;
-    if (int rc = set_smem(k, sm)) return rc;
+    if (int rc = allow_dynamic_smem(k)) return rc;
     k<<<grid, NT, sm, st>>>(loc, (const __nv_bfloat16*)xt, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)z, B,
                             int(D), int(F), L, ldz, zw, ldxt);
   });
@@ -532,7 +525,7 @@ int launch_bwd_features(const void* w, const int32_t* loc, const void* dy, float
   const size_t sm = bwx_smem(int(G), int(F));
   HASTE_DISPATCH_G(G, HASTE_DISPATCH_F(F, {
     auto k = ffi_bwd_features_kernel<G_, F_>;
-    if (int rc = set_smem(k, sm)) return rc;
+    if (int rc = allow_dynamic_smem(k)) return rc;
     k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)w, loc, (const __nv_bfloat16*)dy, dxt, B, int(D), int(F), L, ldy);
   }));
   return check_launch("ffi_bwd_features_kernel");
@@ -548,11 +541,11 @@ int launch_bwd_weights(const void* xt, const int32_t* loc, const void* dy, void*
   HASTE_DISPATCH_G(G, HASTE_DISPATCH_F(F, {
     if (upd) {
       auto k = ffi_bwd_weights_kernel<G_, F_, true>;
-      if (int rc = set_smem(k, sm)) return rc;
+      if (int rc = allow_dynamic_smem(k)) return rc;
       k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)xt, loc, (const __nv_bfloat16*)dy, nullptr, nullptr, u, B, int(D), int(F), L, ldy, ldxt);
     } else {
       auto k = ffi_bwd_weights_kernel<G_, F_, false>;
-      if (int rc = set_smem(k, sm)) return rc;
+      if (int rc = allow_dynamic_smem(k)) return rc;
       k<<<grid, NT, sm, st>>>((const __nv_bfloat16*)xt, loc, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dw, (__nv_bfloat16*)dbias, u, B,
                               int(D), int(F), L, ldy, ldxt);
     }
@@ -570,7 +563,7 @@ int launch_train_step_mma(const int32_t* loc, const void* xt, const int32_t* tgt
 #define HASTE_LAUNCH_STEP(LOSSK, WL)                                                                          \
   {                                                                                                           \
     auto k = ffi_train_step_mma_kernel<G_, F_, LOSSK, WL>;                                                    \
-    if (int rc = set_smem(k, sm)) return rc;                                                                  \
+    if (int rc = allow_dynamic_smem(k)) return rc;                                                                  \
     k<<<grid, NT, sm, st>>>(loc, (const __nv_bfloat16*)xt, tgt_ptr, tgt_ent, dxt, loss, u, B, int(D), int(F), L, grad_scale, ldxt); \
   }
   HASTE_DISPATCH_G(G, HASTE_DISPATCH_F(F, {

@@ -6,6 +6,19 @@
 
 namespace haste {
 
+// Dynamic shared memory of the kernels whose need depends on the call.  The limit that cudaFuncSetAttribute sets belongs to the
+// function (per device), not to a launch, and calls come from several threads: a limit of each call's own size could be lowered by
+// another thread between this thread's setting and its launch.  So every call sets the same constant, which leaves 27 KB of an
+// SM's 227 for static arrays; what a launch takes is still its own size.
+constexpr int DYN_SMEM_MAX = 200 * 1024;
+template <class K>
+int allow_dynamic_smem(K kernel) {
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
+  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute(%d B): %s", DYN_SMEM_MAX, cudaGetErrorString(e));
+  return HASTE_OK;
+}
+
+
 // Everything the fused weight/bias update needs.  mom_* are NULL when momentum is off.
 struct UpdateArgs {
   __nv_bfloat16* w;

@@ -380,8 +380,7 @@ int launch_rewire_select_begin(const void* w, int64_t F, int64_t L, int64_t G, i
   SelectScratch s = select_scratch(scratch, NG, F);
   cudaError_t e = cudaMemsetAsync(s.sel, 0, sizeof(uint32_t) * static_cast<size_t>(2 + NG + 2 * 65536 + 8), st);
   if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaMemsetAsync: %s", cudaGetErrorString(e));
-  e = cudaFuncSetAttribute(ffi_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(size_t(G) * F * 2));
-  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  if (int rc = allow_dynamic_smem(ffi_scores_kernel)) return rc;
   ffi_scores_kernel<<<static_cast<unsigned>(NG), RW_THREADS, size_t(G) * F * 2, st>>>((const uint16_t*)w, int(F), L, int(G), score_mode, s.scores, s.hist_hi);
   return check_launch("ffi_scores_kernel");
 }
@@ -417,8 +416,7 @@ int launch_rewire(void* w, int32_t* loc, float* mom, int64_t D, int64_t F, int64
                   void* scratch, int32_t* changed, cudaStream_t st, uint32_t tie_base) {
   const int64_t NG = (L + G - 1) / G;
   const size_t sm = size_t(G) * F * 2 + size_t(F) * 4 * 4;
-  cudaError_t e = cudaFuncSetAttribute(ffi_rewire_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
-  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  if (int rc = allow_dynamic_smem(ffi_rewire_kernel)) return rc;
   if (changed != nullptr) cudaMemsetAsync(changed, 0, sizeof(int32_t), st);
   const uint32_t* sel = nullptr;
   if (prune_mode == 2) {

@@ -493,7 +493,7 @@ static size_t rows_smem(int64_t B, int64_t D, int64_t seg, int k) {
 static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
   if (B <= TS_ROWS && (F == 16 || F == 32 || F == 64 || F == 128)) {
     const int64_t seg = rows_seg(L, G), parts = (L + seg - 1) / seg;
-    if (rows_smem(B, D, seg, k) <= 200 * 1024 && keep_bound(parts * k, k, parts * k <= 4096 ? TS_THREADS : TS_MERGE) * 8 <= 200 * 1024) return 1;
+    if (rows_smem(B, D, seg, k) <= DYN_SMEM_MAX && keep_bound(parts * k, k, parts * k <= 4096 ? TS_THREADS : TS_MERGE) * 8 <= DYN_SMEM_MAX) return 1;
   }
   const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
   // (the candidate lists take 64 KiB a row: beyond a few thousand rows the chunked path needs less memory)
@@ -522,13 +522,6 @@ int64_t topk_fused_scratch_bytes(int64_t B, int64_t D, int64_t F, int64_t L, int
   }
 }
 
-template <class K>
-static int allow_smem(K kernel, size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return fail(HASTE_ERR_LAUNCH, "cudaFuncSetAttribute(%zu B): %s", bytes, cudaGetErrorString(e));
-  return HASTE_OK;
-}
-
 int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t B, int64_t D, int64_t F, int64_t L,
                       int64_t G, int k, int64_t label0, float* vals, int32_t* idx, cudaStream_t st) {
   const int route = topk_route(B, D, F, L, G, k);
@@ -539,7 +532,7 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
 #define HASTE_TOPK_ROWS(F_, NB_)                                                                                             \
   {                                                                                                                          \
     auto kern = topk_rows_kernel<F_, NB_>;                                                                                   \
-    if (int rc = allow_smem(kern, sm)) return rc;                                                                            \
+    if (int rc = allow_dynamic_smem(kern)) return rc;                                                                            \
     kern<<<static_cast<unsigned>(parts), TS_THREADS, sm, st>>>(loc, (const uint16_t*)x, (const uint16_t*)w, (const uint16_t*)bias, int(B), int(D), L, \
                                                                int(G), int(seg), k, static_cast<uint32_t>(label0), keep_lanes(seg, k, TS_THREADS), part);    \
   }
@@ -555,7 +548,7 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
     const int nt = n <= 4096 ? TS_THREADS : TS_MERGE;
     auto merge = nt == TS_THREADS ? topk_parts_kernel<TS_THREADS> : topk_parts_kernel<TS_MERGE>;
     const size_t sm2 = static_cast<size_t>(keep_bound(n, k, nt)) * 8;
-    if (int rc = allow_smem(merge, sm2)) return rc;
+    if (int rc = allow_dynamic_smem(merge)) return rc;
     merge<<<static_cast<unsigned>(B), nt, sm2, st>>>(part, int(n), k, keep_lanes(n, k, nt), vals, idx);
     return check_launch("topk_parts_kernel");
   }
@@ -576,7 +569,7 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
   if (int rc = launch_forward(loc, xt, w, bias, z, B, D, F, first, G, ldz, (first + 7) / 8 * 8, ldxt, st)) return rc;
   const int cap = static_cast<int>(k * ((first + TF_THREADS - 1) / TF_THREADS));      // the bound of keep_candidates with single threads
   const size_t sm = static_cast<size_t>(cap) * 8;
-  if (int rc = allow_smem(topk_first_kernel, sm)) return rc;
+  if (int rc = allow_dynamic_smem(topk_first_kernel)) return rc;
   topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, sm, st>>>(z, ldz, int(first), static_cast<uint32_t>(label0), k, cap, vals, idx, thr, cnt);
   if (int rc = check_launch("topk_first_kernel")) return rc;
   for (int64_t l0 = first; l0 < L;) {
