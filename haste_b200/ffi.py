@@ -15,7 +15,12 @@ def _stream(t):
     return _raw_stream(t.device.index)
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream      # the cudaStream_t itself: no Stream object per call
+def _stream_object_handle(index):
+    return torch.cuda.current_stream(index).cuda_stream
+
+
+# the cudaStream_t itself, without a Stream object per call (absent from a torch without CUDA)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _stream_object_handle)
 _STAY = contextlib.nullcontext()
 
 

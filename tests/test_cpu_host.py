@@ -282,3 +282,12 @@ def test_pipeline_reserve_choice(built_lib):
     assert [choice(n, 512, 670091, 64) for n in (2, 4, 8)] == [8, 12, 16]           # 670K labels, B=512
     assert [choice(n, 1024, 2812281, 64) for n in (2, 4, 8)] == [8, 8, 8]           # 2.8M labels, B=1024: long kernels
     assert choice(16, 512, 670091, 64) == 16
+
+
+def test_import_with_a_torch_that_has_no_cuda(built_lib):
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda_')]: delattr(torch._C, name)\n"
+            "import haste_b200.ffi, haste_b200.fused, haste_b200.infer, haste_b200.shared_ffi\n"
+            "assert not torch.cuda.is_available()\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
