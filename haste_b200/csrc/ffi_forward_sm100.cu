@@ -15,8 +15,9 @@
 // warps 4-11 drain the accumulator: TMEM -> bf16 -> staging tile; one thread issues the store.
 // All waits are bounded (see mbar_wait).
 //
-// The TOPK instantiations write no logits: the epilogue warps compare each logit (rounded to bf16, as it would have been
-// stored) with the k-th best value its row had before the launch and keep the few that beat it — expected k times the
+// A launch may take every n-th label tile only (TileSet), which is how top-k samples a layer.  The TOPK instantiations write no
+// logits: the epilogue warps compare each logit (rounded to bf16, as it would have been
+// stored) with the k-th best its row had before the launch and keep the few that beat it — expected k times the
 // ratio of labels in this launch to labels before it — as keys for the merge kernel in topk.cu.  A maximum tree over 32
 // logits decides per chunk whether anything passed; what did is collected in a list per warp in the shared
 // memory the staging tiles would use, and flushed 32 entries at a time, so that the latency of the atomics on the
@@ -82,10 +83,11 @@ struct FwdArgs {
   __nv_bfloat16* z;
   int* err;
   int64_t B, L, ldz, zw;
-  int D, NG, NGR;      // NG: tiles of G labels; NGR: label groups
+  int D, NG, NGR;      // NG: tiles (of G labels) of this launch; NGR: label groups of the layer
+  TileSet set;
   long long wait_limit;
   // TOPK
-  const float* thr;            // [B] current k-th best value of every row (-inf: none yet)
+  const RowCut* cut;           // [B] current k-th best of every row
   unsigned long long* cand;    // [B][cap] keys of the logits that beat it
   int* cnt;                    // [B] number of them, also beyond cap; TopkFilter::CNT_STRIDE apart
   int cap, label0;
@@ -157,7 +159,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
     // issues its share of the gathers (four index rows per instruction, landing at their swizzled positions).
     int it = 0, w_armed = 0, my_last = -1;
     for (int gi = 0; gi < n_my_groups; ++gi) {
-      const int g = blockIdx.x + gi * gridDim.x;
+      const int g = a.set.tile(blockIdx.x + gi * gridDim.x);
       const int ws = gi & 1;
       const int64_t l0 = static_cast<int64_t>(g) * G;
       const int rows_real = static_cast<int>(imin64(G, a.L - l0));
@@ -311,13 +313,14 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
         __syncwarp();
       };
       for (int gi = 0; gi < n_my_groups; ++gi) {
-        const int l0 = (blockIdx.x + gi * gridDim.x) * G;
-        const int rows_real = static_cast<int>(imin64(G, a.L - l0));
+        const int l0 = a.set.tile(blockIdx.x + gi * gridDim.x) * G;
+        const int rows_real = static_cast<int>(imin64(G, a.L - l0)), first_label = a.label0 + l0;
         for (int t = 0; t < T; ++t, ++it) {
           const int zs = it & 1;
           const int b = t * BT + row;
-          const float thr = b < a.B ? __ldg(a.thr + b) : INFINITY;       // rows beyond the batch never pass; a bf16 value
-          const uint32_t thr2 = pack2(thr, thr);
+          const uint2 cut = b < a.B ? __ldg(reinterpret_cast<const uint2*>(a.cut) + b) : make_uint2(0x7F807F80u, 0u);   // rows beyond the batch: +inf, never passed
+          const uint32_t thr2 = __byte_perm(cut.x, 0u, first_label < static_cast<int>(cut.y) ? 0x1010 : 0x3232);
+          const float thr = __uint_as_float(thr2 & 0xFFFF0000u);
           const bool ok = mbar_wait(bar(C::B_ZFULL + zs), (it >> 1) & 1, abort_flag, a.err, 27, WL);
           tc_fence_after();
           const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + zs * G + h * C::EC;
@@ -355,7 +358,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
                 for (int y = 1; y < CW / 2; ++y) v = (x & 15) == y ? p[y] : v;
                 const uint32_t bits = (x & 16) ? (v & 0xFFFF0000u) : (v << 16);
                 list[count + __popc(any & ((1u << lane) - 1u))] =
-                    make_uint2(static_cast<uint32_t>(a.label0 + l0 + col0 + 2 * (x & 15) + (x >> 4)), bits | static_cast<uint32_t>(b));
+                    make_uint2(static_cast<uint32_t>(first_label + col0 + 2 * (x & 15) + (x >> 4)), bits | static_cast<uint32_t>(b));
                 hit &= hit - 1u;
               }
               count += __popc(any);
@@ -436,18 +439,19 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
 
 template <int GG_, int FF_, int P_>
 static int launch_shape(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t L,
-                        int64_t ldz, int64_t zw, int64_t ldxt, const TopkFilter* tk, cudaStream_t st) {
+                        int64_t ldz, int64_t zw, int64_t ldxt, const TileSet& set, const TopkFilter* tk, cudaStream_t st) {
   using C = Cfg<GG_, FF_, P_>;
   if (int rc = report_pending_status("tcgen05 forward")) return rc;
   int* err_dev = nullptr;
   if (int rc = device_status_word(&err_dev)) return rc;
   FwdArgs a;
   a.loc = loc; a.bias = static_cast<const __nv_bfloat16*>(bias); a.z = static_cast<__nv_bfloat16*>(z); a.err = err_dev;
-  a.B = B; a.L = L; a.ldz = ldz; a.zw = zw; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::G - 1) / C::G);
+  a.B = B; a.L = L; a.ldz = ldz; a.zw = zw; a.D = static_cast<int>(D); a.set = set;
+  a.NG = set.count(static_cast<int>((L + C::G - 1) / C::G));
   a.NGR = static_cast<int>((L + C::GG - 1) / C::GG);
   a.wait_limit = wait_limit_cycles();
-  a.thr = nullptr; a.cand = nullptr; a.cnt = nullptr; a.cap = 0; a.label0 = 0;
-  if (tk) { a.thr = tk->thr; a.cand = tk->cand; a.cnt = tk->cnt; a.cap = tk->cap; a.label0 = tk->label0; }
+  a.cut = nullptr; a.cand = nullptr; a.cnt = nullptr; a.cap = 0; a.label0 = 0;
+  if (tk) { a.cut = tk->cut; a.cand = tk->cand; a.cnt = tk->cnt; a.cap = tk->cap; a.label0 = tk->label0; }
   CUtensorMap tm_x, tm_w, tm_z;
   if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc;
   if (int rc = make_tmap_bf16_2d(&tm_w, w, static_cast<uint64_t>(C::FF), static_cast<uint64_t>(L), static_cast<uint64_t>(C::FF) * 2, C::FF == 32 ? 32 : 64, C::G)) return rc;
@@ -476,27 +480,32 @@ bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64
          aligned16(w) && L < (int64_t(1) << 31) && ldxt < (int64_t(1) << 31);
 }
 
+#define HASTE_F100_SHAPES(...)                                                     \
+  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(__VA_ARGS__);    \
+  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(__VA_ARGS__);    \
+  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(__VA_ARGS__);      \
+  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(__VA_ARGS__);      \
+  if (G == 32 && F == 128) return f100::launch_shape<32, 128, 1>(__VA_ARGS__);    \
+  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(__VA_ARGS__);      \
+  return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
+
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
                          int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st) {
-  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  if (G == 32 && F == 128) return f100::launch_shape<32, 128, 1>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, nullptr, st);
-  return fail(HASTE_ERR_UNSUPPORTED, "tcgen05 forward: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
+  HASTE_F100_SHAPES(loc, xt, w, bias, z, B, D, L, ldz, zw, ldxt, TileSet(), nullptr, st)
+}
+
+int forward_tile_labels_sm100(int64_t F, int64_t G) { return G == 32 && F < 128 ? 64 : static_cast<int>(G); }
+
+int launch_forward_tiles_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
+                               int64_t L, int64_t G, int64_t ldz, int64_t cols, int64_t ldxt, const TileSet& set, cudaStream_t st) {
+  HASTE_F100_SHAPES(loc, xt, w, bias, z, B, D, L, ldz, (cols + 7) / 8 * 8, ldxt, set, nullptr, st)
 }
 
 int launch_topk_filter_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, int64_t B, int64_t D, int64_t F, int64_t L,
                              int64_t G, int64_t ldxt, const TopkFilter& tk, cudaStream_t st) {
   if (B > 65536) return fail(HASTE_ERR_UNSUPPORTED, "top-k filter: batch %lld too large", (long long)B);      // 16 bits of a list entry
-  if (G == 128 && F == 64) return f100::launch_shape<128, 64, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  if (G == 64 && F == 128) return f100::launch_shape<64, 128, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  if (G == 64 && F == 64) return f100::launch_shape<64, 64, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  if (G == 32 && F == 64) return f100::launch_shape<32, 64, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  if (G == 32 && F == 128) return f100::launch_shape<32, 128, 1>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  if (G == 32 && F == 32) return f100::launch_shape<32, 32, 2>(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, &tk, st);
-  return fail(HASTE_ERR_UNSUPPORTED, "top-k filter: no kernel for group size %lld, fan-in %lld", (long long)G, (long long)F);
+  HASTE_F100_SHAPES(loc, xt, w, bias, nullptr, B, D, L, 0, 0, ldxt, tk.set, &tk, st)
 }
+#undef HASTE_F100_SHAPES
 
 }  // namespace haste

@@ -39,15 +39,45 @@ int launch_forward(const int32_t* loc, const void* xt, const void* w, const void
 bool forward_sm100_supported(const void* z, const void* xt, const void* w, int64_t B, int64_t F, int64_t L, int64_t G, int64_t ldz, int64_t ldxt);
 int launch_forward_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
                          int64_t L, int64_t G, int64_t ldz, int64_t zw, int64_t ldxt, cudaStream_t st);
-// Forward whose epilogue keeps only the logits above thr[b], as keys in cand[b][0 .. cap) (cnt[b] counts them all).
+// The label tiles a launch of the tcgen05 forward works on: every step-th tile of the layer (skip == 0), or every step-th tile but not
+// every (step * skip)-th one, which an earlier launch has done (skip in 3 .. 2^12).  Tile i of the second kind is
+// step * (i + i / (skip - 1) + 1); the division is a multiplication, exact for i < 2^20 * (4096 / skip).
+struct TileSet {
+  int step = 1, skip = 0;
+  uint32_t inv = 0;                                    // 2^32 / (skip - 1), rounded up; 0 for skip == 0
+  TileSet() = default;
+  TileSet(int step_, int skip_) : step(step_), skip(skip_), inv(skip_ == 0 ? 0u : static_cast<uint32_t>((1ull << 32) / (skip_ - 1) + 1)) {}
+  __device__ int tile(int i) const {
+    return step * (i + static_cast<int>(__umulhi(static_cast<uint32_t>(i), inv)) + (skip == 0 ? 0 : 1));
+  }
+  int count(int n_tiles) const {
+    const int with = (n_tiles + step - 1) / step;
+    return skip == 0 ? with : with - (with + skip - 1) / skip;
+  }
+};
+// Logits of the tiles of `set` only, side by side in z (label tile set.tile(i) in columns i * tile ...); z has `cols` real columns,
+// rounded up to a multiple of 8 they receive zeros.
+int launch_forward_tiles_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, void* z, int64_t B, int64_t D, int64_t F,
+                               int64_t L, int64_t G, int64_t ldz, int64_t cols, int64_t ldxt, const TileSet& set, cudaStream_t st);
+int forward_tile_labels_sm100(int64_t F, int64_t G);      // labels of a tile
+
+// What a logit of a row has to beat: the row's k-th best (value, label) so far.  Labels before `label` win with an equal value,
+// labels after it do not; .bits holds the value (bf16) in the upper half and a bf16 just below it in the lower half.
+struct RowCut {
+  uint32_t bits;
+  int label;
+};
+// Forward whose epilogue keeps only the logits of the tiles of `set` that beat cut[b] (and a few more: those of a tile that
+// holds cut[b].label itself may only equal it), as keys in cand[b][0 .. cap) (cnt[b] counts them all).
 struct TopkFilter {
   // One counter per 128-byte line.  Side by side, the counters of 512 rows filled 16 lines, on which the 358 thousand
   // atomics of a 131 K-label launch queued: 88 us for the launch, 69 so.
   static constexpr int CNT_STRIDE = 32;
-  const float* thr;
+  const RowCut* cut;
   unsigned long long* cand;
   int* cnt;
   int cap, label0;
+  TileSet set;
 };
 int launch_topk_filter_sm100(const int32_t* loc, const void* xt, const void* w, const void* bias, int64_t B, int64_t D, int64_t F, int64_t L,
                              int64_t G, int64_t ldxt, const TopkFilter& tk, cudaStream_t st);

@@ -137,14 +137,18 @@ int launch_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t
 
 // ================================================================ whole top-k with a filtered forward
 // The chunked path above writes every logit to L2 and reads it back once (670 K labels, 512 rows: 686 MB each way).  Here
-// only a first chunk of TF_FIRST labels is stored; its k-th best logit is a threshold that all but k * (labels of the
-// launch / labels before it) of the remaining logits fail, so the forward's epilogue filters them in registers
-// (TOPK instantiations of the tcgen05 forward) and a merge kernel folds the survivors in.  Each launch covers TF_GROW
-// times the labels seen before it: for random label order that is TF_GROW * k candidates a row, against a list of
-// TF_CAP.  A row whose list overflows (labels laid out so that later ones are systematically better for it) is computed
-// again by the merge kernel on the CUDA cores: slower, the same result up to the order of the fp32 sums.
+// only the logits of a sample of at most TF_FIRST labels are stored, whole label tiles evenly spread over the layer; a row's k-th
+// best of them is a bar that all but k * (labels of the launch / labels before it) of the other logits fail, so the forward's
+// epilogue filters them in registers (TOPK instantiations of the tcgen05 forward) and a merge kernel folds the survivors in.
+// Each launch covers at most TF_GROW times the labels seen before it, again evenly spread: TF_GROW * k candidates a row
+// are expected, against a list of TF_CAP.  The spread makes that hold for any order of the labels: where logits rise with the
+// label id at most about TF_GROW * (k + a tile) pass, where all are equal the label ids decide likewise.  (With the first 16 K
+// labels as the sample, 670 K labels whose biases rise with the id took 14.2 ms for 512 rows, a masked first 16 K labels
+// 5.2 ms, against 0.28 ms in random order.)
+// A row whose list overflows all the same (logits periodic in the sample's step) is computed again by the merge kernel on the
+// CUDA cores: slower, the same result up to the order of the fp32 sums.
 constexpr int TF_THREADS = 256;
-constexpr int64_t TF_FIRST = 16384, TF_GROW = 8;
+constexpr int64_t TF_FIRST = 148 * 128, TF_GROW = 8;      // the sample: a tile on every SM at G = 128
 constexpr int TF_CAP = 8192;
 typedef unsigned long long u64;
 
@@ -188,14 +192,24 @@ static int keep_lanes(int64_t n, int k, int nt) {
 }
 static int64_t keep_bound(int64_t n, int k, int nt) { return static_cast<int64_t>(k) * ((n + nt - 1) / nt) * keep_lanes(n, k, nt); }
 
-// The k best of keys[0..s) in order, to vals / idx (label ids as in the keys; -inf / -1 where there are fewer); returns
-// nothing, writes *thr = the k-th value when thr != NULL.
-template <int NT>
-__device__ __forceinline__ void write_best(const u64* keys, int s, int k, float* vals, int32_t* idx, float* thr) {
+// The bar that the k-th best key sets (0: fewer than k so far, any number passes).  Just below 0 stands the largest normal
+// negative number: compares may flush what lies between, and what passes in addition only has to be looked at.
+__device__ __forceinline__ RowCut row_cut(u64 key, int label) {
+  if (key == 0) return {0xFF80FF80u, 0};
+  const uint32_t v = __float_as_uint(topk_key_value(key)) >> 16;           // a bf16 above -inf, not -0
+  const uint32_t below = (v & 0x8000u) ? v + 1u : v <= 0x0080u ? 0x8080u : v - 1u;
+  return {(v << 16) | below, label};
+}
+
+// The k best of keys[0..s) in order, to vals / idx (label ids: label(what the keys hold); -inf / -1 where there are fewer), and the
+// bar they set to *cut when cut != NULL.
+struct SameLabel { __device__ int operator()(int l) const { return l; } };
+template <int NT, class LABEL = SameLabel>
+__device__ __forceinline__ void write_best(const u64* keys, int s, int k, float* vals, int32_t* idx, RowCut* cut, LABEL label = LABEL()) {
   const int tid = threadIdx.x;
   for (int i = tid; i < k; i += NT)
     if (i >= s) { vals[i] = -INFINITY; idx[i] = -1; }
-  if (tid == 0 && thr != nullptr && s < k) *thr = -INFINITY;
+  if (tid == 0 && cut != nullptr && s < k) *cut = row_cut(0, 0);
   for (int i = tid; i < s; i += NT) {
     const u64 v = keys[i];
     int rank = 0;
@@ -203,8 +217,8 @@ __device__ __forceinline__ void write_best(const u64* keys, int s, int k, float*
     for (int j = 0; j < s; ++j) rank += keys[j] > v;
     if (rank < k) {
       vals[rank] = topk_key_value(v);
-      idx[rank] = topk_key_label(v);
-      if (thr != nullptr && rank == k - 1) *thr = topk_key_value(v);
+      idx[rank] = label(topk_key_label(v));
+      if (cut != nullptr && rank == k - 1) *cut = row_cut(v, idx[rank]);
     }
   }
 }
@@ -213,8 +227,8 @@ __device__ __forceinline__ u64 logit_key(uint16_t bits, uint32_t label) {
   return v > -INFINITY ? topk_key(v, label) : 0ull;                 // -inf and NaN are never selected
 }
 
-// First chunk: the k best of z[b, 0..C), labels col0 + c; also the row's threshold and its empty candidate list.  Rows are
-// 16-byte aligned and their length is that of whole chunks (the forward writes zeros past C, which are masked here).
+// The sample: the k best of z[b, 0..C) (column c holds label col0 + c / tile * stride + c % tile, tile a power of two); also the
+// bar they set and the row's empty candidate list.  Rows are 16-byte aligned and their length is that of whole chunks (the forward writes zeros past C, which are masked here).
 // The threads' maxima are found on packed bf16 pairs, eight logits per load; equal logits around the k-th maximum may let more
 // through than the list holds, and then the keys decide (which order equal logits by label).
 // The kernel with keys throughout took 33 us for 512 rows.
@@ -226,9 +240,9 @@ __device__ __forceinline__ float max8(const uint4& v) {
   const uint32_t m = max2u(max2u(v.x, v.y), max2u(v.z, v.w));
   return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
 }
-__global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* __restrict__ z, int64_t ldz, int C, uint32_t col0, int k,
-                                                                int cap, float* __restrict__ vals, int32_t* __restrict__ idx,
-                                                                float* __restrict__ thr, int* __restrict__ cnt) {
+__global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* __restrict__ z, int64_t ldz, int C, uint32_t col0, int tile,
+                                                                uint32_t stride, int k, int cap, float* __restrict__ vals, int32_t* __restrict__ idx,
+                                                                RowCut* __restrict__ row_cuts, int* __restrict__ cnt) {
   extern __shared__ __align__(16) u64 kept[];
   __shared__ u64 s_max[TF_THREADS], s_tau;
   __shared__ __align__(16) float s_val[TF_THREADS];
@@ -239,6 +253,8 @@ __global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* 
   const uint16_t* zr = z + b * ldz;
   const uint4* z4 = reinterpret_cast<const uint4*>(zr);
   const int whole = C >> 3;                                                  // chunks without a masked column
+  const int tile_log = __ffs(tile) - 1;
+  auto label_of = [&](int c) { return static_cast<int>(col0 + static_cast<uint32_t>(c >> tile_log) * stride + static_cast<uint32_t>(c & (tile - 1))); };
   float m = -INFINITY;
 #pragma unroll 4
   for (int c = tid; c < whole; c += TF_THREADS) m = fmaxf(m, max8(z4[c]));   // fmaxf drops a NaN
@@ -260,7 +276,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* 
     const float v = bf16_bits_to_float(bits);
     if (v >= cut && v > -INFINITY) {
       const int slot = atomicAdd(&s_n, 1);
-      if (slot < cap) kept[slot] = topk_key(v, col0 + static_cast<uint32_t>(c));
+      if (slot < cap) kept[slot] = topk_key(v, static_cast<uint32_t>(c));
     }
   };
 #pragma unroll 4
@@ -277,9 +293,9 @@ __global__ void __launch_bounds__(TF_THREADS) topk_first_kernel(const uint16_t* 
   int s = s_n;
   if (s > cap) {                                                             // uniform
     __syncthreads();
-    s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], col0 + static_cast<uint32_t>(i)); }, C, k, 1, kept, s_max, &s_tau, &s_n);
+    s = keep_candidates<TF_THREADS>([&](int i) { return logit_key(zr[i], static_cast<uint32_t>(i)); }, C, k, 1, kept, s_max, &s_tau, &s_n);
   }
-  write_best<TF_THREADS>(kept, s, k, vals + b * k, idx + b * k, thr + b);
+  write_best<TF_THREADS>(kept, s, k, vals + b * k, idx + b * k, row_cuts + b, label_of);      // the keys hold columns
   if (tid == 0) cnt[b * TopkFilter::CNT_STRIDE] = 0;
 }
 
@@ -291,13 +307,16 @@ static_assert(TM_LIST + TM_KEEP <= TM_KEYS, "the recomputation works inside the 
 
 struct TopkMergeArgs {
   const int32_t* loc;
-  const uint16_t *xt, *w, *bias;                    // of the launch's labels
+  const uint16_t *xt, *w, *bias;
   const u64* cand;
-  float *vals, *thr;
+  float* vals;
+  RowCut* cut;
   int32_t* idx;
   int* cnt;
   int64_t L, ldxt;
-  int D, F, G, k;
+  int D, F, G, k, tile;                             // tile: labels of a tile
+  TileSet set;                                      // tiles of the launch the candidates come from ...
+  int n_tiles;                                      // ... and their number
   uint32_t label0;
 };
 
@@ -322,13 +341,16 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
     u64* best = keys + TM_LIST;
     if (tid == 0) s_list = k;
     if (tid < k) keys[tid] = kept(tid);
-    float thr = a.thr[b];
+    u64 kth = kept(k - 1);
     __syncthreads();
     const int per = TF_THREADS / a.G, gl = tid / a.G, r = tid % a.G;
-    const int64_t NG = (a.L + a.G - 1) / a.G;
-    for (int64_t g0 = 0; g0 < NG; g0 += per) {
+    const int gpt = a.tile / a.G;                   // groups of a tile
+    const int64_t NG = (a.L + a.G - 1) / a.G;       // of the layer
+    const int n_groups = a.n_tiles * gpt;       // of the launch
+    for (int g0 = 0; g0 < n_groups; g0 += per) {
+      auto group = [&](int i) { return g0 + i < n_groups ? static_cast<int64_t>(a.set.tile((g0 + i) / gpt)) * gpt + (g0 + i) % gpt : NG; };
       for (int i = tid; i < per * a.F; i += TF_THREADS) {
-        const int64_t g = g0 + i / a.F;
+        const int64_t g = group(i / a.F);
         float v = 0.f;
         if (g < NG) {
           const int d = min(max(__ldg(a.loc + g * a.F + i % a.F), 0), a.D - 1);
@@ -337,7 +359,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
         xs[i / a.F][i % a.F] = v;
       }
       __syncthreads();
-      const int64_t l = (g0 + gl) * a.G + r;
+      const int64_t l = group(gl) * a.G + r;
       if (l < a.L) {
         float acc = 0.f;
         const uint4* wr = reinterpret_cast<const uint4*>(a.w + l * a.F);
@@ -352,7 +374,10 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
         }
         if (a.bias != nullptr) acc += bf16_bits_to_float(a.bias[l]);
         const float z = round_to_bf16_f(acc);
-        if (z > thr) keys[atomicAdd(&s_list, 1)] = topk_key(z, a.label0 + static_cast<uint32_t>(l));
+        if (z > -INFINITY) {
+          const u64 key = topk_key(z, a.label0 + static_cast<uint32_t>(l));
+          if (key > kth) keys[atomicAdd(&s_list, 1)] = key;
+        }
       }
       __syncthreads();
       if (s_list > TM_LIST - TF_THREADS) {          // uniform; room for one more round of labels is kept
@@ -364,7 +389,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
         }
         if (tid == 0) s_list = min(m, k);
         __syncthreads();
-        if (m >= k) thr = topk_key_value(s_max[0]);
+        if (m >= k) kth = s_max[0];
         __syncthreads();
       }
     }
@@ -374,7 +399,7 @@ __global__ void __launch_bounds__(TF_THREADS) topk_merge_kernel(TopkMergeArgs a)
     s = m;
   }
   __syncthreads();
-  write_best<TF_THREADS>(keys, s, k, vals, idx, a.thr + b);
+  write_best<TF_THREADS>(keys, s, k, vals, idx, a.cut + b);
   if (tid == 0) a.cnt[b * TopkFilter::CNT_STRIDE] = 0;
 }
 
@@ -501,23 +526,56 @@ static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int
   return 0;
 }
 
-// Scratch of the filtered path, in bytes from a 16-byte aligned base: xt | logits of the first chunk | candidates | thresholds | counters
-struct FusedScratch { int64_t xt, z, cand, thr, cnt, total; };
-static FusedScratch fused_layout(int64_t B, int64_t D, int64_t L, int64_t G) {
-  const int64_t ldxt = (B + 7) / 8 * 8, first = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
+// The launches of the filtered path: a sample (every `step`-th tile), then `launches` filter launches whose tile sets complete it,
+// each TF_GROW times the labels before it at most.
+struct FilterPlan {
+  int tile, n_tiles, step = 1, launches = 0;
+  int64_t sample;                                     // labels of the sample
+  TileSet set[8];
+};
+static FilterPlan filter_plan(int64_t F, int64_t L, int64_t G) {
+  FilterPlan p;
+  p.tile = forward_tile_labels_sm100(F, G);
+  p.n_tiles = static_cast<int>((L + p.tile - 1) / p.tile);
+  const int first = static_cast<int>(TF_FIRST / p.tile);
+  int64_t ratio = (p.n_tiles + first - 1) / first;    // at most 2^17: six launches
+  for (int64_t reach = 1; reach < ratio; reach *= TF_GROW + 1) ++p.launches;
+  int skip[8];
+  for (int i = 0; i < p.launches; ++i) {              // factors as equal as whole numbers allow, their product is at least the ratio
+    int r = 3;
+    for (;; ++r) {
+      int64_t reach = 1;
+      for (int k = i; k < p.launches; ++k) reach *= r;
+      if (reach >= ratio) break;
+    }
+    skip[i] = r;
+    p.step *= r;
+    ratio = (ratio + r - 1) / r;
+  }
+  for (int i = 0, step = p.step; i < p.launches; ++i) p.set[i] = TileSet(step /= skip[i], skip[i]);
+  const int64_t sampled = (p.n_tiles + p.step - 1) / p.step, last = (sampled - 1) * p.step;
+  p.sample = (sampled - 1) * p.tile + imin64(p.tile, L - last * p.tile);
+  return p;
+}
+
+// Scratch of the filtered path, in bytes from a 16-byte aligned base: xt | logits of the sample | candidates | bars | counters
+struct FusedScratch { int64_t xt, z, ldz, cand, cut, cnt, total; };
+static FusedScratch fused_layout(int64_t B, int64_t D, const FilterPlan& p) {
+  const int64_t ldxt = (B + 7) / 8 * 8;
   FusedScratch s;
+  s.ldz = (p.sample + 7) / 8 * 8;
   s.xt = 0;
   s.z = round16(s.xt + D * ldxt * 2);
-  s.cand = round16(s.z + B * first * 2);
-  s.thr = s.cand + (L > first ? B * TF_CAP * 8 : 0);
-  s.cnt = round16(s.thr + B * 4);
+  s.cand = round16(s.z + B * s.ldz * 2);
+  s.cut = s.cand + (p.launches > 0 ? B * TF_CAP * 8 : 0);
+  s.cnt = round16(s.cut + B * static_cast<int64_t>(sizeof(RowCut)));
   s.total = round16(s.cnt + B * 4 * TopkFilter::CNT_STRIDE);
   return s;
 }
 int64_t topk_fused_scratch_bytes(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
   switch (topk_route(B, D, F, L, G, k)) {
     case 1: { const int64_t seg = rows_seg(L, G); return B * ((L + seg - 1) / seg) * k * 8; }
-    case 2: return fused_layout(B, D, L, G).total;
+    case 2: return fused_layout(B, D, filter_plan(F, L, G)).total;
     default: return 0;
   }
 }
@@ -553,38 +611,32 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
     return check_launch("topk_parts_kernel");
   }
   if (route != 2) return fail(HASTE_ERR_UNSUPPORTED, "top-k: group size %lld, fan-in %lld, batch %lld take the chunked call", (long long)G, (long long)F, (long long)B);
-  const FusedScratch fs = fused_layout(B, D, L, G);
+  const FilterPlan plan = filter_plan(F, L, G);
+  const FusedScratch fs = fused_layout(B, D, plan);
   char* base = static_cast<char*>(scratch);
-  const int64_t ldxt = (B + 7) / 8 * 8;
   void* xt = base + fs.xt;
   uint16_t* z = reinterpret_cast<uint16_t*>(base + fs.z);
-  float* thr = reinterpret_cast<float*>(base + fs.thr);
+  RowCut* cut = reinterpret_cast<RowCut*>(base + fs.cut);
   int* cnt = reinterpret_cast<int*>(base + fs.cnt);
   u64* cand = reinterpret_cast<u64*>(base + fs.cand);
-  const char* wb = static_cast<const char*>(w);
-  const char* bb = static_cast<const char*>(bias);
-  if (int rc = launch_transpose(x, xt, B, D, ldxt, false, st)) return rc;
-  const int64_t ldz = imin64(TF_FIRST / G * G, (L + G - 1) / G * G);
-  const int64_t first = imin64(ldz, L);
-  if (int rc = launch_forward(loc, xt, w, bias, z, B, D, F, first, G, ldz, (first + 7) / 8 * 8, ldxt, st)) return rc;
-  const int cap = static_cast<int>(k * ((first + TF_THREADS - 1) / TF_THREADS));      // the bound of keep_candidates with single threads
-  const size_t sm = static_cast<size_t>(cap) * 8;
+  const int cap = static_cast<int>(k * ((plan.sample + TF_THREADS - 1) / TF_THREADS));      // the bound of keep_candidates with single threads
   if (int rc = allow_dynamic_smem(topk_first_kernel)) return rc;
-  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, sm, st>>>(z, ldz, int(first), static_cast<uint32_t>(label0), k, cap, vals, idx, thr, cnt);
+  const int64_t ldxt = (B + 7) / 8 * 8;
+  if (int rc = launch_transpose(x, xt, B, D, ldxt, false, st)) return rc;
+  if (int rc = launch_forward_tiles_sm100(loc, xt, w, bias, z, B, D, F, L, G, fs.ldz, plan.sample, ldxt, TileSet(plan.step, 0), st)) return rc;
+  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, static_cast<size_t>(cap) * 8, st>>>(
+      z, fs.ldz, static_cast<int>(plan.sample), static_cast<uint32_t>(label0), plan.tile, static_cast<uint32_t>(plan.tile) * plan.step, k, cap, vals, idx, cut, cnt);
   if (int rc = check_launch("topk_first_kernel")) return rc;
-  for (int64_t l0 = first; l0 < L;) {
-    const int64_t n = imin64(TF_GROW * l0, L - l0), g0 = l0 / G;          // first is a multiple of G when there is more, so l0 always is
-    TopkFilter tk{thr, cand, cnt, TF_CAP, static_cast<int>(label0 + l0)};
-    const void* w0 = wb + l0 * F * 2;
-    const void* b0 = bb ? bb + l0 * 2 : nullptr;
-    if (int rc = launch_topk_filter_sm100(loc + g0 * F, xt, w0, b0, B, D, F, n, G, ldxt, tk, st)) return rc;
+  for (int i = 0; i < plan.launches; ++i) {
+    const TopkFilter tk{cut, cand, cnt, TF_CAP, static_cast<int>(label0), plan.set[i]};
+    if (int rc = launch_topk_filter_sm100(loc, xt, w, bias, B, D, F, L, G, ldxt, tk, st)) return rc;
     TopkMergeArgs a;
-    a.loc = loc + g0 * F; a.xt = static_cast<const uint16_t*>(xt); a.w = static_cast<const uint16_t*>(w0); a.bias = static_cast<const uint16_t*>(b0);
-    a.cand = cand; a.vals = vals; a.thr = thr; a.idx = idx; a.cnt = cnt; a.L = n; a.ldxt = ldxt;
-    a.D = int(D); a.F = int(F); a.G = int(G); a.k = k; a.label0 = static_cast<uint32_t>(label0 + l0);
+    a.loc = loc; a.xt = static_cast<const uint16_t*>(xt); a.w = static_cast<const uint16_t*>(w); a.bias = static_cast<const uint16_t*>(bias);
+    a.cand = cand; a.vals = vals; a.cut = cut; a.idx = idx; a.cnt = cnt; a.L = L; a.ldxt = ldxt;
+    a.D = int(D); a.F = int(F); a.G = int(G); a.k = k; a.tile = plan.tile; a.set = plan.set[i]; a.n_tiles = plan.set[i].count(plan.n_tiles);
+    a.label0 = static_cast<uint32_t>(label0);
     topk_merge_kernel<<<static_cast<unsigned>(B), TF_THREADS, 0, st>>>(a);
     if (int rc = check_launch("topk_merge_kernel")) return rc;
-    l0 += n;
   }
   return HASTE_OK;
 }

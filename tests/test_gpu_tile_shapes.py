@@ -249,3 +249,58 @@ def test_hinge_step_with_any_gradient_scale(G, F, scale):
     assert abs(float(loss_dev) - ref["loss"] * scale) <= 2e-3 * abs(ref["loss"] * scale)
     want = ref["dXt"].double() * scale
     assert float((dxt.cpu().double() - want).norm()) <= 1e-2 * float(want.norm())
+
+
+@pytest.mark.parametrize("L", [20011, 18944 * 9 + 70])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_topk_fused_ties_and_any_label_order(G, F, L):
+    """The filtered path samples every n-th label tile.  equal: the label id alone decides, whichever launch a label belongs to;
+    rising, falling: the best labels lie at one end; other_tiles: every label outside the sample beats the sample, so that the
+    candidate lists overflow (more than 8192 labels) and the rows are computed again."""
+    from haste_b200 import ffi
+    from haste_b200.infer import ffi_topk
+    B, D, k = 9, 128, 100
+    tile = 64 if G == 32 and F < 128 else G
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=12, x_kind="normal", bias_zero=True)
+    dev = {n: v.cuda() for n, v in inp.items()}
+    x = dev["X"]
+    ramp = torch.arange(L, device="cuda").float()
+    n = 3 if L < 40000 else 12                    # the sample: every n-th tile
+    for kind, bias in (("equal", torch.zeros_like(ramp)), ("rising", ramp / L * 8), ("falling", -ramp / L * 8),
+                       ("other_tiles", 4.0 * (torch.arange(L, device="cuda") // tile % n != 0))):
+        bias = bias.to(torch.bfloat16)
+        features = torch.zeros_like(x) if kind == "equal" else x
+        vals, idx = ffi_topk(dev["loc"], dev["W"], bias, features, k, G, label0=3)
+        z = ffi.forward(dev["loc"], ffi.transpose_padded(features), dev["W"], bias, G, B=B).float()
+        _check_topk(vals, idx, z, k, 3)
+        if kind == "equal":
+            assert torch.equal(idx.cpu(), (3 + torch.arange(k, dtype=torch.int32)).expand(B, k))
+
+
+def test_topk_cost_does_not_depend_on_the_label_order():
+    """Biases that rise with the label id, a first 16 K labels that are masked, a block of labels ahead of all others: the call takes
+    about as long as with biases in random order.  (A bar set by the first labels made these 20 to 50 times slower.)"""
+    from haste_b200.infer import ffi_topk
+    B, D, L, F, G, k = 256, 768, 300007, 64, 128, 100
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=12, x_kind="l2norm", bias_zero=True)
+    dev = {n: v.cuda() for n, v in inp.items()}
+    random = torch.rand(L, generator=torch.Generator().manual_seed(1)) * 0.05
+    masked, block = random.clone(), random.clone()
+    masked[:16384] = float("-inf")
+    block[100000:130000] += 1.0
+
+    def ms(bias):
+        bias = bias.to(torch.bfloat16).cuda()
+        best = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ffi_topk(dev["loc"], dev["W"], bias, dev["X"], k, G)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    base = ms(random)
+    for name, bias in (("rising", torch.sort(random).values), ("masked", masked), ("block", block)):
+        assert ms(bias) <= 4.0 * base, name
