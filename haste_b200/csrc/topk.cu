@@ -144,12 +144,16 @@ int launch_topk_update(const void* z, int64_t ldz, int64_t B, int64_t C, int64_t
 // are expected, against a list of TF_CAP.  The spread makes that hold for any order of the labels: where logits rise with the
 // label id at most about TF_GROW * (k + a tile) pass, where all are equal the label ids decide likewise.  (With the first 16 K
 // labels as the sample, 670 K labels whose biases rise with the id took 14.2 ms for 512 rows, a masked first 16 K labels
-// 5.2 ms, against 0.28 ms in random order.)
+// 5.2 ms, against 0.28 ms in random order; now 0.28 to 0.30 for all of them.)
 // A row whose list overflows all the same (logits periodic in the sample's step) is computed again by the merge kernel on the
-// CUDA cores: slower, the same result up to the order of the fp32 sums.
+// CUDA cores, the same result up to the order of the fp32 sums: all 512 rows of 670 K labels 3.9 ms.
 constexpr int TF_THREADS = 256;
 constexpr int64_t TF_FIRST = 148 * 128, TF_GROW = 8;      // the sample: a tile on every SM at G = 128
 constexpr int TF_CAP = 8192;
+// Rows per pass over the layer: a row takes 64 KiB of candidates and up to 37 KiB of sample logits, so larger batches go through
+// in slices that reuse the same 430 MB.  A slice costs one more set of launches and one more read of the weights: with 1024 rows
+// 8192 rows of 670 K labels took 4,069 us, undivided (820 MB) 3,723; the chunked path takes 7,650.
+constexpr int64_t TF_ROWS = 4096;
 typedef unsigned long long u64;
 
 // The keys that can be among the k best of n: all that are not below the k-th largest of the maxima of NT / lanes groups of
@@ -514,15 +518,18 @@ static size_t rows_smem(int64_t B, int64_t D, int64_t seg, int k) {
   return static_cast<size_t>((nb * D + 7) / 8 * 16 + nb * seg * 2 + keep_bound(seg, k, TS_THREADS) * 8);
 }
 // Which path: 0 the chunked one (above), 1 few rows, 2 filtered forward.
-// Few rows up to TS_ROWS: the filtered forward reads the same weights but pays five launches and a 128-row tile.
+// Few rows up to TS_ROWS: the filtered forward reads the same weights but pays five launches or more and a 128-row tile.  Few rows /
+// filtered, us a call:  k = 5, 131 K labels (G=64, F=128): 1 row 26 / 67, 4 rows 28 / 66, 8 rows 44 / 66; 670 K labels (G=128, F=64):
+// 40 / 102, 56 / 105, 83 / 105; 2.8 M labels: 115 / 289, 181 / 291, 320 / 292.  k = 100, where picking the best of every
+// segment weighs more: 131 K 51 / 73, 77 / 74, 116 / 74; 670 K 72 / 110, 106 / 114, 156 / 114.  The line is drawn by the rows
+// alone, so that a row's logits do not depend on k; it is right for small k and late for large.
 static int topk_route(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int k) {
   if (B <= TS_ROWS && (F == 16 || F == 32 || F == 64 || F == 128)) {
     const int64_t seg = rows_seg(L, G), parts = (L + seg - 1) / seg;
     if (rows_smem(B, D, seg, k) <= DYN_SMEM_MAX && keep_bound(parts * k, k, parts * k <= 4096 ? TS_THREADS : TS_MERGE) * 8 <= DYN_SMEM_MAX) return 1;
   }
   const bool shape = (G == 128 && F == 64) || (G == 64 && (F == 128 || F == 64)) || (G == 32 && (F == 128 || F == 64 || F == 32));
-  // (the candidate lists take 64 KiB a row: beyond a few thousand rows the chunked path needs less memory)
-  if (shape && B <= 8192 && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
+  if (shape && L < (int64_t(1) << 31) && D < (int64_t(1) << 31)) return 2;
   return 0;
 }
 
@@ -561,6 +568,7 @@ static FilterPlan filter_plan(int64_t F, int64_t L, int64_t G) {
 // Scratch of the filtered path, in bytes from a 16-byte aligned base: xt | logits of the sample | candidates | bars | counters
 struct FusedScratch { int64_t xt, z, ldz, cand, cut, cnt, total; };
 static FusedScratch fused_layout(int64_t B, int64_t D, const FilterPlan& p) {
+  B = imin64(B, TF_ROWS);
   const int64_t ldxt = (B + 7) / 8 * 8;
   FusedScratch s;
   s.ldz = (p.sample + 7) / 8 * 8;
@@ -621,22 +629,26 @@ int launch_topk_fused(const int32_t* loc, const void* x, const void* w, const vo
   u64* cand = reinterpret_cast<u64*>(base + fs.cand);
   const int cap = static_cast<int>(k * ((plan.sample + TF_THREADS - 1) / TF_THREADS));      // the bound of keep_candidates with single threads
   if (int rc = allow_dynamic_smem(topk_first_kernel)) return rc;
-  const int64_t ldxt = (B + 7) / 8 * 8;
-  if (int rc = launch_transpose(x, xt, B, D, ldxt, false, st)) return rc;
-  if (int rc = launch_forward_tiles_sm100(loc, xt, w, bias, z, B, D, F, L, G, fs.ldz, plan.sample, ldxt, TileSet(plan.step, 0), st)) return rc;
-  topk_first_kernel<<<static_cast<unsigned>(B), TF_THREADS, static_cast<size_t>(cap) * 8, st>>>(
-      z, fs.ldz, static_cast<int>(plan.sample), static_cast<uint32_t>(label0), plan.tile, static_cast<uint32_t>(plan.tile) * plan.step, k, cap, vals, idx, cut, cnt);
-  if (int rc = check_launch("topk_first_kernel")) return rc;
-  for (int i = 0; i < plan.launches; ++i) {
-    const TopkFilter tk{cut, cand, cnt, TF_CAP, static_cast<int>(label0), plan.set[i]};
-    if (int rc = launch_topk_filter_sm100(loc, xt, w, bias, B, D, F, L, G, ldxt, tk, st)) return rc;
-    TopkMergeArgs a;
-    a.loc = loc; a.xt = static_cast<const uint16_t*>(xt); a.w = static_cast<const uint16_t*>(w); a.bias = static_cast<const uint16_t*>(bias);
-    a.cand = cand; a.vals = vals; a.cut = cut; a.idx = idx; a.cnt = cnt; a.L = L; a.ldxt = ldxt;
-    a.D = int(D); a.F = int(F); a.G = int(G); a.k = k; a.tile = plan.tile; a.set = plan.set[i]; a.n_tiles = plan.set[i].count(plan.n_tiles);
-    a.label0 = static_cast<uint32_t>(label0);
-    topk_merge_kernel<<<static_cast<unsigned>(B), TF_THREADS, 0, st>>>(a);
-    if (int rc = check_launch("topk_merge_kernel")) return rc;
+  for (int64_t b0 = 0; b0 < B; b0 += TF_ROWS) {
+    const int64_t n = imin64(TF_ROWS, B - b0), ldxt = (n + 7) / 8 * 8;
+    float* v = vals + b0 * k;
+    int32_t* id = idx + b0 * k;
+    if (int rc = launch_transpose(static_cast<const uint16_t*>(x) + b0 * D, xt, n, D, ldxt, false, st)) return rc;
+    if (int rc = launch_forward_tiles_sm100(loc, xt, w, bias, z, n, D, F, L, G, fs.ldz, plan.sample, ldxt, TileSet(plan.step, 0), st)) return rc;
+    topk_first_kernel<<<static_cast<unsigned>(n), TF_THREADS, static_cast<size_t>(cap) * 8, st>>>(
+        z, fs.ldz, static_cast<int>(plan.sample), static_cast<uint32_t>(label0), plan.tile, static_cast<uint32_t>(plan.tile) * plan.step, k, cap, v, id, cut, cnt);
+    if (int rc = check_launch("topk_first_kernel")) return rc;
+    for (int i = 0; i < plan.launches; ++i) {
+      const TopkFilter tk{cut, cand, cnt, TF_CAP, static_cast<int>(label0), plan.set[i]};
+      if (int rc = launch_topk_filter_sm100(loc, xt, w, bias, n, D, F, L, G, ldxt, tk, st)) return rc;
+      TopkMergeArgs a;
+      a.loc = loc; a.xt = static_cast<const uint16_t*>(xt); a.w = static_cast<const uint16_t*>(w); a.bias = static_cast<const uint16_t*>(bias);
+      a.cand = cand; a.vals = v; a.cut = cut; a.idx = id; a.cnt = cnt; a.L = L; a.ldxt = ldxt;
+      a.D = int(D); a.F = int(F); a.G = int(G); a.k = k; a.tile = plan.tile; a.set = plan.set[i]; a.n_tiles = plan.set[i].count(plan.n_tiles);
+      a.label0 = static_cast<uint32_t>(label0);
+      topk_merge_kernel<<<static_cast<unsigned>(n), TF_THREADS, 0, st>>>(a);
+      if (int rc = check_launch("topk_merge_kernel")) return rc;
+    }
   }
   return HASTE_OK;
 }

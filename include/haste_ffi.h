@@ -308,10 +308,11 @@ int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void
                    float* vals, int32_t* idx, haste_stream_t stream);
 
 /* The same top-k without a chunk loop over stored logits, straight from the features x bf16 [B,D]: for few rows one
- * weight-streaming kernel and a merge; otherwise the logits of a first chunk set a threshold per row, and the forward
+ * weight-streaming kernel and a merge; otherwise the logits of a sample of the labels set a threshold per row, and the forward
  * kernels of the remaining labels keep only what beats it.  vals / idx are outputs (no start values).  `scratch`: 16-byte
  * aligned, haste_ffi_topk_fused_scratch(...) bytes; that function returns 0 for shapes that need haste_ffi_topk (and for
- * invalid ones).  Results as haste_ffi_topk up to the order of the fp32 sums of a logit. */
+ * invalid ones).  It is up to 0.1 MB a row for at most 4096 rows at a time (54 MB for 512 rows of 670 K labels, 430 MB at
+ * most); larger batches reuse it slice by slice.  Up to 8 rows take kilobytes.  Results as haste_ffi_topk up to the order of the fp32 sums of a logit. */
 int64_t haste_ffi_topk_fused_scratch(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k);
 int haste_ffi_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t scratch_bytes,
                          int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k, int64_t label0,

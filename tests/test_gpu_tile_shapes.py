@@ -304,3 +304,18 @@ def test_topk_cost_does_not_depend_on_the_label_order():
     base = ms(random)
     for name, bias in (("rising", torch.sort(random).values), ("masked", masked), ("block", block)):
         assert ms(bias) <= 4.0 * base, name
+
+
+def test_topk_of_a_batch_larger_than_a_slice():
+    """Batches beyond 4096 rows go through in slices that share their scratch."""
+    from haste_b200 import ffi
+    from haste_b200.infer import ffi_topk
+    B, D, L, F, G, k = 8201, 64, 20011, 32, 32, 10
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=5, x_kind="normal", bias_zero=False)
+    dev = {n: v.cuda() for n, v in inp.items()}
+    vals, idx = ffi_topk(dev["loc"], dev["W"], dev["bias"], dev["X"], k, G)
+    z = ffi.forward(dev["loc"], ffi.transpose_padded(dev["X"]), dev["W"], dev["bias"], G, B=B).float()
+    _check_topk(vals, idx, z, k, 0)
+    from haste_b200._lib import lib
+    n = [lib.haste_ffi_topk_fused_scratch(b, 768, 64, 670091, 128, 100) for b in (512, 4096, 8192, 20000)]
+    assert n[0] < n[1] == n[2] == n[3] < 410 << 20
