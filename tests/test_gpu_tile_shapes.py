@@ -319,3 +319,102 @@ def test_topk_of_a_batch_larger_than_a_slice():
     from haste_b200._lib import lib
     n = [lib.haste_ffi_topk_fused_scratch(b, 768, 64, 670091, 128, 100) for b in (512, 4096, 8192, 20000)]
     assert n[0] < n[1] == n[2] == n[3] < 410 << 20
+
+
+# ------------------------------------------------------------------------------------------------ accuracy and variants
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_step_bce_gradient_accuracy_at_a_multiple_of_8(G, F):
+    """Logits around -12 again, at the batch sizes where (128, 64) and (64, 128) take the sigmoid from tanh.approx: an absolute
+    error of up to 2^-12 per logit there (half of the instruction's 2^-11), a relative one elsewhere."""
+    from haste_b200.fused import FusedFFIShard
+    B, D, L = 104, 264, 3 * G
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=5, x_kind="l2norm", bias_zero=True)
+    inp["bias"] -= 12.0
+    sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss="bce", lr=0.0, momentum=0.9, seed=1)
+    sh.step(inp["X"].cuda(), torch.zeros(0, 2, dtype=torch.int32, device="cuda"))
+    z = fo.forward(inp["loc"], inp["X"], inp["W"], inp["bias"], G).double()
+    want = torch.sigmoid(z).sum(0)
+    tanh = G * F == 128 * 64
+    assert ((sh.mom_b.cpu().double() - want).abs() <= 2 ** -7 * want + (B * 2.0 ** -12 if tanh else 0.0)).all()
+
+
+def test_rewire_prunes_the_slots_with_nan_scores_and_the_lowest_others():
+    """A NaN compares with nothing: its slot has rank 0 and is pruned, and the other slots' ranks do not count it."""
+    from haste_b200 import ffi
+    D, L, F, G, n_prune = 512, 300, 64, 64, 19
+    gen = torch.Generator().manual_seed(3)
+    W = (torch.rand(L, F, generator=gen) - 0.5).to(torch.bfloat16)
+    W[::17, ::5] = float("nan")
+    NG = (L + G - 1) // G
+    loc0 = torch.stack([torch.randperm(D, generator=gen)[:F] for _ in range(NG)]).to(torch.int32)
+    w, loc = W.clone().cuda(), loc0.clone().cuda()
+    ffi.rewire(w, loc, None, D, G, 0, 1, 0.0, n_prune, 1, 0, False, 5, 1)
+    for g in range(NG):
+        rows = W[g * G:(g + 1) * G].float()
+        score = torch.zeros(F)
+        for r in rows:                                        # fp32, one row after the other, as the kernel sums
+            score = score + r.abs()
+        score = score / rows.shape[0]
+        ahead = (score[None, :] < score[:, None]) | ((score[None, :] == score[:, None]) & (torch.arange(F)[None, :] < torch.arange(F)[:, None]))
+        pruned = ahead.sum(1) < n_prune
+        got = w[g * G:(g + 1) * G].cpu()
+        assert (got[:, pruned] == 0).all()
+        assert torch.equal(got[:, ~pruned], W[g * G:(g + 1) * G][:, ~pruned])
+        assert torch.equal(loc[g].cpu()[~pruned], loc0[g][~pruned])
+        assert len(set(loc[g].tolist())) == F                 # 'unused' regrowth
+
+
+@pytest.mark.parametrize("rng", ["reference", "packed"])
+@pytest.mark.parametrize("G,F,L", [(64, 64, 64 * 160 + 33), (32, 64, 32 * 7), (32, 64, 32 * 310 + 1), (32, 128, 32 * 160 + 9), (32, 32, 32 * 401 + 7)])
+def test_update_variant_of_the_backward(G, F, L, rng):
+    """Backward-weights fused with the update against the unfused kernel and the oracle's update, bit for bit."""
+    import numpy as np
+    from haste_b200 import ffi
+    B, D, label0, seed, step, lr, wd = 136, 200, 640, 123, 4, 0.05, 1e-4
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=L, x_kind="normal", bias_zero=False)
+    dev = {k: v.cuda() for k, v in inp.items()}
+    xt = ffi.transpose_bf16(dev["X"])
+    gen = torch.Generator().manual_seed(2)
+    dY = (torch.randn(B, L, generator=gen) * 0.3).to(torch.bfloat16).cuda()
+    dw, db = ffi.backward_weights(xt, dev["W"], dev["loc"], dY, G, want_dbias=True)
+    for mu in (0.0, 0.9):
+        mom, momb = torch.randn(L, F, generator=gen) * 0.01, torch.randn(L, generator=gen) * 0.01
+        want_w, want_m = fo.sgd_update(inp["W"], dw.cpu(), mom, lr, wd, mu, True, True, fo.rand16_for((L, F), seed, step, rng, label0))
+        want_b, want_mb = fo.sgd_update(inp["bias"], db.cpu(), momb, lr, wd, mu, True, True,
+                                        fo.rand16_for((L, 1), seed, step, rng, label0, is_bias=True).reshape(L))
+        w, b, m, mb = dev["W"].clone(), dev["bias"].clone(), mom.clone().cuda(), momb.clone().cuda()
+        ffi.bww_sr_sgd(xt, dev["loc"], dY, w, b, m, mb, G, label0, lr, wd, mu, seed, step, ffi.make_flags(sr=True, contract=True, rng=rng))
+        assert np.array_equal(fo._bf16_to_bits(w.cpu()), fo._bf16_to_bits(want_w)) and np.array_equal(fo._bf16_to_bits(b.cpu()), fo._bf16_to_bits(want_b))
+        if mu:
+            assert torch.equal(m.cpu(), want_m) and torch.equal(mb.cpu(), want_mb)
+
+
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_step_on_fewer_ctas(G, F):
+    """set_max_ctas: the same weights and bias, in a time that shows that the limit holds."""
+    from haste_b200 import _lib
+    from haste_b200.fused import FusedFFIShard
+    B, D, L = 104, 264, G * 592 + 5                           # at least two tiles for each of 148 CTAs
+    inp = fo.make_inputs(B, D, L, F, G, 3, 1.1, seed=4, x_kind="l2norm", bias_zero=False)
+    x, t = inp["X"].cuda(), inp["targets"].cuda()
+
+    def run():
+        sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss="bce", lr=0.05, seed=42)
+        sh.step(x, t)
+        w, b = sh.w.clone(), sh.bias.clone()
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(5):
+            sh.step(x, t)
+        end.record()
+        end.synchronize()
+        return w, b, start.elapsed_time(end)
+
+    want_w, want_b, base = run()
+    try:
+        _lib.check(_lib.lib.haste_ffi_set_max_ctas(3), "set_max_ctas")
+        w, b, few = run()
+    finally:
+        _lib.check(_lib.lib.haste_ffi_set_max_ctas(0), "set_max_ctas")
+    assert torch.equal(w, want_w) and torch.equal(b, want_b)
+    assert few >= 3.0 * base
