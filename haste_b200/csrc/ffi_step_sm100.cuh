@@ -192,7 +192,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE;
   constexpr int N_EA = C::N_EA, N_EB = C::N_EB, N_UP = C::N_UP, EA_COLS = C::EA_COLS, UPS = C::UPS;
-  // Paired fp32 instructions: 670 K labels, hinge, 266 -> 260 us; no gain for BCE, whose loop waits for the MUFU (2.8 M labels: 2,234
+  // Paired fp32 instructions: 670 K labels, hinge, 276.4 -> 271.5 us a step (three runs of each in turn); no gain for BCE, whose loop waits for the MUFU (2.8 M labels: 2,234
   // against 2,243 us), and a loss at 128 slots (501 K labels: 352 against 364 us), where 64 registers per thread spill.
   constexpr bool PAIRED = LOSS == HASTE_LOSS_SQHINGE && F == 64;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
@@ -927,7 +927,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
 
 // Launch one shape.  `dump` selects the debug instantiation (always accumulates the loss).
 // The batch sizes and shapes that the warp-mma kernel used to serve computed the sigmoid to fp32 accuracy; they keep
-// that here (LOSS_BCE_EXP): the newer shapes always, (128, 64) and (64, 128) when B is not a multiple of 8.
+// that here (LOSS_BCE_EXP): the newer shapes always, (128, 64) and (64, 128) when B is not a multiple of 8.  The others keep
+// tanh.approx: with LOSS_BCE_EXP a step of 2.8 M labels takes 2,707 instead of 2,322 us, 501 K 356 instead of 345, 131 K (B=512)
+// 151 instead of 148.
 template <int GG_, int FF_, int P_>
 int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr, const uint32_t* tgt_ent, float* dxt, float* loss,
                       const UpdateArgs& u, int64_t B, int64_t D, int64_t L, int loss_kind, float grad_scale, int64_t ldxt, int max_ctas, cudaStream_t st,

@@ -1,9 +1,15 @@
 """Inference helpers for the FFI layer: per-row top-k labels without materialising the [B, L] logits.
 
 The reference's evaluation computes all logits and calls ``torch.topk(logits, 100)`` (src/evaluate.py:151-156;
-``topk(5)`` at :219).  At 670 K labels and a batch of 512 that matrix is 686 MB.  Here the label groups are
-processed in chunks sized to stay in L2: the forward kernel writes one chunk of logits, ``haste_topk_update`` folds
-it into the running top-k of every row, and the chunk buffer is reused.
+``topk(5)`` at :219).  At 670 K labels and a batch of 512 that matrix is 686 MB.  Three ways
+around it:
+
+  up to 8 rows    one kernel streams the weights on the CUDA cores and keeps k labels per segment, a second one merges
+  more rows       the logits of a sample of the labels set a bar per row, the forward kernels of the other labels keep only
+                  what beats it (the layer shapes the tcgen05 kernels have)
+  chunked         other shapes, or ``groups_per_chunk`` given: the label groups are processed in chunks sized to stay in L2,
+                  the forward kernel writes one chunk of logits, ``haste_topk_update`` folds it into the running top-k of
+                  every row, and the chunk buffer is reused
 """
 import torch
 
@@ -14,8 +20,9 @@ def ffi_topk(group_locations, weights, bias, features, k, group_size, *, groups_
     """Top-k logits and label ids of every row of ``features`` [B, D] (bf16, CUDA) under the FFI layer
     (``group_locations`` int32 [NG, F], ``weights`` bf16 [L, F], ``bias`` bf16 [L] or None).
 
-    Returns ``(values fp32 [B, k] descending, labels int32 [B, k])``; equal logits are ordered by label id, which
-    makes the result unique (``torch.topk`` leaves that order open).  ``label0`` is added to the label ids (for a
+    Returns ``(values fp32 [B, k] descending, labels int32 [B, k])``; equal logits are ordered by label id (``torch.topk``
+    leaves that order open).  Logits are rounded to bf16 after an fp32 sum; batches of up to 8 rows sum in another order than
+    larger ones, so the same row may get the neighbouring bf16 value at another batch size.  ``label0`` is added to the label ids (for a
     shard of a larger layer).  1 <= k <= 128.
     """
     if not 1 <= k <= 128:

@@ -88,9 +88,10 @@ int haste_ffi_backward_weights(const void* xt, const int32_t* loc, const void* d
                                haste_stream_t stream);
 
 /* Both gradients of the autograd backward from one pass over dy: dxt as haste_ffi_backward_features, dw / dbias
- * as haste_ffi_backward_weights (dbias may be NULL).  For (G=128, F=64) and (G=64, F=128) one
- * tcgen05 kernel reads dy once (xt rows at a stride that is a multiple of 8); its rows need no alignment beyond that of a bf16 (a contiguous [B, L] gradient
- * with odd L is read in place) and whatever lies in columns L..ldy-1 is ignored.  Otherwise the two warp-mma
+ * as haste_ffi_backward_weights (dbias may be NULL).  For (G, F) = (128, 64), (64, 128), (64, 64), (32, 64),
+ * (32, 32) and (32, 128), with xt rows at a stride that is a multiple of 8 (B % 8 == 0, or the ..._ldx form below), one
+ * tcgen05 kernel reads dy once; its rows need no alignment beyond that of a bf16 (a contiguous [B, L] gradient with odd L is read
+ * in place) and whatever lies in columns L..ldy-1 is ignored.  Otherwise the two warp-mma
  * kernels run back to back.  flags: HASTE_F_ZERO_DXT.
  * Replaces the pair of calls at shared_ffi/bindings.py:44 and :52. */
 int haste_ffi_backward(const void* xt, const void* w, const int32_t* loc, const void* dy, float* dxt, void* dw, void* dbias,
@@ -156,6 +157,9 @@ int haste_targets_bucket_noalloc(const int32_t* coo, int64_t nnz, int64_t label0
  *   dxt += backward-features; w,bias <- SGD(+wd)(+momentum) + stochastic rounding of backward-weights.
  * Neither z nor dy nor dw is written to memory.  Targets come from haste_targets_bucket.
  * loss (optional fp32 device scalar) is accumulated into when HASTE_F_LOSS is set.
+ * Accuracy of the BCE gradient: the sigmoid is that of fp32 exp (relative error about 2^-22), except for (G, F) = (128, 64) and
+ * (64, 128) with B % 8 == 0, where it comes from one tanh.approx (absolute error up to 2^-12, which exceeds the sigmoid itself
+ * for logits below about -8.3).  The loss value has the same errors.
  * Replaces GroupFFIMulFunction.forward/backward (shared_ffi/bindings.py:12-54), the loss of
  * src/runner.py:469-494 and SRSgd.step (shared_ffi/optim_sr.py:46-114) for this layer. */
 int haste_ffi_train_step(const int32_t* loc, const void* xt, void* w, void* bias,
@@ -312,7 +316,8 @@ int haste_ffi_topk(const int32_t* loc, const void* xt, const void* w, const void
  * kernels of the remaining labels keep only what beats it.  vals / idx are outputs (no start values).  `scratch`: 16-byte
  * aligned, haste_ffi_topk_fused_scratch(...) bytes; that function returns 0 for shapes that need haste_ffi_topk (and for
  * invalid ones).  It is up to 0.1 MB a row for at most 4096 rows at a time (54 MB for 512 rows of 670 K labels, 430 MB at
- * most); larger batches reuse it slice by slice.  Up to 8 rows take kilobytes.  Results as haste_ffi_topk up to the order of the fp32 sums of a logit. */
+ * most); larger batches reuse it slice by slice.  Up to 8 rows take kilobytes.  Results as haste_ffi_topk up to the order of the
+ * fp32 sums of a logit, which differs between the few-rows kernel and the others: a logit may round to the neighbouring bf16. */
 int64_t haste_ffi_topk_fused_scratch(int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k);
 int haste_ffi_topk_fused(const int32_t* loc, const void* x, const void* w, const void* bias, void* scratch, int64_t scratch_bytes,
                          int64_t B, int64_t D, int64_t F, int64_t L, int64_t G, int32_t k, int64_t label0,
