@@ -418,3 +418,20 @@ def test_step_on_fewer_ctas(G, F):
         _lib.check(_lib.lib.haste_ffi_set_max_ctas(0), "set_max_ctas")
     assert torch.equal(w, want_w) and torch.equal(b, want_b)
     assert few >= 3.0 * base
+
+
+@pytest.mark.parametrize("L", [18944 * 9 + 70, 18944 + 1, 200])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_topk_fused_sees_every_tile(G, F, L):
+    """One label of every tile in turn is the best there is: the sample and the filter launches together hold each tile once."""
+    from haste_b200.infer import ffi_topk
+    B, D, tile, k = 9, 16 * F, 64 if G == 32 and F < 128 else G, 128
+    loc = torch.arange((L + G - 1) // G * F, dtype=torch.int32, device="cuda").reshape(-1, F) % D
+    W, x = torch.zeros(L, F, dtype=torch.bfloat16, device="cuda"), torch.ones(B, D, dtype=torch.bfloat16, device="cuda")
+    for t0 in range(0, (L + tile - 1) // tile, k):
+        best = torch.arange(t0, min(t0 + k, (L + tile - 1) // tile)) * tile
+        best = torch.minimum(best + (best * 7 // tile) % tile, torch.tensor(L - 1))
+        bias = torch.zeros(L, dtype=torch.bfloat16)
+        bias[best] = 1.0
+        vals, idx = ffi_topk(loc, W, bias.cuda(), x, len(best), G)
+        assert torch.equal(idx.cpu(), best.to(torch.int32).expand(B, -1)) and (vals == 1.0).all()
