@@ -195,6 +195,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // Paired fp32 instructions: 670 K labels, hinge, 276.4 -> 271.5 us a step (three runs of each in turn); no gain for BCE, whose loop waits for the MUFU (2.8 M labels: 2,234
   // against 2,243 us), and a loss at 128 slots (501 K labels: 352 against 364 us), where 64 registers per thread spill.
   constexpr bool PAIRED = LOSS == HASTE_LOSS_SQHINGE && F == 64;
+  // Hinge without the loss sum, which is what tells of a NaN logit: max drops it.  Not for (128, 64) and (64, 128), which never did at
+  // multiples of 8 rows: 300 K labels (128, 64) 80 -> 84.5 us a step, the other shapes 0.5 to 1 %.
+  constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
 
   extern __shared__ uint8_t smem_raw[];
@@ -461,13 +464,27 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           // Y(t) complete implies forward(t) complete, so the tile's X stage is loaded as well
           const bool ok = mbar_wait(bar(C::B_YFULL + jy), jyph, abort_flag, a.err, 9, WL) && okd;
           tc_fence_after();
+          const int valid = static_cast<int>(imin64(BT, a.B - static_cast<int64_t>(tile_b0(t)))), nks = (valid + 15) / 16;
+          if (valid & 15) {
+            // A last tile with fewer rows: whole steps of 16 rows beyond the batch are left out, and dY of the rows that fill up the last
+            // step becomes 0 whatever their logits are (features of 0 times an infinite weight, an infinite bias).
+            // Backward-features reads these rows at the same time; what it makes of them is not used.  (In the loss
+            // epilogue, zeros after its loop cost every step 1 to 5 %, predicated stores in the loop 2 to 7 %.)
+            uint8_t* yst = sm + C::OFF_Y + jy * YSTAGE + valid * 128;
+            for (int i = lane; i < (nks * 16 - valid) * 8; i += 32) {
+#pragma unroll
+              for (int blk = 0; blk < C::NYB; ++blk) *reinterpret_cast<uint4*>(yst + blk * YBLK + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            fence_proxy_async();
+            __syncwarp();
+          }
           const uint32_t ym = ym_lo + static_cast<uint32_t>(jy) * (YSTAGE >> 4), xb = xb_lo + static_cast<uint32_t>(xs) * (XSTAGE >> 4);
           // dW[l,k] += sum over batch chunks of Y[b-chunk, l]^T * X[k, b-chunk]
           if (ok && elect_one()) {
             umma_bf16_lohi_rt(tdw, ym, ym_hi, xb, xb_hi, id_bww, t > 0);
 #pragma unroll
             for (int ks = 1; ks < BT / 16; ++ks)
-              umma_bf16_lohi<true>(tdw, ym + ((ks * 2048) >> 4), ym_hi, xb + (((ks >> 2) * XBLK + (ks & 3) * 32) >> 4), xb_hi, id_bww);
+              if (ks < nks) umma_bf16_lohi<true>(tdw, ym + ((ks * 2048) >> 4), ym_hi, xb + (((ks >> 2) * XBLK + (ks & 3) * 32) >> 4), xb_hi, id_bww);
             tc_commit(bar(C::B_YEMPTY + jy));
             tc_commit(bar(C::B_XEMPTY + xs));
             if (t + 1 == T) tc_commit(bar(C::B_DWFULL));
@@ -590,8 +607,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   // logits are rounded to bf16 first, as the unfused forward stores them
                   const F2 z2 = {round_bf16_as_f32(__uint_as_float(r[e8 + i])), round_bf16_as_f32(__uint_as_float(r[e8 + i + 1]))};
                   const F2 x2 = fma2<PAIRED>({gs2, gs2}, z2, {gs2, gs2});
-                  // (without the loss sum nothing would tell of a NaN: max drops it here)
-                  x[i] = WITH_LOSS ? x2.x : fmaxf(x2.x, 0.f); x[i + 1] = WITH_LOSS ? x2.y : fmaxf(x2.y, 0.f);
+                  x[i] = DROP_NAN ? fmaxf(x2.x, 0.f) : x2.x; x[i + 1] = DROP_NAN ? fmaxf(x2.y, 0.f) : x2.y;
                   if (WITH_LOSS) { const F2 m2 = {x2.x + fabsf(x2.x), x2.y + fabsf(x2.y)}; fh[(i >> 1) & 1] = fma2<PAIRED>(m2, m2, fh[(i >> 1) & 1]); }
                 }
                 pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
@@ -668,9 +684,8 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             }
           }
         }
-        // Hinge: a logit that is infinite or NaN (a label masked by its bias) leaves x + |x| undefined, and in a row beyond the batch, where
-        // s = 0 and the logits are the biases, x itself.  Such a tile goes through the general branch, which has a value for it;
-        // so does one whose sum of squares overflows.  (max(x, 0) in place of x + |x| needs no second pass and took 1.6 % more
+        // Hinge: a logit that is infinite or NaN (a label masked by its bias) leaves x + |x| undefined.  Such a tile goes through the
+        // general branch, which has a value for it; so does one whose sum of squares overflows.  (max(x, 0) in place of x + |x| needs no second pass and took 1.6 % more
         // of the 670 K step: 276.9 against 272.5 us; this way 274.3.  BCE sums max(z, 0): 2.8 M labels 2,310 against 2,320 us.)
         if (LOSS != HASTE_LOSS_SQHINGE || !WITH_LOSS || DEBUG || ragged || !__any_sync(0xffffffffu, !(fast_loss < INFINITY))) break;
         ragged = true;

@@ -235,6 +235,31 @@ def test_step_with_masked_labels(G, F, loss, B, mask):
         assert not torch.equal(sh.w.cpu()[~masked], inp["W"][~masked])
 
 
+@pytest.mark.parametrize("loss", ["bce", "squared_hinge"])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_step_rows_beyond_the_batch_never_reach_the_gradients(G, F, loss):
+    """Infinite weights and biases give those rows logits that are not finite.  Weight gradients are sums over the batch's rows
+    alone: with B = 1 and finite loss gradients they stay finite, and an infinite one stays infinite."""
+    from haste_b200.fused import FusedFFIShard
+    B, D, L = 1, 264, 3 * G + 7
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=2, x_kind="relu", bias_zero=False)
+    inp["X"] += 0.25                                        # positive: an infinite weight gives an infinite logit, not a NaN
+    inp["W"][5, 3], inp["W"][G, 1] = float("-inf"), float("-inf")
+    inp["bias"][9] = float("inf")
+    sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), inp["bias"].clone().cuda(), G, D, loss=loss, lr=0.05, momentum=0.9, seed=3)
+    sh.step(inp["X"].cuda(), torch.zeros(0, 2, dtype=torch.int32, device="cuda"))
+    mom_w, mom_b = sh.mom_w.cpu(), sh.mom_b.cpu()           # gradients (weight decay 0 leaves a NaN where the weight is infinite)
+    at = torch.isinf(inp["W"].float())
+    assert torch.isfinite(mom_w[[5, G]][~at[[5, G]]]).all() and (mom_b[[5, G]] == 0).all()
+    if loss == "squared_hinge":
+        assert torch.isinf(mom_w[9]).all()
+    else:
+        assert torch.isfinite(mom_w[9]).all()
+    rest = torch.ones(L, dtype=torch.bool)
+    rest[[5, G, 9]] = False
+    assert torch.isfinite(mom_w[rest]).all() and torch.isfinite(mom_b[rest]).all()
+
+
 @pytest.mark.parametrize("scale", [0.0, -0.5, 1e-22, 1e-9, 2.0 ** 40])
 @pytest.mark.parametrize("G,F", [(32, 32), (128, 64)])
 def test_hinge_step_with_any_gradient_scale(G, F, scale):
