@@ -25,13 +25,16 @@
 //   backward-weights   dW [l,k] (TMEM, F+16 cols, accumulated over the batch tiles; M = G)
 //                                                = Y^T (MN-major A) * X (K-major B),         K = 128; column F of the
 //                                                  result (the ones row) is the bias gradient
-// Warp roles: 4 producer warps (warp 0 loads the W tile through a tensor map; all four gather X tiles with TMA
-// tile::gather4, one instruction per lane and tile — the gather rate grows with the number of issuing warps),
-// warp 1 issues forward + backward-features, warp 3 issues backward-weights, 8 loss-epilogue warps turn Z into dY
-// (bf16 rounding of the logit, loss gradient, target bits) and store it swizzled, 4 (F=64) or 8 (F=128) scatter
-// warps drain dXg (TMEM -> registers -> coalesced red.global.add into dxt rows), 8 update warps apply SGD + weight
-// decay (+ momentum) + stochastic rounding to the weights and bias straight from the dW accumulator.  Logits, dY
+// Warp roles (31 warps): warp 0 brings a group's weights (tensor map), index row, bias and targets; 4 warps gather X tiles with TMA
+// tile::gather4, warp 1 issues forward + backward-features, warp 3 issues backward-weights, 8 loss-epilogue warps turn Z into dY
+// (bf16 rounding of the logit, loss gradient, target bits) and store it swizzled, 8 scatter warps drain dXg (TMEM ->
+// registers -> shared memory -> 16-byte reductions into dxt rows), 8 update warps apply SGD + weight
+// decay (+ momentum) + stochastic rounding to the weights and bias from the dW accumulator.  Logits, dY
 // and dW never reach global memory.
+// What bounds the kernel is what its roles share: issue slots (0.66 of them used, 670 K labels), the instruction cache (31 warps run six
+// different loops; with the loops unrolled a quarter of the warps' stalls were for instructions), the L1 data
+// pipe (tensor core operands, shared memory and global accesses: 82 % busy) and at 128 slots the L2's reductions.  So
+// the hot loops are small and rolled, and what a role writes to memory leaves in whole lines.
 // All hand-offs are mbarriers with bounded waits; a wait that gives up raises a CTA-wide abort flag, every role
 // drains its loops without touching global memory, TMEM is freed and the host sees HASTE_ERR_TIMEOUT.
 #pragma once
@@ -64,7 +67,7 @@ struct Cfg {
   static_assert(P == 1 || P == 2, "groups per tile");
   static_assert(FF == 32 || FF % 64 == 0, "a weight row fills 64-byte or 128-byte swizzled rows");
   static constexpr int FR = F + 16;                   // rows of an X block: F gathered rows, one row of ones, 15 zero rows
-  static constexpr int NXS = (F == 64) ? 5 : 4;       // X ring stages
+  static constexpr int NXS = (F == 64) ? 4 : 3;       // X ring stages
   static constexpr int NYS = 2;                       // dY ring stages
   static constexpr int NDX = (F == 64) ? 2 : 1;       // dXg accumulator stages in TMEM
   static constexpr int XBLK = FR * 128;               // one 64-batch block of an X stage (bytes)
@@ -73,6 +76,7 @@ struct Cfg {
   static constexpr int NWB = FF == 32 ? 1 : FF / 64;  // blocks of a W stage (64 slots each, 32 at fan-in 32)
   static constexpr int WBLK = G * WROW;
   static constexpr int WSTAGE = NWB * WBLK;
+  static constexpr int WBYTES = NWB * LS * WROW;      // what is loaded and stored of it
   static constexpr int NYB = G / 64;                  // 64-label blocks of a dY stage
   static constexpr int YBLK = BT * 128;
   static constexpr int YSTAGE = NYB * YBLK;
@@ -82,9 +86,15 @@ struct Cfg {
   static constexpr int OFF_Y = OFF_W + 2 * WSTAGE;
   static constexpr int OFF_BT = OFF_Y + NYS * YSTAGE;
   static constexpr int OFF_LOC = OFF_BT + 2 * BTILE;           // u32 [2][F]: element offset loc * B of each slot's dxt row
-  static constexpr int OFF_LOCR = OFF_LOC + 2 * F * 4;         // int [4][F]: each producer warp's copy of the group's (clamped) indices, for the gather
-  static constexpr int OFF_YB = OFF_LOCR + 4 * F * 4;          // u32 [2][BT][G/32]: target bits
-  static constexpr int OFF_BAR = OFF_YB + 2 * BT * (G / 32) * 4;
+  static constexpr int OFF_YB = OFF_LOC + 2 * F * 4;           // u32 [2][BT][G/32]: target bits
+  static constexpr int NTE = 8;                                // target entries of a group that go through shared memory
+  static constexpr int OFF_TGT = OFF_YB + 2 * BT * (G / 32) * 4;     // u32 [2][4 + NTE]: first, middle and last entry of the tile's groups, entries
+  // (8 slots: 131 K labels 145 -> 164 us; 32: 670 K 252 -> 263)
+  static constexpr int EBP = 16;                               // slots of dXg a scatter warp turns around at a time
+  static constexpr int OFF_EB = (OFF_TGT + 2 * (4 + NTE) * 4 + 127) / 128 * 128;      // float [8 scatter warps][EBP][32 batch rows]
+  static constexpr int OFF_G = OFF_EB + 8 * EBP * 128;         // bf16 [8 update warps][label rows][slots]: gradients on their way to the update
+  static constexpr int GSTAGE = (G / 4) * (FF / 2) * 2;        // of one update warp: the rows of a TMEM lane quarter (absent labels too), half the slots
+  static constexpr int OFF_BAR = OFF_G + 8 * GSTAGE;
   static constexpr int OFF_MISC = OFF_BAR + 32 * 8;            // tmem base address, abort flag
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;      // + slack for the 1024-byte alignment of the base
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
@@ -102,14 +112,15 @@ struct Cfg {
   static_assert(TM_DW + FR <= TM_COLS, "TMEM budget");
 
   static constexpr int N_EA = 8;                      // loss-epilogue warps: 4 TMEM lane quarters x 2 column halves
-  static constexpr int EBS = 64;                      // slots per scatter warp
-  static constexpr int N_EB = 4 * (F / EBS);          // scatter warps: 4 TMEM lane quarters x 64-slot chunks
+  static constexpr int N_EB = 8;                      // scatter warps: 4 TMEM lane quarters x 2 slot halves
+  static constexpr int EBS = F / 2;                   // slots per scatter warp
   static constexpr int N_UP = 8;                      // update warps: 4 TMEM lane quarters x 2 slot halves
   static constexpr int W_EA = 4, W_EB = W_EA + N_EA, W_UP = W_EB + N_EB;
-  static constexpr int NPW = 4;                       // producer warps: warp 0, warp 2, then extra warps after the update warps
-  static_assert(NPW >= 1 && NPW <= NXS, "a producer must not run more than one phase ahead on any stage barrier");
+  static constexpr int NPW = 4;                       // X producer warps: warp 2, then extra warps after the update warps
+  static constexpr int NSH = G * F == 64 * 64 ? 4 : 2;          // producer warps that share a tile
+  static_assert(NPW / NSH <= NXS, "a producer must not run more than one phase ahead on any stage barrier");
   static constexpr int W_XP = W_UP + N_UP;            // first extra producer warp
-  static constexpr int NTHREADS = (W_XP + (NPW > 2 ? NPW - 2 : 0)) * 32;
+  static constexpr int NTHREADS = (W_XP + NPW - 1) * 32;
   static_assert(NTHREADS <= 1024, "thread budget");
   static constexpr int EA_COLS = G * 4 / N_EA;        // label columns of a tile handled by one loss-epilogue warp
   static constexpr int UPS = FF / 2;                  // slots updated by one update warp
@@ -134,6 +145,7 @@ struct StepArgs {
   int D, NG;           // NG: tiles of LS labels
   int NGR;             // label groups (index rows, target buckets)
   float grad_scale;
+  int dxt_v4;          // rows of dxt are 16-byte aligned
   long long wait_limit;
   int stall_tile;      // debug builds: the first loss-epilogue warp withholds its "dY ready" arrival at this tile (-1 = never)
   // optional debug outputs (NULL in production): the bf16 logits and the bf16 gradients the update consumed
@@ -198,6 +210,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // Hinge without the loss sum, which is what tells of a NaN logit: max drops it.  Not for (128, 64) and (64, 128), which never did at
   // multiples of 8 rows: 300 K labels (128, 64) 80 -> 84.5 us a step, the other shapes 0.5 to 1 %.
   constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
+  // Positives put right after the plain loop: 31 K labels, B=64, G=32 21.0 -> 20.2 us; not for (128, 64), whose tiles hardly ever have one (670 K
+  // labels, hinge 240 -> 247 us, 2.8 M, BCE 2,233 -> 2,418: the loop's registers).
+  constexpr bool PATCH = GG != 128;
+  // Two chunks per pass of the loss epilogue's plain loop hide some of the MUFU's latency: 2.8 M labels, BCE, 2,284 -> 2,235 us; the other
+  // instantiations lose by it (501 K labels 278 -> 297, hinge 670 K 252 -> 253: instruction cache).
+  constexpr int UNROLL = LOSS == HASTE_LOSS_BCE && F == 64 ? 2 : 1;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
 
   extern __shared__ uint8_t smem_raw[];
@@ -222,7 +240,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
 
   // ---------------- one-time setup
   if (tid == 0) {
-    for (int i = 0; i < NXS; ++i) { mbar_init(bar(C::B_XFULL + i), 1); mbar_init(bar(C::B_XEMPTY + i), 1); }   // X stage: one arrival that announces the gathered bytes
+    for (int i = 0; i < NXS; ++i) { mbar_init(bar(C::B_XFULL + i), C::NSH); mbar_init(bar(C::B_XEMPTY + i), 1); }   // X stage: each producer announces its bytes
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(C::B_WFULL + i), 1);  mbar_init(bar(C::B_WEMPTY + i), 1);
       mbar_init(bar(C::B_ZFULL + i), 1);  mbar_init(bar(C::B_ZEMPTY + i), N_EA);
@@ -266,23 +284,21 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   const int n_my_groups = full_rounds + (cta >= n_cta - rem_groups ? 1 : 0);
   auto group_of = [&](int gi) { return gi < full_rounds ? cta + gi * n_cta : full_rounds * n_cta + (cta - (n_cta - rem_groups)); };
 
-  const int prod_id = warp == 0 ? 0 : (warp == 2 ? 1 : (warp >= C::W_XP ? 2 + warp - C::W_XP : -1));
-  if (prod_id >= 0 && prod_id < C::NPW) {
-    // ================================================================ producers
-    // Per group: the index row (as dxt row offsets for the scatter warps) and the bias column go to shared memory
-    // with ordinary stores, the W tile comes through the tensor map.  Per batch tile: F index rows of xt, 256 bytes
-    // each, as F/4 TMA gather4 loads per 64-batch block (four index rows per instruction, landing at their swizzled
-    // positions); lane 0 arms the stage's barrier with the byte count, then every lane issues its share.
-    // The W item of every group belongs to producer 0; the X items (one per batch tile) are dealt round-robin.
-    int it = 0;                  // X items so far (all producers count all of them)
+  const int prod_id = warp == 2 ? 0 : (warp >= C::W_XP ? 1 + warp - C::W_XP : -1);
+  if (warp == 0) {
+    // ================================================================ group producer
+    // Per group: the index row (as dxt row offsets for the scatter warps), the bias column and the group's targets go to shared
+    // memory with ordinary stores, the W tile comes through the tensor map.  (One of the X producers used to do this: its wait for the
+    // stage, which ends when the update of the group before last has finished, then held up its X tiles.)
     int w_armed = 0;             // W stages armed so far
-    int my_last = -1;            // last X item this warp actually issued
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int ws = gi & 1;
       const int64_t l0 = static_cast<int64_t>(g) * LS;
       const int rows_real = static_cast<int>(imin64(LS, a.L - l0));
       const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
+      const int t_beg = __ldg(a.tgt_ptr + g * P), t_end = __ldg(a.tgt_ptr + min(g * P + P, a.NGR));
+      const int t_mid = P == 1 ? t_end : __ldg(a.tgt_ptr + g * P + 1);
       int locv[F / 32];
 #pragma unroll
       for (int j = 0; j < F / 32; ++j) {
@@ -290,7 +306,6 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const bool there = P == 1 || lane + 32 * j < (a.NGR - g * P) * FF;
         locv[j] = there ? min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1) : 0;   // clamped: never addresses outside xt / dxt
       }
-      if (prod_id == 0) {
       uint16_t bv[G / 32];
 #pragma unroll
       for (int j = 0; j < G / 32; ++j) {
@@ -300,10 +315,25 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 1, WL, 100);
       ok = mbar_wait(bar(C::B_MEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 1, WL, 100) && ok;
       __syncwarp();
+      const bool go = __all_sync(0xffffffffu, ok && !*abort_flag);
+      if (go) {
+        // the weights first: their way from memory is the longest
+        if (lane == 0) {
+          mbar_expect_tx(bar(C::B_WFULL + ws), C::WBYTES);
+#pragma unroll
+          for (int kb = 0; kb < C::NWB; ++kb)
+            tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
+        }
+        ++w_armed;
+      }
+      // lanes 0 .. 2: entry range of the tile's groups, lanes 4 .. 4 + NTE - 1: the first entries
+      uint32_t tv = lane == 0 ? t_beg : (lane == 1 ? t_mid : t_end);
+      if (lane >= 4 && t_beg + lane - 4 < t_end && lane < 4 + C::NTE) tv = __ldg(a.tgt_ent + t_beg + lane - 4);
 #pragma unroll
       for (int j = 0; j < F / 32; ++j) {
         loc_s[ws * F + lane + 32 * j] = static_cast<uint32_t>(locv[j]) * static_cast<uint32_t>(a.B);   // D * B < 2^32 is a launch condition
       }
+      if (lane < 4 + C::NTE) reinterpret_cast<uint32_t*>(sm + C::OFF_TGT)[ws * (4 + C::NTE) + lane] = tv;
 #pragma unroll
       for (int j = 0; j < G / 32; ++j) {
         const int c = lane + 32 * j;
@@ -311,49 +341,52 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       }
       fence_proxy_async();
       __syncwarp();
-      if (ok && !*abort_flag) {
-        if (lane == 0) {
-          mbar_arrive_expect_tx(bar(C::B_WFULL + ws), WSTAGE);
-#pragma unroll
-          for (int kb = 0; kb < C::NWB; ++kb)
-            tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
-        }
-        ++w_armed;
-      }
+      if (go && lane == 0) mbar_arrive(bar(C::B_WFULL + ws));
       __syncwarp();
-      }
-      // this warp's own copy of the index row, read back four slots at a time for the gathers
-      int* locr = reinterpret_cast<int*>(sm + C::OFF_LOCR) + prod_id * F;
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < F / 32; ++j) locr[lane + 32 * j] = locv[j];
-      __syncwarp();
-      const int4* lr4 = reinterpret_cast<const int4*>(locr);
-      for (int t = 0; t < T; ++t, ++it) {
-        if (it % C::NPW != prod_id) continue;
-        const int xs = it % NXS;
-        const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 2, WL, 100);
-        __syncwarp();
-        if (!okx || *abort_flag) continue;
-        const int b0 = tile_b0(t);
-        const uint32_t xb = sbase + C::OFF_X + xs * XSTAGE;
-        if (lane == 0) mbar_arrive_expect_tx(bar(C::B_XFULL + xs), F * 256);
-        __syncwarp();
-#pragma unroll
-        for (int i = lane; i < 2 * (F / 4); i += 32) {        // one gather4 per four slots and 64-batch block
-          const int blk = i / (F / 4), r4 = i % (F / 4);
-          const int4 lr = lr4[r4];
-          tma_gather4(xb + blk * XBLK + r4 * 512, &tm_x, b0 + blk * 64, lr.x, lr.y, lr.z, lr.w, bar(C::B_XFULL + xs));
-        }
-        my_last = it;
-      }
     }
     // Every copy this warp started has to land before the CTA may exit (normally the consumers have long seen them;
     // after an abort nobody else waits any more).
-    // (only the most recent use of each stage: an older phase of the same barrier can no longer be waited for)
-    for (int j = max(0, it - NXS); j < it; ++j)
-      if (j % C::NPW == prod_id && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
     for (int j = max(0, w_armed - 2); j < w_armed; ++j) mbar_wait_final(bar(C::B_WFULL + (j & 1)), (j >> 1) & 1, WL);
+  } else if (prod_id >= 0 && prod_id < C::NPW) {
+    // ================================================================ X producers
+    // Per batch tile: F index rows of xt, 256 bytes each, as F/4 TMA gather4 loads per 64-batch block (four index rows per
+    // instruction, landing at their swizzled positions).  Every warp loads its share of every tile, one instruction per lane, and
+    // announces its own bytes: a warp issues one of these loads per 80 to 130 cycles, so that a tile of 64 slots from one warp was 4,300
+    // cycles on its way.  Two warps to a tile: 501 K labels 298 -> 280 us (four: 284), 670 K unchanged; four where tiles are small:
+    // 31 K labels 21.5 -> 21.0 us.
+    constexpr int NLD = 2 * (F / 4) / C::NSH, STEP = C::NPW / C::NSH;            // loads per warp and tile; tiles between two of a warp
+    static_assert(NLD * C::NSH == 2 * (F / 4) && NLD <= 32, "one load per lane");
+    const int li = (prod_id % C::NSH) * NLD + lane, blk = li / (F / 4), r4 = li % (F / 4);
+    int4 lr = make_int4(0, 0, 0, 0);
+    int t = prod_id / C::NSH, gi = 0, g_have = -1, my_last = -1;
+    const int n_items = n_my_groups * T;
+    for (int it = t; it < n_items; it += STEP, t += STEP) {
+      while (t >= T) { t -= T; ++gi; }
+      if (gi != g_have) {
+        g_have = gi;
+        const int g = group_of(gi);
+        const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F + r4 * 4;
+        // the last tile may hold one group less: its slots gather row 0 and meet zero weights and zero dY
+        const bool there = lane < NLD && (P == 1 || r4 * 4 < (a.NGR - g * P) * FF);
+        const int top = a.D - 1;                         // clamped: never addresses outside xt
+        lr.x = there ? min(max(__ldg(lrow), 0), top) : 0; lr.y = there ? min(max(__ldg(lrow + 1), 0), top) : 0;
+        lr.z = there ? min(max(__ldg(lrow + 2), 0), top) : 0; lr.w = there ? min(max(__ldg(lrow + 3), 0), top) : 0;
+      }
+      const int xs = it % NXS;
+      const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 2, WL, 100);
+      __syncwarp();
+      if (!okx || *abort_flag) continue;
+      const uint32_t full = bar(C::B_XFULL + xs);
+      if (lane == 0) mbar_arrive_expect_tx(full, NLD * 512);
+      __syncwarp();
+      if (lane < NLD)
+        tma_gather4(sbase + C::OFF_X + xs * XSTAGE + blk * XBLK + r4 * 512, &tm_x, tile_b0(t) + blk * 64, lr.x, lr.y, lr.z, lr.w, full);
+      my_last = it;
+    }
+    // Every copy this warp started lands before the CTA may exit.  (Only the most recent use of each stage: an older phase of the same
+    // barrier can no longer be waited for.)
+    for (int j = max(0, n_items - NXS); j < n_items; ++j)
+      if (j % STEP == prod_id / C::NSH && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
   } else if (warp == 1 || warp == 3) {
     // ================================================================ MMA issuers (one elected lane each)
     // Feeding the tensor pipe from a single thread costs more cycles per tcgen05.mma than the small (N = 64..144)
@@ -401,7 +434,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             constexpr int KS = GG / 16;
             umma_bf16_lohi<false>(tdx + p * FF, ya + ((((p * KS) >> 2) * YBLK + ((p * KS) & 3) * 32) >> 4), ya_hi,
                                   wm + ((p * KS * 16 * C::WROW) >> 4), wm_hi, id_bwx);
-#pragma unroll
+#pragma unroll 1
             for (int ks = p * KS + 1; ks < (p + 1) * KS; ++ks)
               umma_bf16_lohi<true>(tdx + p * FF, ya + (((ks >> 2) * YBLK + (ks & 3) * 32) >> 4), ya_hi, wm + ((ks * 16 * C::WROW) >> 4), wm_hi, id_bwx);
           }
@@ -418,10 +451,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const int ws = gi & 1;
         // the W stage of this group was last used by group gi - 2: its products must all be issued before the
         // stage can be refilled (matters only when a group has a single tile)
-        while (j < it && j_g + 2 <= gi) backward_x();
+        // Nor does a backward product that is due wait for weights or features that are still on their way.
+        while (j < it && (j_g + 2 <= gi || !__all_sync(0xffffffffu, mbar_test(bar(C::B_WFULL + ws), (gi >> 1) & 1)))) backward_x();
         const bool okw = mbar_wait(bar(C::B_WFULL + ws), (gi >> 1) & 1, abort_flag, a.err, 5, WL);
         for (int t = 0; t < T; ++t, ++it) {
           const int zs = it & 1;
+          if (j < it && !__all_sync(0xffffffffu, mbar_test(bar(C::B_XFULL + xs), xph))) backward_x();
           bool ok = mbar_wait(bar(C::B_XFULL + xs), xph, abort_flag, a.err, 6, WL) && okw;
           ok = mbar_wait(bar(C::B_ZEMPTY + zs), ((it >> 1) & 1) ^ 1, abort_flag, a.err, 7, WL) && ok;
           tc_fence_after();
@@ -434,7 +469,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             for (int p = 0; p < P; ++p) {        // group p of the tile: its slots against its labels' weight rows
               const uint32_t xp = xa + ((p * FF * 128) >> 4), wp = wb + ((p * GG * C::WROW) >> 4);
               umma_bf16_lohi<false>(tz + p * GG, xp, xa_hi, wp, wb_hi, id_fwd);
-#pragma unroll
+#pragma unroll 1
               for (int ks = 1; ks < FF / 16; ++ks)
                 umma_bf16_lohi<true>(tz + p * GG, xp + ((ks * 2048) >> 4), xa_hi, wp + (((ks >> 2) * WBLK + (ks & 3) * 32) >> 4), wb_hi, id_fwd);
             }
@@ -443,7 +478,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           }
           __syncwarp();
           if (++xs == NXS) { xs = 0; xph ^= 1; }
-          if (it >= 1) backward_x();
+          if (j < it) backward_x();
         }
       }
       while (j < it) backward_x();
@@ -482,7 +517,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           // dW[l,k] += sum over batch chunks of Y[b-chunk, l]^T * X[k, b-chunk]
           if (ok && elect_one()) {
             umma_bf16_lohi_rt(tdw, ym, ym_hi, xb, xb_hi, id_bww, t > 0);
-#pragma unroll
+#pragma unroll 1
             for (int ks = 1; ks < BT / 16; ++ks)
               if (ks < nks) umma_bf16_lohi<true>(tdw, ym + ((ks * 2048) >> 4), ym_hi, xb + (((ks >> 2) * XBLK + (ks & 3) * 32) >> 4), xb_hi, id_bww);
             tc_commit(bar(C::B_YEMPTY + jy));
@@ -511,24 +546,31 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       const int g = group_of(gi);
       const int ws = gi & 1;
       const int rows_real = static_cast<int>(imin64(LS, a.L - static_cast<int64_t>(g) * LS));
-      // entries of the tile's groups are contiguous; those from t_mid on belong to the second group of a pair
-      const int t_beg = __ldg(a.tgt_ptr + g * P), t_end = __ldg(a.tgt_ptr + min(g * P + P, a.NGR));
-      const int t_mid = P == 1 ? t_end : __ldg(a.tgt_ptr + g * P + 1);
-      const bool has_t = t_end > t_beg;
+      // the group producer left the entry range (contiguous; entries from t_mid on belong to the second group of a pair) and the first entries
+      const uint32_t* tgt_s = reinterpret_cast<const uint32_t*>(sm + C::OFF_TGT) + ws * (4 + C::NTE);
+      mbar_wait(bar(C::B_WFULL + ws), (gi >> 1) & 1, abort_flag, a.err, 16, WL);
+      const uint4 tr = *reinterpret_cast<const uint4*>(tgt_s);
+      const int t_beg = static_cast<int>(tr.x), t_mid = static_cast<int>(tr.y), t_end = static_cast<int>(tr.z);
       for (int t = 0; t < T; ++t) {
         const int zs = it & 1;
         const int b0 = tile_b0(t);
         uint64_t ym = 0ull;                              // target bits of this thread's row, EA_COLS label columns
-        if (has_t && t_end - t_beg <= 8) {
-          // Few targets in this group (the common case): each thread picks the bits of its own row and its label
-          // columns straight from the entry list — no shared bitmap, no barrier between the epilogue warps.
+        // Few targets in the tile's groups (the common case).  PATCH: the plain loop treats every label as a negative, and the few
+        // positives are put right one by one afterwards; their bits are only collected where the other loop is taken.
+        // Otherwise each thread picks the bits of its own row and its label columns from the entry list (no shared
+        // bitmap, no barrier between the epilogue warps), and tiles with targets take the other loop.
+        const bool few = t_end - t_beg <= C::NTE;
+        auto few_bits = [&]() {
           const uint32_t rowkey = static_cast<uint32_t>(b0 + row);
           for (int i = t_beg; i < t_end; ++i) {
-            const uint32_t e = __ldg(a.tgt_ent + i);
+            const uint32_t e = tgt_s[4 + i - t_beg];
             const uint32_t c = (e & 0xFFu) + (P == 2 && i >= t_mid ? GG : 0) - static_cast<uint32_t>(h * EA_COLS);
             if ((e >> 8) == rowkey && c < static_cast<uint32_t>(EA_COLS)) ym |= 1ull << c;
           }
-        } else if (has_t) {
+        };
+        if (few) {
+          if (!PATCH) few_bits();
+        } else {
           uint32_t* yb = ybits + (it & 1) * BT * YBW;
           for (int i = et; i < BT * YBW; i += N_EA * 32) yb[i] = 0u;
           named_bar_sync(1, N_EA * 32);
@@ -565,13 +607,110 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         bool ragged = col0 + EA_COLS > rows_real;     // only the last tile of the layer can be ragged (and absent columns)
         float tile_loss = 0.f, fast_loss = 0.f;             // fast_loss: hinge (4s)^2-scaled squares, or BCE raw log2 terms
         const float hgs = 0.5f * gs;
-        // 16 label columns per iteration.  Nearly every chunk has no positive label in the warp's 32 rows and no
-        // ragged edge: one warp vote per chunk sends those down a branch with no per-element tests; the rest take
-        // the general branch with target bits and a column-valid mask.
-        // (not unrolled: two iterations per loop body cost 27 % of the kernel's time, four 40 %, measured; moving the
-        // general branch out of line, to shrink the loop instead, changed nothing)
         constexpr int CH = 16;                             // label columns per TMEM load
+        // One chunk without targets or absent columns: gradients of its 16 logits, stored swizzled; loss terms into fh / fl / bce_prod.
+        F2 fh[2] = {{0.f, 0.f}, {0.f, 0.f}};               // hinge: (4s)^2-scaled squares
+        float fl[4] = {0.f, 0.f, 0.f, 0.f};                // BCE: max(z, 0); partial sums, no serial dependency through one accumulator
+        auto plain_chunk = [&](const uint32_t (&r)[CH], uint8_t* yblk, int chunk0) {
+          float bp[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+          for (int e8 = 0; e8 < CH; e8 += 8) {
+            uint4 pk;
+            float x[8];
+            if (LOSS == HASTE_LOSS_SQHINGE) {
+              // dLoss/dz = 2 s max(0, 1 + z) with s = grad_scale, evaluated as max(0, fma(2s, z, 2s)); 1 + z is
+              // exact in fp32 for a bf16 z (down to |z| ~ 2^-16), so this is the same single rounding as
+              // (1 + z) * 2s.  The max is left to the bf16 conversion.  The loss term max(0,1+z)^2 is accumulated
+              // as (x + |x|)^2 = (2 max(0,x))^2 and rescaled by 1/(4s)^2 once per tile.
+#pragma unroll
+              for (int i = 0; i < 8; i += 2) {
+                // logits are rounded to bf16 first, as the unfused forward stores them
+                const F2 z2 = {round_bf16_as_f32(__uint_as_float(r[e8 + i])), round_bf16_as_f32(__uint_as_float(r[e8 + i + 1]))};
+                const F2 x2 = fma2<PAIRED>({gs2, gs2}, z2, {gs2, gs2});
+                x[i] = DROP_NAN ? fmaxf(x2.x, 0.f) : x2.x; x[i + 1] = DROP_NAN ? fmaxf(x2.y, 0.f) : x2.y;
+                if (WITH_LOSS) { const F2 m2 = {x2.x + fabsf(x2.x), x2.y + fabsf(x2.y)}; fh[(i >> 1) & 1] = fma2<PAIRED>(m2, m2, fh[(i >> 1) & 1]); }
+              }
+              pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
+            } else if (LOSS == LOSS_BCE_EXP) {
+              // dLoss/dz = s sigmoid(z) = s / (1 + e^-z); loss term softplus(z) = max(z,0) - ln(0.5 + |sigmoid - 0.5|),
+              // whose logarithm arguments lie in [0.5, 1] as below
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
+                const float sg = sigmoid_exp(zr);
+                x[i] = sg * gs;
+                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & 3] *= 0.5f + fabsf(sg - 0.5f); }
+              }
+              pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+            } else {
+              // dLoss/dz = s sigmoid(z) = s/2 + s/2 tanh(z/2) (one MUFU op, one fma); loss term softplus(z) =
+              // max(z,0) - ln(0.5 + 0.5 |tanh(z/2)|).  The logarithm arguments
+              // lie in [0.5, 1], so the 16 of a chunk are multiplied together (>= 2^-16) and one log2 is taken.
+              // (twice each argument is multiplied, 1 + |tanh| being one instruction, and 2^-16 taken off the product: the same bits)
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
+                const float th = tanh_approx(0.5f * zr);
+                x[i] = fmaf(hgs, th, hgs);
+                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & 3] *= 1.f + fabsf(th); }
+              }
+              pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+            }
+            *reinterpret_cast<uint4*>(yblk + (((chunk0 + (e8 >> 3)) ^ (row & 7)) << 4)) = pk;
+          }
+          if (WITH_LOSS && LOSS != HASTE_LOSS_SQHINGE)
+            fast_loss += __log2f(((bp[0] * bp[1]) * (bp[2] * bp[3])) * (LOSS == HASTE_LOSS_BCE ? 0x1p-16f : 1.f));
+        };
+        // Without a target in a warp's 32 rows and 64 columns, or with few, and without a ragged edge: a loop with nothing but the arithmetic.
+        bool plain = !DEBUG && !ragged && ((PATCH && few) || !__any_sync(0xffffffffu, ym != 0ull));
+        if (PATCH && few && !plain) few_bits();
         for (;;) {                                         // one pass; rarely a second (below)
+        bool again = false;
+        if (plain) {
+          __syncwarp();
+#pragma unroll UNROLL
+          for (int c16 = 0; c16 < EA_COLS; c16 += CH) {
+            uint32_t r[CH];
+            tmem_ld(ta + c16, r);
+            tmem_ld_wait();
+            plain_chunk(r, yrow + ((col0 + c16) >> 6) * YBLK, ((col0 + c16) & 63) >> 3);
+          }
+          if (PATCH && few) {
+#pragma unroll 1
+            for (int i = t_beg; i < t_end; ++i) {
+              const uint32_t e = tgt_s[4 + i - t_beg];
+              const uint32_t c = (e & 0xFFu) + (P == 2 && i >= t_mid ? GG : 0) - static_cast<uint32_t>(h * EA_COLS);
+              const uint32_t rw = (e >> 8) - static_cast<uint32_t>(b0 + q * 32);           // row and column of the warp's part of the tile
+              if (rw >= 32u || c >= static_cast<uint32_t>(EA_COLS)) continue;             // (uniform)
+              bool twice = false;                                                         // the same target listed before
+              for (int k = t_beg; k < i; ++k) twice = twice || (tgt_s[4 + k - t_beg] == e && (P == 1 || (k >= t_mid) == (i >= t_mid)));
+              __syncwarp();
+              const uint32_t zb = tmem_ld1(ta + c);
+              tmem_ld_wait();
+              if (lane == static_cast<int>(rw) && !twice) {
+                const float zr = round_bf16_as_f32(__uint_as_float(zb));
+                float gl, la;                              // gradient as a positive; its loss less the loss counted as a negative
+                if (LOSS == HASTE_LOSS_SQHINGE) {
+                  const float m = fmaxf(1.f - zr, 0.f), n = fmaxf(1.f + zr, 0.f);
+                  gl = -m * gs2;
+                  la = m * m - n * n;
+                } else {
+                  // softplus(-z) - softplus(z) = -z
+                  gl = ((LOSS == LOSS_BCE_EXP ? sigmoid_exp(zr) : fmaf(0.5f, tanh_approx(0.5f * zr), 0.5f)) - 1.f) * gs;
+                  la = -zr;
+                }
+                const int cc = col0 + static_cast<int>(c);
+                *reinterpret_cast<__nv_bfloat16*>(yrow + (cc >> 6) * YBLK + ((((cc & 63) >> 3) ^ (row & 7)) << 4) + (cc & 7) * 2) = __float2bfloat16_rn(gl);
+                if (WITH_LOSS) tile_loss += la;
+                // a logit so large that the difference says nothing (or infinite, or NaN): once more through the other loop
+                again = !(fabsf(zr) < 1024.f);
+              }
+            }
+            again = __any_sync(0xffffffffu, again);
+          }
+        } else {
+        // 16 label columns per iteration; chunks without a target in the warp's 32 rows and without a ragged edge still take the plain
+        // form, the rest the general branch with target bits and a column-valid mask.
 #pragma unroll 1
         for (int c16 = 0; c16 < EA_COLS; c16 += CH) {
           if (LS < G && col0 + c16 >= LS) {                // columns no tile of this shape has
@@ -585,62 +724,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           __syncwarp();
           tmem_ld(ta + c16, r);
           tmem_ld_wait();
-          const uint32_t ym16 = static_cast<uint32_t>(ym >> c16) & (CH == 32 ? 0xFFFFFFFFu : 0xFFFFu);
+          const uint32_t ym16 = static_cast<uint32_t>(ym >> c16) & 0xFFFFu;
           const bool general = DEBUG || ragged || __any_sync(0xffffffffu, ym16 != 0u);
           uint8_t* yblk = yrow + ((col0 + c16) >> 6) * YBLK;
           const int chunk0 = ((col0 + c16) & 63) >> 3;       // 16-byte chunk inside the 128-byte row of the block
           if (!general) {
-            float bce_prod = 1.f;
-            float fl[4] = {0.f, 0.f, 0.f, 0.f};        // partial sums: no serial dependency through one accumulator
-            F2 fh[2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-            for (int e8 = 0; e8 < CH; e8 += 8) {
-              uint4 pk;
-              float x[8];
-              if (LOSS == HASTE_LOSS_SQHINGE) {
-                // dLoss/dz = 2 s max(0, 1 + z) with s = grad_scale, evaluated as max(0, fma(2s, z, 2s)); 1 + z is
-                // exact in fp32 for a bf16 z (down to |z| ~ 2^-16), so this is the same single rounding as
-                // (1 + z) * 2s.  The max is left to the bf16 conversion.  The loss term max(0,1+z)^2 is accumulated
-                // as (x + |x|)^2 = (2 max(0,x))^2 and rescaled by 1/(4s)^2 once per tile.
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                  // logits are rounded to bf16 first, as the unfused forward stores them
-                  const F2 z2 = {round_bf16_as_f32(__uint_as_float(r[e8 + i])), round_bf16_as_f32(__uint_as_float(r[e8 + i + 1]))};
-                  const F2 x2 = fma2<PAIRED>({gs2, gs2}, z2, {gs2, gs2});
-                  x[i] = DROP_NAN ? fmaxf(x2.x, 0.f) : x2.x; x[i + 1] = DROP_NAN ? fmaxf(x2.y, 0.f) : x2.y;
-                  if (WITH_LOSS) { const F2 m2 = {x2.x + fabsf(x2.x), x2.y + fabsf(x2.y)}; fh[(i >> 1) & 1] = fma2<PAIRED>(m2, m2, fh[(i >> 1) & 1]); }
-                }
-                pk = make_uint4(pack_bf16x2_relu(x[0], x[1]), pack_bf16x2_relu(x[2], x[3]), pack_bf16x2_relu(x[4], x[5]), pack_bf16x2_relu(x[6], x[7]));
-              } else if (LOSS == LOSS_BCE_EXP) {
-                // dLoss/dz = s sigmoid(z) = s / (1 + e^-z); loss term softplus(z) = max(z,0) - ln(0.5 + |sigmoid - 0.5|),
-                // whose logarithm arguments lie in [0.5, 1] as below
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
-                  const float sg = sigmoid_exp(zr);
-                  x[i] = sg * gs;
-                  if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bce_prod *= 0.5f + fabsf(sg - 0.5f); }
-                }
-                pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
-              } else {
-                // dLoss/dz = s sigmoid(z) = s/2 + s/2 tanh(z/2) (one MUFU op, one fma); loss term softplus(z) =
-                // max(z,0) - ln(0.5 + 0.5 |tanh(z/2)|).  The logarithm arguments
-                // lie in [0.5, 1], so the 16 of a chunk are multiplied together (>= 2^-16) and one log2 is taken.
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
-                  const float th = tanh_approx(0.5f * zr);
-                  x[i] = fmaf(hgs, th, hgs);
-                  if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bce_prod *= fmaf(0.5f, fabsf(th), 0.5f); }
-                }
-                pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
-              }
-              *reinterpret_cast<uint4*>(yblk + (((chunk0 + (e8 >> 3)) ^ (row & 7)) << 4)) = pk;
-            }
-            if (WITH_LOSS) {
-              if (LOSS != HASTE_LOSS_SQHINGE) { fast_loss += __log2f(bce_prod); tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]); }
-              else fast_loss += (fh[0].x + fh[0].y) + (fh[1].x + fh[1].y);
-            }
+            plain_chunk(r, yblk, chunk0);
           } else {
             const int nvalid = rows_real - (col0 + c16);           // columns of this chunk that are real labels
 #pragma unroll
@@ -684,13 +773,19 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             }
           }
         }
+        }
+        if (LOSS == HASTE_LOSS_SQHINGE) fast_loss = (fh[0].x + fh[0].y) + (fh[1].x + fh[1].y);
         // Hinge: a logit that is infinite or NaN (a label masked by its bias) leaves x + |x| undefined.  Such a tile goes through the
         // general branch, which has a value for it; so does one whose sum of squares overflows.  (max(x, 0) in place of x + |x| needs no second pass and took 1.6 % more
         // of the 670 K step: 276.9 against 272.5 us; this way 274.3.  BCE sums max(z, 0): 2.8 M labels 2,310 against 2,320 us.)
-        if (LOSS != HASTE_LOSS_SQHINGE || !WITH_LOSS || DEBUG || ragged || !__any_sync(0xffffffffu, !(fast_loss < INFINITY))) break;
-        ragged = true;
+        if (!again && (LOSS != HASTE_LOSS_SQHINGE || !WITH_LOSS || DEBUG || ragged || !__any_sync(0xffffffffu, !(fast_loss < INFINITY)))) break;
+        if (PATCH && few && plain) few_bits();
+        ragged = true; plain = false;
         tile_loss = fast_loss = 0.f;
+        fh[0] = fh[1] = {0.f, 0.f};
+        fl[0] = fl[1] = fl[2] = fl[3] = 0.f;
         }
+        if (LOSS != HASTE_LOSS_SQHINGE) tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
         tc_fence_before();                             // this warp's part of the Z stage has been read
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
@@ -717,45 +812,52 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     }
   } else if (warp >= C::W_EB && warp < C::W_UP) {
     // ================================================================ scatter: dXg -> dxt
-    const int e = warp - C::W_EB;
+    // dXg[b,k] of TMEM lane b goes to dxt[loc[k], b].  The L2 takes reductions of 16 bytes a lane, whole 128-byte lines, at 5.4 TB/s
+    // beside the gathers, 4-byte ones at 3.0 (four warps a SM) to 3.4 (eight), and each of those costs five
+    // instructions.  TMEM gives a lane one batch row, so the warp turns EBP slots around in 2 KB of its own shared memory: lane l then takes
+    // slot 4i + l/8 and batch rows 4 (l%8) .. +3.  (Bulk reductions from shared memory: a warp issues one per 100 cycles and is
+    // held meanwhile; 462 us where this takes 252.)  Rows of dxt that are not 16-byte aligned take the 4-byte form.
     const int q = warp & 3;
+    const int kc = (warp - C::W_EB) >> 2;        // which EBS-slot chunk this warp scatters
     const int row = q * 32 + lane;               // TMEM lane == batch row inside the tile
-    const int kc = e >> 2;                       // which EBS-slot chunk this warp scatters
+    float* buf = reinterpret_cast<float*>(sm + C::OFF_EB) + (warp - C::W_EB) * C::EBP * 32;
     int it = 0;
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int ws = gi & 1;
       mbar_wait(bar(C::B_WFULL + ws), (gi >> 1) & 1, abort_flag, a.err, 12, WL);   // loc_s of this group is in place
-      const uint4* loc4 = reinterpret_cast<const uint4*>(loc_s + ws * F + kc * C::EBS);
+      const uint32_t* loc_g = loc_s + ws * F + kc * C::EBS;
       for (int t = 0; t < T; ++t, ++it) {
-        const int b0 = tile_b0(t);
         const int ds = it % NDX;
         mbar_wait(bar(C::B_DXFULL + ds), (it / NDX) & 1, abort_flag, a.err, 13, WL);
         tc_fence_after();
         const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DX + ds * F + kc * C::EBS;
-        // dXg[b,k] of this thread's batch row goes to dxt[loc[k], b]: for a fixed k the warp's 32 lanes hit 32
-        // consecutive floats, so each red below is one 128-byte transaction.  Two halves of 32 slots, so that only
-        // 32 accumulator values are live at a time; the stage goes back to the tensor core after the second load.
-        const bool do_red = (b0 + row < a.B) && !*abort_flag;
-        float* dbase = a.dxt + b0 + row;
-#pragma unroll
-        for (int half = 0; half < C::EBS / 32; ++half) {
-          uint32_t r0[32];
-          tmem_ld32(ta + half * 32, r0);
+        const bool live = !*abort_flag;
+        const int b1 = tile_b0(t) + row, b4 = tile_b0(t) + q * 32 + 4 * (lane & 7);
+#pragma unroll 1
+        for (int c = 0; c < C::EBS; c += C::EBP) {
+          uint32_t r[C::EBP];
+          __syncwarp();
+          tmem_ld(ta + c, r);
           tmem_ld_wait();
-          if (half == C::EBS / 32 - 1) {
+          if (c == C::EBS - C::EBP) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::B_DXEMPTY + ds));
           }
-          if (do_red) {
+          if (a.dxt_v4) {
 #pragma unroll
-            for (int k4 = 0; k4 < 32; k4 += 4) {
-              const uint4 lc = loc4[half * 8 + (k4 >> 2)];      // 32-bit row offsets: one widening add per address
-              atomicAdd(dbase + lc.x, __uint_as_float(r0[k4 + 0]));
-              atomicAdd(dbase + lc.y, __uint_as_float(r0[k4 + 1]));
-              atomicAdd(dbase + lc.z, __uint_as_float(r0[k4 + 2]));
-              atomicAdd(dbase + lc.w, __uint_as_float(r0[k4 + 3]));
+            for (int k = 0; k < C::EBP; ++k) buf[k * 32 + lane] = __uint_as_float(r[k]);
+            __syncwarp();
+            if (live && b4 < a.B) {
+              float* dst = a.dxt + b4;
+#pragma unroll
+              for (int k = 0; k < C::EBP / 4; ++k)
+                red_add_v4(dst + loc_g[c + 4 * k + (lane >> 3)], *reinterpret_cast<const float4*>(buf + k * 128 + lane * 4));
             }
+          } else if (live && b1 < a.B) {
+            float* dst = a.dxt + b1;
+#pragma unroll
+            for (int k = 0; k < C::EBP; ++k) atomicAdd(dst + loc_g[c + k], __uint_as_float(r[k]));
           }
         }
       }
@@ -766,21 +868,21 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     // ================================================================ update warps: SGD + stochastic rounding
     // Weight / bias update of each finished group from its dW accumulator: warp (q, kh) owns the label rows of TMEM
     // lane quarter q (32 rows for G = 128; 16 for G = 64, where an M = 64 accumulator occupies lanes 0-15 of each
-    // quarter) and slots kh*UPS .. kh*UPS+UPS-1.  The accumulator slice is read, rounded to bf16 (as the unfused
-    // kernel would store the gradient) and handed back to the tensor core at once; the old weights come out of the
-    // group's W tile in shared memory.
+    // quarter) and slots kh*UPS .. kh*UPS+UPS-1.  It reads its accumulator slice, rounds it to bf16 (as the unfused
+    // kernel would store the gradient) into shared memory and hands the accumulator back; then a lane takes one 16-byte chunk of a row
+    // at a time: 8 slots, which are one Philox call, old weights out of the group's W tile, new ones to memory.  Neighbouring
+    // lanes have neighbouring chunks, so a store covers runs of 64 or 128 bytes (one row per lane: 32 accesses per
+    // instruction, a quarter of all that the L1 data pipe did in the 670 K step).
+    // The loops are rolled: the roles' loops share the instruction cache (two chunks per pass: 254 -> 274 us, 670 K labels).
     const int e = warp - C::W_UP;
     const int q = warp & 3;
     const int kh = e >> 2;
-    // G = 64: only lanes 0-15 of a TMEM lane quarter hold accumulator rows, so lane l and lane l+16 share label row
-    // l: lane l keeps the lower 8 slots of every 16-slot piece, lane l+16 gets the upper 8 by shuffle — the whole
-    // warp works and a lane's 8 slots are exactly one Philox call, one 16-byte chunk of W and one 16-byte store.
-    constexpr bool SPLIT = C::ROWS_PER_Q == 16;
-    constexpr int NSL = SPLIT ? 8 : 16;            // slots per lane and piece
-    const int lrow = SPLIT ? (lane & 15) : lane;
-    const int half = SPLIT ? (lane >> 4) : 0;
-    const int row = q * C::ROWS_PER_Q + lrow;      // label row inside the group
-    constexpr int NPC = UPS / 16;                  // pieces of 16 slots
+    constexpr int ROWS = C::ROWS_PER_Q, CPR = UPS / 8;      // label rows of a warp, chunks of a row
+    constexpr int RPI = 32 / CPR;                           // rows per pass of the update
+    static_assert(ROWS * UPS * 2 == C::GSTAGE && N_UP == 8, "the warps' gradient buffers");
+    uint8_t* gst = sm + C::OFF_G + e * C::GSTAGE;
+    // byte offset of chunk c of row r: swizzled so that neither eight rows of a chunk nor the chunks of a row share a bank
+    auto g_chunk = [](int r, int c) { return r * (CPR * 16) + ((c ^ ((r * CPR >> 3) & (CPR - 1))) << 4); };
     for (int gu = 0; gu < n_my_groups; ++gu) {
       const int gg = group_of(gu);
       const int wsu = gu & 1;
@@ -790,144 +892,111 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       mbar_wait(bar(C::B_DWFULL), gu & 1, abort_flag, a.err, 15, WL);
       tc_fence_after();
       const uint32_t tdw = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW;
-      const uint32_t tdg = tdw + (P == 1 ? 0 : (q * C::ROWS_PER_Q) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
-      uint32_t gw[UPS / 2];                       // this TMEM lane's gradients, bf16 pairs (garbage in lanes 16-31 when SPLIT)
+      const uint32_t tdg = tdw + (P == 1 ? 0 : (q * ROWS) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
       float gb = 0.f;
-      {
-        __syncwarp();
-#pragma unroll
-        for (int pc = 0; pc < NPC; ++pc) {
-          uint32_t rr[16];
-          tmem_ld16(tdg + kh * UPS + pc * 16, rr);
-          tmem_ld_wait();
-#pragma unroll
-          for (int x = 0; x < 8; ++x) gw[pc * 8 + x] = pack_bf16x2(__uint_as_float(rr[2 * x]), __uint_as_float(rr[2 * x + 1]));
-        }
-        if (kh == 0) {
-          uint32_t rb[8];
-          tmem_ld8(tdw + F, rb);
-          tmem_ld_wait();
-          gb = round_to_bf16_f(__uint_as_float(rb[0]));
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(C::B_DWEMPTY));
-      }
-      const bool do_row = row < rows_real_u && !*abort_flag;
-      const unsigned row_mask = __ballot_sync(0xffffffffu, do_row);      // lanes l and l+16 always agree
-      const int64_t l = l0 + row, gl = u.label0 + l;
-      const bool sr = u.flags & HASTE_F_SR, packed = u.flags & HASTE_F_RNG_PACKED, contract = u.flags & HASTE_F_CONTRACT;
-      // the old bias comes from the group's bias column in shared memory
-      const uint16_t b_old = (has_bias && kh == 0 && half == 0)
-                                 ? *reinterpret_cast<const uint16_t*>(sm + C::OFF_BT + wsu * C::BTILE + (row >> 3) * 256 + (row & 7) * 16)
-                                 : uint16_t(0);
-      if (do_row) {
-        __nv_bfloat16* wrow = u.w + l * FF;
 #pragma unroll 1
-        for (int pc = 0; pc < NPC; ++pc) {          // pieces of 16 slots
-          uint32_t p8[8];
+      for (int c = 0; c < CPR; ++c) {
+        uint32_t rr[8];
+        __syncwarp();
+        tmem_ld8(tdg + kh * UPS + c * 8, rr);
+        tmem_ld_wait();
+        if (lane < ROWS)
+          *reinterpret_cast<uint4*>(gst + g_chunk(lane, c)) =
+              make_uint4(pack_bf16x2(__uint_as_float(rr[0]), __uint_as_float(rr[1])), pack_bf16x2(__uint_as_float(rr[2]), __uint_as_float(rr[3])),
+                         pack_bf16x2(__uint_as_float(rr[4]), __uint_as_float(rr[5])), pack_bf16x2(__uint_as_float(rr[6]), __uint_as_float(rr[7])));
+      }
+      if (kh == 0) {
+        uint32_t rb[8];
+        __syncwarp();
+        tmem_ld8(tdw + F, rb);
+        tmem_ld_wait();
+        gb = round_to_bf16_f(__uint_as_float(rb[0]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(C::B_DWEMPTY));
+      const bool live = !*abort_flag;
+      const bool sr = u.flags & HASTE_F_SR, packed = u.flags & HASTE_F_RNG_PACKED, contract = u.flags & HASTE_F_CONTRACT;
+      const uint8_t* wsm = sm + C::OFF_W + wsu * WSTAGE;
+#pragma unroll 1
+      for (int r0 = 0; r0 < ROWS; r0 += RPI) {
+        const int r = r0 + lane / CPR, row = q * ROWS + r;      // row of the warp, of the tile
+        if (!live || row >= rows_real_u) continue;
+        const int s0 = kh * UPS + (lane % CPR) * 8;             // first slot
+        const int64_t l = l0 + row, gl = u.label0 + l;
+        const uint4 ga = *reinterpret_cast<const uint4*>(gst + g_chunk(r, lane % CPR));
+        const uint4 wa = *reinterpret_cast<const uint4*>(wsm + C::w_chunk(row, s0 >> 3));
+        const uint32_t g8[4] = {ga.x, ga.y, ga.z, ga.w}, w8[4] = {wa.x, wa.y, wa.z, wa.w};
+        float* mrow = MOM ? u.mom_w + l * FF + s0 : nullptr;
+        float mv[8];
+        if (MOM) {
 #pragma unroll
-          for (int x = 0; x < 8; ++x) p8[x] = gw[x];
+          for (int x = 0; x < 2; ++x) {
+            const float4 m4 = reinterpret_cast<const float4*>(mrow)[x];
+            mv[4 * x] = m4.x; mv[4 * x + 1] = m4.y; mv[4 * x + 2] = m4.z; mv[4 * x + 3] = m4.w;
+          }
+        }
+        if (DEBUG) {
+          if (a.dw_dump != nullptr) {
 #pragma unroll
-          for (int p2 = 1; p2 < NPC; ++p2)       // register select (a dynamic index would put gw in local memory)
-            if (p2 == pc) {
-#pragma unroll
-              for (int x = 0; x < 8; ++x) p8[x] = gw[p2 * 8 + x];
-            }
-          uint32_t g8[NSL / 2], w8[NSL / 2];
-          if (SPLIT) {
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-              const uint32_t up = __shfl_sync(row_mask, p8[4 + x], lane & 15);     // upper 8 slots of the piece, from the lane that read TMEM
-              g8[x] = half ? up : p8[x];
-            }
+            for (int x = 0; x < 4; ++x) reinterpret_cast<uint32_t*>(a.dw_dump + l * FF + s0)[x] = g8[x];
+          }
+        }
+        uint32_t rnd[4] = {0u, 0u, 0u, 0u};                     // 8 x 16 random bits, two per word
+        if (sr) {
+          if (packed) {
+            const uint4 rp = rand_packed8_call(u.seed, u.step, gl, s0 >> 3);
+            rnd[0] = rp.x; rnd[1] = rp.y; rnd[2] = rp.z; rnd[3] = rp.w;
           } else {
 #pragma unroll
-            for (int x = 0; x < NSL / 2; ++x) g8[x] = p8[x];
+            for (int x = 0; x < 4; ++x)
+              rnd[x] = rand16_reference_call(u.seed, gl * FF + s0 + 2 * x) | (rand16_reference_call(u.seed, gl * FF + s0 + 2 * x + 1) << 16);
           }
-          const int s0 = kh * UPS + pc * 16 + half * 8;        // first slot of this lane's part of the piece
-          {
-            // the old weights: one (SPLIT) or two 16-byte chunks of the row in the W tile
-            const uint8_t* wsm = sm + C::OFF_W + wsu * WSTAGE;
-            const uint4 wa = *reinterpret_cast<const uint4*>(wsm + C::w_chunk(row, s0 >> 3));
-            w8[0] = wa.x; w8[1] = wa.y; w8[2] = wa.z; w8[3] = wa.w;
-            if (!SPLIT) {
-              const uint4 wb = *reinterpret_cast<const uint4*>(wsm + C::w_chunk(row, (s0 >> 3) + 1));
-              w8[NSL / 2 - 4] = wb.x; w8[NSL / 2 - 3] = wb.y; w8[NSL / 2 - 2] = wb.z; w8[NSL / 2 - 1] = wb.w;
-            }
-          }
-          if (DEBUG) {
-            if (a.dw_dump != nullptr) {
-#pragma unroll
-              for (int x = 0; x < NSL / 2; ++x) reinterpret_cast<uint32_t*>(a.dw_dump + l * FF + s0)[x] = g8[x];
-            }
-          }
-          uint32_t rnd[NSL / 2];           // NSL x 16 random bits, two per word
-#pragma unroll
-          for (int x = 0; x < NSL / 2; ++x) rnd[x] = 0u;
-          if (sr) {
-            if (packed) {
-              const uint4 rp0 = rand_packed8_call(u.seed, u.step, gl, s0 >> 3);
-              rnd[0] = rp0.x; rnd[1] = rp0.y; rnd[2] = rp0.z; rnd[3] = rp0.w;
-              if (!SPLIT) {
-                const uint4 rp1 = rand_packed8_call(u.seed, u.step, gl, (s0 >> 3) + 1);
-                rnd[NSL / 2 - 4] = rp1.x; rnd[NSL / 2 - 3] = rp1.y; rnd[NSL / 2 - 2] = rp1.z; rnd[NSL / 2 - 1] = rp1.w;
-              }
-            } else {
-#pragma unroll
-              for (int x = 0; x < NSL; x += 2)
-                rnd[x >> 1] = rand16_reference_call(u.seed, gl * FF + s0 + x) | (rand16_reference_call(u.seed, gl * FF + s0 + x + 1) << 16);
-            }
-          }
-          uint32_t ob[NSL / 2];
-          if (!MOM && sr && contract) {
-            // the configuration every benchmark and the reference's compiled kernel use, without per-element flag
-            // tests: w' = fma(-lr, fma(wd, w, g), w), then add 16 random bits and keep the high half
-#pragma unroll
-            for (int p = 0; p < NSL / 2; ++p) {
-              const float g0 = __uint_as_float(g8[p] << 16), g1 = __uint_as_float(g8[p] & 0xFFFF0000u);
-              const float w0 = __uint_as_float(w8[p] << 16), w1 = __uint_as_float(w8[p] & 0xFFFF0000u);
-              const F2 wv = {w0, w1}, nv = fma2<PAIRED>({-u.lr, -u.lr}, fma2<PAIRED>({u.wd, u.wd}, wv, {g0, g1}), wv);
-              const uint32_t rr = rnd[p];
-              const uint32_t s0b = __float_as_uint(nv.x) + (rr & 0xFFFFu), s1b = __float_as_uint(nv.y) + (rr >> 16);
-              ob[p] = __byte_perm(s0b, s1b, 0x7632);              // high halves: s0b -> low 16 bits, s1b -> high 16 bits
-            }
-          } else {
-            float mv[NSL];
-            float* mrow = MOM ? u.mom_w + l * FF + s0 : nullptr;
-            if (MOM) {
-#pragma unroll
-              for (int x = 0; x < NSL / 4; ++x) {
-                const float4 m4 = reinterpret_cast<const float4*>(mrow)[x];
-                mv[4 * x] = m4.x; mv[4 * x + 1] = m4.y; mv[4 * x + 2] = m4.z; mv[4 * x + 3] = m4.w;
-              }
-            }
-#pragma unroll
-            for (int p = 0; p < NSL / 2; ++p) {
-              const float g0 = __uint_as_float(g8[p] << 16), g1 = __uint_as_float(g8[p] & 0xFFFF0000u);
-              const float w0 = __uint_as_float(w8[p] << 16), w1 = __uint_as_float(w8[p] & 0xFFFF0000u);
-              float n0, n1;
-              if (contract) { n0 = sgd_math<true>(w0, g0, MOM ? &mv[2 * p] : nullptr, u.lr, u.wd, u.mu); n1 = sgd_math<true>(w1, g1, MOM ? &mv[2 * p + 1] : nullptr, u.lr, u.wd, u.mu); }
-              else          { n0 = sgd_math<false>(w0, g0, MOM ? &mv[2 * p] : nullptr, u.lr, u.wd, u.mu); n1 = sgd_math<false>(w1, g1, MOM ? &mv[2 * p + 1] : nullptr, u.lr, u.wd, u.mu); }
-              const uint32_t rr = rnd[p];
-              const uint32_t o0 = sr ? ((__float_as_uint(n0) + (rr & 0xFFFFu)) >> 16) : rn_bf16_bits(n0);
-              const uint32_t o1 = sr ? ((__float_as_uint(n1) + (rr >> 16)) >> 16) : rn_bf16_bits(n1);
-              ob[p] = (o0 & 0xFFFFu) | (o1 << 16);
-            }
-            if (MOM) {
-#pragma unroll
-              for (int x = 0; x < NSL / 4; ++x) reinterpret_cast<float4*>(mrow)[x] = make_float4(mv[4 * x], mv[4 * x + 1], mv[4 * x + 2], mv[4 * x + 3]);
-            }
-          }
-          *reinterpret_cast<uint4*>(wrow + s0) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
-          if (!SPLIT) *reinterpret_cast<uint4*>(wrow + s0 + 8) = make_uint4(ob[NSL / 2 - 4], ob[NSL / 2 - 3], ob[NSL / 2 - 2], ob[NSL / 2 - 1]);
         }
-        if (has_bias && kh == 0 && half == 0) {
-          if (DEBUG) if (a.db_dump != nullptr) a.db_dump[l] = __float2bfloat16_rn(gb);
-          uint32_t r16 = 0;
-          if (sr) r16 = rand16_call(u.flags, u.seed ^ (packed ? 0x62696173ull : 0ull), u.step, gl);
-          u.bias[l] = __ushort_as_bfloat16(sgd_update_bits(b_old, gb, (MOM && u.mom_b != nullptr) ? u.mom_b + l : nullptr, u.lr, u.wd, u.mu, u.flags, r16));
+        uint32_t ob[4];
+        if (sr && contract) {
+          // the configuration every benchmark and the reference's compiled kernel use, without per-element flag
+          // tests: w' = fma(-lr, m', w) with m' = fma(wd, w, g), or fma(mu, m, .) of that with momentum; then add 16 random bits and
+          // keep the high half
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const float g0 = __uint_as_float(g8[p] << 16), g1 = __uint_as_float(g8[p] & 0xFFFF0000u);
+            const float w0 = __uint_as_float(w8[p] << 16), w1 = __uint_as_float(w8[p] & 0xFFFF0000u);
+            const F2 wv = {w0, w1};
+            F2 gv = fma2<PAIRED>({u.wd, u.wd}, wv, {g0, g1});
+            if (MOM) { gv = fma2<PAIRED>({u.mu, u.mu}, {mv[2 * p], mv[2 * p + 1]}, gv); mv[2 * p] = gv.x; mv[2 * p + 1] = gv.y; }
+            const F2 nv = fma2<PAIRED>({-u.lr, -u.lr}, gv, wv);
+            const uint32_t s0b = __float_as_uint(nv.x) + (rnd[p] & 0xFFFFu), s1b = __float_as_uint(nv.y) + (rnd[p] >> 16);
+            ob[p] = __byte_perm(s0b, s1b, 0x7632);              // high halves: s0b -> low 16 bits, s1b -> high 16 bits
+          }
+        } else {
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const float g0 = __uint_as_float(g8[p] << 16), g1 = __uint_as_float(g8[p] & 0xFFFF0000u);
+            const float w0 = __uint_as_float(w8[p] << 16), w1 = __uint_as_float(w8[p] & 0xFFFF0000u);
+            float n0, n1;
+            if (contract) { n0 = sgd_math<true>(w0, g0, MOM ? &mv[2 * p] : nullptr, u.lr, u.wd, u.mu); n1 = sgd_math<true>(w1, g1, MOM ? &mv[2 * p + 1] : nullptr, u.lr, u.wd, u.mu); }
+            else          { n0 = sgd_math<false>(w0, g0, MOM ? &mv[2 * p] : nullptr, u.lr, u.wd, u.mu); n1 = sgd_math<false>(w1, g1, MOM ? &mv[2 * p + 1] : nullptr, u.lr, u.wd, u.mu); }
+            const uint32_t o0 = sr ? ((__float_as_uint(n0) + (rnd[p] & 0xFFFFu)) >> 16) : rn_bf16_bits(n0);
+            const uint32_t o1 = sr ? ((__float_as_uint(n1) + (rnd[p] >> 16)) >> 16) : rn_bf16_bits(n1);
+            ob[p] = (o0 & 0xFFFFu) | (o1 << 16);
+          }
         }
+        *reinterpret_cast<uint4*>(u.w + l * FF + s0) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
+        if (MOM) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) reinterpret_cast<float4*>(mrow)[x] = make_float4(mv[4 * x], mv[4 * x + 1], mv[4 * x + 2], mv[4 * x + 3]);
+        }
+      }
+      if (has_bias && kh == 0 && lane < ROWS && live && q * ROWS + lane < rows_real_u) {
+        const int row = q * ROWS + lane;
+        const int64_t l = l0 + row, gl = u.label0 + l;
+        // the old bias comes from the group's bias column in shared memory
+        const uint16_t b_old = *reinterpret_cast<const uint16_t*>(sm + C::OFF_BT + wsu * C::BTILE + (row >> 3) * 256 + (row & 7) * 16);
+        if (DEBUG) if (a.db_dump != nullptr) a.db_dump[l] = __float2bfloat16_rn(gb);
+        uint32_t r16 = 0;
+        if (sr) r16 = rand16_call(u.flags, u.seed ^ (packed ? 0x62696173ull : 0ull), u.step, gl);
+        u.bias[l] = __ushort_as_bfloat16(sgd_update_bits(b_old, gb, (MOM && u.mom_b != nullptr) ? u.mom_b + l : nullptr, u.lr, u.wd, u.mu, u.flags, r16));
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::B_MEMPTY + wsu));   // this warp no longer needs the group's W tile / bias column
@@ -957,6 +1026,7 @@ int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
   if (int rc = device_status_word(&a.err)) return rc;
   a.B = B; a.L = L; a.D = static_cast<int>(D); a.NG = static_cast<int>((L + C::LS - 1) / C::LS);
   a.NGR = static_cast<int>((L + GG_ - 1) / GG_); a.grad_scale = grad_scale;
+  a.dxt_v4 = (B & 3) == 0 && aligned16(dxt);
   a.wait_limit = wait_limit_cycles();
   a.stall_tile = dump ? take_stall_tile() : -1;
   a.z_dump = dump ? static_cast<__nv_bfloat16*>(dump->z) : nullptr; a.ldz = dump ? dump->ldz : 0;
@@ -964,7 +1034,7 @@ int launch_step_shape(const int32_t* loc, const void* xt, const int32_t* tgt_ptr
   CUtensorMap tm_x, tm_w;
   // xt [D][ldxt]: one box = 64 batch columns of one row (gather4 stacks four rows); W [L][FF]: one box = 64 slots (32 at fan-in 32) x G labels
   if (int rc = make_tmap_bf16_2d(&tm_x, xt, static_cast<uint64_t>(ldxt), static_cast<uint64_t>(D), static_cast<uint64_t>(ldxt) * 2, 64, 1)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tm_w, u.w, static_cast<uint64_t>(FF_), static_cast<uint64_t>(L), static_cast<uint64_t>(FF_) * 2, FF_ == 32 ? 32 : 64, C::G)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tm_w, u.w, static_cast<uint64_t>(FF_), static_cast<uint64_t>(L), static_cast<uint64_t>(FF_) * 2, FF_ == 32 ? 32 : 64, C::LS)) return rc;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
