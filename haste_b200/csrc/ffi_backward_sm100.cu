@@ -56,7 +56,9 @@ struct Cfg {
   static constexpr int OFF_YSIDE = OFF_Y + NYS * YSTAGE;
   static constexpr int OFF_LOC = OFF_YSIDE + NYS * YSIDE;      // u32 [2][F]: element offset loc * B of each slot's dxt row
   static constexpr int OFF_LOCR = OFF_LOC + 2 * F * 4;         // int [4][F]: each producer warp's copy of the group's indices
-  static constexpr int OFF_BAR = OFF_LOCR + 4 * F * 4;
+  static constexpr int WST = (G / 4) * 64;                     // one writer warp's gradients on their way out: bf16 [label rows][32 slots]
+  static constexpr int OFF_WST = OFF_LOCR + 4 * F * 4;
+  static constexpr int OFF_BAR = OFF_WST + 4 * WST;
   static constexpr int OFF_MISC = OFF_BAR + 40 * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
@@ -249,31 +251,33 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         const uint32_t sh = static_cast<uint32_t>((dy_base + 2ull * static_cast<uint64_t>((b0 + k) * a.ldy + l0)) & 15u);
         const bool mask_cols = l0 + LS > a.L;
         if ((sh != 0 || mask_cols) && !*abort_flag) {
-          const uint32_t wo = sh >> 2, hb = (sh & 2u) << 3;     // whole words, then 0 or 16 bits
+          const uint32_t hb = (sh & 2u) << 3;
           uint8_t* yb = sm + C::OFF_Y + ys * YSTAGE;
           const uint8_t* yside = sm + C::OFF_YSIDE + ys * C::YSIDE;
-          // (Unrolling this over the four row sets, so that their shared-memory latencies overlap, made the whole
-          // kernel slower in measurement — aligned inputs included — and is therefore not done.)
-#pragma unroll 1
+          // Per set of four rows every chunk is read, with its right neighbour, before any is rewritten.
+          // Unrolled, so that the shared-memory latencies of the sets overlap (one set at a time: 670 K labels 289 -> 303 us of backward).
+#pragma unroll
           for (int set = 0; set < 4; ++set) {
             const int r = k + 8 * (4 * set + rr);
+            uint8_t* pr = yb + r * 128;
+            uint4 v[C::NYB][2];
 #pragma unroll
-            for (int blk = 0; blk < C::NYB; ++blk) {           // ascending: chunk 8 is read (as a neighbour) before it is rewritten
+            for (int blk = 0; blk < C::NYB; ++blk) {
               const int cj = blk * 8 + c;
-              uint8_t* p = yb + blk * YBLK + r * 128 + ((c ^ (r & 7)) << 4);
               // (a chunk no label has: nothing is read beyond the tile, nothing is written)
-              const uint8_t* pn = cj >= NCH ? p : (cj + 1 == NCH) ? yside + r * 16
-                                                  : yb + ((cj + 1) >> 3) * YBLK + r * 128 + ((((cj + 1) & 7) ^ (r & 7)) << 4);
-              const uint4 v0 = *reinterpret_cast<const uint4*>(p);
-              const uint4 v1 = *reinterpret_cast<const uint4*>(pn);
-              __syncwarp();                            // every lane has read its neighbour's chunk before anyone rewrites one
-              uint32_t w0, w1, w2, w3, w4;
-              switch (wo) {                            // warp-uniform
-                case 0: w0 = v0.x; w1 = v0.y; w2 = v0.z; w3 = v0.w; w4 = v1.x; break;
-                case 1: w0 = v0.y; w1 = v0.z; w2 = v0.w; w3 = v1.x; w4 = v1.y; break;
-                case 2: w0 = v0.z; w1 = v0.w; w2 = v1.x; w3 = v1.y; w4 = v1.z; break;
-                default: w0 = v0.w; w1 = v1.x; w2 = v1.y; w3 = v1.z; w4 = v1.w; break;
-              }
+              const uint8_t* pn = cj >= NCH ? pr : (cj + 1 == NCH) ? yside + r * 16 : pr + ((cj + 1) >> 3) * YBLK + ((((cj + 1) & 7) ^ (r & 7)) << 4);
+              v[blk][0] = *reinterpret_cast<const uint4*>(pr + blk * YBLK + ((c ^ (r & 7)) << 4));
+              v[blk][1] = *reinterpret_cast<const uint4*>(pn);
+            }
+            __syncwarp();                              // every lane has read its neighbour's chunk before anyone rewrites one
+#pragma unroll
+            for (int blk = 0; blk < C::NYB; ++blk) {
+              const int cj = blk * 8 + c;
+              const uint4 v0 = v[blk][0], v1 = v[blk][1];
+              // left by 8, 4 and 2 bytes as the misalignment (uniform) asks
+              const bool s8 = sh & 8u, s4 = sh & 4u;
+              const uint32_t t0 = s8 ? v0.z : v0.x, t1 = s8 ? v0.w : v0.y, t2 = s8 ? v1.x : v0.z, t3 = s8 ? v1.y : v0.w, t4 = s8 ? v1.z : v1.x, t5 = s8 ? v1.w : v1.y;
+              const uint32_t w0 = s4 ? t1 : t0, w1 = s4 ? t2 : t1, w2 = s4 ? t3 : t2, w3 = s4 ? t4 : t3, w4 = s4 ? t5 : t4;
               uint4 o = make_uint4(__funnelshift_r(w0, w1, hb), __funnelshift_r(w1, w2, hb), __funnelshift_r(w2, w3, hb),
                                    __funnelshift_r(w3, w4, hb));
               if (mask_cols) {
@@ -285,7 +289,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
                   o.w = nv == 7 ? (o.w & 0xFFFFu) : 0u;
                 }
               }
-              if (cj < NCH) *reinterpret_cast<uint4*>(p) = o;
+              if (cj < NCH) *reinterpret_cast<uint4*>(pr + blk * YBLK + ((c ^ (r & 7)) << 4)) = o;
             }
           }
         }
@@ -302,21 +306,38 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
           const int64_t l0 = static_cast<int64_t>(group_of(gi_i)) * LS;
           const int64_t b0 = static_cast<int64_t>(t_i) * BT;
           const uint32_t yb = sbase + C::OFF_Y + ys * YSTAGE, yside = sbase + C::OFF_YSIDE + ys * C::YSIDE;
+          // Away from the tensor's ends every chunk that covers a row slice lies in the tensor, and a lane's chunks are a constant distance
+          // apart: lane = (row within a set of four, chunk within a 64-label block), as in the shifting.  (The Y warps bound the kernel,
+          // half with this and half with the shifting; with a division, a 64-bit product and five comparisons per chunk the backward of 670 K labels
+          // took 350 us, with this 305, and 280 with the shifting's loads overlapped.)
+          const bool inside = b0 + BT <= a.B && (b0 != 0 || l0 != 0) && (b0 + BT - 1) * a.ldy + l0 + LS + 8 <= (a.B - 1) * a.ldy + a.L;
+          if (inside) {
+            const uintptr_t row_addr = dy_base + 2ull * static_cast<uint64_t>((b0 + k + 8 * rr) * a.ldy + l0);
+            const bool side = c == 0 && (row_addr & 15) != 0;        // (all rows of this warp have the same misalignment)
+            const uint8_t* src = reinterpret_cast<const uint8_t*>(row_addr & ~static_cast<uintptr_t>(15)) + 16 * c;
+            const uint32_t dst = yb + (k + 8 * rr) * 128 + ((c ^ k) << 4), dst_side = yside + (k + 8 * rr) * 16;
+            const int64_t set_step = 64 * a.ldy;                     // 32 rows
+#pragma unroll 1
+            for (int set = 0; set < 4; ++set, src += set_step) {
 #pragma unroll
-          for (int j = 0; j < (N_CP + 31) / 32; ++j) {
-            const int idx = lane + 32 * j;
-            if (idx < N_CP) {
-              const int ri = idx / PER_ROW, ch = idx % PER_ROW;
-              const int r = k + 8 * ri;
-              const int64_t b = b0 + r;
-              const uintptr_t row_addr = dy_base + 2ull * static_cast<uint64_t>(b * a.ldy + l0);
-              const uintptr_t src = (row_addr & ~static_cast<uintptr_t>(15)) + 16u * ch;
-              // a chunk is read when it holds at least one byte of the tensor (it lies in the same 16-byte granule as
-              // that byte); everything else is zero-filled
-              const bool valid = b < a.B && src + 16 > dy_base && src < dy_end && (ch < NCH || (row_addr & 15) != 0);
-              const uint32_t dst = ch < NCH ? yb + (ch >> 3) * YBLK + r * 128 + (((ch & 7) ^ (r & 7)) << 4) : yside + r * 16;
-              cp_async16(dst, valid ? reinterpret_cast<const void*>(src) : reinterpret_cast<const void*>(dy_base & ~static_cast<uintptr_t>(15)), valid);
+              for (int blk = 0; blk < (NCH + 7) / 8; ++blk)
+                if (NCH % 8 == 0 || c < NCH) cp_async16(dst + set * (32 * 128) + blk * YBLK, src + blk * 128, true);
+              if (side) cp_async16(dst_side + set * (32 * 16), src + NCH * 16, true);
             }
+          } else {
+#pragma unroll 1
+          for (int idx = lane; idx < N_CP; idx += 32) {
+            const int ri = idx / PER_ROW, ch = idx % PER_ROW;
+            const int r = k + 8 * ri;
+            const int64_t b = b0 + r;
+            const uintptr_t row_addr = dy_base + 2ull * static_cast<uint64_t>(b * a.ldy + l0);
+            const uintptr_t src = (row_addr & ~static_cast<uintptr_t>(15)) + 16u * ch;
+            // a chunk is read when it holds at least one byte of the tensor (it lies in the same 16-byte granule as
+            // that byte); everything else is zero-filled
+            const bool valid = b < a.B && src + 16 > dy_base && src < dy_end && (ch < NCH || (row_addr & 15) != 0);
+            const uint32_t dst = ch < NCH ? yb + (ch >> 3) * YBLK + r * 128 + (((ch & 7) ^ (r & 7)) << 4) : yside + r * 16;
+            cp_async16(dst, valid ? reinterpret_cast<const void*>(src) : reinterpret_cast<const void*>(dy_base & ~static_cast<uintptr_t>(15)), valid);
+          }
           }
         }
         if (++t_i == T) { t_i = 0; ++gi_i; }
@@ -447,14 +468,13 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     }
   } else if (DW && warp >= C::W_EC && warp < C::W_Y) {
     // ================================================================ dW / dbias rows out of the accumulator
-    // G = 128: TMEM lane == label row, every lane takes its row's 32 columns of each piece.  G = 64: an M = 64
-    // accumulator occupies lanes 0-15 of each lane quarter, so lane l and lane l + 16 share label row l: the upper 16
-    // columns of every 32-column piece go to lane l + 16 by shuffle and the whole warp works.
-    constexpr bool SPLIT = C::ROWS_PER_Q == 16;
-    constexpr int NCL = SPLIT ? 2 : 4;              // 8-slot chunks per lane and piece
+    // TMEM lane == label row (G = 64: an M = 64 accumulator occupies lanes 0-15 of each lane quarter).  32 slots at a time go through
+    // shared memory, so that a lane then has one 16-byte chunk of a row and neighbouring lanes neighbouring chunks: stores
+    // (and the update's loads) cover runs of 64 bytes instead of one row per lane (670 K labels 563 -> 551 us a layer step).
+    constexpr int ROWS = C::ROWS_PER_Q;
     const int q = warp & 3;
-    const int half = SPLIT ? (lane >> 4) : 0;
-    const int row = q * C::ROWS_PER_Q + (lane & (C::ROWS_PER_Q - 1));
+    uint8_t* gst = sm + C::OFF_WST + q * C::WST;
+    auto g_chunk = [](int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); };        // no bank twice, by rows and by chunks
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int dws = gi % NDW;
@@ -463,78 +483,77 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       mbar_wait(bar(C::B_DWFULL + dws), (gi / NDW) & 1, abort_flag, a.err, 42, WL);
       tc_fence_after();
       const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW + dws * FR;
-      const uint32_t tg = ta + (P == 1 ? 0 : (q * C::ROWS_PER_Q) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
-      const bool do_row = row < rows_real && !*abort_flag;
-      const int64_t l = l0 + row, gl = u.label0 + l;
+      const uint32_t tg = ta + (P == 1 ? 0 : (q * ROWS) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
+      const bool live = !*abort_flag;
       const bool fast = UPD && u.mom_w == nullptr && (u.flags & HASTE_F_SR) && (u.flags & HASTE_F_CONTRACT);
-#pragma unroll
+#pragma unroll 1
       for (int pc = 0; pc < FF / 32; ++pc) {
-        uint32_t r0[32];
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r0[8];
+          __syncwarp();
+          tmem_ld8(tg + pc * 32 + c * 8, r0);
+          tmem_ld_wait();
+          // the gradient as the unfused kernel would store it: rounded to bf16
+          if (lane < ROWS)
+            *reinterpret_cast<uint4*>(gst + g_chunk(lane, c)) =
+                make_uint4(pack2(__uint_as_float(r0[0]), __uint_as_float(r0[1])), pack2(__uint_as_float(r0[2]), __uint_as_float(r0[3])),
+                           pack2(__uint_as_float(r0[4]), __uint_as_float(r0[5])), pack2(__uint_as_float(r0[6]), __uint_as_float(r0[7])));
+        }
         __syncwarp();
-        tmem_ld32(tg + pc * 32, r0);
-        tmem_ld_wait();
-        if (SPLIT) {
-#pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            const uint32_t up = __shfl_sync(0xffffffffu, r0[16 + x], lane & 15);
-            if (half) r0[x] = up;
-          }
-        }
-        if (do_row) {
-#pragma unroll
-          for (int c4 = 0; c4 < NCL; ++c4) {
-            const int s0 = pc * 32 + half * 16 + c4 * 8;        // first of this chunk's 8 slots
-            uint4* out = reinterpret_cast<uint4*>((UPD ? u.w : a.dw) + l * FF + s0);
-            // the gradient as the unfused kernel would store it: rounded to bf16
-            const uint4 g8 = make_uint4(pack2(__uint_as_float(r0[8 * c4]), __uint_as_float(r0[8 * c4 + 1])),
-                                        pack2(__uint_as_float(r0[8 * c4 + 2]), __uint_as_float(r0[8 * c4 + 3])),
-                                        pack2(__uint_as_float(r0[8 * c4 + 4]), __uint_as_float(r0[8 * c4 + 5])),
-                                        pack2(__uint_as_float(r0[8 * c4 + 6]), __uint_as_float(r0[8 * c4 + 7])));
-            if (!UPD) {
-              *out = g8;
-            } else {
-              const uint4 w8 = *out;
-              const uint32_t gw[4] = {g8.x, g8.y, g8.z, g8.w}, ww[4] = {w8.x, w8.y, w8.z, w8.w};
-              uint32_t rnd[4] = {0u, 0u, 0u, 0u};               // 8 x 16 random bits, two per word
-              if (u.flags & HASTE_F_SR) {
-                if (u.flags & HASTE_F_RNG_PACKED) {
-                  const uint4 rp = rand_packed8(u.seed, u.step, gl, s0 >> 3);
-                  rnd[0] = rp.x; rnd[1] = rp.y; rnd[2] = rp.z; rnd[3] = rp.w;
-                } else {
-#pragma unroll
-                  for (int x = 0; x < 4; ++x)
-                    rnd[x] = rand16_reference(u.seed, gl * FF + s0 + 2 * x) | (rand16_reference(u.seed, gl * FF + s0 + 2 * x + 1) << 16);
-                }
-              }
-              uint32_t ob[4];
-              if (fast) {
-                // no momentum, stochastic rounding, fused multiply-add: w' = fma(-lr, fma(wd, w, g), w), then add 16
-                // random bits and keep the high half
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                  const float g0 = __uint_as_float(gw[x] << 16), g1 = __uint_as_float(gw[x] & 0xFFFF0000u);
-                  const float w0 = __uint_as_float(ww[x] << 16), w1 = __uint_as_float(ww[x] & 0xFFFF0000u);
-                  const float n0 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w0, g0), w0), n1 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w1, g1), w1);
-                  ob[x] = __byte_perm(__float_as_uint(n0) + (rnd[x] & 0xFFFFu), __float_as_uint(n1) + (rnd[x] >> 16), 0x7632);
-                }
+#pragma unroll 1
+        for (int r0 = 0; r0 < ROWS; r0 += 8) {
+          const int r = r0 + (lane >> 2), row = q * ROWS + r;
+          if (!live || row >= rows_real) continue;
+          const int s0 = pc * 32 + (lane & 3) * 8;              // first of this lane's 8 slots
+          const int64_t l = l0 + row, gl = u.label0 + l;
+          uint4* out = reinterpret_cast<uint4*>((UPD ? u.w : a.dw) + l * FF + s0);
+          const uint4 g8 = *reinterpret_cast<const uint4*>(gst + g_chunk(r, lane & 3));
+          if (!UPD) {
+            *out = g8;
+          } else {
+            const uint4 w8 = *out;
+            const uint32_t gw[4] = {g8.x, g8.y, g8.z, g8.w}, ww[4] = {w8.x, w8.y, w8.z, w8.w};
+            uint32_t rnd[4] = {0u, 0u, 0u, 0u};               // 8 x 16 random bits, two per word
+            if (u.flags & HASTE_F_SR) {
+              if (u.flags & HASTE_F_RNG_PACKED) {
+                const uint4 rp = rand_packed8(u.seed, u.step, gl, s0 >> 3);
+                rnd[0] = rp.x; rnd[1] = rp.y; rnd[2] = rp.z; rnd[3] = rp.w;
               } else {
-                float* mrow = u.mom_w != nullptr ? u.mom_w + l * FF + s0 : nullptr;
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                  float m0 = 0.f, m1 = 0.f;
-                  if (mrow) { m0 = mrow[2 * x]; m1 = mrow[2 * x + 1]; }
-                  const uint32_t o0 = sgd_update_bits(static_cast<uint16_t>(ww[x] & 0xFFFFu), __uint_as_float(gw[x] << 16), mrow ? &m0 : nullptr,
-                                                      u.lr, u.wd, u.mu, u.flags, rnd[x] & 0xFFFFu);
-                  const uint32_t o1 = sgd_update_bits(static_cast<uint16_t>(ww[x] >> 16), __uint_as_float(gw[x] & 0xFFFF0000u),
-                                                      mrow ? &m1 : nullptr, u.lr, u.wd, u.mu, u.flags, rnd[x] >> 16);
-                  ob[x] = o0 | (o1 << 16);
-                  if (mrow) { mrow[2 * x] = m0; mrow[2 * x + 1] = m1; }
-                }
+                for (int x = 0; x < 4; ++x)
+                  rnd[x] = rand16_reference(u.seed, gl * FF + s0 + 2 * x) | (rand16_reference(u.seed, gl * FF + s0 + 2 * x + 1) << 16);
               }
-              *out = make_uint4(ob[0], ob[1], ob[2], ob[3]);
             }
+            uint32_t ob[4];
+            if (fast) {
+              // no momentum, stochastic rounding, fused multiply-add: w' = fma(-lr, fma(wd, w, g), w), then add 16
+              // random bits and keep the high half
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {
+                const float g0 = __uint_as_float(gw[x] << 16), g1 = __uint_as_float(gw[x] & 0xFFFF0000u);
+                const float w0 = __uint_as_float(ww[x] << 16), w1 = __uint_as_float(ww[x] & 0xFFFF0000u);
+                const float n0 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w0, g0), w0), n1 = __fmaf_rn(-u.lr, __fmaf_rn(u.wd, w1, g1), w1);
+                ob[x] = __byte_perm(__float_as_uint(n0) + (rnd[x] & 0xFFFFu), __float_as_uint(n1) + (rnd[x] >> 16), 0x7632);
+              }
+            } else {
+              float* mrow = u.mom_w != nullptr ? u.mom_w + l * FF + s0 : nullptr;
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {
+                float m0 = 0.f, m1 = 0.f;
+                if (mrow) { m0 = mrow[2 * x]; m1 = mrow[2 * x + 1]; }
+                const uint32_t o0 = sgd_update_bits(static_cast<uint16_t>(ww[x] & 0xFFFFu), __uint_as_float(gw[x] << 16), mrow ? &m0 : nullptr,
+                                                    u.lr, u.wd, u.mu, u.flags, rnd[x] & 0xFFFFu);
+                const uint32_t o1 = sgd_update_bits(static_cast<uint16_t>(ww[x] >> 16), __uint_as_float(gw[x] & 0xFFFF0000u),
+                                                    mrow ? &m1 : nullptr, u.lr, u.wd, u.mu, u.flags, rnd[x] >> 16);
+                ob[x] = o0 | (o1 << 16);
+                if (mrow) { mrow[2 * x] = m0; mrow[2 * x + 1] = m1; }
+              }
+            }
+            *out = make_uint4(ob[0], ob[1], ob[2], ob[3]);
           }
         }
+        __syncwarp();                                           // the buffer is free for the next 32 slots
       }
       uint32_t rb[8];
       __syncwarp();
@@ -543,10 +562,12 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(C::B_DWEMPTY + dws));
-      if (half == 0) {
+      const int row = q * ROWS + lane;
+      const int64_t l = l0 + row, gl = u.label0 + l;
+      if (lane < ROWS && live && row < rows_real) {
         if (!UPD) {
-          if (do_row && a.dbias != nullptr) a.dbias[l] = __float2bfloat16_rn(__uint_as_float(rb[0]));
-        } else if (do_row && u.bias != nullptr) {
+          if (a.dbias != nullptr) a.dbias[l] = __float2bfloat16_rn(__uint_as_float(rb[0]));
+        } else if (u.bias != nullptr) {
           const float gb = round_to_bf16_f(__uint_as_float(rb[0]));
           uint32_t r16 = 0;
           if (u.flags & HASTE_F_SR) r16 = rand16(u.flags, u.seed ^ ((u.flags & HASTE_F_RNG_PACKED) ? 0x62696173ull : 0ull), u.step, gl, 0, 1);

@@ -54,3 +54,27 @@ def test_step_targets_few_many_twice_and_large_logits(G, F, loss, B):
         else:
             tol = 1e-2 * want_w.abs() + 1e-3 * max(1.0, float(want_w.abs().max()))
             assert ((sh.mom_w.cpu() - want_w).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("off", [0, 1, 6])
+@pytest.mark.parametrize("B,tail", [(128, 0), (129, 1), (256, 7), (300, 63)])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_backward_reads_dy_at_any_offset_and_nothing_else(G, F, B, tail, off):
+    """The rows of dY are copied in aligned 16-byte chunks: all of them with one pointer away from the tensor's ends, chunk by chunk at the
+    ends.  What lies before and after the gradient in memory is NaN here and must not be seen."""
+    from haste_b200 import ffi
+    D = 200
+    full = fo.make_inputs(B, D, 3 * G + tail, F, G, 1, 1.1, seed=B, x_kind="normal", bias_zero=False)
+    for L in (3 * G + tail, max(tail, 1)):
+        inp = dict(loc=full["loc"][:(L + G - 1) // G].contiguous(), X=full["X"], W=full["W"][:L].contiguous())
+        buf = torch.full((off + B * L + 16,), float("nan"), dtype=torch.bfloat16)
+        buf[off:off + B * L] = (torch.randn(B * L, generator=torch.Generator().manual_seed(L)) * 0.5).to(torch.bfloat16)
+        dev = {k: inp[k].cuda() for k in ("loc", "X", "W")}
+        gbuf = buf.cuda()
+        dY, dY_dev = buf[off:off + B * L].view(B, L), gbuf[off:off + B * L].view(B, L)
+        dxt, dw, db = ffi.backward_both(ffi.transpose_padded(dev["X"]), dev["W"], dev["loc"], dY_dev, G, B=B)
+        for got, want in ((dxt, fo.backward_features(inp["loc"], inp["W"], dY, G, D)),
+                          (dw, fo.backward_weights(inp["loc"], inp["X"], dY, G, L, round_bf16=False)), (db, dY.float().sum(0))):
+            got, want = got.float().cpu(), want.float()
+            # bf16 outputs of fp32 sums
+            assert ((got - want).abs() <= 1e-3 * max(1.0, float(want.abs().max())) + 1e-2 * want.abs()).all()
