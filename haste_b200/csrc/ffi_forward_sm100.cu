@@ -8,11 +8,11 @@
 // tiles.  Same shared-memory operand layout as the fused train step (128-byte-swizzled row blocks; X tile as
 // MN-major A with a row of ones under the gathered rows, W tile as K-major B, the bias as one more K step).
 // Everything that moves a tile is a TMA copy: the W tile through a 2-D tensor map, the X rows by tile::gather4
-// from four producer warps (the gather rate grows with the number of issuing warps), and the logits leave
+// from four or eight producer warps (the gather rate grows with the number of issuing warps), and the logits leave
 // through a tensor-map store from a swizzled staging tile, which also clips the ragged last group and the
 // ragged last batch tile (in whole 16-byte chunks: the store's extent is the writable width rounded down to 8
-// columns, and the up to 7 columns left over are written with ordinary 2-byte stores).  Warp roles (416 threads): warps 0, 2, 3, 12 produce, warp 1 issues the MMAs,
-// warps 4-11 drain the accumulator: TMEM -> bf16 -> staging tile; one thread issues the store.
+// columns, and the up to 7 columns left over are written with ordinary 2-byte stores).  Warp roles (448 or 576 threads): warp 0 brings
+// weights and bias, warps 2, 3, 12, 13 (to 17) gather, warp 1 issues the MMAs, warps 4-11 drain the accumulator: TMEM -> bf16 -> staging tile; one thread issues the store.
 // All waits are bounded (see mbar_wait).
 //
 // A launch may take every n-th label tile only (TileSet), which is how top-k samples a layer.  The TOPK instantiations write no
@@ -54,8 +54,7 @@ struct Cfg {
   static constexpr int OFF_W = OFF_X + NXS * XSTAGE;
   static constexpr int OFF_C = OFF_W + 2 * WSTAGE;
   static constexpr int OFF_BT = OFF_C + 2 * CSTAGE;
-  static constexpr int OFF_LOCR = OFF_BT + 2 * BTILE;          // int [4][F]: each producer warp's copy of the group's (clamped) indices
-  static constexpr int OFF_BAR = OFF_LOCR + 4 * F * 4;
+  static constexpr int OFF_BAR = OFF_BT + 2 * BTILE;
   static constexpr int OFF_MISC = OFF_BAR + 32 * 8;
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
@@ -65,10 +64,15 @@ struct Cfg {
   static_assert(NBAR <= 32, "barrier space");
   static constexpr int N_EPI = 8;                     // epilogue warps: 4 TMEM lane quarters x 2 column halves
   static constexpr int EC = G / 2;                    // label columns of a tile drained by one epilogue warp
-  static constexpr int NPW = 4;                       // producer warps: 0, 2, 3 and the warp after the epilogue warps
-  static_assert(NPW <= NXS, "a producer must not run more than one phase ahead on any stage barrier");
+  // The products waited for their X tiles: a warp issues one gather per 100 cycles or so, and one of four producers also waited for
+  // the weights' stage.  Now a warp of its own brings the weights, and two warps share a tile.  Forward of 670 K labels, 512 rows:
+  // 170 -> 147 us (four warps to a tile: 158; eight producers, two to a tile: 166); 131 K labels, G=32, F=64, 256 rows, 128 slots to a tile: a layer
+  // step 149 -> 138 us with eight producers, 149 with four.
+  static constexpr int NPW = F == 64 ? 4 : 8;         // X producer warps: 2, 3 and those after the epilogue warps ...
+  static constexpr int NSH = 2;                       // ... of which so many share a tile
+  static_assert(NPW / NSH <= NXS, "a producer must not run more than one phase ahead on any stage barrier");
   static constexpr int W_EPI = 4, W_XP = W_EPI + N_EPI;
-  static constexpr int NTHREADS = (W_XP + 1) * 32;
+  static constexpr int NTHREADS = (W_XP + NPW - 2) * 32;
   static constexpr uint32_t TM_COLS = 2 * G;          // two accumulator stages
   // byte offset of 16-byte chunk c (8 labels) of batch row `row` in a staging tile: as the tensor map's swizzle expects it
   __device__ static __forceinline__ int c_chunk(int row, int c) {
@@ -124,7 +128,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
   const int T = static_cast<int>((a.B + BT - 1) / BT);
 
   if (tid == 0) {
-    for (int i = 0; i < NXS; ++i) { mbar_init(bar(C::B_XFULL + i), 1); mbar_init(bar(C::B_XEMPTY + i), 1); }
+    for (int i = 0; i < NXS; ++i) { mbar_init(bar(C::B_XFULL + i), C::NSH); mbar_init(bar(C::B_XEMPTY + i), 1); }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(C::B_WFULL + i), 1);  mbar_init(bar(C::B_WEMPTY + i), 1);
       mbar_init(bar(C::B_ZFULL + i), 1);  mbar_init(bar(C::B_ZEMPTY + i), C::N_EPI);
@@ -151,83 +155,81 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
   const uint32_t tmem = *tmem_slot;
   const int n_my_groups = (a.NG > static_cast<int>(blockIdx.x)) ? (a.NG - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
 
-  const int prod_id = warp == 0 ? 0 : (warp == 2 ? 1 : (warp == 3 ? 2 : (warp == C::W_XP ? 3 : -1)));
-  if (prod_id >= 0) {
-    // ================================================================ producers
-    // Producer 0 also loads every group's W tile and writes its bias column; the X tiles (one per batch tile) are
-    // dealt round-robin over the four warps.  Lane 0 arms the stage's barrier with the byte count, then every lane
-    // issues its share of the gathers (four index rows per instruction, landing at their swizzled positions).
-    int it = 0, w_armed = 0, my_last = -1;
+  const int prod_id = warp == 2 || warp == 3 ? warp - 2 : (warp >= C::W_XP ? 2 + warp - C::W_XP : -1);
+  if (warp == 0) {
+    // ================================================================ group producer: W tile (tensor map) and bias column
+    int w_armed = 0;
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = a.set.tile(blockIdx.x + gi * gridDim.x);
       const int ws = gi & 1;
       const int64_t l0 = static_cast<int64_t>(g) * G;
       const int rows_real = static_cast<int>(imin64(G, a.L - l0));
-      const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F;
-      int locv[F / 32];
+      uint16_t bv[G / 32];
 #pragma unroll
-      for (int j = 0; j < F / 32; ++j) {
-        // the last tile may hold one group less: its slots gather row 0 and meet zero weights
-        const bool there = P == 1 || lane + 32 * j < (a.NGR - g * P) * FF;
-        locv[j] = there ? min(max(__ldg(lrow + lane + 32 * j), 0), a.D - 1) : 0;   // clamped: never addresses outside xt
+      for (int j = 0; j < G / 32; ++j) {
+        const int c = lane + 32 * j;
+        bv[j] = (a.bias != nullptr && c < rows_real) ? __bfloat16_as_ushort(a.bias[l0 + c]) : uint16_t(0);
       }
-      if (prod_id == 0) {
-        uint16_t bv[G / 32];
-#pragma unroll
-        for (int j = 0; j < G / 32; ++j) {
-          const int c = lane + 32 * j;
-          bv[j] = (a.bias != nullptr && c < rows_real) ? __bfloat16_as_ushort(a.bias[l0 + c]) : uint16_t(0);
-        }
-        const bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 21, WL, 100);
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < G / 32; ++j) {
-          const int c = lane + 32 * j;
-          *reinterpret_cast<uint16_t*>(sm + C::OFF_BT + ws * C::BTILE + (c >> 3) * 256 + (c & 7) * 16) = bv[j];
-        }
-        fence_proxy_async();
-        __syncwarp();
-        if (ok && !*abort_flag) {
-          if (lane == 0) {
-            mbar_arrive_expect_tx(bar(C::B_WFULL + ws), WSTAGE);
-#pragma unroll
-            for (int kb = 0; kb < C::NWB; ++kb)
-              tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
-          }
-          ++w_armed;
-        }
-        __syncwarp();
-      }
-      int* locr = reinterpret_cast<int*>(sm + C::OFF_LOCR) + prod_id * F;
+      const bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 21, WL, 100);
       __syncwarp();
+      const bool go = __all_sync(0xffffffffu, ok && !*abort_flag);
+      if (go) {
+        if (lane == 0) {
+          mbar_expect_tx(bar(C::B_WFULL + ws), WSTAGE);
 #pragma unroll
-      for (int j = 0; j < F / 32; ++j) locr[lane + 32 * j] = locv[j];
-      __syncwarp();
-      const int4* lr4 = reinterpret_cast<const int4*>(locr);
-      for (int t = 0; t < T; ++t, ++it) {
-        if (it % C::NPW != prod_id) continue;
-        const int xs = it % NXS;
-        const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 22, WL, 100);
-        __syncwarp();
-        if (!okx || *abort_flag) continue;
-        const int b0 = t * BT;
-        const uint32_t xb = sbase + C::OFF_X + xs * XSTAGE;
-        if (lane == 0) mbar_arrive_expect_tx(bar(C::B_XFULL + xs), F * 256);
-        __syncwarp();
-#pragma unroll
-        for (int i = lane; i < 2 * (F / 4); i += 32) {
-          const int blk = i / (F / 4), r4 = i % (F / 4);
-          const int4 lr = lr4[r4];
-          tma_gather4(xb + blk * XBLK + r4 * 512, &tm_x, b0 + blk * 64, lr.x, lr.y, lr.z, lr.w, bar(C::B_XFULL + xs));
+          for (int kb = 0; kb < C::NWB; ++kb)
+            tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
         }
-        my_last = it;
+        ++w_armed;
       }
+#pragma unroll
+      for (int j = 0; j < G / 32; ++j) {
+        const int c = lane + 32 * j;
+        *reinterpret_cast<uint16_t*>(sm + C::OFF_BT + ws * C::BTILE + (c >> 3) * 256 + (c & 7) * 16) = bv[j];
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (go && lane == 0) mbar_arrive(bar(C::B_WFULL + ws));
+      __syncwarp();
     }
-    // every copy this warp started has to land before the CTA may exit (only the most recent use of each stage:
-    // an older phase of the same barrier can no longer be waited for)
-    for (int j = max(0, it - NXS); j < it; ++j)
-      if (j % C::NPW == prod_id && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
+    // every copy this warp started has to land before the CTA may exit (only the most recent use of each stage: an older phase of the same
+    // barrier can no longer be waited for)
     for (int j = max(0, w_armed - 2); j < w_armed; ++j) mbar_wait_final(bar(C::B_WFULL + (j & 1)), (j >> 1) & 1, WL);
+  } else if (prod_id >= 0) {
+    // ================================================================ X producers
+    // F index rows of xt per batch tile, 256 bytes each, as gathers of four rows that land at their swizzled positions.  NSH warps share a tile,
+    // one load per lane, and each announces its own bytes.
+    constexpr int NLD = 2 * (F / 4) / C::NSH, STEP = C::NPW / C::NSH;            // loads per warp and tile; tiles between two of a warp
+    static_assert(NLD * C::NSH == 2 * (F / 4) && NLD <= 32, "one load per lane");
+    const int li = (prod_id % C::NSH) * NLD + lane, blk = li / (F / 4), r4 = li % (F / 4);
+    int4 lr = make_int4(0, 0, 0, 0);
+    int t = prod_id / C::NSH, gi = 0, g_have = -1, my_last = -1;
+    const int n_items = n_my_groups * T;
+    for (int it = t; it < n_items; it += STEP, t += STEP) {
+      while (t >= T) { t -= T; ++gi; }
+      if (gi != g_have) {
+        g_have = gi;
+        const int g = a.set.tile(blockIdx.x + gi * gridDim.x);
+        const int32_t* lrow = a.loc + static_cast<int64_t>(g) * F + r4 * 4;
+        // the last tile may hold one group less: its slots gather row 0 and meet zero weights
+        const bool there = lane < NLD && (P == 1 || r4 * 4 < (a.NGR - g * P) * FF);
+        const int top = a.D - 1;                         // clamped: never addresses outside xt
+        lr.x = there ? min(max(__ldg(lrow), 0), top) : 0; lr.y = there ? min(max(__ldg(lrow + 1), 0), top) : 0;
+        lr.z = there ? min(max(__ldg(lrow + 2), 0), top) : 0; lr.w = there ? min(max(__ldg(lrow + 3), 0), top) : 0;
+      }
+      const int xs = it % NXS;
+      const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 22, WL, 100);
+      __syncwarp();
+      if (!okx || *abort_flag) continue;
+      const uint32_t full = bar(C::B_XFULL + xs);
+      if (lane == 0) mbar_arrive_expect_tx(full, NLD * 512);
+      __syncwarp();
+      if (lane < NLD)
+        tma_gather4(sbase + C::OFF_X + xs * XSTAGE + blk * XBLK + r4 * 512, &tm_x, t * BT + blk * 64, lr.x, lr.y, lr.z, lr.w, full);
+      my_last = it;
+    }
+    for (int j = max(0, n_items - NXS); j < n_items; ++j)
+      if (j % STEP == prod_id / C::NSH && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
   } else if (warp == 1) {
     // ================================================================ MMA issuer
     // The warp runs its control flow converged; one elected lane issues the products and commits (descriptors stay
@@ -325,12 +327,19 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
           tc_fence_after();
           const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + zs * G + h * C::EC;
           constexpr int CW = C::EC < 32 ? C::EC : 32;            // columns per TMEM load
-#pragma unroll 1
+          // All of the tile's columns at once, so that the accumulator goes back before they are looked at (chunk by chunk: 670 K labels, 512
+          // rows 280 us for the whole top-k, so 258).
+          uint32_t ra[C::EC / CW][CW];
+          __syncwarp();
+#pragma unroll
+          for (int x = 0; x < C::EC / CW; ++x) tmem_ld(ta + x * CW, ra[x]);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
+#pragma unroll
           for (int c0 = 0; c0 < C::EC; c0 += CW) {
-            uint32_t r[CW];
-            __syncwarp();
-            tmem_ld(ta + c0, r);
-            tmem_ld_wait();
+            const uint32_t (&r)[CW] = ra[c0 / CW];
             uint32_t p[CW / 2], m[CW / 2];
 #pragma unroll
             for (int x = 0; x < CW / 2; ++x) m[x] = p[x] = pack2(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1]));
@@ -364,9 +373,6 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
               count += __popc(any);
             }
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
         }
       }
       flush();
