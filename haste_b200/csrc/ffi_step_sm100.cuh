@@ -210,9 +210,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // Hinge without the loss sum, which is what tells of a NaN logit: max drops it.  Not for (128, 64) and (64, 128), which never did at
   // multiples of 8 rows: 300 K labels (128, 64) 80 -> 84.5 us a step, the other shapes 0.5 to 1 %.
   constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
-  // Positives put right after the plain loop: 31 K labels, B=64, G=32 21.0 -> 20.2 us; not for (128, 64), whose tiles hardly ever have one (670 K
-  // labels, hinge 240 -> 247 us, 2.8 M, BCE 2,233 -> 2,418: the loop's registers).
-  constexpr bool PATCH = GG != 128;
+  // Columns with positives put right after the plain loop: 31 K labels, B=64, G=32 21.0 -> 18.6 us; not for (128, 64), whose tiles hardly ever
+  // have one (up to 12 columns: 670 K labels, hinge 240 -> 249 us, 2.8 M, BCE 2,217 -> 2,308: the loop's registers).
+  constexpr int PATCH = GG != 128 ? 12 : 0;
   // Two chunks per pass of the loss epilogue's plain loop hide some of the MUFU's latency: 2.8 M labels, BCE, 2,284 -> 2,235 us; the other
   // instantiations lose by it (501 K labels 278 -> 297, hinge 670 K 252 -> 253: instruction cache).
   constexpr int UNROLL = LOSS == HASTE_LOSS_BCE && F == 64 ? 2 : 1;
@@ -555,21 +555,15 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const int zs = it & 1;
         const int b0 = tile_b0(t);
         uint64_t ym = 0ull;                              // target bits of this thread's row, EA_COLS label columns
-        // Few targets in the tile's groups (the common case).  PATCH: the plain loop treats every label as a negative, and the few
-        // positives are put right one by one afterwards; their bits are only collected where the other loop is taken.
-        // Otherwise each thread picks the bits of its own row and its label columns from the entry list (no shared
-        // bitmap, no barrier between the epilogue warps), and tiles with targets take the other loop.
-        const bool few = t_end - t_beg <= C::NTE;
-        auto few_bits = [&]() {
+        if (t_end - t_beg <= C::NTE) {
+          // Few targets in the tile's groups (the common case): each thread picks the bits of its own row and its label
+          // columns straight from the entry list — no shared bitmap, no barrier between the epilogue warps.
           const uint32_t rowkey = static_cast<uint32_t>(b0 + row);
           for (int i = t_beg; i < t_end; ++i) {
             const uint32_t e = tgt_s[4 + i - t_beg];
             const uint32_t c = (e & 0xFFu) + (P == 2 && i >= t_mid ? GG : 0) - static_cast<uint32_t>(h * EA_COLS);
             if ((e >> 8) == rowkey && c < static_cast<uint32_t>(EA_COLS)) ym |= 1ull << c;
           }
-        };
-        if (few) {
-          if (!PATCH) few_bits();
         } else {
           uint32_t* yb = ybits + (it & 1) * BT * YBW;
           for (int i = et; i < BT * YBW; i += N_EA * 32) yb[i] = 0u;
@@ -661,9 +655,18 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
           if (WITH_LOSS && LOSS != HASTE_LOSS_SQHINGE)
             fast_loss += __log2f(((bp[0] * bp[1]) * (bp[2] * bp[3])) * (LOSS == HASTE_LOSS_BCE ? 0x1p-16f : 1.f));
         };
-        // Without a target in a warp's 32 rows and 64 columns, or with few, and without a ragged edge: a loop with nothing but the arithmetic.
-        bool plain = !DEBUG && !ragged && ((PATCH && few) || !__any_sync(0xffffffffu, ym != 0ull));
-        if (PATCH && few && !plain) few_bits();
+        // Tiles without a target in a warp's 32 rows and its columns take a loop with nothing but the arithmetic.  With PATCH so do those with
+        // targets in up to PATCH columns: the loop treats every label as a negative, and these columns are put right one by one
+        // afterwards.
+        uint32_t pos_lo = 0u, pos_hi = 0u;                  // columns with a target in any of the warp's rows
+        bool plain = !DEBUG && !ragged;
+        if (PATCH > 0) {
+          pos_lo = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(ym));
+          if (EA_COLS > 32) pos_hi = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(ym >> 32));
+          plain = plain && __popc(pos_lo) + __popc(pos_hi) <= PATCH;
+        } else {
+          plain = plain && !__any_sync(0xffffffffu, ym != 0ull);
+        }
         for (;;) {                                         // one pass; rarely a second (below)
         bool again = false;
         if (plain) {
@@ -675,19 +678,14 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
             tmem_ld_wait();
             plain_chunk(r, yrow + ((col0 + c16) >> 6) * YBLK, ((col0 + c16) & 63) >> 3);
           }
-          if (PATCH && few) {
-#pragma unroll 1
-            for (int i = t_beg; i < t_end; ++i) {
-              const uint32_t e = tgt_s[4 + i - t_beg];
-              const uint32_t c = (e & 0xFFu) + (P == 2 && i >= t_mid ? GG : 0) - static_cast<uint32_t>(h * EA_COLS);
-              const uint32_t rw = (e >> 8) - static_cast<uint32_t>(b0 + q * 32);           // row and column of the warp's part of the tile
-              if (rw >= 32u || c >= static_cast<uint32_t>(EA_COLS)) continue;             // (uniform)
-              bool twice = false;                                                         // the same target listed before
-              for (int k = t_beg; k < i; ++k) twice = twice || (tgt_s[4 + k - t_beg] == e && (P == 1 || (k >= t_mid) == (i >= t_mid)));
+          if (PATCH > 0) {
+            while ((pos_lo | pos_hi) != 0u) {              // (uniform)
+              const int c = pos_lo != 0u ? __ffs(pos_lo) - 1 : 31 + __ffs(pos_hi);
+              if (pos_lo != 0u) pos_lo &= pos_lo - 1u; else pos_hi &= pos_hi - 1u;
               __syncwarp();
               const uint32_t zb = tmem_ld1(ta + c);
               tmem_ld_wait();
-              if (lane == static_cast<int>(rw) && !twice) {
+              if ((ym >> c) & 1u) {
                 const float zr = round_bf16_as_f32(__uint_as_float(zb));
                 float gl, la;                              // gradient as a positive; its loss less the loss counted as a negative
                 if (LOSS == HASTE_LOSS_SQHINGE) {
@@ -699,11 +697,11 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                   gl = ((LOSS == LOSS_BCE_EXP ? sigmoid_exp(zr) : fmaf(0.5f, tanh_approx(0.5f * zr), 0.5f)) - 1.f) * gs;
                   la = -zr;
                 }
-                const int cc = col0 + static_cast<int>(c);
+                const int cc = col0 + c;
                 *reinterpret_cast<__nv_bfloat16*>(yrow + (cc >> 6) * YBLK + ((((cc & 63) >> 3) ^ (row & 7)) << 4) + (cc & 7) * 2) = __float2bfloat16_rn(gl);
                 if (WITH_LOSS) tile_loss += la;
                 // a logit so large that the difference says nothing (or infinite, or NaN): once more through the other loop
-                again = !(fabsf(zr) < 1024.f);
+                again = again || !(fabsf(zr) < 1024.f);
               }
             }
             again = __any_sync(0xffffffffu, again);
@@ -779,7 +777,6 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         // general branch, which has a value for it; so does one whose sum of squares overflows.  (max(x, 0) in place of x + |x| needs no second pass and took 1.6 % more
         // of the 670 K step: 276.9 against 272.5 us; this way 274.3.  BCE sums max(z, 0): 2.8 M labels 2,310 against 2,320 us.)
         if (!again && (LOSS != HASTE_LOSS_SQHINGE || !WITH_LOSS || DEBUG || ragged || !__any_sync(0xffffffffu, !(fast_loss < INFINITY)))) break;
-        if (PATCH && few && plain) few_bits();
         ragged = true; plain = false;
         tile_loss = fast_loss = 0.f;
         fh[0] = fh[1] = {0.f, 0.f};
@@ -833,31 +830,55 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DX + ds * F + kc * C::EBS;
         const bool live = !*abort_flag;
         const int b1 = tile_b0(t) + row, b4 = tile_b0(t) + q * 32 + 4 * (lane & 7);
+        // two loops, although they differ in their last lines only: one loop with both forms inside took 151 us for 131 K labels and 290 for 501 K, so 138
+        // and 271 (instruction cache; the BCE step of 2.8 M labels 2,217 and 2,272)
+        if (a.dxt_v4) {
+          const bool on = live && b4 < a.B;
+          float* dst = a.dxt + b4;
 #pragma unroll 1
-        for (int c = 0; c < C::EBS; c += C::EBP) {
-          uint32_t r[C::EBP];
-          __syncwarp();
-          tmem_ld(ta + c, r);
-          tmem_ld_wait();
-          if (c == C::EBS - C::EBP) {
-            tc_fence_before();
+          for (int c = 0; c < C::EBS; c += C::EBP) {
+            uint32_t r[C::EBP];
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar(C::B_DXEMPTY + ds));
-          }
-          if (a.dxt_v4) {
+            tmem_ld(ta + c, r);
+            tmem_ld_wait();
+            if (c == C::EBS - C::EBP) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(C::B_DXEMPTY + ds));
+            }
 #pragma unroll
             for (int k = 0; k < C::EBP; ++k) buf[k * 32 + lane] = __uint_as_float(r[k]);
             __syncwarp();
-            if (live && b4 < a.B) {
-              float* dst = a.dxt + b4;
+            if (on) {
 #pragma unroll
               for (int k = 0; k < C::EBP / 4; ++k)
                 red_add_v4(dst + loc_g[c + 4 * k + (lane >> 3)], *reinterpret_cast<const float4*>(buf + k * 128 + lane * 4));
             }
-          } else if (live && b1 < a.B) {
-            float* dst = a.dxt + b1;
+          }
+        } else {
+          const bool on = live && b1 < a.B;
+          float* dst = a.dxt + b1;
+#pragma unroll 1
+          for (int c = 0; c < C::EBS; c += C::EBP) {
+            uint32_t r[C::EBP];
+            __syncwarp();
+            tmem_ld(ta + c, r);
+            tmem_ld_wait();
+            if (c == C::EBS - C::EBP) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(C::B_DXEMPTY + ds));
+            }
+            if (on) {
 #pragma unroll
-            for (int k = 0; k < C::EBP; ++k) atomicAdd(dst + loc_g[c + k], __uint_as_float(r[k]));
+              for (int k = 0; k < C::EBP; k += 4) {
+                const uint4 lc = *reinterpret_cast<const uint4*>(loc_g + c + k);
+                atomicAdd(dst + lc.x, __uint_as_float(r[k + 0]));
+                atomicAdd(dst + lc.y, __uint_as_float(r[k + 1]));
+                atomicAdd(dst + lc.z, __uint_as_float(r[k + 2]));
+                atomicAdd(dst + lc.w, __uint_as_float(r[k + 3]));
+              }
+            }
           }
         }
       }
