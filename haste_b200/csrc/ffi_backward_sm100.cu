@@ -116,6 +116,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
   uint32_t* loc_s = reinterpret_cast<uint32_t*>(sm + C::OFF_LOC);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 8);
+  volatile int* x_last = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 16);      // [NPW] the last tile each X producer announced
   auto bar = [&](int i) { return sbase + C::OFF_BAR + i * 8; };
   const long long WL = a.wait_limit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -163,7 +164,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     // through the tensor map.  Per batch tile: F index rows of xt, 256 bytes each, as TMA gather4 loads (four index
     // rows per instruction, landing at their swizzled positions), dealt round-robin over the four warps.
     int it = 0, w_armed = 0, my_last = -1;
-    for (int gi = 0; gi < n_my_groups; ++gi) {
+    bool go = true;
+    for (int gi = 0; go && gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
       const int ws = gi & 1;
       const int64_t l0 = static_cast<int64_t>(g) * LS;
@@ -179,20 +181,20 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 31, WL, 100);
         ok = mbar_wait(bar(C::B_LEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 31, WL, 100) && ok;
         __syncwarp();
+        // After an abort (the flag stays up) the stage may still have readers: nothing of it is touched any more.
+        if (!__all_sync(0xffffffffu, ok && !*abort_flag)) break;
 #pragma unroll
         for (int j = 0; j < F / 32; ++j)
           loc_s[ws * F + lane + 32 * j] = static_cast<uint32_t>(locv[j]) * static_cast<uint32_t>(a.B);   // D * B < 2^32 is a launch condition
         __syncwarp();
-        if (ok && !*abort_flag) {
-          if (lane == 0) {
-            // the arrival also releases the index row written above to the warps that wait for this barrier
-            mbar_arrive_expect_tx(bar(C::B_WFULL + ws), WSTAGE);
+        if (lane == 0) {
+          // the arrival also releases the index row written above to the warps that wait for this barrier
+          mbar_arrive_expect_tx(bar(C::B_WFULL + ws), WSTAGE);
 #pragma unroll
-            for (int kb = 0; kb < C::NWB; ++kb)
-              tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
-          }
-          ++w_armed;
+          for (int kb = 0; kb < C::NWB; ++kb)
+            tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
         }
+        ++w_armed;
         __syncwarp();
       }
       int* locr = reinterpret_cast<int*>(sm + C::OFF_LOCR) + prod_id * F;
@@ -206,7 +208,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         const int xs = it % NXS;
         const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 32, WL, 100);
         __syncwarp();
-        if (!okx || *abort_flag) continue;
+        go = __all_sync(0xffffffffu, okx && !*abort_flag);
+        if (!go) break;
         const int b0 = t * BT;
         const uint32_t xb = sbase + C::OFF_X + xs * XSTAGE;
         if (lane == 0) mbar_arrive_expect_tx(bar(C::B_XFULL + xs), F * 256);
@@ -220,9 +223,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
         my_last = it;
       }
     }
+    if (lane == 0) x_last[prod_id] = my_last;
     // every copy this warp started has to land before the CTA may exit (only the most recent use of each stage)
-    for (int j = max(0, it - NXS); j < it; ++j)
-      if (j % C::NPW == prod_id && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
     for (int j = max(0, w_armed - 2); j < w_armed; ++j) mbar_wait_final(bar(C::B_WFULL + (j & 1)), (j >> 1) & 1, WL);
   } else if (warp >= C::W_Y && warp < C::W_XP) {
     // ================================================================ Y warps: dY slice -> aligned, swizzled Y tile
@@ -583,6 +585,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, C::TM_COLS);
+  // every copy into this CTA's shared memory lands before it exits (without an abort the issuer has waited for all of them)
+  if (warp == 2 && lane == 0 && *abort_flag) drain_x_ring<NXS, C::NPW, 1>(bar(C::B_XFULL), x_last, WL);
 }
 
 template <int GG_, int FF_, int P_>

@@ -122,6 +122,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
   const uint32_t sbase = smem_u32(sm);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 8);
+  volatile int* x_last = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 16);      // [NPW] the last tile each X producer announced
   auto bar = [&](int i) { return sbase + C::OFF_BAR + i * 8; };
   const long long WL = a.wait_limit;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -220,7 +221,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
       const int xs = it % NXS;
       const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 22, WL, 100);
       __syncwarp();
-      if (!okx || *abort_flag) continue;
+      if (!__all_sync(0xffffffffu, okx && !*abort_flag)) break;          // (the flag stays up)
       const uint32_t full = bar(C::B_XFULL + xs);
       if (lane == 0) mbar_arrive_expect_tx(full, NLD * 512);
       __syncwarp();
@@ -228,8 +229,7 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
         tma_gather4(sbase + C::OFF_X + xs * XSTAGE + blk * XBLK + r4 * 512, &tm_x, t * BT + blk * 64, lr.x, lr.y, lr.z, lr.w, full);
       my_last = it;
     }
-    for (int j = max(0, n_items - NXS); j < n_items; ++j)
-      if (j % STEP == prod_id / C::NSH && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
+    if (lane == 0) x_last[prod_id] = my_last;
   } else if (warp == 1) {
     // ================================================================ MMA issuer
     // The warp runs its control flow converged; one elected lane issues the products and commits (descriptors stay
@@ -441,6 +441,8 @@ ffi_forward_sm100_kernel(FwdArgs a, const __grid_constant__ CUtensorMap tm_x, co
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, C::TM_COLS);
+  // every copy into this CTA's shared memory lands before it exits (without an abort the issuer has waited for all of them)
+  if (warp == 2 && lane == 0 && *abort_flag) drain_x_ring<NXS, C::NPW, C::NSH>(bar(C::B_XFULL), x_last, WL);
 }
 
 template <int GG_, int FF_, int P_>

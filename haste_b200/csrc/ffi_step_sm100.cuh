@@ -95,7 +95,7 @@ struct Cfg {
   static constexpr int OFF_G = OFF_EB + 8 * EBP * 128;         // bf16 [8 update warps][label rows][slots]: gradients on their way to the update
   static constexpr int GSTAGE = (G / 4) * (FF / 2) * 2;        // of one update warp: the rows of a TMEM lane quarter (absent labels too), half the slots
   static constexpr int OFF_BAR = OFF_G + 8 * GSTAGE;
-  static constexpr int OFF_MISC = OFF_BAR + 32 * 8;            // tmem base address, abort flag
+  static constexpr int OFF_MISC = OFF_BAR + 32 * 8;            // tmem base address, abort flag, last tiles of the X producers
   static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;      // + slack for the 1024-byte alignment of the base
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
   static_assert(XSTAGE % 1024 == 0 && WBLK % 1024 == 0 && YBLK % 1024 == 0 && OFF_BT % 128 == 0, "tile alignment");
@@ -225,6 +225,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   uint32_t* ybits = reinterpret_cast<uint32_t*>(sm + C::OFF_YB);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + C::OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 8);
+  volatile int* x_last = reinterpret_cast<volatile int*>(sm + C::OFF_MISC + 16);      // [NPW] the last tile each X producer announced
   auto bar = [&](int i) { return sbase + C::OFF_BAR + i * 8; };
   const long long WL = a.wait_limit;
 
@@ -375,7 +376,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       const int xs = it % NXS;
       const bool okx = mbar_wait(bar(C::B_XEMPTY + xs), ((it / NXS) & 1) ^ 1, abort_flag, a.err, 2, WL, 100);
       __syncwarp();
-      if (!okx || *abort_flag) continue;
+      if (!__all_sync(0xffffffffu, okx && !*abort_flag)) break;          // (the flag stays up)
       const uint32_t full = bar(C::B_XFULL + xs);
       if (lane == 0) mbar_arrive_expect_tx(full, NLD * 512);
       __syncwarp();
@@ -383,10 +384,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         tma_gather4(sbase + C::OFF_X + xs * XSTAGE + blk * XBLK + r4 * 512, &tm_x, tile_b0(t) + blk * 64, lr.x, lr.y, lr.z, lr.w, full);
       my_last = it;
     }
-    // Every copy this warp started lands before the CTA may exit.  (Only the most recent use of each stage: an older phase of the same
-    // barrier can no longer be waited for.)
-    for (int j = max(0, n_items - NXS); j < n_items; ++j)
-      if (j % STEP == prod_id / C::NSH && j <= my_last) mbar_wait_final(bar(C::B_XFULL + j % NXS), (j / NXS) & 1, WL);
+    if (lane == 0) x_last[prod_id] = my_last;
   } else if (warp == 1 || warp == 3) {
     // ================================================================ MMA issuers (one elected lane each)
     // Feeding the tensor pipe from a single thread costs more cycles per tcgen05.mma than the small (N = 64..144)
@@ -1028,6 +1026,8 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, C::TM_COLS);
+  // every copy into this CTA's shared memory lands before it exits (without an abort the issuer has waited for all of them)
+  if (warp == 2 && lane == 0 && *abort_flag) drain_x_ring<NXS, C::NPW, C::NSH>(bar(C::B_XFULL), x_last, WL);
 }
 
 // Launch one shape.  `dump` selects the debug instantiation (always accumulates the loss).

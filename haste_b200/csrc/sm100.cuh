@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ring.h"
+
 namespace haste {
 namespace sm100 {
 
@@ -88,13 +90,27 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Bounded wait that ignores the abort flag: for work that has to finish before the CTA may exit (copies in flight
-// into its shared memory, tensor-core products writing its TMEM), also on the way out after an abort.
+// into its shared memory, tensor-core products writing its TMEM), also on the way out after an abort.  However short the limit of the
+// other waits, this one leaves copies and products the milliseconds they could need.
 __device__ __noinline__ static bool mbar_wait_final(uint32_t bar, uint32_t parity, long long limit) {
   const long long t0 = clock64();
+  if (limit < (1ll << 24)) limit = 1ll << 24;
   while (!mbar_try_wait_hint(bar, parity, 4000u)) {
     if (clock64() - t0 > limit) return false;
   }
   return true;
+}
+// One thread, after every producer warp has left its loop because the abort flag is up: ends the phases that wait for announcements
+// nobody will make any more, and waits until what was announced has landed.  (Without an abort the consumers have waited for every item.)
+template <int NXS, int NPW, int NSH>
+__device__ __noinline__ void drain_x_ring(uint32_t full0, const volatile int* last, long long limit) {
+#pragma unroll 1
+  for (int s = 0; s < NXS; ++s) {
+    const RingDrain d = ring_drain<NXS, NPW, NSH>(s, [&](int p) { return last[p]; });
+    if (d.item < 0) continue;
+    for (int i = 0; i < d.missing; ++i) mbar_arrive(full0 + 8 * s);
+    mbar_wait_final(full0 + 8 * s, (d.item / NXS) & 1, limit);
+  }
 }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
