@@ -104,7 +104,7 @@ struct Cfg {
   static constexpr int B_XFULL = 0, B_XEMPTY = NXS, B_WFULL = 2 * NXS, B_WEMPTY = B_WFULL + 2, B_ZFULL = B_WEMPTY + 2,
                        B_ZEMPTY = B_ZFULL + 2, B_YFULL = B_ZEMPTY + 2, B_YEMPTY = B_YFULL + NYS, B_DXFULL = B_YEMPTY + NYS,
                        B_DXEMPTY = B_DXFULL + NDX, B_DWFULL = B_DXEMPTY + NDX, B_DWEMPTY = B_DWFULL + 1, B_MEMPTY = B_DWEMPTY + 1,
-                       B_FIN = B_MEMPTY + 2, NBAR = B_FIN + 2;   // B_FIN: one per issuer warp, "all my products have completed"
+                       B_FIN = B_MEMPTY + 2, B_YBITS = B_FIN + 2, NBAR = B_YBITS + 1;   // B_FIN: one per issuer warp, "all my products have completed"
   static_assert(NBAR <= 32, "barrier space");
 
   // TMEM columns: Z double-buffered, dXg NDX stages, dW single (F + 16)
@@ -253,6 +253,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     mbar_init(bar(C::B_DWEMPTY), N_UP);
     mbar_init(bar(C::B_FIN), 1);
     mbar_init(bar(C::B_FIN + 1), 1);
+    mbar_init(bar(C::B_YBITS), N_EA);
     mbar_fence_init();
     *abort_flag = 0;
   }
@@ -316,17 +317,16 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       bool ok = mbar_wait(bar(C::B_WEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 1, WL, 100);
       ok = mbar_wait(bar(C::B_MEMPTY + ws), ((gi >> 1) & 1) ^ 1, abort_flag, a.err, 1, WL, 100) && ok;
       __syncwarp();
-      const bool go = __all_sync(0xffffffffu, ok && !*abort_flag);
-      if (go) {
-        // the weights first: their way from memory is the longest
-        if (lane == 0) {
-          mbar_expect_tx(bar(C::B_WFULL + ws), C::WBYTES);
+      // After an abort (the flag stays up) the stage may still have readers: nothing of it is touched any more.
+      if (!__all_sync(0xffffffffu, ok && !*abort_flag)) break;
+      // the weights first: their way from memory is the longest
+      if (lane == 0) {
+        mbar_expect_tx(bar(C::B_WFULL + ws), C::WBYTES);
 #pragma unroll
-          for (int kb = 0; kb < C::NWB; ++kb)
-            tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
-        }
-        ++w_armed;
+        for (int kb = 0; kb < C::NWB; ++kb)
+          tma_load_2d(sbase + C::OFF_W + ws * WSTAGE + kb * WBLK, &tm_w, kb * 64, static_cast<int>(l0), bar(C::B_WFULL + ws));
       }
+      ++w_armed;
       // lanes 0 .. 2: entry range of the tile's groups, lanes 4 .. 4 + NTE - 1: the first entries
       uint32_t tv = lane == 0 ? t_beg : (lane == 1 ? t_mid : t_end);
       if (lane >= 4 && t_beg + lane - 4 < t_end && lane < 4 + C::NTE) tv = __ldg(a.tgt_ent + t_beg + lane - 4);
@@ -342,7 +342,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       }
       fence_proxy_async();
       __syncwarp();
-      if (go && lane == 0) mbar_arrive(bar(C::B_WFULL + ws));
+      if (lane == 0) mbar_arrive(bar(C::B_WFULL + ws));
       __syncwarp();
     }
     // Every copy this warp started has to land before the CTA may exit (normally the consumers have long seen them;
@@ -539,6 +539,14 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     const int et = tid - C::W_EA * 32;           // thread index inside the role
     float loss_acc = 0.f;
     const float inv_4gs2_sq = 0.0625f / (a.grad_scale * a.grad_scale);   // undoes the (4 s)^2 carried by the fast loss sum
+    // The role's warps meet twice per tile with a bitmap.  Not at a named barrier, which knows no limit: after a wait that gave up the warps
+    // need not agree on which tiles have one.
+    auto warps_meet = [&](int phase) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(C::B_YBITS));
+      mbar_wait(bar(C::B_YBITS), phase, abort_flag, a.err, 17, WL);
+      __syncwarp();
+    };
     int it = 0, ys = 0, yph = 0;                 // global tile counter, its dY stage and phase
     for (int gi = 0; gi < n_my_groups; ++gi) {
       const int g = group_of(gi);
@@ -546,8 +554,8 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
       const int rows_real = static_cast<int>(imin64(LS, a.L - static_cast<int64_t>(g) * LS));
       // the group producer left the entry range (contiguous; entries from t_mid on belong to the second group of a pair) and the first entries
       const uint32_t* tgt_s = reinterpret_cast<const uint32_t*>(sm + C::OFF_TGT) + ws * (4 + C::NTE);
-      mbar_wait(bar(C::B_WFULL + ws), (gi >> 1) & 1, abort_flag, a.err, 16, WL);
-      const uint4 tr = *reinterpret_cast<const uint4*>(tgt_s);
+      const bool there = __all_sync(0xffffffffu, mbar_wait(bar(C::B_WFULL + ws), (gi >> 1) & 1, abort_flag, a.err, 16, WL));
+      const uint4 tr = there ? *reinterpret_cast<const uint4*>(tgt_s) : make_uint4(0u, 0u, 0u, 0u);      // (what a wait that gave up left behind is no range)
       const int t_beg = static_cast<int>(tr.x), t_mid = static_cast<int>(tr.y), t_end = static_cast<int>(tr.z);
       for (int t = 0; t < T; ++t) {
         const int zs = it & 1;
@@ -565,7 +573,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         } else {
           uint32_t* yb = ybits + (it & 1) * BT * YBW;
           for (int i = et; i < BT * YBW; i += N_EA * 32) yb[i] = 0u;
-          named_bar_sync(1, N_EA * 32);
+          warps_meet(0);
           // head groups of a long-tailed label distribution hold thousands of entries: eight independent loads in
           // flight per thread, so that the scan runs at L2 throughput rather than one L2 latency per entry
           for (int i0 = t_beg + et; i0 < t_end; i0 += 8 * N_EA * 32) {
@@ -582,7 +590,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
               if (rb >= 0 && rb < BT && c < G) atomicOr(&yb[rb * YBW + (c >> 5)], 1u << (c & 31));
             }
           }
-          named_bar_sync(1, N_EA * 32);
+          warps_meet(1);
           if (EA_COLS == 32) ym = yb[row * YBW + h];
           else ym = static_cast<uint64_t>(yb[row * YBW + h * 2]) | (static_cast<uint64_t>(yb[row * YBW + h * 2 + 1]) << 32);
         }

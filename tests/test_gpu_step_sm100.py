@@ -252,3 +252,31 @@ def test_sm100_step_wait_runs_out_and_recovers(hb):
     _close(z, z_ref, 1e-2, 1e-3 * max(1.0, float(z_ref.abs().max())), "logits after recovery")
     want_w, _ = fo.sgd_update(inp["W"], dw.cpu(), None, 0.05, 1e-4, 0.0, False, True, fo.rand16_for((L, F), 123, 3, "packed", 0))
     assert np.array_equal(_bits(w), fo._bf16_to_bits(want_w))
+
+
+@pytest.mark.parametrize("tile", [0, 3, 8])
+@pytest.mark.parametrize("kind", KINDS, ids=["G128F64", "G64F128"])
+def test_sm100_step_wait_runs_out_among_listed_and_bitmap_groups(hb, kind, tile):
+    """As above with six groups a CTA, some without targets, some with a short list and some with a bitmap, for which the loss-epilogue warps
+    meet: after the wait has given up they need not agree on which tile has one, and must come to an end all the same."""
+    ffi, lib = hb
+    G, F = kind
+    B, D, NG = 256, 256, 148 * 6
+    L = G * NG
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=10, bias_zero=False)
+    pairs = [((7 * i + g) % B, g * G + (11 * i) % G) for g in range(NG) for i in range((0, 3, 40)[g % 3])]
+    inp["targets"] = torch.tensor(sorted(set(pairs)), dtype=torch.int32)
+    assert lib.lib.haste_poll_status() == lib.OK
+    try:
+        assert lib.lib.haste_debug_set_wait_limit(2_000_000) == lib.OK       # about 1 ms
+        assert lib.lib.haste_debug_stall_next_step(tile) == lib.OK
+        _run(ffi, lib, inp, B, D, L, lib.LOSS_SQHINGE, 1.0, "packed", G=G)      # returns by itself; outputs invalid
+    finally:
+        lib.lib.haste_debug_set_wait_limit(4_000_000_000)
+    assert lib.lib.haste_poll_status() == lib.ERR_TIMEOUT
+    w, b, dxt, loss, z, dw, db = _run(ffi, lib, inp, B, D, L, lib.LOSS_SQHINGE, 1.0, "packed", G=G)
+    assert lib.lib.haste_poll_status() == lib.OK
+    loss_ref, dY = fo.loss_and_grad(z.cpu(), inp["targets"], fo.LOSS_SQHINGE, 1.0)
+    assert abs(loss - loss_ref) <= 1e-3 * abs(loss_ref)
+    want_w, _ = fo.sgd_update(inp["W"], dw.cpu(), None, 0.05, 1e-4, 0.0, False, True, fo.rand16_for((L, F), 123, 3, "packed", 0))
+    assert np.array_equal(_bits(w), fo._bf16_to_bits(want_w))
