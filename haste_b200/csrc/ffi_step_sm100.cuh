@@ -211,8 +211,10 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // multiples of 8 rows: 300 K labels (128, 64) 80 -> 84.5 us a step, the other shapes 0.5 to 1 %.
   constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
   // Columns with positives put right after the plain loop: 31 K labels, B=64, G=32 21.0 -> 18.6 us; not for (128, 64), whose tiles hardly ever
-  // have one (up to 12 columns: 670 K labels, hinge 240 -> 249 us, 2.8 M, BCE 2,217 -> 2,308: the loop's registers).
-  constexpr int PATCH = GG != 128 ? 12 : 0;
+  // have one (up to 12 columns: 670 K labels, hinge 240 -> 249 us, 2.8 M, BCE 2,217 -> 2,308: the loop's registers).  Nor for the hinge loss:
+  // a confident positive counted as a negative first, with (1 + z)^2, costs the sum its low bits, and what is left when it is taken out again has
+  // either sign (z near 50: relative error 9e-5 instead of 2e-7 of the loss).  For BCE the two differ by z, which bf16 logits add up exactly.
+  constexpr int PATCH = GG != 128 && !(LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS) ? 12 : 0;
   // Two chunks per pass of the loss epilogue's plain loop hide some of the MUFU's latency: 2.8 M labels, BCE, 2,284 -> 2,235 us; the other
   // instantiations lose by it (501 K labels 278 -> 297, hinge 670 K 252 -> 253: instruction cache).
   constexpr int UNROLL = LOSS == HASTE_LOSS_BCE && F == 64 ? 2 : 1;
@@ -695,9 +697,8 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 const float zr = round_bf16_as_f32(__uint_as_float(zb));
                 float gl, la;                              // gradient as a positive; its loss less the loss counted as a negative
                 if (LOSS == HASTE_LOSS_SQHINGE) {
-                  const float m = fmaxf(1.f - zr, 0.f), n = fmaxf(1.f + zr, 0.f);
-                  gl = -m * gs2;
-                  la = m * m - n * n;
+                  gl = -fmaxf(1.f - zr, 0.f) * gs2;
+                  la = 0.f;                                // (no loss sum)
                 } else {
                   // softplus(-z) - softplus(z) = -z
                   gl = ((LOSS == LOSS_BCE_EXP ? sigmoid_exp(zr) : fmaf(0.5f, tanh_approx(0.5f * zr), 0.5f)) - 1.f) * gs;

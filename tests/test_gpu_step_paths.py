@@ -78,3 +78,33 @@ def test_backward_reads_dy_at_any_offset_and_nothing_else(G, F, B, tail, off):
             got, want = got.float().cpu(), want.float()
             # bf16 outputs of fp32 sums
             assert ((got - want).abs() <= 1e-3 * max(1.0, float(want.abs().max())) + 1e-2 * want.abs()).all()
+
+
+@pytest.mark.parametrize("z_pos", [8.0, 50.0, 300.0, 900.0])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_hinge_loss_beside_confident_positives(G, F, z_pos):
+    """A positive beyond the margin has no loss, however far.  Every negative lies on the margin but one per row and group, which is all there is
+    to sum: beside positives of z_pos its loss must come out to the accuracy of an fp32 sum."""
+    from haste_b200.fused import FusedFFIShard
+    B, NG, D, scale = 64, 5, 160, 0.3
+    L, gen = NG * G, torch.Generator().manual_seed(F)
+    loc = torch.stack([torch.randperm(D, generator=gen)[:F].sort().values for _ in range(NG)]).int()
+    X = torch.zeros(B, D, dtype=torch.bfloat16)
+    X[torch.arange(B), torch.arange(B)] = 1.0                      # row b has feature b alone: weights set the logits one by one
+    W, bias = torch.zeros(L, F, dtype=torch.bfloat16), torch.full((L,), -1.0, dtype=torch.bfloat16)
+    pairs, n_off = [], 0
+    for g in range(NG):
+        slots = [k for k in range(F) if int(loc[g, k]) < B]
+        for i in (0, 1):                                           # two rows with a positive and, in the same columns' half, a negative off the margin
+            b, k = int(loc[g, slots[i]]), slots[i]
+            W[g * G + 3 + i, k] = z_pos + 1.0                      # logit z_pos
+            W[g * G + 9 + i, k] = 0.25                             # logit -0.75: loss 1/16
+            pairs.append((b, g * G + 3 + i))
+            n_off += 1
+    z = fo.forward(loc, X, W, bias, G).double()
+    assert float(z[pairs[0][0], pairs[0][1]]) == pytest.approx(z_pos, rel=2 ** -8)
+    sh = FusedFFIShard(loc.cuda(), W.cuda(), bias.cuda(), G, D, loss="squared_hinge", lr=0.0, seed=1, grad_scale=scale)
+    _, loss = sh.step(X.cuda(), torch.tensor(sorted(pairs), dtype=torch.int32).cuda())
+    want = n_off / 16.0 * scale
+    # ten equal terms, each rounded a few times to 2^-24
+    assert abs(float(loss) - want) <= 1e-5 * want
