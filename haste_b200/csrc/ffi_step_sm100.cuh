@@ -210,11 +210,13 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // Hinge without the loss sum, which is what tells of a NaN logit: max drops it.  Not for (128, 64) and (64, 128), which never did at
   // multiples of 8 rows: 300 K labels (128, 64) 80 -> 84.5 us a step, the other shapes 0.5 to 1 %.
   constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
-  // Columns with positives put right after the plain loop: 31 K labels, B=64, G=32 21.0 -> 18.6 us; not for (128, 64), whose tiles hardly ever
-  // have one (up to 12 columns: 670 K labels, hinge 240 -> 249 us, 2.8 M, BCE 2,217 -> 2,308: the loop's registers).  Nor for the hinge loss:
+  // Up to so many columns with positives are put right after the plain loop: 31 K labels, G=32, B=64 (BCE) 20.6 -> 18.6 us a step.  One column
+  // after the other, and each waits for its logits: with up to 12 the kernel took 33 us for 8.8 K labels, G=32, B=1024, one positive a row, where
+  // no tile of the SM's hides it; with up to 4 27, and nothing else became slower.  Not for (128, 64), whose tiles hardly ever have one at the
+  // sizes of 670 K and 2.8 M labels (4 % slower there: the loop's registers).  Nor for the hinge loss:
   // a confident positive counted as a negative first, with (1 + z)^2, costs the sum its low bits, and what is left when it is taken out again has
   // either sign (z near 50: relative error 9e-5 instead of 2e-7 of the loss).  For BCE the two differ by z, which bf16 logits add up exactly.
-  constexpr int PATCH = GG != 128 && !(LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS) ? 12 : 0;
+  constexpr int PATCH = GG != 128 && !(LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS) ? 4 : 0;
   // Two chunks per pass of the loss epilogue's plain loop hide some of the MUFU's latency: 2.8 M labels, BCE, 2,284 -> 2,235 us; the other
   // instantiations lose by it (501 K labels 278 -> 297, hinge 670 K 252 -> 253: instruction cache).
   constexpr int UNROLL = LOSS == HASTE_LOSS_BCE && F == 64 ? 2 : 1;
