@@ -473,6 +473,9 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     // TMEM lane == label row (G = 64: an M = 64 accumulator occupies lanes 0-15 of each lane quarter).  32 slots at a time go through
     // shared memory, so that a lane then has one 16-byte chunk of a row and neighbouring lanes neighbouring chunks: stores
     // (and the update's loads) cover runs of 64 bytes instead of one row per lane (670 K labels 563 -> 551 us a layer step).
+    // A batch of one tile gives a group no more time than this takes, and the accumulator goes back only afterwards: 32 columns per TMEM load, and
+    // with G = 64, where a lane quarter has 16 rows, unrolled: backward of 131 K labels, 64 rows, (64, 128) 54.7 -> 45.2 us, (32, 128) 93.9 -> 78.1
+    // against 8 columns per load and rolled loops.  With G = 128 unrolling costs 4 % (131 K labels, 512 rows: 64.0 -> 66.9).
     constexpr int ROWS = C::ROWS_PER_Q;
     const int q = warp & 3;
     uint8_t* gst = sm + C::OFF_WST + q * C::WST;
@@ -488,22 +491,22 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       const uint32_t tg = ta + (P == 1 ? 0 : (q * ROWS) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
       const bool live = !*abort_flag;
       const bool fast = UPD && u.mom_w == nullptr && (u.flags & HASTE_F_SR) && (u.flags & HASTE_F_CONTRACT);
-#pragma unroll 1
+#pragma unroll (G == 64 ? 4 : 1)
       for (int pc = 0; pc < FF / 32; ++pc) {
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r0[8];
-          __syncwarp();
-          tmem_ld8(tg + pc * 32 + c * 8, r0);
-          tmem_ld_wait();
-          // the gradient as the unfused kernel would store it: rounded to bf16
-          if (lane < ROWS)
+        uint32_t rv[32];
+        __syncwarp();
+        tmem_ld32(tg + pc * 32, rv);
+        tmem_ld_wait();
+        // the gradient as the unfused kernel would store it: rounded to bf16
+        if (lane < ROWS) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
             *reinterpret_cast<uint4*>(gst + g_chunk(lane, c)) =
-                make_uint4(pack2(__uint_as_float(r0[0]), __uint_as_float(r0[1])), pack2(__uint_as_float(r0[2]), __uint_as_float(r0[3])),
-                           pack2(__uint_as_float(r0[4]), __uint_as_float(r0[5])), pack2(__uint_as_float(r0[6]), __uint_as_float(r0[7])));
+                make_uint4(pack2(__uint_as_float(rv[8 * c]), __uint_as_float(rv[8 * c + 1])), pack2(__uint_as_float(rv[8 * c + 2]), __uint_as_float(rv[8 * c + 3])),
+                           pack2(__uint_as_float(rv[8 * c + 4]), __uint_as_float(rv[8 * c + 5])), pack2(__uint_as_float(rv[8 * c + 6]), __uint_as_float(rv[8 * c + 7])));
         }
         __syncwarp();
-#pragma unroll 1
+#pragma unroll (G == 64 ? 4 : 1)
         for (int r0 = 0; r0 < ROWS; r0 += 8) {
           const int r = r0 + (lane >> 2), row = q * ROWS + r;
           if (!live || row >= rows_real) continue;
