@@ -142,3 +142,38 @@ def test_hinge_loss_beside_confident_positives(G, F, z_pos):
     want = n_off / 16.0 * scale
     # ten equal terms, each rounded a few times to 2^-24
     assert abs(float(loss) - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("B,off", [(64, 0), (64, 1), (136, 3), (100, 6)])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_single_gradients_against_both_over_several_groups_a_cta(G, F, B, off):
+    """The kernels that make one gradient, or update with it, have accumulator stages and copy loops of their own.  The sums are the same in the
+    same order: dW, dbias and the updated weights bit for bit, dX up to the order of its reductions."""
+    from haste_b200 import ffi
+    D, L = 160, (5 if G == 128 or F == 128 else 9) * 148 * G // 2 + 3        # more than two tiles for most CTAs, the last one ragged
+    gen = torch.Generator(device="cuda").manual_seed(B + F)
+    loc = torch.rand((L + G - 1) // G, D, generator=gen, device="cuda").topk(F, dim=1).indices.sort(dim=1).values.int()
+    W = ((torch.rand(L, F, generator=gen, device="cuda") * 2 - 1) / F ** 0.5).to(torch.bfloat16)
+    bias = torch.randn(L, generator=gen, device="cuda").to(torch.bfloat16)
+    X = torch.randn(B, D, generator=gen, device="cuda").to(torch.bfloat16)
+    buf = torch.randn(off + B * L + 16, generator=gen, device="cuda").to(torch.bfloat16)
+    dY, xt = buf[off:off + B * L].view(B, L), ffi.transpose_padded(X)
+    dxt, dw, db = ffi.backward_both(xt, W, loc, dY, G, B=B)
+    want = torch.zeros(B, D, device="cuda", dtype=torch.float64)
+    for g0 in range(0, loc.shape[0], 256):                                   # dX[b, loc[g, k]] += sum over the group's labels of dY W
+        for g in range(g0, min(g0 + 256, loc.shape[0])):
+            rows = slice(g * G, min(g * G + G, L))
+            want.index_add_(1, loc[g].long(), dY[:, rows].double() @ W[rows].double())
+    # fp32 sums of L F / D label terms in any order
+    tol = 2.0 ** -20 * (L * F / D) * float(dY.float().std() * W.float().std()) + 1e-5 * want.abs()
+    for got in (dxt, ffi.backward_features(xt, W, loc, dY, G, B=B)):
+        assert ((got[:, :B].t().double() - want).abs() <= tol).all()
+    dw1, db1 = ffi.backward_weights(xt, W, loc, dY, G, want_dbias=True, B=B)
+    assert torch.equal(dw1, dw) and torch.equal(db1, db)
+    if B % 8 == 0:
+        for rng in ("packed", "reference"):
+            flags = ffi.make_flags(rng=rng)
+            w1, b1, w2 = W.clone(), bias.clone(), W.clone()
+            ffi.bww_sr_sgd(xt, loc, dY, w1, b1, None, None, G, 0, 0.05, 1e-4, 0.0, 7, 2, flags)
+            ffi.sgd_sr_update(w2, dw, None, 0, 0.05, 1e-4, 0.0, 7, 2, flags)
+            assert torch.equal(w1, w2)
