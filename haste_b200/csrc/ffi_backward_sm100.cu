@@ -44,7 +44,9 @@ struct Cfg {
   static constexpr int NXS = (F == 64) ? 2 : 3;       // X ring stages
   static constexpr int NYS = 4;                       // dY ring stages
   static constexpr int NDX = 2;                       // dXg accumulator stages
-  static constexpr int NDW = (F == 64) ? 2 : 1;       // dW accumulator stages
+  // dW accumulator stages beside those of dXg.  Alone dW has two at every shape: with one the next group's products wait until the writer warps are
+  // done with a group, and longest where they update: 131 K labels, 512 rows, (64, 128) 131.5 -> 94.3 us, (32, 128) 247.8 -> 176.5.
+  static constexpr int NDW = (F == 64) ? 2 : 1;
   static constexpr int XBLK = FR * 128, XSTAGE = 2 * XBLK;
   static constexpr int NWB = FF == 32 ? 1 : FF / 64, WBLK = G * WROW, WSTAGE = NWB * WBLK;
   static constexpr int NYB = G / 64, YBLK = BT * 128, YSTAGE = NYB * YBLK;
@@ -65,7 +67,7 @@ struct Cfg {
   static_assert(XSTAGE % 1024 == 0 && WBLK % 1024 == 0 && YBLK % 1024 == 0, "tile alignment");
   static constexpr int B_XFULL = 0, B_XEMPTY = NXS, B_YFULL = 2 * NXS, B_YEMPTY = B_YFULL + NYS, B_WFULL = B_YEMPTY + NYS,
                        B_WEMPTY = B_WFULL + 2, B_DXFULL = B_WEMPTY + 2, B_DXEMPTY = B_DXFULL + NDX, B_DWFULL = B_DXEMPTY + NDX,
-                       B_DWEMPTY = B_DWFULL + NDW, B_LEMPTY = B_DWEMPTY + NDW, B_FIN = B_LEMPTY + 2, NBAR = B_FIN + 2;
+                       B_DWEMPTY = B_DWFULL + 2, B_LEMPTY = B_DWEMPTY + 2, B_FIN = B_LEMPTY + 2, NBAR = B_FIN + 2;
   static_assert(NBAR <= 40, "barrier space");
   static constexpr int N_EB = 8;                      // scatter warps: 4 TMEM lane quarters x 2 slot halves
   static constexpr int EBS = F / 2;                   // slots per scatter warp
@@ -76,7 +78,7 @@ struct Cfg {
   static constexpr int W_EB = 4, W_EC = W_EB + N_EB, W_Y = W_EC + N_EC, W_XP = W_Y + N_Y;
   static constexpr int NTHREADS = (W_XP + NPW - 2) * 32;
   static constexpr uint32_t TM_DX = 0, TM_DW = NDX * F, TM_COLS = 512;
-  static_assert(TM_DW + NDW * FR <= TM_COLS, "TMEM budget");
+  static_assert(TM_DW + NDW * FR <= TM_COLS && 2 * FR <= TM_COLS, "TMEM budget");
   static constexpr int ROWS_PER_Q = G / 4;            // label rows of the dW accumulator in one TMEM lane quarter
   static_assert(GG % ROWS_PER_Q == 0, "the rows of a lane quarter belong to one group");
 };
@@ -108,7 +110,8 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
   static_assert(!UPD || DW, "the update consumes the weight gradient");
   using C = Cfg<GG_, FF_, P_>;
   constexpr int GG = C::GG, FF = C::FF, P = C::P, LS = C::LS;
-  constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX, NDW = C::NDW;
+  constexpr int G = C::G, F = C::F, BT = C::BT, FR = C::FR, NXS = C::NXS, NYS = C::NYS, NDX = C::NDX, NDW = DX ? C::NDW : 2;
+  constexpr uint32_t TM_DW = DX ? C::TM_DW : 0;
   constexpr int XBLK = C::XBLK, XSTAGE = C::XSTAGE, WBLK = C::WBLK, WSTAGE = C::WSTAGE, YBLK = C::YBLK, YSTAGE = C::YSTAGE, NCH = C::NCH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -409,7 +412,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       int it = 0, xs = 0, xph = 0, ys = 0, yph = 0;
       for (int gi = 0; gi < n_my_groups; ++gi) {
         const int dws = gi % NDW;
-        const uint32_t tdw = tmem + C::TM_DW + dws * FR;
+        const uint32_t tdw = tmem + TM_DW + dws * FR;
         const bool okd = mbar_wait(bar(C::B_DWEMPTY + dws), ((gi / NDW) & 1) ^ 1, abort_flag, a.err, 37, WL);
         for (int t = 0; t < T; ++t, ++it) {
           bool ok = mbar_wait(bar(C::B_XFULL + xs), xph, abort_flag, a.err, 38, WL) && okd;
@@ -497,7 +500,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
       const int rows_real = static_cast<int>(imin64(LS, a.L - l0));
       mbar_wait(bar(C::B_DWFULL + dws), (gi / NDW) & 1, abort_flag, a.err, 42, WL);
       tc_fence_after();
-      const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + C::TM_DW + dws * FR;
+      const uint32_t ta = tmem + (static_cast<uint32_t>(q * 32) << 16) + TM_DW + dws * FR;
       const uint32_t tg = ta + (P == 1 ? 0 : (q * ROWS) / GG * FF);      // the columns of this quarter's group: its block on the diagonal
       const bool live = !*abort_flag;
       const bool fast = UPD && u.mom_w == nullptr && (u.flags & HASTE_F_SR) && (u.flags & HASTE_F_CONTRACT);
