@@ -19,8 +19,8 @@
 //
 // Warp roles (24 or 25 warps): warps 0, 2 (and 24) gather X tiles with TMA tile::gather4 (warp 0 also loads the W tile
 // through a tensor map), warp 1 issues backward-features, warp 3 backward-weights, warps 4-11 drain dXg (TMEM ->
-// registers -> coalesced red.global.add.f32), warps 12-15 turn the dW accumulator into bf16 rows of dw / dbias at
-// the end of each group, warps 16-23 are the Y warps.  All waits are bounded (see mbar_wait).
+// registers -> coalesced red.global.add.f32), warps 12-15 turn the dW accumulator into bf16 rows of dw / dbias (or update the
+// weights with them) at the end of each group, warps 16-23 are the Y warps.  All waits are bounded (see mbar_wait).
 #include "common.cuh"
 #include "launchers.h"
 #include "runtime.h"
@@ -165,7 +165,7 @@ ffi_backward_sm100_kernel(BwdArgs a, UpdateArgs u, const __grid_constant__ CUten
     // ================================================================ X / W producers
     // Per group: producer 0 writes the index row (as dxt row offsets for the scatter warps) and loads the W tile
     // through the tensor map.  Per batch tile: F index rows of xt, 256 bytes each, as TMA gather4 loads (four index
-    // rows per instruction, landing at their swizzled positions), dealt round-robin over the four warps.
+    // rows per instruction, landing at their swizzled positions), dealt round-robin over the two or three warps.
     int it = 0, w_armed = 0, my_last = -1;
     bool go = true;
     for (int gi = 0; go && gi < n_my_groups; ++gi) {

@@ -1,6 +1,6 @@
 // sm_100a primitives in inline PTX: mbarrier with bounded waits, TMA loads (tiled and tile::gather4, never
 // multicast) and tiled stores, tcgen05 (alloc / mma / commit / ld), UMMA shared-memory and instruction descriptors, cp.async with
-// zero fill, bulk reduce-add to global.
+// zero fill, 16-byte reductions into global memory.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -157,8 +157,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // ---------------------------------------------------------------- reductions into global memory
 // Four consecutive floats (16-byte aligned) per lane.
 __device__ __forceinline__ void red_add_v4(float* p, float4 v) {
@@ -264,14 +262,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8(taddr, r); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// Wait for outstanding TMEM loads and tie the wait to the registers of one earlier 8-column load, so that no use
-// of those registers can be scheduled ahead of the wait when other work sits between load and wait.
-__device__ __forceinline__ void tmem_ld_wait8(uint32_t (&r)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
-               :
-               : "memory");
-}
 
 // ---------------------------------------------------------------- descriptors
 // Shared-memory matrix descriptor, 128-byte swizzle.  The operand lives in "row blocks": rows of 128 bytes
