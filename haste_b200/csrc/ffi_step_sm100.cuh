@@ -35,8 +35,11 @@
 // different loops; with the loops unrolled a quarter of the warps' stalls were for instructions), the L1 data
 // pipe (tensor core operands, shared memory and global accesses: 82 % busy) and at 128 slots the L2's reductions.  So
 // the hot loops are small and rolled, and what a role writes to memory leaves in whole lines.
+// (Where a comment here gives two times, they are of two builds that differ in that one thing, measured in turn.  The same step's time differs by some
+// per cent between builds further apart.)
 // All hand-offs are mbarriers with bounded waits; a wait that gives up raises a CTA-wide abort flag, every role
-// drains its loops without touching global memory, TMEM is freed and the host sees HASTE_ERR_TIMEOUT.
+// drains its loops without touching global memory, copies and products in flight are waited for, TMEM is freed and the host sees
+// HASTE_ERR_TIMEOUT.
 #pragma once
 #include "common.cuh"
 #include "launchers.h"
@@ -212,14 +215,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   constexpr bool DROP_NAN = !WITH_LOSS && GG * FF != 128 * 64;
   // Up to so many columns with positives are put right after the plain loop: 31 K labels, G=32, B=64 (BCE) 20.6 -> 18.6 us a step.  One column
   // after the other, and each waits for its logits: with up to 12 the kernel took 33 us for 8.8 K labels, G=32, B=1024, one positive a row, where
-  // no tile of the SM's hides it; with up to 4 27, and nothing else became slower.  Not for (128, 64), whose tiles hardly ever have one at the
-  // sizes of 670 K and 2.8 M labels (4 % slower there: the loop's registers).  Nor for the hinge loss:
+  // no tile of the SM's hides it; with up to 4 27, and nothing else became slower.  Not for (128, 64), where BCE steps lose 2 to 5 % from
+  // 5 K labels (B=200: 18.6 -> 19.5 us) over 670 K (313 -> 321) to 2.8 M (2,307 -> 2,343) and only few rows of many labels gain (246 K, B=64: 60.6 ->
+  // 55.9).  Nor for the hinge loss:
   // a confident positive counted as a negative first, with (1 + z)^2, costs the sum its low bits, and what is left when it is taken out again has
   // either sign (z near 50: relative error 9e-5 instead of 2e-7 of the loss).  For BCE the two differ by z, which bf16 logits add up exactly.
   constexpr int PATCH = GG != 128 && !(LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS) ? 4 : 0;
-  // Two chunks per pass of the loss epilogue's plain loop hide some of the MUFU's latency: 2.8 M labels, BCE, 2,284 -> 2,235 us; the other
-  // instantiations lose by it (501 K labels 278 -> 297, hinge 670 K 252 -> 253: instruction cache).
-  constexpr int UNROLL = LOSS == HASTE_LOSS_BCE && F == 64 ? 2 : 1;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
 
   extern __shared__ uint8_t smem_raw[];
@@ -681,7 +682,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         bool again = false;
         if (plain) {
           __syncwarp();
-#pragma unroll UNROLL
+#pragma unroll 1           // (two chunks per pass: 2.8 M labels 2,293 -> 2,307 us, 131 K at (128, 64) 76.7 -> 78.5; at 128 slots 501 K 278 -> 297: instruction cache)
           for (int c16 = 0; c16 < EA_COLS; c16 += CH) {
             uint32_t r[CH];
             tmem_ld(ta + c16, r);
@@ -840,7 +841,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         const bool live = !*abort_flag;
         const int b1 = tile_b0(t) + row, b4 = tile_b0(t) + q * 32 + 4 * (lane & 7);
         // two loops, although they differ in their last lines only: one loop with both forms inside took 151 us for 131 K labels and 290 for 501 K, so 138
-        // and 271 (instruction cache; the BCE step of 2.8 M labels 2,217 and 2,272)
+        // and 271 (instruction cache); the BCE step of 2.8 M labels goes the other way by 2 %
         if (a.dxt_v4) {
           const bool on = live && b4 < a.B;
           float* dst = a.dxt + b4;
