@@ -270,6 +270,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
     *reinterpret_cast<uint4*>(sm + C::OFF_X + blk * XBLK + (F + row) * 128 + chunk * 16) = make_uint4(v, v, v, v);
   }
   for (int i = tid; i < 2 * C::BTILE / 16; i += C::NTHREADS) *reinterpret_cast<uint4*>(sm + C::OFF_BT + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+  // No targets in either group stage: after an abort that came before a stage was first filled, a later wait on its barrier finds the parity it
+  // asks for all the same, and the range it then reads has to be one.
+  if (tid < 2 * (4 + C::NTE)) reinterpret_cast<uint32_t*>(sm + C::OFF_TGT)[tid] = 0u;
   fence_proxy_async();
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), C::TM_COLS);
