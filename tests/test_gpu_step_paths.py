@@ -11,6 +11,51 @@ from oracle import ffi_oracle as fo
 SHAPES = [(32, 32), (32, 64), (64, 64), (32, 128), (128, 64), (64, 128)]
 
 
+@pytest.mark.parametrize("B", [36, 61, 132])
+@pytest.mark.parametrize("loss", ["bce", "squared_hinge"])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_step_targets_few_many_twice_and_large_logits(G, F, loss, B):
+    from haste_b200.fused import FusedFFIShard
+    D, L, scale, lr = 264, 7 * G + 5, 0.5, 0.05
+    inp = fo.make_inputs(B, D, L, F, G, 1, 1.1, seed=B + F, x_kind="normal", bias_zero=False)
+    bias = inp["bias"].clone()
+    bias[2 * G + 3], bias[2 * G + 4] = 3000.0, -3000.0          # beyond what a difference of two losses can carry
+    rows = [0, 31, 32 % B, min(63, B - 1), B - 1]
+    pairs = [(r, c) for r in rows for c in (0,)]                                              # group 0: the first label in the edge rows
+    pairs += [(0, G + G - 1), (0, G + G - 1), (B - 1, G), (B - 1, G), (B - 1, G + 15)]          # group 1: the last label twice, the first twice
+    pairs += [(1, 2 * G + 3), (2, 2 * G + 4), (3, 2 * G + 5)]                                 # group 2: large logits as positives
+    pairs += [(r % B, 3 * G + (5 * r) % G) for r in range(40)]                                # group 3: more than the entry list holds
+    pairs += [(0, 7 * G + 4), (B - 1, 7 * G)]                                                 # the ragged last group
+    pairs += [(r % B, 5 * G + r) for r in range(8)]                                           # group 5: exactly a full list
+    targets = torch.tensor(pairs, dtype=torch.int32)
+    z = fo.forward(inp["loc"], inp["X"], inp["W"], bias, G).double()
+    y = torch.zeros(B, L, dtype=torch.float64)
+    y[targets[:, 0].long(), targets[:, 1].long()] = 1.0
+    if loss == "bce":
+        term, dY = torch.nn.functional.softplus(z) - y * z, torch.sigmoid(z) - y
+    else:
+        s = 2.0 * y - 1.0
+        m = (1.0 - s * z).clamp_min(0.0)
+        term, dY = m * m, -2.0 * s * m
+    want_loss, dY = float(term.sum()) * scale, (dY * scale).to(torch.bfloat16)
+    want_x, want_w = fo.backward_features(inp["loc"], inp["W"], dY, G, D), fo.backward_weights(inp["loc"], inp["X"], dY, G, L, round_bf16=False)
+    for mu in (0.0, 0.9):
+        sh = FusedFFIShard(inp["loc"].cuda(), inp["W"].clone().cuda(), bias.clone().cuda(), G, D, loss=loss, lr=lr, momentum=mu, seed=42, grad_scale=scale)
+        dxt, loss_dev = sh.step(inp["X"].cuda(), targets.cuda())
+        # the logits are bf16, some one rounding away from the oracle's
+        assert abs(float(loss_dev) - want_loss) <= 2e-3 * want_loss
+        big = 1e-3 * max(1.0, float(want_x.abs().max())) + 1e-2 * want_x.abs()
+        assert ((dxt.cpu() - want_x).abs() <= big).all()
+        if mu == 0.0:
+            # w' = w - lr g, stochastically rounded to bf16: one unit in the last place (2^-7) of w', and g as far off as dW may be
+            want = inp["W"].float() - lr * want_w
+            tol = want.abs() / 128 + lr * (1e-2 * want_w.abs() + 1e-3 * max(1.0, float(want_w.abs().max()))) + 1e-6
+            assert ((sh.w.float().cpu() - want).abs() <= tol).all()
+        else:
+            tol = 1e-2 * want_w.abs() + 1e-3 * max(1.0, float(want_w.abs().max()))
+            assert ((sh.mom_w.cpu() - want_w).abs() <= tol).all()
+
+
 def step_case(G, F, B, large):
     """Inputs whose negatives have next to no hinge loss and little BCE loss (bias -3), so that every positive shows in the loss, in its batch row
     of dX and in its label's row of dW.  ``large``: two labels with logits near +-3000, positive for one row each, instead of the patterns."""
@@ -67,7 +112,7 @@ STEP_SCALE, STEP_LR = 0.5, 0.05
 @pytest.mark.parametrize("B", [36, 61, 132, 136])
 @pytest.mark.parametrize("loss", ["bce", "squared_hinge"])
 @pytest.mark.parametrize("G,F", SHAPES)
-def test_step_targets_few_many_twice_and_large_logits(G, F, loss, B, large):
+def test_step_positives_by_row_and_by_label(G, F, loss, B, large):
     from haste_b200.fused import FusedFFIShard
     inp = step_case(G, F, B, large)
     want_loss, want_x, want_w = step_expected(inp, G, loss, STEP_SCALE)
