@@ -616,11 +616,19 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         float tile_loss = 0.f, fast_loss = 0.f;             // fast_loss: hinge (4s)^2-scaled squares, or BCE raw log2 terms
         const float hgs = 0.5f * gs;
         constexpr int CH = 16;                             // label columns per TMEM load
-        // One chunk without targets or absent columns: gradients of its 16 logits, stored swizzled; loss terms into fh / fl / bce_prod.
+        // One chunk without targets or absent columns: gradients of its 16 logits, stored swizzled; loss terms into fh / fl / fast_loss.
         F2 fh[2] = {{0.f, 0.f}, {0.f, 0.f}};               // hinge: (4s)^2-scaled squares
-        float fl[4] = {0.f, 0.f, 0.f, 0.f};                // BCE: max(z, 0); partial sums, no serial dependency through one accumulator
+        // BCE: max(z, 0) in partial sums, and the logarithms' arguments in partial products: no serial dependency through one accumulator.
+        // With FOLD the sums go into tile_loss chunk by chunk and two products do: four of each kept over the tile's chunks hold registers that the
+        // loop lacks.  BCE, (128, 64), 500 rows of 670 K labels 381 -> 355 us a step, 1,020 of 300 K 330 -> 310; (64, 128), 512 of 131 K 135.3 -> 133.4.
+        // Not for (32, 32): 1,024 rows of 8.8 K labels 28.9 -> 30.9, 31 K labels the same.
+        constexpr bool FOLD = FF != 32;
+        constexpr int NBP = FOLD ? 2 : 4;
+        float fl[4] = {0.f, 0.f, 0.f, 0.f};
         auto plain_chunk = [&](const uint32_t (&r)[CH], uint8_t* yblk, int chunk0) {
-          float bp[4] = {1.f, 1.f, 1.f, 1.f};
+          float bp[NBP];
+#pragma unroll
+          for (int i = 0; i < NBP; ++i) bp[i] = 1.f;
 #pragma unroll
           for (int e8 = 0; e8 < CH; e8 += 8) {
             uint4 pk;
@@ -647,7 +655,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
                 const float sg = sigmoid_exp(zr);
                 x[i] = sg * gs;
-                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & 3] *= 0.5f + fabsf(sg - 0.5f); }
+                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & (NBP - 1)] *= 0.5f + fabsf(sg - 0.5f); }
               }
               pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
             } else {
@@ -660,14 +668,20 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 const float zr = round_bf16_as_f32(__uint_as_float(r[e8 + i]));
                 const float th = tanh_approx(0.5f * zr);
                 x[i] = fmaf(hgs, th, hgs);
-                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & 3] *= 1.f + fabsf(th); }
+                if (WITH_LOSS) { fl[i & 3] += fmaxf(zr, 0.f); bp[i & (NBP - 1)] *= 1.f + fabsf(th); }
               }
               pk = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
             }
             *reinterpret_cast<uint4*>(yblk + (((chunk0 + (e8 >> 3)) ^ (row & 7)) << 4)) = pk;
           }
-          if (WITH_LOSS && LOSS != HASTE_LOSS_SQHINGE)
-            fast_loss += __log2f(((bp[0] * bp[1]) * (bp[2] * bp[3])) * (LOSS == HASTE_LOSS_BCE ? 0x1p-16f : 1.f));
+          if (WITH_LOSS && LOSS != HASTE_LOSS_SQHINGE) {
+            const float prod = FOLD ? bp[0] * bp[1] : (bp[0] * bp[1]) * (bp[NBP - 2] * bp[NBP - 1]);
+            fast_loss += __log2f(prod * (LOSS == HASTE_LOSS_BCE ? 0x1p-16f : 1.f));
+            if (FOLD) {
+              tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
+              fl[0] = fl[1] = fl[2] = fl[3] = 0.f;
+            }
+          }
         };
         // Tiles without a target in a warp's 32 rows and its columns take a loop with nothing but the arithmetic.  With PATCH so do those with
         // targets in up to PATCH columns: the loop treats every label as a negative, and these columns are put right one by one
@@ -795,7 +809,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         fh[0] = fh[1] = {0.f, 0.f};
         fl[0] = fl[1] = fl[2] = fl[3] = 0.f;
         }
-        if (LOSS != HASTE_LOSS_SQHINGE) tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
+        if (LOSS != HASTE_LOSS_SQHINGE && !FOLD) tile_loss += (fl[0] + fl[1]) + (fl[2] + fl[3]);
         tc_fence_before();                             // this warp's part of the Z stage has been read
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_ZEMPTY + zs));
