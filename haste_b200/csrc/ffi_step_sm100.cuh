@@ -217,10 +217,13 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
   // after the other, and each waits for its logits: with up to 12 the kernel took 33 us for 8.8 K labels, G=32, B=1024, one positive a row, where
   // no tile of the SM's hides it; with up to 4 27, and nothing else became slower.  Not for (128, 64), where BCE steps lose 2 to 5 % from
   // 5 K labels (B=200: 18.6 -> 19.5 us) over 670 K (313 -> 321) to 2.8 M (2,307 -> 2,343) and only few rows of many labels gain (246 K, B=64: 60.6 ->
-  // 55.9).  Nor for the hinge loss:
-  // a confident positive counted as a negative first, with (1 + z)^2, costs the sum its low bits, and what is left when it is taken out again has
-  // either sign (z near 50: relative error 9e-5 instead of 2e-7 of the loss).  For BCE the two differ by z, which bf16 logits add up exactly.
-  constexpr int PATCH = GG != 128 && !(LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS) ? 4 : 0;
+  // 55.9).
+  constexpr int PATCH = GG != 128 ? 4 : 0;
+  // A positive beyond this logit sends the warp's part through the other loop.  What it was counted with as a negative has to leave the sum again, and the
+  // sum's low bits are gone: for the hinge loss that is (1 + z)^2, at most 25 here and with z up to 1,000 a million (a relative error of 9e-5 of the loss
+  // at z near 50 already).  For BCE the two losses differ by z, which bf16 logits add up exactly.  Without the correction 184 rows of 1.4 M labels,
+  // (32, 32), hinge, take 580 us a step, with it 518; 31 K labels, 64 rows, 18.6 and 16.6.
+  constexpr float PATCH_TOP = LOSS == HASTE_LOSS_SQHINGE && WITH_LOSS ? 4.f : 1024.f;
   constexpr int YBW = G / 32;                          // 32-bit words of target bits per batch row
 
   extern __shared__ uint8_t smem_raw[];
@@ -715,10 +718,12 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
               tmem_ld_wait();
               if ((ym >> c) & 1u) {
                 const float zr = round_bf16_as_f32(__uint_as_float(zb));
-                float gl, la;                              // gradient as a positive; its loss less the loss counted as a negative
+                float gl, la;                              // gradient as a positive; its loss (BCE: less the loss counted as a negative)
                 if (LOSS == HASTE_LOSS_SQHINGE) {
-                  gl = -fmaxf(1.f - zr, 0.f) * gs2;
-                  la = 0.f;                                // (no loss sum)
+                  const float m = fmaxf(1.f - zr, 0.f), x2 = fmaf(gs2, zr, gs2), m2 = x2 + fabsf(x2);
+                  gl = -m * gs2;
+                  la = m * m;
+                  fh[0].x = fmaf(-m2, m2, fh[0].x);        // out in the form it went in
                 } else {
                   // softplus(-z) - softplus(z) = -z
                   gl = ((LOSS == LOSS_BCE_EXP ? sigmoid_exp(zr) : fmaf(0.5f, tanh_approx(0.5f * zr), 0.5f)) - 1.f) * gs;
@@ -728,7 +733,7 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
                 *reinterpret_cast<__nv_bfloat16*>(yrow + (cc >> 6) * YBLK + ((((cc & 63) >> 3) ^ (row & 7)) << 4) + (cc & 7) * 2) = __float2bfloat16_rn(gl);
                 if (WITH_LOSS) tile_loss += la;
                 // a logit so large that the difference says nothing (or infinite, or NaN): once more through the other loop
-                again = again || !(fabsf(zr) < 1024.f);
+                again = again || !(zr > -1024.f && zr < PATCH_TOP);
               }
             }
             again = __any_sync(0xffffffffu, again);

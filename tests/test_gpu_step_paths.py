@@ -159,11 +159,9 @@ def test_backward_reads_dy_at_any_offset_and_nothing_else(G, F, B, tail, off):
             assert ((got - want).abs() <= 1e-3 * max(1.0, float(want.abs().max())) + 1e-2 * want.abs()).all()
 
 
-@pytest.mark.parametrize("z_pos", [8.0, 50.0, 300.0, 900.0])
-@pytest.mark.parametrize("G,F", SHAPES)
-def test_hinge_loss_beside_confident_positives(G, F, z_pos):
-    """A positive beyond the margin has no loss, however far.  Every negative lies on the margin but one per row and group, which is all there is
-    to sum: beside positives of z_pos its loss must come out to the accuracy of an fp32 sum."""
+def hinge_loss_beside(G, F, z_pos):
+    """(loss, what it should be, number of positives, scale).  A positive beyond the margin has no loss, however far.  Every negative lies on the margin but one per row and group, which is all there is
+    to sum."""
     from haste_b200.fused import FusedFFIShard
     B, NG, D, scale = 64, 5, 160, 0.3
     L, gen = NG * G, torch.Generator().manual_seed(F)
@@ -185,8 +183,25 @@ def test_hinge_loss_beside_confident_positives(G, F, z_pos):
     sh = FusedFFIShard(loc.cuda(), W.cuda(), bias.cuda(), G, D, loss="squared_hinge", lr=0.0, seed=1, grad_scale=scale)
     _, loss = sh.step(X.cuda(), torch.tensor(sorted(pairs), dtype=torch.int32).cuda())
     want = n_off / 16.0 * scale
+    return float(loss), want, len(pairs), scale
+
+
+@pytest.mark.parametrize("z_pos", [8.0, 50.0, 300.0, 900.0])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_hinge_loss_beside_confident_positives(G, F, z_pos):
+    """Beside positives of z_pos the loss must come out to the accuracy of an fp32 sum."""
+    loss, want, _, _ = hinge_loss_beside(G, F, z_pos)
     # ten equal terms, each rounded a few times to 2^-24
-    assert abs(float(loss) - want) <= 1e-5 * want
+    assert abs(loss - want) <= 1e-5 * want
+
+
+@pytest.mark.parametrize("z_pos", [1.0, 1.5, 3.0, 3.9375])
+@pytest.mark.parametrize("G,F", SHAPES)
+def test_hinge_loss_beside_positives_taken_out_again(G, F, z_pos):
+    """Positives that may have been counted as negatives first, with (1 + z)^2, and taken out again: at most six roundings to 2^-24 of that
+    each (a partial sum's other terms are 0 but one), beside those of the sum itself."""
+    loss, want, n, scale = hinge_loss_beside(G, F, z_pos)
+    assert abs(loss - want) <= 1e-5 * want + 6 * n * 2.0 ** -24 * (1.0 + z_pos) ** 2 * scale
 
 
 @pytest.mark.parametrize("B,off", [(64, 0), (64, 1), (136, 3), (100, 6)])
