@@ -624,8 +624,9 @@ ffi_train_step_sm100_kernel(StepArgs a, UpdateArgs u, const __grid_constant__ CU
         // BCE: max(z, 0) in partial sums, and the logarithms' arguments in partial products: no serial dependency through one accumulator.
         // With FOLD the sums go into tile_loss chunk by chunk and two products do: four of each kept over the tile's chunks hold registers that the
         // loop lacks.  BCE, (128, 64), 500 rows of 670 K labels 381 -> 355 us a step, 1,020 of 300 K 330 -> 310; (64, 128), 512 of 131 K 135.3 -> 133.4.
-        // Not for (32, 32): 1,024 rows of 8.8 K labels 28.9 -> 30.9, 31 K labels the same.
-        constexpr bool FOLD = FF != 32;
+        // Not for (32, 32): 1,024 rows of 8.8 K labels 28.9 -> 30.9, 31 K labels the same.  Nor for (32, 128): reference stream, 120 rows of 164 K labels 290 -> 296,
+        // 160 of 2.8 M 5,172 -> 5,227; packed, 184 of 1.4 M 1,473 -> 1,464, 131 K the same.
+        constexpr bool FOLD = FF != 32 && !(GG == 32 && FF == 128);
         constexpr int NBP = FOLD ? 2 : 4;
         float fl[4] = {0.f, 0.f, 0.f, 0.f};
         auto plain_chunk = [&](const uint32_t (&r)[CH], uint8_t* yblk, int chunk0) {
